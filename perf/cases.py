@@ -9,8 +9,8 @@ A case names a model, a number of decoding requests with the context that they h
 * both: the step a scheduler makes while requests decode and others arrive.
 
 The layers have the sizes that ``bench.py`` measures, fewer of them (a layer's work does not depend on how many there
-are) and a vocabulary cut in proportion.  Weights are random, drawn on the device; a router's are three times as large
-as the rest, so that it prefers some experts, as a trained one does.
+are) and a vocabulary cut in proportion.  Weights are random, drawn on the device; a router's are six times as large as
+the rest, so that it prefers some experts clearly, as a trained one does, and a rounding seldom changes the outcome.
 """
 from __future__ import annotations
 
@@ -116,9 +116,11 @@ def listed():
         _case("mixed-7+53", "moe", decode=7, context=700, prompts=1, tokens=53),
         # a larger model, a full batch of prompts admitted together
         _case("wide-prompt-4096", "moe-wide", prompts=3, tokens=4096),
-        # the true 32-bit engine, which checkpoints are checked with: a prompt of odd length, and its decoding
-        _case("f32-prompt-517", "moe", dtype="f32", prompts=1, tokens=517),
-        _case("f32-decode-4", "moe", dtype="f32", decode=4, context=700),
+        # the true 32-bit engine, which checkpoints are checked with: a prompt of odd length, and its decoding (without
+        # experts: two correct engines that differ in the last bit choose other ones now and then, and then their
+        # results cannot be compared at the precision that this engine is for)
+        _case("f32-prompt-517", "dense", dtype="f32", prompts=1, tokens=517),
+        _case("f32-decode-4", "dense", dtype="f32", decode=4, context=700),
         # models that carry a state from token to token beside their attention: long prompts, one and several
         _case("safepel-prompt-2048", "safepel", prompts=1, tokens=2048),
         _case("sesuzen-prompt-3001", "sesuzen", prompts=3, tokens=3001),
@@ -135,7 +137,7 @@ def _log(rng, lo, hi):
 def draw(rng):
     model = rng.choice(sorted(MODELS))
     kind = rng.choice(("decode", "prompt", "mixed"))
-    f32 = model in ("moe", "dense") and rng.random() < 0.35
+    f32 = model == "dense" and rng.random() < 0.5
     decode = context = prompts = tokens = 0
     if kind != "prompt":
         decode = _log(rng, 1, (8 if f32 else 64) if kind == "decode" else 16)
@@ -164,7 +166,7 @@ def _tensor(decl, seed, dtype):
         return torch.ones(decl.shape, dtype=dtype, device="cuda")
     name, std, mean = decl.name, 0.02, decl.mean
     if name.endswith(".mlp.gate.weight"):
-        std = 0.06                                   # the router
+        std = 0.12                                   # the router
     elif name == "model.embed_tokens.weight":
         std = 1.0                                    # a residual stream that layers add to, as in a deep model
     elif name.endswith(".conv"):
