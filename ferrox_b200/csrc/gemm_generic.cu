@@ -1,8 +1,9 @@
 // C[M,N] (+)= A[M,K] . W[N,K]^T (+ bias): the matrix product every projection is.
 //
 // CUDA-core kernel (FFMA, 32-bit accumulate, no tensor-core or reduced-precision
-// mode): it is the whole 32-bit path and the fallback of the bfloat16 path for
-// shapes the tensor-core kernels refuse.  Takes any M, N, K.
+// mode): the fallback of the bfloat16 path for shapes the tensor-core kernels
+// refuse, and of the 32-bit path for what gemm_f32.cu refuses (rows that are no
+// multiple of 16 bytes).  Takes any M, N, K.
 //
 //  * rows of A may be gathered through `a_rows` (row r of the product reads row
 //    a_rows[r] of A), which is how expert inputs are picked without a copy;
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(NT) gemm_kernel(
     }
 }
 
-template <typename AT, typename WT, typename CT>
+template <typename AT, typename WT, typename CT, bool MAY_VEC>
 int launch(const void* A, long lda, const int* a_rows, const void* W, long ldw, const void* bias, int bias_dtype,
            void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
            long w_group_stride, cudaStream_t stream)
@@ -132,10 +133,10 @@ int launch(const void* A, long lda, const int* a_rows, const void* W, long ldw, 
     if (M <= 0 || N <= 0) return FX_OK;
     dim3 grid((unsigned)fx_cdiv(N, BN), (unsigned)fx_cdiv(M, BM), group_offsets ? n_groups : 1);
     if (grid.y > 65535u || grid.z > 65535u) return FX_ERR_SIZE;
-    const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (w_group_stride % 4 == 0) &&
+    const bool vec = MAY_VEC && (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && (w_group_stride % 4 == 0) &&
                      ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
     if (vec)
-        gemm_kernel<AT, WT, CT, true><<<grid, NT, 0, stream>>>(
+        gemm_kernel<AT, WT, CT, MAY_VEC><<<grid, NT, 0, stream>>>(
             (const AT*)A, lda, a_rows, (const WT*)W, ldw, bias, bias_dtype, (CT*)C, ldc, accumulate, M, N, K,
             group_offsets, w_group_stride);
     else
@@ -156,15 +157,16 @@ extern "C" int fx_gemm(const void* A, int a_dtype, long lda, const int* a_rows,
                        void* stream)
 {
     cudaStream_t s = (cudaStream_t)stream;
-#define FX_GEMM_CASE(AC, WC, CC, AT, WT, CT)                                                            \
+    // (32-bit operands whose rows can be read in fours go to fx_gemm_f32)
+#define FX_GEMM_CASE(AC, WC, CC, AT, WT, CT, MAY_VEC)                                                     \
     if (a_dtype == AC && w_dtype == WC && c_dtype == CC)                                                  \
-        return launch<AT, WT, CT>(A, lda, a_rows, W, ldw, bias, bias_dtype, C, ldc, accumulate, M, N, K, \
+        return launch<AT, WT, CT, MAY_VEC>(A, lda, a_rows, W, ldw, bias, bias_dtype, C, ldc, accumulate, M, N, K, \
                                   group_offsets, n_groups, w_group_stride, s);
-    FX_GEMM_CASE(FX_F32, FX_F32, FX_F32, float, float, float)
-    FX_GEMM_CASE(FX_BF16, FX_BF16, FX_BF16, bf16, bf16, bf16)
-    FX_GEMM_CASE(FX_BF16, FX_BF16, FX_F32, bf16, bf16, float)
-    FX_GEMM_CASE(FX_BF16, FX_F32, FX_BF16, bf16, float, bf16)
-    FX_GEMM_CASE(FX_BF16, FX_F32, FX_F32, bf16, float, float)
+    FX_GEMM_CASE(FX_F32, FX_F32, FX_F32, float, float, float, false)
+    FX_GEMM_CASE(FX_BF16, FX_BF16, FX_BF16, bf16, bf16, bf16, true)
+    FX_GEMM_CASE(FX_BF16, FX_BF16, FX_F32, bf16, bf16, float, true)
+    FX_GEMM_CASE(FX_BF16, FX_F32, FX_BF16, bf16, float, bf16, true)
+    FX_GEMM_CASE(FX_BF16, FX_F32, FX_F32, bf16, float, float, true)
 #undef FX_GEMM_CASE
     return FX_ERR_DTYPE;
 }

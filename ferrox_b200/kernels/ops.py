@@ -8,6 +8,7 @@ torch fallback, and a CPU tensor is an error.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_double, c_float, c_int, c_long, c_ulonglong, c_void_p
 from typing import Optional
 
@@ -36,6 +37,7 @@ _SIGNATURES = {
     "fx_set_pdl": [_I],
     "fx_set_scan_lanes": [_I],
     "fx_gemm": [_P, _I, _L, _P, _P, _I, _L, _P, _I, _P, _I, _L, _I, _I, _I, _I, _P, _I, _L, _P],
+    "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
     "fx_embed_norm": [_P, _I, _P, _P, _I, _F, _P, _I, _I, _I, _P, _P],
     "fx_scaled_add_norm": [_P, _P, _F, _P, _I, _F, _P, _I, _I, _I, _P],
@@ -300,12 +302,54 @@ def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=N
         ldw = _rows(w)
     if Nw != N or a.shape[1] != K or (a_rows is None and a.shape[0] != M):
         raise KernelError(f"gemm shapes do not agree: a {tuple(a.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
+    if (a.dtype == w.dtype == out.dtype == torch.float32 and M > 0 and N > 0 and K > 0 and K % 4 == 0 and _rows(a) % 4 == 0
+            and ldw % 4 == 0 and wstride % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and a.is_cuda):
+        form, splits = gemm_f32_plan(M, N, K, G if group_offsets is not None else None)
+        part = torch.empty(splits * M * N, dtype=torch.float32, device=out.device) if splits > 1 else None
+        call("fx_gemm_f32", _ptr(a), _rows(a), _ptr(a_rows), _ptr(w), ldw, _ptr(bias), code(bias) if bias is not None else 0,
+             _ptr(out), _rows(out), int(accumulate), M, N, K, _ptr(group_offsets), G, wstride, form, splits, _ptr(part),
+             stream if stream is not None else stream_ptr())
+        return out
     call(
         "fx_gemm", _ptr(a), code(a), _rows(a), _ptr(a_rows), _ptr(w), code(w), ldw,
         _ptr(bias), code(bias) if bias is not None else 0, _ptr(out), code(out), _rows(out), int(accumulate),
         M, N, K, _ptr(group_offsets), G, wstride, stream if stream is not None else stream_ptr(),
     )
     return out
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
+    """(form, runs of K) of the 32-bit product's kernel (gemm_f32.cu): minus the rows a pass of the weight-streaming
+    kernel, or the rows a tile of the tiled one.
+
+    Up to 4 rows the weights are streamed once, whatever their size.  Beyond, the two kernels' times are compared, in
+    microseconds as measured on a B200: a pass of 8 rows streams the weights at 3.1 TB/s; a round of the tiled kernel
+    (four warps an SM: one 64-row tile, two 32-row tiles or half a 128-row one) takes 0.0555 us an element of K, and a
+    product cut into runs of K writes and reads its partial sums (16 x 6144 x 2048: 30.6 us streamed, 28.2 us in 32-row
+    tiles and 6 runs; 16 x 2048 x 2048: 12.3 against 20.2 us; 60 x 2048 x 5632: 46 us in 8 runs, 312 us in one).
+    Of groups, the mean number of rows decides: 4 rows a pass up to 6 rows a group (60 experts of 2816 x 2048, 4 rows
+    each: 332 us against 532 us in 32-row tiles; 13 rows each: 922 against 536 us)."""
+    if groups is not None:
+        if M > 6 * groups or groups > 1024:
+            return (32 if M <= 1 << 20 else 128), 1
+        return (-2 if M <= groups else -4), 1
+    if M <= 4:
+        return -(1 if M == 1 else 2 if M == 2 else 4), 1
+    sms, n_tiles = sm_count(), -(-N // 128)
+    best = (-(-M // 8) * (2.0 + 4.0 * N * K / 3.1e6), -8, 1)
+    for bm in (128, 64, 32):
+        tiles = n_tiles * -(-M // bm)
+        if tiles // n_tiles > 65535:     # (rows of blocks in a grid)
+            continue
+        for splits in range(1, max(1, min(16, K // 128)) + 1):
+            rounds = -(-tiles * splits * (bm // 16) // (4 * sms))
+            t = rounds * 0.0555 * K / splits + 4.0
+            if splits > 1:
+                t += 3.0 + splits * 8.0 * M * N / 5e6
+            if t < best[0]:
+                best = (t, bm, splits)
+    return best[1], best[2]
 
 
 def embed(table, ids, out, status=None, stream=None, scale=1.0):

@@ -46,6 +46,49 @@ def test_gemm_generic(dtype, M, N, K):
     assert rel(acc, base + a.float() @ w.float().T) < (3e-6 if dtype == "float32" else 1e-5)
 
 
+# sums of K products in another order: each is off by at most K roundings, in practice by about sqrt(K) of them
+F32_FORMS = [(-1, 1), (-2, 1), (-4, 1), (-8, 1), (32, 1), (64, 1), (128, 1), (32, 3), (64, 2), (128, 5)]
+
+
+@pytest.mark.parametrize("form,splits", F32_FORMS)
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (5, 61, 128), (9, 130, 1028), (33, 127, 20), (65, 257, 2048), (129, 128, 132)])
+def test_gemm_f32_forms(form, splits, M, N, K, monkeypatch):
+    """Both kernels of the 32-bit product at the edges of their tiles, passes and runs of K: with a bias, added to what
+    is there, rows wider than K, and their error against 64-bit sums no larger than that of the same sums in order."""
+    o = ops()
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (form, splits))
+    a, w, bias = rnd(M, K + 4)[:, :K], rnd(N, K + 8)[:, :K], rnd(N)
+    want = a.double() @ w.double().T
+    out = torch.full((M, N + 3), 7.0, device=DEV)
+    o.gemm(a, w, out[:, :N], bias=bias)
+    assert rel(out[:, :N], want + bias) < 3e-6 and bool((out[:, N:] == 7).all())
+    acc = rnd(M, N, seed=5)
+    base = acc.clone()
+    o.gemm(a, w, acc, accumulate=True)
+    assert rel(acc, base + want) < 3e-6
+
+
+@pytest.mark.parametrize("form", [-1, -4, -8, 32, 64, 128])
+def test_gemm_f32_groups(form, monkeypatch):
+    """Groups without rows, of one row, of a tile's rows and one more, with gathered rows, more groups than a warp."""
+    o = ops()
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (form, 1))
+    G, N, K, T = 40, 130, 68, 50
+    x, w = rnd(T, K), rnd(G, N, K)
+    counts = [0] * G
+    for g, c in ((1, 1), (2, 32), (5, 33), (31, 9), (32, 64), (33, 129), (39, 2)):
+        counts[g] = c
+    off = [0]
+    for c in counts:
+        off.append(off[-1] + c)
+    rows = torch.randint(0, T, (off[-1],), generator=torch.Generator().manual_seed(1)).to(torch.int32).to(DEV)
+    offsets = torch.tensor(off, dtype=torch.int32, device=DEV)
+    want = torch.cat([x[rows[off[g]:off[g + 1]].long()].double() @ w[g].double().T for g in range(G)])
+    out = torch.empty(off[-1], N, device=DEV)
+    o.gemm(x, w, out, a_rows=rows, group_offsets=offsets)
+    assert rel(out, want) < 3e-6
+
+
 def test_gemm_mixed_precision_weights_stay_32_bit():
     o = ops()
     a, w = rnd(5, 96, dtype=torch.bfloat16), rnd(40, 96, dtype=torch.float32)
