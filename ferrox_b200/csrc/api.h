@@ -17,6 +17,12 @@ int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long 
                 void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
                 long w_group_stride, int form, int splits, void* part, void* stream);
 
+// Prompt attention in 32 bits (attention_f32.cu); tiles as for fx_prefill_attention, of 32 queries at most.
+int fx_prefill_attention_f32(const void* q, long ldq, const void* k_pages, const void* v_pages, const int* block_table,
+                             int table_width, int page_size, const int* tiles, int n_tiles, const int* seq_slot, void* out,
+                             long ldo, int n_heads, int n_kv_heads, int head_dim, int window, float scale, float softcap,
+                             void* stream);
+
 // Streaming multiprocessors of the current device (asked once).
 int fx_sm_count();
 

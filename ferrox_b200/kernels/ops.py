@@ -38,6 +38,7 @@ _SIGNATURES = {
     "fx_set_scan_lanes": [_I],
     "fx_gemm": [_P, _I, _L, _P, _P, _I, _L, _P, _I, _P, _I, _L, _I, _I, _I, _I, _P, _I, _L, _P],
     "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
+    "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
     "fx_embed_norm": [_P, _I, _P, _P, _I, _F, _P, _I, _I, _I, _P, _P],
     "fx_scaled_add_norm": [_P, _P, _F, _P, _I, _F, _P, _I, _I, _I, _P],
@@ -962,6 +963,28 @@ def paged_attention(q, k_pages, v_pages, block_table, page_size, positions, toke
     call("fx_paged_attention", _ptr(q), _rows(q), _ptr(k_pages), _ptr(v_pages), code(q), _ptr(block_table),
          block_table.shape[1], page_size, _ptr(positions), _ptr(token_seq), _ptr(seq_slot), _ptr(out), _rows(out), T,
          n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), float(softcap or 0.0),
+         stream if stream is not None else stream_ptr())
+    return out
+
+
+F32_PREFILL_TILE = 32     # queries a tile of the 32-bit prompt attention holds
+
+
+def prefill_f32_ok(q, out, k_pages, head_dim) -> bool:
+    """Whether :func:`prefill_attention_f32` takes these operands: 32-bit rows on the 16-byte grid, heads of at most 128
+    elements in steps of 4."""
+    return (q.dtype == torch.float32 and k_pages.dtype == torch.float32 and out.dtype == torch.float32 and head_dim <= 128
+            and head_dim % 4 == 0 and _rows(q) % 4 == 0 and _rows(out) % 4 == 0 and q.data_ptr() % 16 == 0
+            and out.data_ptr() % 16 == 0)
+
+
+def prefill_attention_f32(q, k_pages, v_pages, block_table, page_size, tiles, seq_slot, out, n_heads, n_kv_heads, head_dim,
+                          window, scale, stream=None, softcap=None):
+    """Prompt attention in 32 bits; ``tiles``: int32 [n, 4] rows of (first token, rows, entry, position of the first
+    row), at most F32_PREFILL_TILE rows each."""
+    call("fx_prefill_attention_f32", _ptr(q), _rows(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+         block_table.shape[1], page_size, _ptr(tiles), tiles.shape[0], _ptr(seq_slot), _ptr(out), _rows(out), n_heads,
+         n_kv_heads, head_dim, int(window or 0), float(scale), float(softcap or 0.0),
          stream if stream is not None else stream_ptr())
     return out
 

@@ -316,8 +316,15 @@ class GqaAttention(Mixer):
                 batch.seq_slot, attn,
                 s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream, softcap=self.softcap,
             )
+        elif ops.prefill_f32_ok(qkv, attn, cache.k, s.head_dim):
+            # prompt portions in 32 bits: tiles of 32 queries
+            ops.prefill_attention_f32(
+                qkv, cache.k, cache.v, cache.block_table, cache.page_size, query_tiles(batch, ops.F32_PREFILL_TILE),
+                batch.seq_slot, attn,
+                s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream, softcap=self.softcap,
+            )
         else:
-            # 32-bit, and head sizes that are no multiple of 16: a warp per (token, head)
+            # head sizes that no tiled kernel takes: a warp per (token, head)
             ops.paged_attention(
                 qkv, cache.k, cache.v, cache.block_table, cache.page_size, batch.positions, batch.token_seq,
                 batch.seq_slot, attn, s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream,

@@ -385,6 +385,54 @@ ATT_CASES = [
 ]
 
 
+@pytest.mark.parametrize("case", [
+    # nh, nkv, d, page, window, softcap, [(keys before the portion, tokens of the portion)]
+    (4, 2, 16, 4, 0, None, [(0, 1), (0, 33), (63, 2)]),
+    (6, 3, 48, 8, 7, 5.0, [(30, 40), (0, 9)]),
+    (16, 16, 128, 64, 0, None, [(64, 65), (0, 64), (127, 1)]),
+    (28, 4, 124, 128, 100, 30.0, [(200, 70)]),
+    (3, 1, 68, 96, 0, None, [(95, 97)]),
+])
+def test_prefill_attention_f32(case):
+    """The 32-bit tiled prompt attention against the plain statement, and, where a portion's last key and value are not
+    numbers, every query before it as if they were not there."""
+    o = ops()
+    nh, nkv, d, ps, window, cap, portions = case
+    lens = [a + n for a, n in portions]
+    kp, vp, table, ks, vs = build_cache(torch.float32, lens, nkv, d, ps, n_pages=sum(-(-L // ps) for L in lens) + 3)
+    T = sum(n for _, n in portions)
+    q = rnd(T, nh * d + 8)
+    tiles, flat = [], 0
+    for b, (start, n) in enumerate(portions):
+        tiles += [(flat + i, min(32, n - i), b, start + i) for i in range(0, n, 32)]
+        flat += n
+    tiles = torch.tensor(tiles, dtype=torch.int32, device=DEV)
+    slots = torch.tensor([b + 1 for b in range(len(lens))], dtype=torch.int32, device=DEV)
+    out = torch.empty(T, nh * d, device=DEV)
+    assert o.prefill_f32_ok(q, out, kp, d)
+    args = (table, ps, tiles, slots, out, nh, nkv, d, window, d ** -0.5)
+    o.prefill_attention_f32(q, kp, vp, *args, softcap=cap)
+    flat, last = 0, []
+    for b, (start, n) in enumerate(portions):
+        for i in range(n):
+            pos, qi = start + i, q[flat + i, :nh * d].cpu().view(nh, d)
+            lo = max(0, pos - window + 1) if window else 0
+            for h in range(nh):
+                s = (ks[b][lo:pos + 1, h * nkv // nh] @ qi[h]) * d ** -0.5
+                s = cap * torch.tanh(s / cap) if cap else s
+                want = torch.softmax(s, 0) @ vs[b][lo:pos + 1, h * nkv // nh]
+                assert rel(out[flat + i].view(nh, d)[h].cpu(), want) < 5e-6
+        flat += n
+        last.append(flat - 1)
+    before = out.clone()
+    for b, L in enumerate(lens):
+        page = int(table[b + 1, (L - 1) // ps])
+        kp[page, :, (L - 1) % ps], vp[page, :, (L - 1) % ps] = float("nan"), float("inf")
+    o.prefill_attention_f32(q, kp, vp, *args, softcap=cap)
+    keep = [t for t in range(T) if t not in last]
+    assert torch.equal(out[keep], before[keep])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("case", ATT_CASES)
 @pytest.mark.parametrize("kernel", ["generic", "decode"])
