@@ -162,7 +162,11 @@ class SoftmaxTopkMoe(FeedForward):
             self.w_route = torch.cat([self.w_router.to(dtr), self.w_shared_gate.to(dtr)], dim=0).contiguous()
         self._scratch = torch.zeros(2 * E, dtype=torch.int32, device=rt.device)
         if self.w_shared_gu is not None and rt.device.type == "cuda":
-            self._side = torch.cuda.Stream(device=rt.device)
+            # one second stream for all such layers of a model (they run one after the other): its buffers are the
+            # same in every layer, and a new model's first step asks the device for them once
+            self._side = rt.groups.get("side stream")
+            if self._side is None:
+                self._side = rt.groups["side stream"] = torch.cuda.Stream(device=rt.device)
             self._fork, self._join = torch.cuda.Event(), torch.cuda.Event()
 
     def _load_table(self, src, rt):
