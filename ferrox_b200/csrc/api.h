@@ -17,6 +17,19 @@ int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long 
                 void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
                 long w_group_stride, int form, int splits, void* part, void* stream);
 
+// The recurrences of matrix-state mixers in chunks of tokens (chunk_scan.cu).
+int fx_chunk_size();
+int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const float* v, long ldv, const float* g, const float* beta,
+                  const float* take, float q_scale, float* p, float* gam, float* e, float* wr, const float* norm_in, float* norm,
+                  int copies, const float* floor_m, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,
+                  const int* seq_slot, int n_tokens, int n_entries, int H, int G, int D, int V, void* stream);
+int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, float* u, float* au,
+                          float* w, float* p, float* gam, float* wr, float* state, float* out, const int* tiles, int n_tiles,
+                          const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream);
+int fx_mlstm_gates(const float* gates, long ldg, const void* i_bias, const void* f_bias, int bias_dtype, float cap, float* m,
+                   int copies, const float* norm, float* norm_in, int D, float* keep, float* take, float* floor_m,
+                   const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, void* stream);
+
 // Prompt attention in 32 bits (attention_f32.cu); tiles as for fx_prefill_attention, of 32 queries at most.
 int fx_prefill_attention_f32(const void* q, long ldq, const void* k_pages, const void* v_pages, const int* block_table,
                              int table_width, int page_size, const int* tiles, int n_tiles, const int* seq_slot, void* out,

@@ -1,0 +1,845 @@
+// Recurrences of a matrix state per head over the tokens of a prompt, CHUNK tokens at a time instead of one by one:
+//
+//   mLSTM      S <- keep_t S + take_t k_t v_t^T, n likewise with k_t alone         o_t = S^T q_t / max(|n.q_t|, ..)
+//   delta      S <- g_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T     o_t = S^T q_t
+//   general    S <- diag(w_t) S - (a_t u_t)(u_t^T S) + k_t v_t^T                  o_t = S^T r_t
+//
+// (linear_state.cu, general_delta.cu, mlstm.cu state them and take steps of few tokens.)  Within a
+// chunk the tokens meet through products of their keys and queries alone, so that everything but the state itself is
+// worked out for all chunks at once, and what remains in the tokens' order is three small matrix products a chunk.
+// With R_ts the product of the decays of tokens s+1 .. t and G_t = R_t0 that of the chunk's tokens up to t:
+//
+//   delta:    (I + L) U = diag(beta) V - diag(beta G) K S_0,  L_ts = beta_t R_ts k_t.k_s  (s < t)
+//             U = U0 - W S_0 with [U0 | W] = (I + L)^-1 [diag(beta) V | diag(beta G) K]
+//             o_t = G_t S_0^T q_t + sum_{s <= t} R_ts (q_t.k_s) u_s,   S_C = G_C S_0 + sum_s R_Cs k_s u_s^T
+//   mLSTM:    the same with U = V and no product with W
+//   general:  decays per key channel: rows scaled by the channels' products, u'_t = u_t G_(t-1), r'_t = r_t G_t,
+//             k'_s = k_s / G_s, a'_s = a_s u_s / G_s;  y_t = u_t^T S_(t-1) solves
+//             (I + A) Y = u' S_0 + B V,  A_ts = u'_t.a'_s, B_ts = u'_t.k'_s (s < t);  Y = Y0 + W S_0
+//             o_t = S_0^T r'_t + sum_{s <= t} (r'_t.k'_s) v_s - (r'_t.a'_s) y_s
+//             S_C = diag(G_C) S_0 + sum_s (G_C k'_s) v_s^T - (G_C a'_s) y_s^T
+//             (its decays lie in (0.54, 1): over 32 tokens the products stay above 3e-9, and every term is a ratio <= 1)
+//
+// Everything is 32-bit FFMA arithmetic; products of decays are taken in 64 bits and rounded once, because one of a
+// chunk's is raised to the power of the chunks that a memory travels through.  State [slots, H, V, D], as before.
+//
+// Kernels: *_chunks make what a chunk needs (a block a chunk and head); walk_kernel goes through an entry's chunks in
+// order (a block 16 columns of a head's state).  A walk's chunk is bound by the chain of its three products and two
+// barriers, at 4 warps an SM: the block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
+// columns: 128 blocks), the next chunk's rows travel by cp.async meanwhile
+// (by untiled bulk copies, one a row, 160 a chunk: 8 us a chunk instead of 3.7).
+#include "common.cuh"
+#include "api.h"
+
+namespace {
+
+constexpr int CHUNK = 32;
+constexpr int COLS = 16;             // columns of the state a walking block owns
+constexpr int WALK_THREADS = 256;
+constexpr int PREP_THREADS = 256;
+typedef unsigned long long u64;
+
+__device__ __forceinline__ void fma2(u64& d, u64 a, u64 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ u64 pair(float x, float y) {
+    return (u64)__float_as_uint(x) | ((u64)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ float lo_of(u64 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi_of(u64 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ float sum_of(u64 v) { return lo_of(v) + hi_of(v); }
+
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
+    const int n = ok ? 16 : 0;       // the rest is filled with zeros, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n));
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, bool ok) {
+    const int n = ok ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n));
+}
+
+// first row r with token_seq[r] >= b
+__device__ __forceinline__ int first_row_of(const int* __restrict__ token_seq, int n_tokens, int b)
+{
+    int lo = 0, hi = n_tokens;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (token_seq[mid] < b) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// D rows of CHUNK tokens into shared memory, `pitch` floats apart, zeros beyond `rows` and beyond `d`.
+template <int D, int THREADS>
+__device__ __forceinline__ void load_rows(float* to, int pitch, const float* from, long ld, int rows, int d)
+{
+    constexpr int P = D / 4;
+    for (int i = threadIdx.x; i < CHUNK * P; i += THREADS) {
+        const int t = i / P, c = (i - t * P) * 4;
+        const bool ok = t < rows && c < d;
+        cp16(to + t * pitch + c, from + (ok ? (long)t * ld + c : 0), ok);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ what a chunk needs
+struct ChunkArgs {
+    const int* tiles;                // [n][4]: first token, tokens, entry, position
+    const float *q, *k, *v; long ldq, ldk, ldv;
+    float *u, *au, *w;               // general: contiguous [T, H * D]; r', G_C k' and -G_C a' take their places
+    const float* g;                  // decays [T, H]
+    const float* gate;               // delta: beta [T, H]; mLSTM: take [T, H]
+    float scale;                     // on q (mLSTM)
+    int H, G, D, V;
+    float *p;                        // [T, H, CHUNK or 2 CHUNK]: weights of the chunk's tokens in a token's read-out
+    float *gam, *e;                  // [T, H]: G_t; R_Cs (mLSTM: times take_s).  general: gam [tiles, H, D], G_C
+    float *x0, *wr;                  // [T, H, V], [T, H, D]: U0 or Y0, W
+};
+
+// Products of a chunk's decays: win[j][t] that of the 2^j tokens up to t (as many as there are), so that any run's product
+// takes at most five factors.  By the first warp; tokens beyond the chunk's rows count as decays of one.
+__device__ __forceinline__ void decay_windows(float g, double (*win)[CHUNK])
+{
+    const int t = threadIdx.x;
+    double w = (double)g;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        win[j][t] = w;
+        if (j == 5) break;
+        const double before = __shfl_up_sync(0xffffffffu, w, 1 << j);
+        if (t >= 1 << j) w *= before;
+    }
+}
+// That of the n tokens up to t (n < 32).
+__device__ __forceinline__ float decay_product(const double (*win)[CHUNK], int t, int n)
+{
+    double r = 1.0;
+#pragma unroll
+    for (int j = 0; j < 5; ++j)
+        if (n >> j & 1) { r *= win[j][t]; t -= 1 << j; }
+    return (float)r;
+}
+
+template <int D, bool DELTA>
+__global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
+{
+    constexpr int PITCH = D + 4, LP = CHUNK + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* k_s = sm;                                  // [CHUNK][PITCH]
+    float* q_s = k_s + CHUNK * PITCH;
+    float* l_s = q_s + CHUNK * PITCH;                 // [CHUNK][LP]
+    __shared__ double win[6][CHUNK];
+    __shared__ float gam[CHUNK], gate_s[CHUNK];
+    fx_pdl_wait();
+    const int4 tile = reinterpret_cast<const int4*>(a.tiles)[blockIdx.x];
+    const int tok0 = tile.x, rows = tile.y, h = blockIdx.y, tid = threadIdx.x;
+    const int kvh = h / (a.H / a.G);
+    load_rows<D, PREP_THREADS>(k_s, PITCH, a.k + (long)tok0 * a.ldk + (long)kvh * a.D, a.ldk, rows, a.D);
+    load_rows<D, PREP_THREADS>(q_s, PITCH, a.q + (long)tok0 * a.ldq + (long)kvh * a.D, a.ldq, rows, a.D);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // (the first column of the substitution below: its values travel while the chunk's products are made)
+    float x[CHUNK];
+    if (DELTA && tid < a.V) {
+        const float* vp = a.v + (long)tok0 * a.ldv + (long)h * a.V + tid;
+#pragma unroll
+        for (int t = 0; t < CHUNK; ++t) x[t] = t < rows ? vp[(long)t * a.ldv] : 0.f;
+    }
+    if (tid < CHUNK) {
+        const bool ok = tid < rows;
+        decay_windows(ok ? a.g[(long)(tok0 + tid) * a.H + h] : 1.f, win);
+        gam[tid] = (float)win[5][tid];
+        gate_s[tid] = ok ? a.gate[(long)(tok0 + tid) * a.H + h] : 0.f;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    // thread (ty, tx): tokens t = ty, ty + 16 against s = tx, tx + 16
+    const int ty = tid >> 4, tx = tid & 15;
+    u64 qk[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, kk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+        ulonglong2 ks[2], qt[2], kt[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
+            qt[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * PITCH + d);
+            if (DELTA) kt[i] = *reinterpret_cast<const ulonglong2*>(k_s + (ty + 16 * i) * PITCH + d);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                fma2(qk[i][j], qt[i].x, ks[j].x); fma2(qk[i][j], qt[i].y, ks[j].y);
+                if (DELTA) { fma2(kk[i][j], kt[i].x, ks[j].x); fma2(kk[i][j], kt[i].y, ks[j].y); }
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = ty + 16 * i, s = tx + 16 * j;
+            const float r = s < t ? decay_product(win, t, t - s) : 1.f;
+            if (DELTA) l_s[t * LP + s] = s < t ? gate_s[t] * (r * sum_of(kk[i][j])) : 0.f;
+            if (t < rows)
+                a.p[((long)(tok0 + t) * a.H + h) * CHUNK + s] =
+                    s <= t ? r * sum_of(qk[i][j]) * (DELTA ? 1.f : a.scale * gate_s[s]) : 0.f;
+        }
+    if (tid < rows) {
+        a.gam[(long)(tok0 + tid) * a.H + h] = gam[tid];
+        a.e[(long)(tok0 + tid) * a.H + h] = decay_product(win, rows - 1, rows - 1 - tid) * (DELTA ? 1.f : gate_s[tid]);
+    }
+    if (!DELTA) return;
+    __syncthreads();
+    // forward substitution, a column a thread
+    for (int c = tid; c < a.V + a.D; c += PREP_THREADS) {
+        const bool val = c < a.V;
+        if (val && c >= PREP_THREADS) {
+            const float* vp = a.v + (long)tok0 * a.ldv + (long)h * a.V + c;
+#pragma unroll
+            for (int t = 0; t < CHUNK; ++t) x[t] = t < rows ? vp[(long)t * a.ldv] : 0.f;
+        } else if (!val) {
+#pragma unroll
+            for (int t = 0; t < CHUNK; ++t) x[t] = gam[t] * k_s[t * PITCH + c - a.V];
+        }
+#pragma unroll
+        for (int t = 0; t < CHUNK; ++t) x[t] *= gate_s[t];
+#pragma unroll
+        for (int t = 1; t < CHUNK; ++t) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(l_s + t * LP + s);     // (zeros from t on)
+                s0 = fmaf(l.x, x[s], s0);
+                if (s + 1 < t) s1 = fmaf(l.y, x[s + 1], s1);
+                if (s + 2 < t) s0 = fmaf(l.z, x[s + 2], s0);
+                if (s + 3 < t) s1 = fmaf(l.w, x[s + 3], s1);
+            }
+            x[t] -= s0 + s1;
+        }
+        float* to = val ? a.x0 + ((long)tok0 * a.H + h) * a.V + c : a.wr + ((long)tok0 * a.H + h) * a.D + (c - a.V);
+        const long ld = (long)a.H * (val ? a.V : a.D);
+#pragma unroll
+        for (int t = 0; t < CHUNK; ++t)
+            if (t < rows) to[t * ld] = x[t];
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
+{
+    constexpr int PITCH = D + 4, LP = CHUNK + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* u_s = sm;                                  // [CHUNK][PITCH] each
+    float* r_s = u_s + CHUNK * PITCH;
+    float* k_s = r_s + CHUNK * PITCH;
+    float* a_s = k_s + CHUNK * PITCH;
+    float* g_s = a_s + CHUNK * PITCH;                 // decays, then their products up to each token
+    float* A_s = g_s + CHUNK * PITCH;                 // [CHUNK][LP]
+    float* B_s = A_s + CHUNK * LP;
+    fx_pdl_wait();
+    const int4 tile = reinterpret_cast<const int4*>(a.tiles)[blockIdx.x];
+    const int tok0 = tile.x, rows = tile.y, h = blockIdx.y, tid = threadIdx.x;
+    const long hd = (long)a.H * a.D, at0 = (long)tok0 * hd + (long)h * a.D;
+    load_rows<D, PREP_THREADS>(u_s, PITCH, a.u + at0, hd, rows, a.D);
+    load_rows<D, PREP_THREADS>(a_s, PITCH, a.au + at0, hd, rows, a.D);
+    load_rows<D, PREP_THREADS>(g_s, PITCH, a.w + at0, hd, rows, a.D);
+    load_rows<D, PREP_THREADS>(r_s, PITCH, a.q + (long)tok0 * a.ldq + (long)h * a.D, a.ldq, rows, a.D);
+    load_rows<D, PREP_THREADS>(k_s, PITCH, a.k + (long)tok0 * a.ldk + (long)h * a.D, a.ldk, rows, a.D);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // (the values of the first column of the substitution below travel meanwhile)
+    float v[CHUNK];
+    if (tid < a.V) {
+        const float* vp = a.v + (long)tok0 * a.ldv + (long)h * a.V + tid;
+#pragma unroll
+        for (int t = 0; t < CHUNK; ++t) v[t] = t < rows ? vp[(long)t * a.ldv] : 0.f;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // a channel's products: runs of RUN tokens a thread, then the runs before it
+    constexpr int RUNS = PREP_THREADS / D, RUN = CHUNK / RUNS;
+    __shared__ double total[RUNS][D];
+    {
+        const int d = tid % D, run = tid / D;
+        double r[RUN], p = 1.0;
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) {
+            const int t = run * RUN + i;
+            if (t < rows && d < a.D) p *= (double)g_s[t * PITCH + d];
+            r[i] = p;
+        }
+        total[run][d] = p;
+        __syncthreads();
+        p = 1.0;
+        for (int i = 0; i < run; ++i) p *= total[i][d];
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) g_s[(run * RUN + i) * PITCH + d] = (float)(p * r[i]);
+        if (run == RUNS - 1 && d < a.D) a.gam[((long)blockIdx.x * a.H + h) * a.D + d] = (float)(p * r[RUN - 1]);
+    }
+    __syncthreads();
+    for (int i = tid; i < CHUNK * D; i += PREP_THREADS) {
+        const int t = i / D, d = i - t * D, at = t * PITCH + d;
+        const float g = g_s[at], inv = 1.0f / g, last = g_s[(CHUNK - 1) * PITCH + d];
+        const float kk = k_s[at] * inv, aa = a_s[at] * inv, rr = r_s[at] * g;
+        u_s[at] *= t ? g_s[at - PITCH] : 1.f;
+        k_s[at] = kk; a_s[at] = aa; r_s[at] = rr;
+        if (t < rows && d < a.D) {
+            const long to = at0 + (long)t * hd + d;
+            a.u[to] = rr; a.au[to] = kk * last; a.w[to] = -aa * last;      // (the block has read these rows)
+        }
+    }
+    __syncthreads();
+    const int ty = tid >> 4, tx = tid & 15;
+    u64 ua[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, uk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+    u64 ra[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, rk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll 2
+    for (int d = 0; d < D; d += 4) {
+        ulonglong2 ks[2], as[2], ut[2], rt[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
+            as[i] = *reinterpret_cast<const ulonglong2*>(a_s + (tx + 16 * i) * PITCH + d);
+            ut[i] = *reinterpret_cast<const ulonglong2*>(u_s + (ty + 16 * i) * PITCH + d);
+            rt[i] = *reinterpret_cast<const ulonglong2*>(r_s + (ty + 16 * i) * PITCH + d);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                fma2(ua[i][j], ut[i].x, as[j].x); fma2(ua[i][j], ut[i].y, as[j].y);
+                fma2(uk[i][j], ut[i].x, ks[j].x); fma2(uk[i][j], ut[i].y, ks[j].y);
+                fma2(ra[i][j], rt[i].x, as[j].x); fma2(ra[i][j], rt[i].y, as[j].y);
+                fma2(rk[i][j], rt[i].x, ks[j].x); fma2(rk[i][j], rt[i].y, ks[j].y);
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = ty + 16 * i, s = tx + 16 * j;
+            A_s[t * LP + s] = s < t ? sum_of(ua[i][j]) : 0.f;
+            B_s[t * LP + s] = s < t ? sum_of(uk[i][j]) : 0.f;
+            if (t < rows) {
+                float* p = a.p + ((long)(tok0 + t) * a.H + h) * (2 * CHUNK);
+                p[s] = s <= t ? sum_of(rk[i][j]) : 0.f;
+                p[CHUNK + s] = s <= t ? -sum_of(ra[i][j]) : 0.f;
+            }
+        }
+    __syncthreads();
+    for (int c = tid; c < a.V + a.D; c += PREP_THREADS) {
+        const bool val = c < a.V;
+        float x[CHUNK];
+        if (val) {
+            x[0] = 0.f;      // (V <= PREP_THREADS: its values are here)
+#pragma unroll
+            for (int t = 1; t < CHUNK; ++t) {
+                float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+                for (int s = 0; s < t; s += 4) {
+                    const float4 b = *reinterpret_cast<const float4*>(B_s + t * LP + s);
+                    s0 = fmaf(b.x, v[s], s0);
+                    if (s + 1 < t) s1 = fmaf(b.y, v[s + 1], s1);
+                    if (s + 2 < t) s0 = fmaf(b.z, v[s + 2], s0);
+                    if (s + 3 < t) s1 = fmaf(b.w, v[s + 3], s1);
+                }
+                x[t] = s0 + s1;
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < CHUNK; ++t) x[t] = u_s[t * PITCH + c - a.V];
+        }
+#pragma unroll
+        for (int t = 1; t < CHUNK; ++t) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(A_s + t * LP + s);
+                s0 = fmaf(l.x, x[s], s0);
+                if (s + 1 < t) s1 = fmaf(l.y, x[s + 1], s1);
+                if (s + 2 < t) s0 = fmaf(l.z, x[s + 2], s0);
+                if (s + 3 < t) s1 = fmaf(l.w, x[s + 3], s1);
+            }
+            x[t] -= s0 + s1;
+        }
+        float* to = val ? a.x0 + ((long)tok0 * a.H + h) * a.V + c : a.wr + ((long)tok0 * a.H + h) * a.D + (c - a.V);
+        const long ld = (long)a.H * (val ? a.V : a.D);
+#pragma unroll
+        for (int t = 0; t < CHUNK; ++t)
+            if (t < rows) to[t * ld] = x[t];
+    }
+}
+
+// The gates of an mLSTM and its running maximum of their logarithms (mlstm.cu states them): a warp an (entry, head), a lane
+// a token.  m_t = max(f_t + m_(t-1), i_t) is a scan under (f, i) o (f', i') = (f + f', max(i + f', i')).
+__device__ __forceinline__ float logsigmoid_f(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
+
+__global__ void __launch_bounds__(32) mlstm_gates_kernel(const float* __restrict__ gates, long ldg, const void* i_bias,
+                                                         const void* f_bias, int bias_dtype, float cap, float* m_state, int copies,
+                                                         const float* __restrict__ norm, float* __restrict__ norm_in, int D, float* __restrict__ keep, float* __restrict__ take, float* __restrict__ floor_out,
+                                                         const int* __restrict__ token_seq, const int* __restrict__ seq_slot,
+                                                         int n_tokens, int H)
+{
+    fx_pdl_wait();
+    const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
+    const int r0 = first_row_of(token_seq, n_tokens, b), r1 = first_row_of(token_seq, n_tokens, b + 1);
+    if (r1 <= r0) return;
+    float* mp = m_state + ((long)seq_slot[b] * H + h) * copies;
+    // (the walk's blocks start from a copy: the first of them moves the state's own on while others may not have begun)
+    for (int d = lane; d < D; d += 32) norm_in[((long)b * H + h) * D + d] = norm[((long)seq_slot[b] * H + h) * copies * D + d];
+    const float bi = load_any(i_bias, bias_dtype, h), bf = load_any(f_bias, bias_dtype, h), inv_cap = 1.0f / cap;
+    float m = mp[0];
+    for (int c0 = r0; c0 < r1; c0 += 32) {
+        const int t = c0 + lane;
+        const float* g = gates + (long)min(t, r1 - 1) * ldg;
+        const float gi = cap * tanhf((g[h] + bi) * inv_cap);
+        const float gf = logsigmoid_f(cap * tanhf((g[H + h] + bf) * inv_cap));
+        float f = gf, i = gi;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float pf = __shfl_up_sync(0xffffffffu, f, o), pi = __shfl_up_sync(0xffffffffu, i, o);
+            if (lane >= o) { i = fmaxf(pi + f, i); f = pf + f; }
+        }
+        const float after = fmaxf(f + m, i);
+        float before = __shfl_up_sync(0xffffffffu, after, 1);
+        if (lane == 0) before = m;
+        if (t < r1) {
+            const long at = (long)t * H + h;
+            // (rounding may leave f + before a last place above the maximum that it is one of)
+            keep[at] = expf(fminf(gf + before - after, 0.f));
+            take[at] = expf(fminf(gi - after, 0.f));
+            floor_out[at] = expf(-after);
+        }
+        m = __shfl_sync(0xffffffffu, after, min(31, r1 - 1 - c0));
+    }
+    for (int i = lane; i < copies; i += 32) mp[i] = m;
+}
+
+// ------------------------------------------------------------------------------------------------------ the walk
+struct WalkArgs {
+    const float* w;                            // rows of W [T, H * D] (not mLSTM)
+    const float* q; long ldq; int q_share;     // rows of q (general: r'), heads that share one
+    const float* k; long ldk;                  // rows of k (general: G_C k')
+    const float* a;                            // general: -G_C a'  [T, H * D]
+    const float* v; long ldv;                  // general, mLSTM: values
+    const float* x0;                           // delta: U0, general: Y0  [T, H * V]
+    const float *p, *gam, *e;
+    const float* floor_m;                      // mLSTM: exp(-m_t) [T, H], or null
+    const float* norm_in;                      // mLSTM: the normaliser before the step [entries, H, D]
+    float* norm; int copies;                   // and its copies in the state [slots, H, copies, D]
+    float q_scale;                             // mLSTM: on q
+    float* state; float* out; long ldo;
+    const int *token_seq, *seq_slot;
+    const int* tiles; int n_tiles;             // general: as for the chunks' kernel
+    int n_tokens, H, D, V;
+};
+
+enum { DELTA_RULE = 1, GENERAL = 2, MLSTM = 3 };
+
+template <int D, int KIND> struct Stage {
+    static constexpr bool HASW = KIND == DELTA_RULE || KIND == GENERAL;
+    static constexpr int C2 = KIND == GENERAL ? 2 * CHUNK : CHUNK;      // rows that update the state
+    static constexpr int PITCH = D + 4, PP = C2 + 4;
+    float w[HASW ? CHUNK * PITCH : 4], q[CHUNK * PITCH], k[C2 * D], p[CHUNK * PP];
+    float v[CHUNK * COLS], y[KIND == GENERAL ? CHUNK * COLS : 4];
+    float gam[KIND == GENERAL ? D : CHUNK], e[CHUNK], fl[CHUNK];
+};
+template <int D, int KIND> struct WalkSmem {
+    Stage<D, KIND> st[2];
+    float s[COLS * (D + 4)];                                     // the state's columns, along the keys
+    float ut[COLS * Stage<D, KIND>::PP];                         // the update's values along the tokens,
+    float2 un[Stage<D, KIND>::C2 * COLS];                        // and along the columns, each twice (an FFMA pair's operand)
+    float part[(WALK_THREADS / D - 1) * COLS * D];               // partial updates of the state
+    float z[D], den[CHUNK];
+};
+
+// Partial sums of 4 tokens x 4 columns, spread over eight neighbouring lanes (kg), added up: lane kg gets column
+// 2 (kg & 1) + (kg >> 1 & 1) of tokens 2 (kg >> 2) and 2 (kg >> 2) + 1.
+__device__ __forceinline__ void over_lanes(const float (&x)[4][4], int kg, float (&y)[2])
+{
+    const bool b0 = kg & 1, b1 = kg & 2, b2 = kg & 4;
+    float m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float m0 = (b0 ? x[i][2] : x[i][0]) + __shfl_xor_sync(0xffffffffu, b0 ? x[i][0] : x[i][2], 1);
+        const float m1 = (b0 ? x[i][3] : x[i][1]) + __shfl_xor_sync(0xffffffffu, b0 ? x[i][1] : x[i][3], 1);
+        m[i] = (b1 ? m1 : m0) + __shfl_xor_sync(0xffffffffu, b1 ? m0 : m1, 2);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) y[i] = (b2 ? m[2 + i] : m[i]) + __shfl_xor_sync(0xffffffffu, b2 ? m[i] : m[2 + i], 4);
+}
+
+// One block an SM where one prompt's heads are walked, so that what counts is a warp's chain of instructions and how many
+// warps share a scheduler: two, on tiles large enough that neither the loads from shared memory (a 16-byte load of a warp
+// takes four cycles of an SM) nor the moves around them outnumber the products.  Eight lanes share out the inner index of
+// a tile of 4 tokens (of W and of Q) x 4 columns and add their sums by exchanges; the update's rows are shared out over
+// parts of the block.  (Heads of 128 x 128, a chunk: 2 x 2 tiles with the whole inner index a thread, 4 warps: 4.1 us;
+// 4 x 4 tiles, 4 warps: 3.7 us, 2,500 instructions a warp at three cycles each.)
+template <int D, int KIND>
+__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
+{
+    using St = Stage<D, KIND>;
+    constexpr bool HASW = St::HASW;
+    constexpr int C2 = St::C2, PITCH = St::PITCH, PP = St::PP;
+    constexpr int DG = D / 4;                                    // a thread holds four keys of four columns of the state
+    constexpr int PARTS = WALK_THREADS / D;                      // parts of the block, each with its share of the update's rows
+    extern __shared__ __align__(16) unsigned char raw[];
+    WalkSmem<D, KIND>& sm = *reinterpret_cast<WalkSmem<D, KIND>*>(raw);
+    const int tid = threadIdx.x, b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
+    fx_pdl_wait_only();
+    const int r0 = first_row_of(a.token_seq, a.n_tokens, b), r1 = first_row_of(a.token_seq, a.n_tokens, b + 1);
+    if (r1 <= r0) return;
+    const int nc = min(COLS, a.V - col0);
+    const long slot = a.seq_slot[b];
+    float* state = a.state + ((slot * a.H + h) * a.V + col0) * a.D;
+
+    const long HD = (long)a.H * a.D, HV = (long)a.H * a.V;
+    int tile0 = 0;                   // general: the entry's first chunk
+    if (KIND == GENERAL) {
+        int hi = a.n_tiles;
+        while (tile0 < hi) {
+            const int mid = (tile0 + hi) >> 1;
+            if (a.tiles[mid * 4 + 2] < b) tile0 = mid + 1; else hi = mid;
+        }
+    }
+    auto fetch = [&](int c0, St& st) {
+        const int rows = min(CHUNK, r1 - c0);
+        if (HASW) load_rows<D, WALK_THREADS>(st.w, PITCH, a.w + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
+        load_rows<D, WALK_THREADS>(st.q, PITCH, a.q + (long)c0 * a.ldq + (long)(h / a.q_share) * a.D, a.ldq, rows, a.D);
+        load_rows<D, WALK_THREADS>(st.k, D, a.k + (long)c0 * a.ldk + (long)(h / a.q_share) * a.D, a.ldk, rows, a.D);
+        if (KIND == GENERAL) load_rows<D, WALK_THREADS>(st.k + CHUNK * D, D, a.a + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
+        for (int i = tid; i < CHUNK * (C2 / 4); i += WALK_THREADS) {
+            const int t = i / (C2 / 4), s = (i - t * (C2 / 4)) * 4;
+            cp16(st.p + t * PP + s, a.p + (t < rows ? ((long)(c0 + t) * a.H + h) * C2 + s : 0), t < rows);
+        }
+        if (tid < 4 * CHUNK) {
+            const int t = tid >> 2, c = (tid & 3) * 4;
+            const bool ok = t < rows && c < nc;
+            const long at = (long)(c0 + t) * HV + (long)h * a.V + col0 + c;
+            if (KIND == DELTA_RULE) cp16(st.v + t * COLS + c, a.x0 + (ok ? at : 0), ok);
+            else cp16(st.v + t * COLS + c, a.v + (ok ? (long)(c0 + t) * a.ldv + (long)h * a.V + col0 + c : 0), ok);
+            if (KIND == GENERAL) cp16(st.y + t * COLS + c, a.x0 + (ok ? at : 0), ok);
+        }
+        if (KIND == GENERAL) {
+            if (tid < DG) cp16(st.gam + tid * 4, a.gam + (tid * 4 < a.D ? ((long)(tile0 + (c0 - r0) / CHUNK) * a.H + h) * a.D + tid * 4 : 0), tid * 4 < a.D);
+        } else if (tid < CHUNK) {
+            const long at = tid < rows ? (long)(c0 + tid) * a.H + h : 0;
+            cp4(st.gam + tid, a.gam + at, tid < rows);
+            cp4(st.e + tid, a.e + at, tid < rows);
+            if (KIND == MLSTM) cp4(st.fl + tid, a.floor_m + at, tid < rows);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // the state: thread (dg, cg) of part 0 holds keys 4 dg .. of columns 4 cg ..; the other parts hold updates only
+    const int dg = tid % DG, cg = (tid / DG) & 3, part = tid / (DG * 4);
+    u64 S[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = cg * 4 + j;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (part == 0 && c < nc && dg * 4 < a.D) x = *reinterpret_cast<const float4*>(state + (long)c * a.D + dg * 4);
+        S[j][0] = pair(x.x, x.y); S[j][1] = pair(x.z, x.w);
+        if (part == 0) *reinterpret_cast<float4*>(sm.s + c * PITCH + dg * 4) = x;
+    }
+    float z = 0.f;                                               // mLSTM: the normaliser's element tid
+    if (KIND == MLSTM && tid < D) {
+        z = tid < a.D ? a.norm_in[((long)b * a.H + h) * a.D + tid] : 0.f;
+        sm.z[tid] = z;
+    }
+    fetch(r0, sm.st[0]);
+    // products: tokens t0 .. t0 + 3 and columns w4 .. w4 + 3, of which this lane ends up with tokens tl, tl + 1 of column c
+    const int kg = tid & 7, t0 = (tid >> 7) * 16 + ((tid >> 3) & 3) * 4, w4 = ((tid >> 5) & 3) * 4;
+    const int tl = t0 + 2 * (kg >> 2), c = w4 + 2 * (kg & 1) + ((kg >> 1) & 1);
+    int buf = 0;
+    for (int c0 = r0; c0 < r1; c0 += CHUNK, buf ^= 1) {
+        const int rows = min(CHUNK, r1 - c0);
+        St& st = sm.st[buf];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();             // this chunk's rows are there, the state is up to date, the other place is free
+        if (c0 + CHUNK < r1) fetch(c0 + CHUNK, sm.st[buf ^ 1]);
+
+        // W S_0 and Q S_0
+        float xq[4][4], xw[4][4];
+        {
+            u64 pq[4][4], pw[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { pq[i][j] = 0ull; pw[i][j] = 0ull; }
+#pragma unroll 2
+            for (int d = kg * 4; d < D; d += 32) {
+                ulonglong2 s[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[j] = *reinterpret_cast<const ulonglong2*>(sm.s + (w4 + j) * PITCH + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(st.q + (t0 + i) * PITCH + d);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { fma2(pq[i][j], q.x, s[j].x); }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { fma2(pq[i][j], q.y, s[j].y); }
+                    if (HASW) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(st.w + (t0 + i) * PITCH + d);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) { fma2(pw[i][j], w.x, s[j].x); }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) { fma2(pw[i][j], w.y, s[j].y); }
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { xq[i][j] = sum_of(pq[i][j]); xw[i][j] = HASW ? sum_of(pw[i][j]) : 0.f; }
+        }
+        {
+            float x[2], u[2], y[2];
+            if (HASW) over_lanes(xw, kg, x);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = tl + i;
+                u[i] = st.v[t * COLS + c];
+                if (KIND == DELTA_RULE) u[i] -= x[i];
+                const float ue = KIND == GENERAL ? u[i] : u[i] * st.e[t];
+                sm.un[t * COLS + c] = make_float2(ue, ue);
+                if (KIND == GENERAL) {
+                    y[i] = st.y[t * COLS + c] + x[i];
+                    sm.un[(CHUNK + t) * COLS + c] = make_float2(y[i], y[i]);
+                }
+            }
+            *reinterpret_cast<float2*>(sm.ut + c * PP + tl) = make_float2(u[0], u[1]);
+            if (KIND == GENERAL) *reinterpret_cast<float2*>(sm.ut + c * PP + CHUNK + tl) = make_float2(y[0], y[1]);
+        }
+        if (KIND == MLSTM) {
+            // n_t . q_t: eight threads a token
+            const int t = tid >> 3;
+            float acc = 0.f;
+            for (int d = kg * 4; d < D; d += 32) {
+                const float4 q = *reinterpret_cast<const float4*>(st.q + t * PITCH + d);
+                const float4 n = *reinterpret_cast<const float4*>(sm.z + d);
+                acc = fmaf(q.x, n.x, acc); acc = fmaf(q.y, n.y, acc); acc = fmaf(q.z, n.z, acc); acc = fmaf(q.w, n.w, acc);
+            }
+            acc *= st.gam[t] * a.q_scale;
+            const float4 p = *reinterpret_cast<const float4*>(st.p + t * PP + kg * 4);
+            acc += (p.x + p.y) + (p.z + p.w);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+            if (kg == 0) sm.den[t] = fmaxf(fabsf(acc), st.fl[t]) + 1e-6f;
+        }
+        __syncthreads();             // the update's values are there, everyone has read the state
+
+        // the read-outs: the chunk's own tokens up to each one, on top of Q S_0 (the later tokens' values are left out, not
+        // multiplied by zero: what is no number must not reach the tokens before it)
+        {
+            u64 o[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[i][j] = 0ull;
+#pragma unroll
+            for (int n = 0; n < C2 / 32; ++n) {
+                const int s = n * 32 + kg * 4, sb = s & (CHUNK - 1);
+                if (sb > t0) continue;
+                const bool full = sb < t0;                       // else s .. s + 3 are the tile's own four tokens
+                u64 ux[4], uy[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(sm.ut + (w4 + j) * PP + s);
+                    ux[j] = u.x; uy[j] = u.y;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(st.p + (t0 + i) * PP + s);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        fma2(o[i][j], p.x, full || i > 0 ? ux[j] : ux[j] & 0xffffffffull);
+                        fma2(o[i][j], p.y, full || i > 2 ? uy[j] : i > 1 ? uy[j] & 0xffffffffull : 0ull);
+                    }
+                }
+            }
+            float y[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float g = KIND == GENERAL ? 1.f : KIND == DELTA_RULE ? st.gam[t0 + i] : st.gam[t0 + i] * a.q_scale;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xq[i][j] = fmaf(g, xq[i][j], sum_of(o[i][j]));
+            }
+            over_lanes(xq, kg, y);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = tl + i;
+                if (t >= rows || c >= nc) continue;
+                if (KIND == MLSTM) y[i] /= sm.den[t];
+                a.out[(long)(c0 + t) * a.ldo + (long)h * a.V + col0 + c] = y[i];
+            }
+        }
+
+        // the state
+        if (KIND == GENERAL) {
+            const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(st.gam + dg * 4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                S[j][0] = pair(lo_of(S[j][0]) * lo_of(g.x), hi_of(S[j][0]) * hi_of(g.x));
+                S[j][1] = pair(lo_of(S[j][1]) * lo_of(g.y), hi_of(S[j][1]) * hi_of(g.y));
+            }
+        } else {
+            const float g = st.gam[rows - 1];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                S[j][0] = pair(lo_of(S[j][0]) * g, hi_of(S[j][0]) * g);
+                S[j][1] = pair(lo_of(S[j][1]) * g, hi_of(S[j][1]) * g);
+            }
+            if (KIND == MLSTM && tid < D) {
+                float acc = 0.f;
+#pragma unroll 8
+                for (int s = 0; s < CHUNK; ++s) acc = fmaf(st.e[s], st.k[s * D + tid], acc);
+                z = fmaf(g, z, acc);
+            }
+        }
+#pragma unroll 8
+        for (int i = 0; i < C2 / PARTS; ++i) {
+            const int s = part * (C2 / PARTS) + i;
+            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(st.k + s * D + dg * 4);
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4);
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4 + 2);
+            fma2(S[0][0], k.x, u.x); fma2(S[0][1], k.y, u.x); fma2(S[1][0], k.x, u.y); fma2(S[1][1], k.y, u.y);
+            fma2(S[2][0], k.x, v.x); fma2(S[2][1], k.y, v.x); fma2(S[3][0], k.x, v.y); fma2(S[3][1], k.y, v.y);
+        }
+        if (part > 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                *reinterpret_cast<ulonglong2*>(sm.part + ((part - 1) * COLS + cg * 4 + j) * D + dg * 4) = make_ulonglong2(S[j][0], S[j][1]);
+                S[j][0] = 0ull; S[j][1] = 0ull;
+            }
+        }
+        __syncthreads();
+        if (part == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int i = 0; i < PARTS - 1; ++i) {
+                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sm.part + (i * COLS + cg * 4 + j) * D + dg * 4);
+                    S[j][0] = pair(lo_of(S[j][0]) + lo_of(x.x), hi_of(S[j][0]) + hi_of(x.x));
+                    S[j][1] = pair(lo_of(S[j][1]) + lo_of(x.y), hi_of(S[j][1]) + hi_of(x.y));
+                }
+                *reinterpret_cast<ulonglong2*>(sm.s + (cg * 4 + j) * PITCH + dg * 4) = make_ulonglong2(S[j][0], S[j][1]);
+            }
+        }
+        if (KIND == MLSTM && tid < D) sm.z[tid] = z;
+    }
+    fx_pdl_trigger();
+    if (part == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int cc = cg * 4 + j;
+            if (cc < nc && dg * 4 < a.D)
+                *reinterpret_cast<float4*>(state + (long)cc * a.D + dg * 4) =
+                    make_float4(lo_of(S[j][0]), hi_of(S[j][0]), lo_of(S[j][1]), hi_of(S[j][1]));
+        }
+    }
+    if (KIND == MLSTM && blockIdx.x == 0 && tid < a.D)
+        for (int i = 0; i < a.copies; ++i) a.norm[((slot * a.H + h) * a.copies + i) * a.D + tid] = z;
+}
+
+template <int D, int KIND> int go_walk(const WalkArgs& a, int n_entries, cudaStream_t s)
+{
+    const int smem = (int)sizeof(WalkSmem<D, KIND>);
+    static const cudaError_t set = cudaFuncSetAttribute(walk_kernel<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (set != cudaSuccess) return (int)set;
+    // (not set up early: its blocks stay for the whole prompt, see fx_launch_pdl_if)
+    fx_launch_pdl_if(false, walk_kernel<D, KIND>, dim3((unsigned)fx_cdiv(a.V, COLS), (unsigned)a.H, (unsigned)n_entries), WALK_THREADS,
+                     (size_t)smem, s, a);
+    return fx_launch_status();
+}
+
+template <typename K> int go_chunks(K kernel, const ChunkArgs& a, int n_tiles, size_t smem, cudaStream_t s)
+{
+    const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (set != cudaSuccess) return (int)set;
+    fx_launch_pdl(kernel, dim3((unsigned)n_tiles, (unsigned)a.H), PREP_THREADS, smem, s, a);
+    return fx_launch_status();
+}
+
+int check(int H, int G, int D, int V, int n_entries)
+{
+    if (H <= 0 || H > 65535 || G <= 0 || H % G || D <= 0 || D > 128 || V <= 0 || n_entries > 65535) return FX_ERR_SIZE;
+    if (D % 4 || V % 4) return FX_ERR_SIZE;
+    return FX_OK;
+}
+bool off_grid(const void* p, long ld) { return (uintptr_t)p % 16 || ld % 4; }
+
+}  // namespace
+
+extern "C" int fx_chunk_size() { return CHUNK; }
+
+// The delta rule (beta [T, H]) or, with take [T, H] (a factor on k v^T), norm_in, norm and floor_m, an mLSTM's recurrence.
+// q, k [T, G * D], v [T, H * V] 32-bit rows; g [T, H] the decays.  Scratch: p [T, H, CHUNK], gam and e [T, H]; delta rule: wr
+// [T, H, D].  norm_in: the normaliser before the step [entries, H, D], norm its copies in the state [slots, H, copies, D],
+// floor_m exp(-m_t) [T, H], as fx_mlstm_gates leaves them.  out contiguous [T, H * V] (the delta rule's U0 until a chunk's
+// read-outs take its place: a block reads a chunk's share of it before it writes it).
+extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const float* v, long ldv, const float* g,
+                             const float* beta, const float* take, float q_scale, float* p, float* gam, float* e, float* wr,
+                             const float* norm_in, float* norm, int copies, const float* floor_m, float* state, float* out,
+                             const int* tiles, int n_tiles, const int* token_seq, const int* seq_slot, int n_tokens, int n_entries,
+                             int H, int G, int D, int V, void* stream)
+{
+    if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
+    int st = check(H, G, D, V, n_entries);
+    if (st != FX_OK) return st;
+    if (beta ? !wr || take || norm : !take || !norm || !norm_in || !floor_m || copies < 1) return FX_ERR_SIZE;
+    if (off_grid(q, ldq) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(p, 0) || off_grid(state, 0) || off_grid(out, 0) ||
+        off_grid(wr, 0) || off_grid(tiles, 0))
+        return FX_ERR_ALIGN;
+    cudaStream_t s = (cudaStream_t)stream;
+    ChunkArgs c = {};
+    c.tiles = tiles; c.q = q; c.k = k; c.v = v; c.ldq = ldq; c.ldk = ldk; c.ldv = ldv; c.g = g;
+    c.gate = beta ? beta : take; c.scale = q_scale; c.H = H; c.G = G; c.D = D; c.V = V; c.p = p; c.gam = gam; c.e = e; c.x0 = out; c.wr = wr;
+    const size_t small = sizeof(float) * (2 * CHUNK * (64 + 4) + CHUNK * (CHUNK + 4)), large = small + sizeof(float) * 2 * CHUNK * 64;
+    if (beta) st = D <= 64 ? go_chunks(scalar_chunks<64, true>, c, n_tiles, small, s) : go_chunks(scalar_chunks<128, true>, c, n_tiles, large, s);
+    else st = D <= 64 ? go_chunks(scalar_chunks<64, false>, c, n_tiles, small, s) : go_chunks(scalar_chunks<128, false>, c, n_tiles, large, s);
+    if (st != FX_OK) return st;
+    WalkArgs a = {};
+    a.w = wr; a.q = q; a.ldq = ldq; a.q_share = H / G; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.x0 = out; a.p = p; a.gam = gam; a.e = e;
+    a.floor_m = floor_m; a.norm_in = norm_in; a.norm = norm; a.copies = copies; a.q_scale = q_scale; a.state = state; a.out = out;
+    a.ldo = (long)H * V; a.token_seq = token_seq; a.seq_slot = seq_slot; a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = V;
+    if (beta) return D <= 64 ? go_walk<64, DELTA_RULE>(a, n_entries, s) : go_walk<128, DELTA_RULE>(a, n_entries, s);
+    return D <= 64 ? go_walk<64, MLSTM>(a, n_entries, s) : go_walk<128, MLSTM>(a, n_entries, s);
+}
+
+// The generalized delta rule.  r, k, v rows [T, H * D]; u, au, w contiguous [T, H * D], overwritten; scratch: p [T, H, 2 CHUNK],
+// gam [tiles, H, D], wr [T, H, D].  out contiguous [T, H * D]: it holds Y0 until a chunk's read-outs take its place.
+extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, float* u, float* au,
+                                     float* w, float* p, float* gam, float* wr, float* state, float* out, const int* tiles, int n_tiles,
+                                     const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream)
+{
+    if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
+    int st = check(H, H, D, D, n_entries);
+    if (st != FX_OK) return st;
+    if (off_grid(r, ldr) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(u, 0) || off_grid(au, 0) || off_grid(w, 0) ||
+        off_grid(p, 0) || off_grid(gam, 0) || off_grid(wr, 0) || off_grid(out, 0) || off_grid(state, 0) || off_grid(tiles, 0))
+        return FX_ERR_ALIGN;
+    cudaStream_t s = (cudaStream_t)stream;
+    ChunkArgs c = {};
+    c.tiles = tiles; c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.u = u; c.au = au; c.w = w;
+    c.H = H; c.G = H; c.D = D; c.V = D; c.p = p; c.gam = gam; c.x0 = out; c.wr = wr;
+    const size_t small = sizeof(float) * (5 * CHUNK * (64 + 4) + 2 * CHUNK * (CHUNK + 4)), large = small + sizeof(float) * 5 * CHUNK * 64;
+    st = D <= 64 ? go_chunks(general_chunks<64>, c, n_tiles, small, s) : go_chunks(general_chunks<128>, c, n_tiles, large, s);
+    if (st != FX_OK) return st;
+    WalkArgs a = {};
+    a.w = wr; a.q = u; a.ldq = (long)H * D; a.q_share = 1; a.k = au; a.ldk = (long)H * D; a.a = w; a.v = v; a.ldv = ldv; a.x0 = out;
+    a.p = p; a.gam = gam; a.q_scale = 1.f; a.state = state; a.out = out; a.ldo = (long)H * D; a.token_seq = token_seq; a.seq_slot = seq_slot;
+    a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles;
+    return D <= 64 ? go_walk<64, GENERAL>(a, n_entries, s) : go_walk<128, GENERAL>(a, n_entries, s);
+}
+
+// The gates of an mLSTM for fx_chunk_scan: keep, take and floor_m [T, H] from the projected [i | f] rows; moves the running
+// maximum's copies [slots, H, copies] on; norm_in [entries, H, D] gets the normaliser as it is.
+extern "C" int fx_mlstm_gates(const float* gates, long ldg, const void* i_bias, const void* f_bias, int bias_dtype, float cap, float* m,
+                              int copies, const float* norm, float* norm_in, int D, float* keep, float* take, float* floor_m, const int* token_seq, const int* seq_slot,
+                              int n_tokens, int n_entries, int H, void* stream)
+{
+    if (n_tokens <= 0 || n_entries <= 0) return FX_OK;
+    if (H <= 0 || H > 65535 || copies < 1 || !(cap > 0.f)) return FX_ERR_SIZE;
+    fx_launch_pdl(mlstm_gates_kernel, dim3((unsigned)n_entries, (unsigned)H), 32, 0, (cudaStream_t)stream, gates, ldg, i_bias, f_bias,
+                  bias_dtype, cap, m, copies, norm, norm_in, D, keep, take, floor_m, token_seq, seq_slot, n_tokens, H);
+    return fx_launch_status();
+}

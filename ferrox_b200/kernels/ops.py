@@ -39,6 +39,10 @@ _SIGNATURES = {
     "fx_gemm": [_P, _I, _L, _P, _P, _I, _L, _P, _I, _P, _I, _L, _I, _I, _I, _I, _P, _I, _L, _P],
     "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
+    "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
+                      _I, _I, _I, _I, _I, _I, _P],
+    "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "fx_mlstm_gates": [_P, _L, _P, _P, _I, _F, _P, _I, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
     "fx_embed_norm": [_P, _I, _P, _P, _I, _F, _P, _I, _I, _I, _P, _P],
     "fx_scaled_add_norm": [_P, _P, _F, _P, _I, _F, _P, _I, _I, _I, _P],
@@ -626,6 +630,59 @@ def state_scan(q, k, v, g, g_ld, beta, state, out, token_seq, seq_slot, n_entrie
          int(g_ld), _ptr(beta), _ptr(state), _ptr(out), _rows(out), _ptr(token_seq), _ptr(seq_slot), T, int(n_entries),
          H, G, D, V, stream if stream is not None else stream_ptr())
     return out
+
+
+SCAN_CHUNK = 32      # tokens a chunk of the chunked recurrences (chunk_scan.cu)
+
+
+def chunk_scan_ok(rows, D, V, state) -> bool:
+    """Whether the chunked recurrences take these 32-bit row views and this state: heads of at most 128 rows, widths in
+    steps of 4, rows on the 16-byte grid."""
+    return (D <= 128 and D % 4 == 0 and V % 4 == 0 and state.data_ptr() % 16 == 0
+            and all(t.dtype == torch.float32 and _rows(t) % 4 == 0 and t.data_ptr() % 16 == 0 for t in rows))
+
+
+def chunk_scan(q, k, v, g, state, out, tiles, token_seq, seq_slot, n_entries, H, G, D, V, *, beta=None, take=None,
+               q_scale=1.0, normalizer=None, scratch, stream=None):
+    """Over a prompt's chunks of SCAN_CHUNK tokens, with ``beta`` [T, H] the delta rule of :func:`state_scan`, with ``take``
+    [T, H] and ``normalizer`` = (its value before the step, the state's copies, exp(-m)), as :func:`mlstm_gates` makes
+    them, the recurrence of :func:`mlstm_scan`.  ``g`` [T, H]: the decays; ``out`` contiguous [T, H * V]; ``tiles``: int32
+    [n, 4] rows of (first token, tokens, entry, position), the entries cut into chunks; ``scratch(*shape)``: 32-bit
+    buffers."""
+    T = q.shape[0]
+    if not (g.is_contiguous() and out.is_contiguous()):
+        raise KernelError("chunk_scan: contiguous decays and read-outs")
+    p, gam, e = scratch(T, H, SCAN_CHUNK), scratch(T, H), scratch(T, H)
+    wr = scratch(T, H, D) if beta is not None else None
+    norm_in, norm, floor_m = normalizer if normalizer is not None else (None, None, None)
+    call("fx_chunk_scan", _ptr(q), _rows(q), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(g), _ptr(beta), _ptr(take),
+         float(q_scale), _ptr(p), _ptr(gam), _ptr(e), _ptr(wr), _ptr(norm_in), _ptr(norm),
+         int(norm.shape[2]) if norm is not None else 0, _ptr(floor_m), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0],
+         _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, G, D, V, stream if stream is not None else stream_ptr())
+    return out
+
+
+def chunk_scan_general(r, k, v, u, au, w, state, out, tiles, token_seq, seq_slot, n_entries, H, D, *, scratch, stream=None):
+    """:func:`general_delta_scan` over a prompt's chunks (see :func:`chunk_scan`); ``u``, ``au`` and ``w`` are overwritten."""
+    T = r.shape[0]
+    if not all(t.is_contiguous() for t in (u, au, w, out)):
+        raise KernelError("chunk_scan_general: contiguous unit keys, decays and read-outs")
+    p, gam, wr = scratch(T, H, 2 * SCAN_CHUNK), scratch(tiles.shape[0], H, D), scratch(T, H, D)
+    call("fx_chunk_scan_general", _ptr(r), _rows(r), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(u), _ptr(au), _ptr(w), _ptr(p),
+         _ptr(gam), _ptr(wr), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0], _ptr(token_seq), _ptr(seq_slot), T,
+         int(n_entries), H, D, stream if stream is not None else stream_ptr())
+    return out
+
+
+def mlstm_gates(gates, i_bias, f_bias, cap, log_max, normalizer, norm_in, keep, take, floor_m, token_seq, seq_slot, n_entries, H, D,
+                stream=None):
+    """An mLSTM's gates for :func:`chunk_scan`: ``keep``, ``take`` and ``floor_m`` = exp(-m) [T, H]; ``log_max`` is moved on,
+    ``norm_in`` [entries, H, D] gets the normaliser as it is before the step."""
+    if i_bias.dtype != f_bias.dtype:
+        raise KernelError("mlstm_gates: both gate biases of one element type")
+    call("fx_mlstm_gates", _ptr(gates), _rows(gates), _ptr(i_bias), _ptr(f_bias), code(i_bias), float(cap), _ptr(log_max),
+         int(log_max.shape[2]), _ptr(normalizer), _ptr(norm_in), int(D), _ptr(keep), _ptr(take), _ptr(floor_m), _ptr(token_seq),
+         _ptr(seq_slot), gates.shape[0], int(n_entries), H, stream if stream is not None else stream_ptr())
 
 
 GROUP_NORM_GATES = {"silu": 0, "sigmoid": 1}

@@ -43,11 +43,31 @@ import torch
 from ..cache.specs import CacheSpec, StateSpec
 from ..kernels import ops
 from ..weights.loader import TensorDecl
+from .attention import query_tiles
 from .base import Mixer, register_part
 
 
 # From this many tokens an entry of the step on, the fixed-decay recurrence takes the kernel made for prompts.
 FIXED_DECAY_MIN_TOKENS = 32
+
+
+def _chunk_tiles(batch, H, V):
+    """The step's entries cut into chunks of tokens (the work list of ``ops.chunk_scan``) where that form of a recurrence
+    is the faster one, else None.
+
+    In microseconds on a B200, 16 heads of 128 x 128 (32 of 64 x 64 likewise): token by token 0.33 to 0.43 a token of the
+    longest entry, and at least 0.13 a token of the step; in chunks 10 and 4.2 a chunk of the longest entry, or of all
+    entries where their blocks (16 columns of a head each) need more than the device's SMs (one prompt of 64 tokens: 31
+    against 19, of 2,048: 868 against 282; 40 tokens beside 16 decoded ones: 39 against 94; four prompts of 500: 267
+    against 289)."""
+    chunk, most, T = ops.SCAN_CHUNK, batch.max_new, batch.n_tokens
+    if most < chunk:
+        return None
+    chunks = sum(-(-len(e.tokens) // chunk) for e in batch.entries)
+    rounds = max(-(-most // chunk), chunks * H * -(-V // 16) / ops.sm_count())
+    if 10 + 4.2 * rounds >= max(0.38 * most, 0.13 * T):
+        return None
+    return query_tiles(batch, chunk)
 
 
 def _cat_rows(tensors):
@@ -60,6 +80,9 @@ class _StateMixer(Mixer):
 
     def forward_add(self, x, h, batch, cache):
         self.forward_into(x, h, batch, cache, accumulate=True)
+
+    def _scratch(self, *shape):
+        return self.rt.empty(*shape, dtype=torch.float32)
 
 
 class GatedDeltaRule(_StateMixer):
@@ -126,8 +149,14 @@ class GatedDeltaRule(_StateMixer):
             ops.conv_tail_update(proj, self.channels, s.conv_taps, tail, batch.token_seq, batch.seq_slot, batch.n_seqs,
                                  stream=batch.stream)
         read = rt.empty(T, self.vv, dtype=f32)
-        ops.state_scan(qkv[:, :self.qk], qkv[:, self.qk:2 * self.qk], qkv[:, 2 * self.qk:], g, H, beta, state, read,
-                       batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V, stream=batch.stream)
+        q, k, v = qkv[:, :self.qk], qkv[:, self.qk:2 * self.qk], qkv[:, 2 * self.qk:]
+        tiles = _chunk_tiles(batch, H, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
+        if tiles is not None:
+            ops.chunk_scan(q, k, v, g, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
+                           beta=beta, scratch=self._scratch, stream=batch.stream)
+        else:
+            ops.state_scan(q, k, v, g, H, beta, state, read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
+                           stream=batch.stream)
         y = rt.empty(T, self.vv)
         ops.gated_group_norm(read, proj[:, self.channels:self.channels + self.vv], self.norm_w, s.norm_eps, "silu", y, H, V, stream=batch.stream)
         ops.linear(y, self.w_o, out, accumulate=accumulate, status=batch.status, stream=batch.stream)
@@ -239,9 +268,15 @@ class GeneralDeltaRule(_StateMixer):
         u, au, w = rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32)
         ops.general_delta_prep(k, proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:], self.w2, self.w0, self.a_bias, s.decay_rate,
                                u, au, w, H, D, stream=batch.stream)
-        read = rt.empty(T, hd, dtype=f32)
-        ops.general_delta_scan(r, k, v, u, au, w, cache.states["matrix"], read, batch.token_seq, batch.seq_slot,
-                               batch.n_seqs, H, D, stream=batch.stream)
+        read, state = rt.empty(T, hd, dtype=f32), cache.states["matrix"]
+        # (decays below e^-1 a token: over a chunk their products would leave 32-bit numbers' range)
+        tiles = _chunk_tiles(batch, H, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v), D, D, state) else None
+        if tiles is not None:
+            ops.chunk_scan_general(r, k, v, u, au, w, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D,
+                                   scratch=self._scratch, stream=batch.stream)
+        else:
+            ops.general_delta_scan(r, k, v, u, au, w, state, read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D,
+                                   stream=batch.stream)
         y = rt.empty(T, hd)
         ops.gated_group_norm(read, gate, self.norm_w, s.norm_eps, "sigmoid", y, H, D, stream=batch.stream)
         ops.linear(y, self.w_o, out, accumulate=accumulate, status=batch.status, stream=batch.stream)
@@ -308,9 +343,19 @@ class Mlstm(_StateMixer):
         gate = proj[:, 2 * self.qk + self.vv:2 * self.qk + 2 * self.vv]
         gates = proj[:, 2 * self.qk + 2 * self.vv:]       # [i | f] as projected
         read = rt.empty(T, self.vv, dtype=f32)
-        ops.mlstm_scan(q, k, v, gates, self.i_bias, self.f_bias, s.gate_cap, float(D) ** -0.5, cache.states["matrix"],
-                       cache.states["normalizer"], cache.states["log_max"], read, batch.token_seq, batch.seq_slot,
-                       batch.n_seqs, H, D, V, stream=batch.stream)
+        matrix, norm, log_max = (cache.states[n] for n in ("matrix", "normalizer", "log_max"))
+        tiles = _chunk_tiles(batch, H, V) if ops.chunk_scan_ok((q, k, v), D, V, matrix) else None
+        if tiles is not None:
+            keep, take, floor = rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32)
+            before = rt.empty(batch.n_seqs, H, D, dtype=f32)
+            ops.mlstm_gates(gates, self.i_bias, self.f_bias, s.gate_cap, log_max, norm, before, keep, take, floor,
+                            batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, stream=batch.stream)
+            ops.chunk_scan(q, k, v, keep, matrix, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, H, D, V,
+                           take=take, q_scale=float(D) ** -0.5, scratch=self._scratch, normalizer=(before, norm, floor),
+                           stream=batch.stream)
+        else:
+            ops.mlstm_scan(q, k, v, gates, self.i_bias, self.f_bias, s.gate_cap, float(D) ** -0.5, matrix, norm, log_max,
+                           read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, V, stream=batch.stream)
         y = rt.empty(T, self.vv)
         ops.gated_group_norm(read, gate, self.norm_w, s.norm_eps, "sigmoid", y, H, V, stream=batch.stream)
         ops.linear(y, self.w_o, out, accumulate=accumulate, status=batch.status, stream=batch.stream)

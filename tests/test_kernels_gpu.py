@@ -1219,3 +1219,138 @@ def test_route_fused_is_product_routing_and_gather(T, E, K, H, extra):
                 assert torch.equal(xp, x[src.long()])
     # what it does not take is said beforehand
     assert not o.route_fused_ok(rnd(9, H, dtype=torch.bfloat16), w, E) and not o.route_fused_ok(x.float(), w, E)
+
+
+# ------------------------------------------------------------------ recurrences in chunks
+def scan_setup(lens, seed):
+    """(token_seq, seq_slot, tiles of 32 tokens) of entries of these lengths."""
+    seq, tiles, flat = [], [], 0
+    for b, n in enumerate(lens):
+        seq += [b] * n
+        tiles += [(flat + i, min(32, n - i), b, i) for i in range(0, n, 32)]
+        flat += n
+    as_int = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    return as_int(seq), as_int([(b + 2) % (len(lens) + 2) for b in range(len(lens))]), as_int(tiles)
+
+
+def scan_scratch(*shape):
+    return torch.full(shape, float("nan"), device=DEV)
+
+
+# (entries' lengths, heads, key heads, D, V)
+SCANS = [([1], 2, 1, 64, 16), ([31, 32, 33], 4, 2, 128, 128), ([100], 3, 3, 20, 36), ([65, 1, 64], 2, 2, 68, 4),
+         ([200, 7], 2, 1, 128, 100)]
+
+
+@pytest.mark.parametrize("case", SCANS)
+@pytest.mark.parametrize("kind", ["delta", "mlstm"])
+def test_chunk_scan(case, kind):
+    """The chunked recurrences against the loop over the tokens in 64 bits: decays from nothing to one, states that
+    are not empty, slots unlike entries; no further from it than the kernels that take the tokens one by one; and what is
+    no number in a token reaches no token before it and no other request."""
+    o = ops()
+    lens, H, G, D, V = case
+    G = H if kind == "mlstm" else G
+    T, (seq, slot, tiles) = sum(lens), scan_setup(lens, 0)
+    wide = rnd(T, 2 * G * D + H * V + 4)
+    q, k, v = wide[:, :G * D], wide[:, G * D:2 * G * D], wide[:, 2 * G * D:2 * G * D + H * V]
+    n_slots = len(lens) + 2
+    state = rnd(n_slots, H, V, D, seed=3)
+    gen = torch.Generator().manual_seed(T)
+    g = torch.sigmoid(torch.randn(T, H, generator=gen) * 3 + 2)
+    g[T // 2] = 0.0
+    g[T // 3] = 1.0
+    beta = torch.rand(T, H, generator=gen)
+    g, beta = g.to(DEV), beta.to(DEV)
+    if kind == "delta":
+        k.div_(k.reshape(T, G, D).norm(dim=-1, keepdim=True).expand(T, G, D).reshape(T, G * D))
+    gates, ib, fb, cap = rnd(T, 2 * H, seed=9) * 4, rnd(H, seed=1), rnd(H, seed=2) + 2, 15.0
+    copies = o.mlstm_column_blocks(D, V)
+    norm0 = rnd(n_slots, H, 1, D, seed=4).expand(n_slots, H, copies, D).contiguous()
+    max0 = rnd(n_slots, H, 1, seed=5).expand(n_slots, H, copies).contiguous()
+
+    def run(chunked, q=q, k=k, v=v):
+        st, out, nm, mx = state.clone(), torch.empty(T, H * V, device=DEV), norm0.clone(), max0.clone()
+        args = (seq, slot, len(lens))
+        if kind == "mlstm" and chunked:
+            keep, take, floor = (torch.empty(T, H, device=DEV) for _ in range(3))
+            before = torch.empty(len(lens), H, D, device=DEV)
+            o.mlstm_gates(gates, ib, fb, cap, mx, nm, before, keep, take, floor, *args, H, D)
+            o.chunk_scan(q, k, v, keep, st, out, tiles, *args, H, G, D, V, take=take, q_scale=D ** -0.5, scratch=scan_scratch,
+                         normalizer=(before, nm, floor))
+        elif kind == "mlstm":
+            o.mlstm_scan(q, k, v, gates, ib, fb, cap, D ** -0.5, st, nm, mx, out, *args, H, D, V)
+        elif chunked:
+            o.chunk_scan(q, k, v, g, st, out, tiles, *args, H, G, D, V, beta=beta, scratch=scan_scratch)
+        else:
+            o.state_scan(q, k, v, g, H, beta, st, out, *args, H, G, D, V)
+        return out, st, nm, mx
+
+    got, old = run(True), run(False)
+    d = lambda t: t.double().cpu()
+    Q, K = (d(x).view(T, G, D).repeat_interleave(H // G, 1) for x in (q, k))
+    Vv, gg, bb = d(v).view(T, H, V), d(g), d(beta)
+    want, S_want, n_want = torch.zeros(T, H, V, dtype=torch.float64), d(state), d(norm0)
+    for b in range(len(lens)):
+        s = int(slot[b])
+        S, n, m = S_want[s].transpose(1, 2).clone(), d(norm0)[s, :, 0].clone(), d(max0)[s, :, 0].clone()
+        for t in [i for i in range(T) if int(seq[i]) == b]:
+            if kind == "delta":
+                S = S * gg[t][:, None, None]
+                u = bb[t][:, None] * (Vv[t] - torch.einsum("hdv,hd->hv", S, K[t]))
+                S = S + K[t][:, :, None] * u[:, None]
+                want[t] = torch.einsum("hdv,hd->hv", S, Q[t])
+            elif kind == "mlstm":
+                gi = cap * torch.tanh((d(gates)[t, :H] + d(ib)) / cap)
+                gf = torch.nn.functional.logsigmoid(cap * torch.tanh((d(gates)[t, H:] + d(fb)) / cap))
+                mn = torch.maximum(gf + m, gi)
+                keep, take = torch.exp(gf + m - mn), torch.exp(gi - mn)
+                S = keep[:, None, None] * S + take[:, None, None] * K[t][:, :, None] * Vv[t][:, None]
+                n, m = keep[:, None] * n + take[:, None] * K[t], mn
+                qs = Q[t] * D ** -0.5
+                want[t] = torch.einsum("hdv,hd->hv", S, qs) / (torch.maximum((n * qs).sum(-1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+        S_want[s] = S.transpose(1, 2)
+        n_want[s] = n[:, None]
+    want = want.reshape(T, H * V)
+    far = lambda a, b: float((d(a) - b).norm() / b.norm())
+    assert far(got[0], want) < max(2e-6, 1.5 * far(old[0], want)) and far(got[1], S_want) < max(1e-6, 1.5 * far(old[1], S_want))
+    if kind == "mlstm":
+        assert far(got[2], n_want) < 2e-6 and float((got[3] - old[3]).abs().max()) < 1e-5
+    t = T // 2
+    bad = wide.clone()
+    bad[t] = float("nan")
+    out = run(True, bad[:, :G * D], bad[:, G * D:2 * G * D], bad[:, 2 * G * D:2 * G * D + H * V])[0]
+    keep = [i for i in range(T) if i < t or int(seq[i]) != int(seq[t])]
+    assert torch.equal(out[keep], got[0][keep]) and bool(out[t].isnan().any())
+
+
+@pytest.mark.parametrize("lens,H,D", [([1], 2, 64), ([31, 32, 33], 3, 64), ([100, 5], 2, 20), ([65], 2, 128), ([130, 1, 64], 1, 100)])
+def test_chunk_scan_general(lens, H, D):
+    """The generalized delta rule in chunks against the loop in 64 bits, with decays over their whole range."""
+    o = ops()
+    T, (seq, slot, tiles) = sum(lens), scan_setup(lens, 0)
+    wide = rnd(T, 3 * H * D + 8)
+    r, k, v = (wide[:, i * H * D:(i + 1) * H * D] for i in range(3))
+    gen = torch.Generator().manual_seed(T)
+    w = torch.exp(-0.6065 * torch.sigmoid(torch.randn(T, H * D, generator=gen) * 4)).to(DEV)
+    w[:, ::7], w[:, 1::7] = 0.5453, 1.0        # channels that forget as fast as they can, and that never do
+    u = k / torch.sqrt((k.reshape(T, H, D) ** 2).sum(-1, keepdim=True) + 1e-6).expand(T, H, D).reshape(T, H * D)
+    au = u * torch.rand(T, H * D, generator=gen).to(DEV)
+    state = rnd(len(lens) + 2, H, D, D, seed=3)
+    st, st_old = state.clone(), state.clone()
+    out, old = torch.empty(T, H * D, device=DEV), torch.empty(T, H * D, device=DEV)
+    o.general_delta_scan(r, k, v, u, au, w, st_old, old, seq, slot, len(lens), H, D)
+    o.chunk_scan_general(r, k, v, u.clone(), au.clone(), w.clone(), st, out, tiles, seq, slot, len(lens), H, D, scratch=scan_scratch)
+    d = lambda t: t.double().cpu()
+    R, K, Vv, U, A, W = (d(x).reshape(T, H, D) for x in (r, k, v, u, au, w))
+    want, S_want = torch.zeros(T, H, D, dtype=torch.float64), d(state)
+    for b in range(len(lens)):
+        S = S_want[int(slot[b])].transpose(1, 2).clone()
+        for t in [i for i in range(T) if int(seq[i]) == b]:
+            y = torch.einsum("hi,hij->hj", U[t], S)
+            S = W[t][:, :, None] * S - A[t][:, :, None] * y[:, None] + K[t][:, :, None] * Vv[t][:, None]
+            want[t] = torch.einsum("hij,hi->hj", S, R[t])
+        S_want[int(slot[b])] = S.transpose(1, 2)
+    far = lambda a, b: float((d(a) - b).norm() / b.norm())
+    want = want.reshape(T, H * D)
+    assert far(out, want) < max(2e-6, 1.5 * far(old, want)) and far(st, S_want) < max(1e-6, 1.5 * far(st_old, S_want))
