@@ -41,6 +41,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels.ops import upload
 from .specs import CacheSpec
 
 
@@ -307,12 +308,12 @@ class CacheManager:
             if n == 0:
                 continue
             rows = [self._dirty[i] for i in range(n)]
+            # (ordered on the stream, without waiting for it: steps that read the old rows are ahead of the copies)
+            new = upload(g.table[rows], self.device)
             if n == 1:
-                r = rows[0]
-                g.table_dev[r].copy_(torch.from_numpy(g.table[r].copy()), non_blocking=False)
+                g.table_dev[rows[0]].copy_(new[0])
             else:
-                idx = torch.tensor(rows, dtype=torch.long)
-                g.table_dev[idx.to(self.device)] = torch.from_numpy(g.table[rows]).to(self.device)
+                g.table_dev[upload(np.asarray(rows, dtype=np.int64), self.device)] = new
 
     def layer_cache(self, cache_index: int, writes: bool = True) -> LayerCache:
         g = self._group_of[cache_index]

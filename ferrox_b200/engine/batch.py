@@ -20,6 +20,8 @@ from typing import List, Sequence
 import numpy as np
 import torch
 
+from ..kernels import ops
+
 
 @dataclass
 class StepEntry:
@@ -73,7 +75,7 @@ def flatten(entries: Sequence[StepEntry], device, status: torch.Tensor, stream: 
         t += n
         max_len = max(max_len, e.start + n)
         max_new = max(max_new, n)
-    dev = torch.from_numpy(buf).to(device, non_blocking=False)
+    dev = ops.upload(buf, device)
     return StepBatch(
         n_tokens=T, n_seqs=B, n_want=W,
         token_ids=dev[:T], positions=dev[T:2 * T], token_seq=dev[2 * T:3 * T],

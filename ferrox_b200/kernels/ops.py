@@ -289,6 +289,17 @@ def _rows(t: torch.Tensor) -> int:
     return t.stride(0)
 
 
+def upload(values, device) -> torch.Tensor:
+    """A numpy array's copy on ``device``, ordered on the current stream without waiting for it: by way of pinned memory,
+    which torch's allocator hands out again only when the copy is done.  (A pageable copy waits for everything the
+    stream holds: the host then prepares a step while the device stands still, 0.3 ms of every prompt.)"""
+    t = torch.from_numpy(values)
+    device = torch.device(device)
+    if device.type != "cuda" or t.numel() == 0:
+        return t.to(device)
+    return t.pin_memory().to(device, non_blocking=True)
+
+
 # ---------------------------------------------------------------------------
 def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=None, stream=None):
     """out[M,N] (+)= a[M,K] . w[N,K]^T (+ bias).  With ``group_offsets`` ([G+1],

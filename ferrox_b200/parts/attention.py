@@ -48,7 +48,7 @@ def query_tiles(batch, rows: int) -> torch.Tensor:
             for i in range(0, n, rows):
                 out.append((flat + i, min(rows, n - i), b, e.start + i))
             flat += n
-        t = torch.from_numpy(np.asarray(out, dtype=np.int32).reshape(-1, 4)).to(batch.token_ids.device)
+        t = ops.upload(np.asarray(out, dtype=np.int32).reshape(-1, 4), batch.token_ids.device)
         batch.shared[key] = t
     return t
 
@@ -61,7 +61,7 @@ def prefill_tc_plan(batch, window, n_heads: int, chunk=None):
     if plan is None:
         items, merges, parts = ops.prefill_tc_plan([(len(e.tokens), e.start) for e in batch.entries], window, n_heads,
                                                    chunk=chunk)
-        both = torch.from_numpy(np.concatenate([items.reshape(-1), merges.reshape(-1)])).to(batch.token_ids.device)
+        both = ops.upload(np.concatenate([items.reshape(-1), merges.reshape(-1)]), batch.token_ids.device)
         plan = (both[:items.size].view(-1, 8), both[items.size:].view(-1, 4) if merges.size else None, parts)
         batch.shared[key] = plan
     return plan
@@ -464,8 +464,8 @@ def general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldoh, 
             key = ("general attention items", n_heads, n_kv_heads)
             items = batch.shared.get(key)
             if items is None:
-                items = torch.from_numpy(ops.general_attention_items([len(e.tokens) for e in batch.entries], n_heads,
-                                                                     n_kv_heads)).to(batch.token_ids.device)
+                items = ops.upload(ops.general_attention_items([len(e.tokens) for e in batch.entries], n_heads, n_kv_heads),
+                                   batch.token_ids.device)
                 batch.shared[key] = items
         return ops.general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, cache.block_table, cache.page_size,
                                      batch.positions, batch.token_seq, batch.seq_slot, items, out, ldo, ldoh, n_heads,

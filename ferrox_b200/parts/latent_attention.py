@@ -198,7 +198,7 @@ class LatentAttention(Mixer):
             items = ops.general_attention_items([len(e.tokens) for e in batch.entries], self.spec.n_heads, self.spec.n_heads)
             flat = np.concatenate([np.concatenate(src).astype(np.int32), table.reshape(-1),
                                    np.arange(len(spans), dtype=np.int32), items.reshape(-1)])
-            dev = torch.from_numpy(flat).to(self.rt.device)
+            dev = ops.upload(flat, self.rt.device)
             a, b2, c = n, n + table.size, n + table.size + len(spans)
             plan = (dev[:a], dev[a:b2].view(len(spans), width), dev[b2:c], dev[c:].view(-1, 5), n)
             batch.shared[key] = plan
