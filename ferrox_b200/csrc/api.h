@@ -23,9 +23,11 @@ int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const floa
                   const float* take, float q_scale, float* p, float* gam, float* e, float* wr, const float* norm_in, float* norm,
                   int copies, const float* floor_m, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,
                   const int* seq_slot, int n_tokens, int n_entries, int H, int G, int D, int V, void* stream);
-int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, float* u, float* au,
-                          float* w, float* p, float* gam, float* wr, float* state, float* out, const int* tiles, int n_tiles,
-                          const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream);
+int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, const float* a_pre, long lda,
+                          const float* low, long ldl, const void* w2, int w2_dtype, const void* w0, int w0_dtype,
+                          const void* a_bias, int ab_dtype, float rate, int rank, float* p, float* gam, float* wr, float* qs,
+                          float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,
+                          const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream);
 int fx_mlstm_gates(const float* gates, long ldg, const void* i_bias, const void* f_bias, int bias_dtype, float cap, float* m,
                    int copies, const float* norm, float* norm_in, int D, float* keep, float* take, float* floor_m,
                    const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, void* stream);
@@ -279,6 +281,12 @@ int fx_state_scan(const void* q, long ldq, const void* k, long ldk, const void* 
                   const float* g, long g_ld, const float* beta, float* state, float* out, long ldo, const int* token_seq,
                   const int* seq_slot, int n_tokens, int n_entries, int H, int G, int D, int V, void* stream);
 int fx_set_scan_lanes(int lanes);   // lanes that share a state column, fixed for measurements (0: the launcher's choice)
+int fx_delta_prep_runs(const float* proj, long ldp, const float* conv_w, const float* tail, const float* ba, long ldba,
+                       const float* a_log, const float* dt_bias, const int* token_seq, const int* seq_slot, float* out,
+                       float* beta, float* g, int n_tokens, int G, int D, int H, int V, void* stream);
+int fx_delta_prep_runs(const float* proj, long ldp, const float* conv_w, const float* tail, const float* ba, long ldba,
+                       const float* a_log, const float* dt_bias, const int* token_seq, const int* seq_slot, float* out,
+                       float* beta, float* g, int n_tokens, int G, int D, int H, int V, void* stream);
 int fx_gated_group_norm(const float* x, const void* gate, int gate_dtype, long ldg, const void* w, int w_dtype, float eps,
                         int act, void* out, int out_dtype, int n_tokens, int groups, int width, long w_stride,
                         void* stream);

@@ -85,7 +85,9 @@ __device__ __forceinline__ void load_rows(float* to, int pitch, const float* fro
 struct ChunkArgs {
     const int* tiles;                // [n][4]: first token, tokens, entry, position
     const float *q, *k, *v; long ldq, ldk, ldv;
-    float *u, *au, *w;               // general: contiguous [T, H * D]; r', G_C k' and -G_C a' take their places
+    const float *a_pre, *low; long lda, ldl; int rank;     // general: rows [T, H * D] and [T, rank], W2 [H * D, rank] and so on
+    const void *w2, *w0, *ab; int w2_dtype, w0_dtype, ab_dtype; float rate;
+    float *qs, *ks, *as;             // general: r', G_C k' and -G_C a'  [T, H * D]
     const float* g;                  // decays [T, H]
     const float* gate;               // delta: beta [T, H]; mLSTM: take [T, H]
     float scale;                     // on q (mLSTM)
@@ -223,10 +225,18 @@ __global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
     }
 }
 
+constexpr int RANK = 64;             // low-rank columns a pass
+
+__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
+
+// The decays and rates come from the projections' rows here as well (general_delta.cu states them: w = exp(-rate sigmoid(W2
+// tanh(low) + w0)), a = sigmoid(a_pre + bias), u = k / sqrt(sum k^2 + 1e-6)): a block has a head's slice of W2 in shared
+// memory for 32 tokens, and u, a u and w never go to memory.  (The kernel that makes them for the token-by-token form,
+// eight tokens a block, took 249 us for 3,001 tokens of 32 heads of 64.)
 template <int D>
 __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
 {
-    constexpr int PITCH = D + 4, LP = CHUNK + 4;
+    constexpr int PITCH = D + 4, LP = CHUNK + 4, RP = RANK + 4;
     extern __shared__ __align__(16) float sm[];
     float* u_s = sm;                                  // [CHUNK][PITCH] each
     float* r_s = u_s + CHUNK * PITCH;
@@ -235,15 +245,16 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
     float* g_s = a_s + CHUNK * PITCH;                 // decays, then their products up to each token
     float* A_s = g_s + CHUNK * PITCH;                 // [CHUNK][LP]
     float* B_s = A_s + CHUNK * LP;
+    float* w2_s = B_s + CHUNK * LP;                   // [D][RP]
+    float* th_s = w2_s + D * RP;                      // [CHUNK][RP]
+    __shared__ float len_s[CHUNK];
     fx_pdl_wait();
     const int4 tile = reinterpret_cast<const int4*>(a.tiles)[blockIdx.x];
     const int tok0 = tile.x, rows = tile.y, h = blockIdx.y, tid = threadIdx.x;
     const long hd = (long)a.H * a.D, at0 = (long)tok0 * hd + (long)h * a.D;
-    load_rows<D, PREP_THREADS>(u_s, PITCH, a.u + at0, hd, rows, a.D);
-    load_rows<D, PREP_THREADS>(a_s, PITCH, a.au + at0, hd, rows, a.D);
-    load_rows<D, PREP_THREADS>(g_s, PITCH, a.w + at0, hd, rows, a.D);
-    load_rows<D, PREP_THREADS>(r_s, PITCH, a.q + (long)tok0 * a.ldq + (long)h * a.D, a.ldq, rows, a.D);
     load_rows<D, PREP_THREADS>(k_s, PITCH, a.k + (long)tok0 * a.ldk + (long)h * a.D, a.ldk, rows, a.D);
+    load_rows<D, PREP_THREADS>(a_s, PITCH, a.a_pre + (long)tok0 * a.lda + (long)h * a.D, a.lda, rows, a.D);
+    load_rows<D, PREP_THREADS>(r_s, PITCH, a.q + (long)tok0 * a.ldq + (long)h * a.D, a.ldq, rows, a.D);
     asm volatile("cp.async.commit_group;" ::: "memory");
     // (the values of the first column of the substitution below travel meanwhile)
     float v[CHUNK];
@@ -252,7 +263,61 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
 #pragma unroll
         for (int t = 0; t < CHUNK; ++t) v[t] = t < rows ? vp[(long)t * a.ldv] : 0.f;
     }
+    // tanh(low) W2^T: thread (zy, zx) tokens zy, zy + 16, channels zx + 16 j
+    const int zy = tid >> 4, zx = tid & 15;
+    u64 zacc[2][D / 16];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j) zacc[i][j] = 0ull;
+    for (int rc = 0; rc < a.rank; rc += RANK) {
+        const int nr = min(RANK, a.rank - rc);
+        __syncthreads();
+        for (int i = tid; i < D * RANK; i += PREP_THREADS) {
+            const int d = i / RANK, r = i - d * RANK;
+            w2_s[d * RP + r] = r < nr && d < a.D ? load_any(a.w2, a.w2_dtype, ((long)h * a.D + d) * a.rank + rc + r) : 0.f;
+        }
+        for (int i = tid; i < CHUNK * RANK; i += PREP_THREADS) {
+            const int t = i / RANK, r = i - t * RANK;
+            th_s[t * RP + r] = r < nr && t < rows ? tanhf(a.low[(long)(tok0 + t) * a.ldl + rc + r]) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int r = 0; r < RANK; r += 4) {
+            ulonglong2 th[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) th[i] = *reinterpret_cast<const ulonglong2*>(th_s + (zy + 16 * i) * RP + r);
+#pragma unroll
+            for (int j = 0; j < D / 16; ++j) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(w2_s + (zx + 16 * j) * RP + r);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) { fma2(zacc[i][j], th[i].x, w.x); fma2(zacc[i][j], th[i].y, w.y); }
+            }
+        }
+    }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    {
+        const int t = tid >> 3;                       // a token's key length, eight threads a token
+        float ss = 0.f;
+        for (int d = tid & 7; d < D; d += 8) ss = fmaf(k_s[t * PITCH + d], k_s[t * PITCH + d], ss);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+        if ((tid & 7) == 0) len_s[t] = sqrtf(ss + 1e-6f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j) {
+            const int t = zy + 16 * i, d = zx + 16 * j, c = h * a.D + d;
+            if (d >= a.D) { u_s[t * PITCH + d] = 0.f; g_s[t * PITCH + d] = 1.f; continue; }
+            const float u = k_s[t * PITCH + d] / len_s[t];
+            u_s[t * PITCH + d] = u;
+            a_s[t * PITCH + d] = sigmoid_f(a_s[t * PITCH + d] + load_any(a.ab, a.ab_dtype, c)) * u;
+            g_s[t * PITCH + d] = expf(-a.rate * sigmoid_f(sum_of(zacc[i][j]) + load_any(a.w0, a.w0_dtype, c)));
+        }
     __syncthreads();
     // a channel's products: runs of RUN tokens a thread, then the runs before it
     constexpr int RUNS = PREP_THREADS / D, RUN = CHUNK / RUNS;
@@ -283,7 +348,7 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
         k_s[at] = kk; a_s[at] = aa; r_s[at] = rr;
         if (t < rows && d < a.D) {
             const long to = at0 + (long)t * hd + d;
-            a.u[to] = rr; a.au[to] = kk * last; a.w[to] = -aa * last;      // (the block has read these rows)
+            a.qs[to] = rr; a.ks[to] = kk * last; a.as[to] = -aa * last;
         }
     }
     __syncthreads();
@@ -386,11 +451,13 @@ __global__ void __launch_bounds__(32) mlstm_gates_kernel(const float* __restrict
     for (int d = lane; d < D; d += 32) norm_in[((long)b * H + h) * D + d] = norm[((long)seq_slot[b] * H + h) * copies * D + d];
     const float bi = load_any(i_bias, bias_dtype, h), bf = load_any(f_bias, bias_dtype, h), inv_cap = 1.0f / cap;
     float m = mp[0];
+    float in_i = gates[(long)min(r0 + lane, r1 - 1) * ldg + h], in_f = gates[(long)min(r0 + lane, r1 - 1) * ldg + H + h];
     for (int c0 = r0; c0 < r1; c0 += 32) {
         const int t = c0 + lane;
-        const float* g = gates + (long)min(t, r1 - 1) * ldg;
-        const float gi = cap * tanhf((g[h] + bi) * inv_cap);
-        const float gf = logsigmoid_f(cap * tanhf((g[H + h] + bf) * inv_cap));
+        const float gi = cap * tanhf((in_i + bi) * inv_cap);
+        const float gf = logsigmoid_f(cap * tanhf((in_f + bf) * inv_cap));
+        const float* g = gates + (long)min(t + 32, r1 - 1) * ldg;      // (the next tokens' inputs travel meanwhile)
+        in_i = g[h]; in_f = g[H + h];
         float f = gf, i = gi;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -805,27 +872,33 @@ extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk,
     return D <= 64 ? go_walk<64, MLSTM>(a, n_entries, s) : go_walk<128, MLSTM>(a, n_entries, s);
 }
 
-// The generalized delta rule.  r, k, v rows [T, H * D]; u, au, w contiguous [T, H * D], overwritten; scratch: p [T, H, 2 CHUNK],
-// gam [tiles, H, D], wr [T, H, D].  out contiguous [T, H * D]: it holds Y0 until a chunk's read-outs take its place.
-extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, float* u, float* au,
-                                     float* w, float* p, float* gam, float* wr, float* state, float* out, const int* tiles, int n_tiles,
+// The generalized delta rule from its projections: r, k, v, a_pre rows [T, H * D], low rows [T, rank], w2 [H * D, rank], w0 and
+// a_bias [H * D], all rows 32-bit.  Scratch: p [T, H, 2 CHUNK], gam [tiles, H, D], wr, qs, ks and as [T, H, D].  out contiguous
+// [T, H * D]: it holds Y0 until a chunk's read-outs take its place.
+extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, const float* a_pre,
+                                     long lda, const float* low, long ldl, const void* w2, int w2_dtype, const void* w0, int w0_dtype,
+                                     const void* a_bias, int ab_dtype, float rate, int rank, float* p, float* gam, float* wr, float* qs,
+                                     float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles,
                                      const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream)
 {
     if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
     int st = check(H, H, D, D, n_entries);
     if (st != FX_OK) return st;
-    if (off_grid(r, ldr) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(u, 0) || off_grid(au, 0) || off_grid(w, 0) ||
-        off_grid(p, 0) || off_grid(gam, 0) || off_grid(wr, 0) || off_grid(out, 0) || off_grid(state, 0) || off_grid(tiles, 0))
+    if (rank <= 0 || !(rate >= 0.f && rate <= 1.f)) return FX_ERR_SIZE;      // (decays below 1/e: see above)
+    if (off_grid(r, ldr) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(a_pre, lda) || off_grid(p, 0) || off_grid(gam, 0) ||
+        off_grid(wr, 0) || off_grid(qs, 0) || off_grid(ks, 0) || off_grid(as, 0) || off_grid(out, 0) || off_grid(state, 0) ||
+        off_grid(tiles, 0))
         return FX_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     ChunkArgs c = {};
-    c.tiles = tiles; c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.u = u; c.au = au; c.w = w;
-    c.H = H; c.G = H; c.D = D; c.V = D; c.p = p; c.gam = gam; c.x0 = out; c.wr = wr;
-    const size_t small = sizeof(float) * (5 * CHUNK * (64 + 4) + 2 * CHUNK * (CHUNK + 4)), large = small + sizeof(float) * 5 * CHUNK * 64;
-    st = D <= 64 ? go_chunks(general_chunks<64>, c, n_tiles, small, s) : go_chunks(general_chunks<128>, c, n_tiles, large, s);
+    c.tiles = tiles; c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.a_pre = a_pre; c.lda = lda; c.low = low; c.ldl = ldl;
+    c.rank = rank; c.w2 = w2; c.w0 = w0; c.ab = a_bias; c.w2_dtype = w2_dtype; c.w0_dtype = w0_dtype; c.ab_dtype = ab_dtype; c.rate = rate;
+    c.H = H; c.G = H; c.D = D; c.V = D; c.p = p; c.gam = gam; c.x0 = out; c.wr = wr; c.qs = qs; c.ks = ks; c.as = as;
+    auto smem = [](int d) { return sizeof(float) * (5 * CHUNK * (d + 4) + 2 * CHUNK * (CHUNK + 4) + (d + CHUNK) * (RANK + 4)); };
+    st = D <= 64 ? go_chunks(general_chunks<64>, c, n_tiles, smem(64), s) : go_chunks(general_chunks<128>, c, n_tiles, smem(128), s);
     if (st != FX_OK) return st;
     WalkArgs a = {};
-    a.w = wr; a.q = u; a.ldq = (long)H * D; a.q_share = 1; a.k = au; a.ldk = (long)H * D; a.a = w; a.v = v; a.ldv = ldv; a.x0 = out;
+    a.w = wr; a.q = qs; a.ldq = (long)H * D; a.q_share = 1; a.k = ks; a.ldk = (long)H * D; a.a = as; a.v = v; a.ldv = ldv; a.x0 = out;
     a.p = p; a.gam = gam; a.q_scale = 1.f; a.state = state; a.out = out; a.ldo = (long)H * D; a.token_seq = token_seq; a.seq_slot = seq_slot;
     a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles;
     return D <= 64 ? go_walk<64, GENERAL>(a, n_entries, s) : go_walk<128, GENERAL>(a, n_entries, s);

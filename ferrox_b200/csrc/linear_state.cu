@@ -109,6 +109,97 @@ __global__ void __launch_bounds__(PREP_THREADS) delta_prep_kernel(
     }
 }
 
+// The same for prompts, four taps and heads of 64 or 128: a warp takes a run of RUN tokens of 128 channels, four a lane,
+// so that an input is read once (and three before the run) instead of once a tap, and a head's length is a sum over lanes.
+// Bound by memory: 2,048 tokens of 4,096 channels, 33 MB in and 33 MB out, 138 us with a block a token and head.  The
+// convolution's sums run in the same order.  The last row of blocks makes the gates.
+constexpr int RUN = 16, RUN_TAPS = 4, RUN_WARPS = 8;
+
+__global__ void __launch_bounds__(RUN_WARPS * 32) delta_prep_runs_kernel(
+    const float* __restrict__ proj, long ldp, const float* __restrict__ conv_w, const float* __restrict__ tail,
+    const float* __restrict__ ba, long ldba, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+    const int* __restrict__ token_seq, const int* __restrict__ seq_slot, float* __restrict__ out, float* __restrict__ beta,
+    float* __restrict__ g, int n_tokens, int G, int D, int H, int C)
+{
+    fx_pdl_wait();
+    if (blockIdx.y == gridDim.y - 1) {
+        const long base = (long)blockIdx.x * RUN * RUN_WARPS * H, end = min(base + (long)RUN * RUN_WARPS * H, (long)n_tokens * H);
+        for (long i = base + threadIdx.x; i < end; i += RUN_WARPS * 32) {
+            const int hd = (int)(i % H);
+            const float* r = ba + i / H * ldba;
+            beta[i] = sigmoid_f(r[hd]);
+            const double sp = log1p(exp((double)(r[H + hd] + dt_bias[hd])));      // (in 64 bits, as above)
+            g[i] = (float)exp(-exp((double)a_log[hd]) * sp);
+        }
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = (blockIdx.x * RUN_WARPS + warp) * RUN, c = blockIdx.y * 128 + lane * 4;
+    if (t0 >= n_tokens) return;
+    const bool live = c < C, normed = blockIdx.y * 128 < 2 * G * D;      // (2 G D is a multiple of 128)
+    const int cc = live ? c : 0, nt = min(RUN, n_tokens - t0);
+    float w[RUN_TAPS][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(conv_w + (long)(cc + i) * RUN_TAPS);
+        w[0][i] = x.x; w[1][i] = x.y; w[2][i] = x.z; w[3][i] = x.w;
+    }
+    float4 win[RUN_TAPS - 1];                                            // the inputs before the token, oldest first
+    int b = token_seq[t0], own = 0;
+    while (own < RUN_TAPS - 1 && t0 - own - 1 >= 0 && token_seq[t0 - own - 1] == b) ++own;
+    auto from_tail = [&](int entry, int j) {
+        return *reinterpret_cast<const float4*>(tail + ((long)seq_slot[entry] * (RUN_TAPS - 1) + j) * C + cc);
+    };
+#pragma unroll
+    for (int j = 0; j < RUN_TAPS - 1; ++j) {
+        const int back = RUN_TAPS - 1 - j;
+        win[j] = back <= own ? *reinterpret_cast<const float4*>(proj + (long)(t0 - back) * ldp + cc) : from_tail(b, RUN_TAPS - 1 - (back - own));
+    }
+#pragma unroll 1
+    for (int i0 = 0; i0 < nt; i0 += 8) {
+        float4 xs[8];
+        int bs[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = min(t0 + i0 + i, n_tokens - 1);
+            xs[i] = *reinterpret_cast<const float4*>(proj + (long)t * ldp + cc);
+            bs[i] = token_seq[t];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = t0 + i0 + i;
+            if (i0 + i >= nt) break;
+            if (bs[i] != b) {                                            // the next request begins
+                b = bs[i];
+#pragma unroll
+                for (int j = 0; j < RUN_TAPS - 1; ++j) win[j] = from_tail(b, j);
+            }
+            const float x[4] = {xs[i].x, xs[i].y, xs[i].z, xs[i].w};
+            const float p0[4] = {win[0].x, win[0].y, win[0].z, win[0].w}, p1[4] = {win[1].x, win[1].y, win[1].z, win[1].w};
+            const float p2[4] = {win[2].x, win[2].y, win[2].z, win[2].w};
+            float y[4], ss = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float acc = fmaf(w[0][k], p0[k], 0.f);
+                acc = fmaf(w[1][k], p1[k], acc); acc = fmaf(w[2][k], p2[k], acc); acc = fmaf(w[3][k], x[k], acc);
+                y[k] = silu_f(acc);
+                ss = fmaf(y[k], y[k], ss);
+            }
+            if (normed) {                                                // (uniform across the block)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (o < D / 4) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                float inv = 1.0f / sqrtf(ss + 1e-6f);
+                inv *= c < G * D ? 1.0f / sqrtf((float)D) : 1.0f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y[k] *= inv;
+            }
+            if (live) *reinterpret_cast<float4*>(out + (long)t * C + c) = make_float4(y[0], y[1], y[2], y[3]);
+            win[0] = win[1]; win[1] = win[2]; win[2] = xs[i];
+        }
+    }
+}
+
 // The convolution's tail after the step: the last taps - 1 inputs of every entry, from its rows of this step and,
 // where the entry brought fewer, from the old tail.  Grid (entries, channels); a thread reads all it needs of a channel
 // before it writes.
@@ -484,6 +575,22 @@ extern "C" int fx_delta_prep(const void* proj, int dtype, long ldp, const void* 
         fx_launch_pdl(delta_prep_kernel<bf16>, grid, PREP_THREADS, smem, s, (const bf16*)proj, ldp, conv_w, cw_dtype, taps,
                       tail, ba, ldba, a_log, dt_bias, token_seq, seq_slot, out, beta, g, G, D, H, V, tail_new);
     else return FX_ERR_DTYPE;
+    return fx_launch_status();
+}
+
+// Refuses (FX_ERR_SIZE / FX_ERR_ALIGN) other than four taps' weights in 32 bits, heads of 64 or 128 whose q and k rows are
+// multiples of 128 channels, value rows in steps of 4, rows off the 16-byte grid.
+extern "C" int fx_delta_prep_runs(const float* proj, long ldp, const float* conv_w, const float* tail, const float* ba, long ldba,
+                                  const float* a_log, const float* dt_bias, const int* token_seq, const int* seq_slot, float* out,
+                                  float* beta, float* g, int n_tokens, int G, int D, int H, int V, void* stream)
+{
+    if (n_tokens <= 0) return FX_OK;
+    const int C = 2 * G * D + H * V;
+    if ((D != 64 && D != 128) || 2 * G * D % 128 || H * V % 4 || H <= 0) return FX_ERR_SIZE;
+    if (ldp % 4 || (uintptr_t)proj % 16 || (uintptr_t)conv_w % 16 || (uintptr_t)tail % 16 || (uintptr_t)out % 16) return FX_ERR_ALIGN;
+    dim3 grid((unsigned)fx_cdiv(n_tokens, RUN * RUN_WARPS), (unsigned)fx_cdiv(C, 128) + 1);
+    fx_launch_pdl(delta_prep_runs_kernel, grid, RUN_WARPS * 32, 0, (cudaStream_t)stream, proj, ldp, conv_w, tail, ba, ldba, a_log, dt_bias,
+                  token_seq, seq_slot, out, beta, g, n_tokens, G, D, H, C);
     return fx_launch_status();
 }
 

@@ -42,6 +42,7 @@ _SIGNATURES = {
     "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
                       _I, _I, _I, _I, _I, _I, _P],
     "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "fx_delta_prep_runs": [_P, _L, _P, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fx_mlstm_gates": [_P, _L, _P, _P, _I, _F, _P, _I, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
     "fx_embed_norm": [_P, _I, _P, _P, _I, _F, _P, _I, _I, _I, _P, _P],
@@ -606,6 +607,9 @@ def scale_(x, factor, stream=None):
     return x
 
 
+DELTA_PREP_RUNS_MIN_TOKENS = 128     # from here on a run of 16 tokens a warp fills the device (4,096 channels)
+
+
 def delta_prep(proj, conv_w, taps, tail, ba, a_log, dt_bias, token_seq, seq_slot, out, beta, g, G, D, H, V, stream=None,
                update_tail=False):
     """What the gated delta rule needs before its recurrence, from rows ``proj`` = [q | k | v | ...] as projected:
@@ -615,6 +619,14 @@ def delta_prep(proj, conv_w, taps, tail, ba, a_log, dt_bias, token_seq, seq_slot
     ``update_tail``: only when every entry of the step brings exactly one token; the kernel then also moves the
     tail on, and :func:`conv_tail_update` is not needed."""
     T = proj.shape[0]
+    # prompts: runs of tokens instead of a block a token (a step of few tokens wants the blocks)
+    if (not update_tail and T >= DELTA_PREP_RUNS_MIN_TOKENS and taps == 4 and D in (64, 128) and 2 * G * D % 128 == 0
+            and H * V % 4 == 0 and proj.dtype == conv_w.dtype == torch.float32 and _rows(proj) % 4 == 0
+            and all(x.data_ptr() % 16 == 0 for x in (proj, conv_w, tail, out))):
+        call("fx_delta_prep_runs", _ptr(proj), _rows(proj), _ptr(conv_w), _ptr(tail), _ptr(ba), _rows(ba), _ptr(a_log),
+             _ptr(dt_bias), _ptr(token_seq), _ptr(seq_slot), _ptr(out), _ptr(beta), _ptr(g), T, G, D, H, V,
+             stream if stream is not None else stream_ptr())
+        return
     call("fx_delta_prep", _ptr(proj), code(proj), _rows(proj), _ptr(conv_w), code(conv_w), int(taps), _ptr(tail), _ptr(ba),
          _rows(ba), _ptr(a_log), _ptr(dt_bias), _ptr(token_seq), _ptr(seq_slot), _ptr(out), _ptr(beta), _ptr(g), T, G, D, H, V,
          int(update_tail), stream if stream is not None else stream_ptr())

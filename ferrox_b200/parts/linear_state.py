@@ -265,16 +265,18 @@ class GeneralDeltaRule(_StateMixer):
         proj = rt.empty(T, 5 * hd + s.decay_rank, dtype=f32)
         ops.linear(x, self.w_in, proj, status=batch.status, stream=batch.stream)
         r, k, v, gate = (proj[:, i * hd:(i + 1) * hd] for i in range(4))
-        u, au, w = rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32)
-        ops.general_delta_prep(k, proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:], self.w2, self.w0, self.a_bias, s.decay_rate,
-                               u, au, w, H, D, stream=batch.stream)
+        a_pre, low = proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:]
         read, state = rt.empty(T, hd, dtype=f32), cache.states["matrix"]
-        # (decays below e^-1 a token: over a chunk their products would leave 32-bit numbers' range)
-        tiles = _chunk_tiles(batch, H, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v), D, D, state) else None
+        # (a rate of at most 1: over a chunk the products of stronger decays would leave 32-bit numbers' range)
+        tiles = _chunk_tiles(batch, H, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
         if tiles is not None:
-            ops.chunk_scan_general(r, k, v, u, au, w, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D,
-                                   scratch=self._scratch, stream=batch.stream)
+            ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, tiles,
+                                   batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, scratch=self._scratch,
+                                   stream=batch.stream)
         else:
+            u, au, w = rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32)
+            ops.general_delta_prep(k, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, u, au, w, H, D,
+                                   stream=batch.stream)
             ops.general_delta_scan(r, k, v, u, au, w, state, read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D,
                                    stream=batch.stream)
         y = rt.empty(T, hd)

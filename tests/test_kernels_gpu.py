@@ -1324,25 +1324,31 @@ def test_chunk_scan(case, kind):
     assert torch.equal(out[keep], got[0][keep]) and bool(out[t].isnan().any())
 
 
-@pytest.mark.parametrize("lens,H,D", [([1], 2, 64), ([31, 32, 33], 3, 64), ([100, 5], 2, 20), ([65], 2, 128), ([130, 1, 64], 1, 100)])
-def test_chunk_scan_general(lens, H, D):
-    """The generalized delta rule in chunks against the loop in 64 bits, with decays over their whole range."""
+@pytest.mark.parametrize("lens,H,D,rank", [([1], 2, 64, 64), ([31, 32, 33], 3, 64, 8), ([100, 5], 2, 20, 3), ([65], 2, 128, 96),
+                                           ([130, 1, 64], 1, 100, 65)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_chunk_scan_general(dtype, lens, H, D, rank):
+    """The generalized delta rule in chunks, from its projections, against the loop in 64 bits, with decays over their whole
+    range."""
     o = ops()
     T, (seq, slot, tiles) = sum(lens), scan_setup(lens, 0)
-    wide = rnd(T, 3 * H * D + 8)
-    r, k, v = (wide[:, i * H * D:(i + 1) * H * D] for i in range(3))
-    gen = torch.Generator().manual_seed(T)
-    w = torch.exp(-0.6065 * torch.sigmoid(torch.randn(T, H * D, generator=gen) * 4)).to(DEV)
-    w[:, ::7], w[:, 1::7] = 0.5453, 1.0        # channels that forget as fast as they can, and that never do
-    u = k / torch.sqrt((k.reshape(T, H, D) ** 2).sum(-1, keepdim=True) + 1e-6).expand(T, H, D).reshape(T, H * D)
-    au = u * torch.rand(T, H * D, generator=gen).to(DEV)
+    wide = rnd(T, 4 * H * D + rank + (-rank) % 4)
+    r, k, v, a_pre = (wide[:, i * H * D:(i + 1) * H * D] for i in range(4))
+    low, w2, w0 = wide[:, 4 * H * D:4 * H * D + rank], rnd(H * D, rank, dtype=DT[dtype], scale=0.3), rnd(H * D, dtype=DT[dtype], scale=2.0)
+    w0[::7], w0[1::7] = 30.0, -30.0            # channels that forget as fast as they can, and that never do
+    a_bias, rate = rnd(H * D, dtype=DT[dtype], seed=2), math.exp(-0.5)
     state = rnd(len(lens) + 2, H, D, D, seed=3)
     st, st_old = state.clone(), state.clone()
     out, old = torch.empty(T, H * D, device=DEV), torch.empty(T, H * D, device=DEV)
+    u, au, w = (torch.empty(T, H * D, device=DEV) for _ in range(3))
+    o.general_delta_prep(k, a_pre, low, w2, w0, a_bias, rate, u, au, w, H, D)
     o.general_delta_scan(r, k, v, u, au, w, st_old, old, seq, slot, len(lens), H, D)
-    o.chunk_scan_general(r, k, v, u.clone(), au.clone(), w.clone(), st, out, tiles, seq, slot, len(lens), H, D, scratch=scan_scratch)
+    o.chunk_scan_general(r, k, v, a_pre, low, w2, w0, a_bias, rate, st, out, tiles, seq, slot, len(lens), H, D, scratch=scan_scratch)
     d = lambda t: t.double().cpu()
-    R, K, Vv, U, A, W = (d(x).reshape(T, H, D) for x in (r, k, v, u, au, w))
+    R, K, Vv = (d(x).reshape(T, H, D) for x in (r, k, v))
+    U = K / torch.sqrt((K * K).sum(-1, keepdim=True) + 1e-6)
+    A = torch.sigmoid(d(a_pre) + d(a_bias)).view(T, H, D) * U
+    W = torch.exp(-rate * torch.sigmoid(torch.tanh(d(low)) @ d(w2).T + d(w0))).view(T, H, D)
     want, S_want = torch.zeros(T, H, D, dtype=torch.float64), d(state)
     for b in range(len(lens)):
         S = S_want[int(slot[b])].transpose(1, 2).clone()
@@ -1354,3 +1360,47 @@ def test_chunk_scan_general(lens, H, D):
     far = lambda a, b: float((d(a) - b).norm() / b.norm())
     want = want.reshape(T, H * D)
     assert far(out, want) < max(2e-6, 1.5 * far(old, want)) and far(st, S_want) < max(1e-6, 1.5 * far(st_old, S_want))
+
+
+@pytest.mark.parametrize("lens,G,D,H,V", [([128], 1, 128, 1, 4), ([1, 2, 3, 200], 1, 64, 2, 36), ([17, 130, 16, 4], 2, 128, 4, 128),
+                                          ([300], 2, 64, 2, 62)])
+def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
+    """What the delta rule needs before its recurrence, in runs of tokens: entries that begin and end inside a run and
+    beside its edges, against the kernel that takes a token a block (the same order of the convolution's sums)."""
+    o = ops()
+    T, C, n = sum(lens), 2 * G * D + H * V, len(lens)
+    seq, slot, _ = scan_setup(lens, 0)
+    proj = rnd(T, C + 2 * H + 4 + (-(C + 2 * H)) % 4)
+    ba, conv, tail = proj[:, C:], rnd(C, 4, seed=1), rnd(n + 2, 3, C, seed=2)
+    a_log, dt = rnd(H, seed=3), rnd(H, seed=4)
+
+    def run(runs):
+        monkeypatch.setattr(o, "DELTA_PREP_RUNS_MIN_TOKENS", 1 if runs else 1 << 30)
+        got = torch.empty(T, C, device=DEV), torch.empty(T, H, device=DEV), torch.empty(T, H, device=DEV)
+        o.delta_prep(proj, conv, 4, tail, ba, a_log, dt, seq, slot, *got, G, D, H, V)
+        return got
+
+    for a, b in zip(run(True), run(False)):
+        assert rel(a, b) < 1e-6
+
+
+@pytest.mark.parametrize("lens,G,D,H,V", [([128], 1, 128, 1, 4), ([1, 2, 3, 200], 1, 64, 2, 36), ([17, 130, 16, 4], 2, 128, 4, 128),
+                                          ([300], 2, 64, 2, 62)])
+def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
+    """What the delta rule needs before its recurrence, in runs of tokens: entries that begin and end inside a run and
+    beside its edges, against the kernel that takes a token a block (the same order of the convolution's sums)."""
+    o = ops()
+    T, C, n = sum(lens), 2 * G * D + H * V, len(lens)
+    seq, slot, _ = scan_setup(lens, 0)
+    proj = rnd(T, C + 2 * H + 4 + (-(C + 2 * H)) % 4)
+    ba, conv, tail = proj[:, C:], rnd(C, 4, seed=1), rnd(n + 2, 3, C, seed=2)
+    a_log, dt = rnd(H, seed=3), rnd(H, seed=4)
+
+    def run(runs):
+        monkeypatch.setattr(o, "DELTA_PREP_RUNS_MIN_TOKENS", 1 if runs else 1 << 30)
+        got = torch.empty(T, C, device=DEV), torch.empty(T, H, device=DEV), torch.empty(T, H, device=DEV)
+        o.delta_prep(proj, conv, 4, tail, ba, a_log, dt, seq, slot, *got, G, D, H, V)
+        return got
+
+    for a, b in zip(run(True), run(False)):
+        assert rel(a, b) < 1e-6
