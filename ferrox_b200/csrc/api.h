@@ -284,9 +284,6 @@ int fx_set_scan_lanes(int lanes);   // lanes that share a state column, fixed fo
 int fx_delta_prep_runs(const float* proj, long ldp, const float* conv_w, const float* tail, const float* ba, long ldba,
                        const float* a_log, const float* dt_bias, const int* token_seq, const int* seq_slot, float* out,
                        float* beta, float* g, int n_tokens, int G, int D, int H, int V, void* stream);
-int fx_delta_prep_runs(const float* proj, long ldp, const float* conv_w, const float* tail, const float* ba, long ldba,
-                       const float* a_log, const float* dt_bias, const int* token_seq, const int* seq_slot, float* out,
-                       float* beta, float* g, int n_tokens, int G, int D, int H, int V, void* stream);
 int fx_gated_group_norm(const float* x, const void* gate, int gate_dtype, long ldg, const void* w, int w_dtype, float eps,
                         int act, void* out, int out_dtype, int n_tokens, int groups, int width, long w_stride,
                         void* stream);

@@ -41,7 +41,8 @@ _SIGNATURES = {
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
     "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
                       _I, _I, _I, _I, _I, _I, _P],
-    "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _F, _I, _P, _P, _P, _P, _P, _P, _P,
+                              _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
     "fx_delta_prep_runs": [_P, _L, _P, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fx_mlstm_gates": [_P, _L, _P, _P, _I, _F, _P, _I, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
@@ -685,15 +686,20 @@ def chunk_scan(q, k, v, g, state, out, tiles, token_seq, seq_slot, n_entries, H,
     return out
 
 
-def chunk_scan_general(r, k, v, u, au, w, state, out, tiles, token_seq, seq_slot, n_entries, H, D, *, scratch, stream=None):
-    """:func:`general_delta_scan` over a prompt's chunks (see :func:`chunk_scan`); ``u``, ``au`` and ``w`` are overwritten."""
+def chunk_scan_general(r, k, v, a_pre, low, w2, w0, a_bias, rate, state, out, tiles, token_seq, seq_slot, n_entries, H, D, *,
+                       scratch, stream=None):
+    """:func:`general_delta_prep` and :func:`general_delta_scan` over a prompt's chunks (see :func:`chunk_scan`): ``r``,
+    ``k``, ``v``, ``a_pre`` 32-bit row views [T, H*D], ``low`` [T, rank], ``w2`` contiguous [H*D, rank]; a ``rate`` of at
+    most 1, so that a chunk's products of decays stay inside 32-bit numbers' range."""
     T = r.shape[0]
-    if not all(t.is_contiguous() for t in (u, au, w, out)):
-        raise KernelError("chunk_scan_general: contiguous unit keys, decays and read-outs")
+    if not (out.is_contiguous() and w2.is_contiguous()) or low.dtype != torch.float32:
+        raise KernelError("chunk_scan_general: 32-bit low-rank rows, a contiguous matrix and read-outs")
     p, gam, wr = scratch(T, H, 2 * SCAN_CHUNK), scratch(tiles.shape[0], H, D), scratch(T, H, D)
-    call("fx_chunk_scan_general", _ptr(r), _rows(r), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(u), _ptr(au), _ptr(w), _ptr(p),
-         _ptr(gam), _ptr(wr), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0], _ptr(token_seq), _ptr(seq_slot), T,
-         int(n_entries), H, D, stream if stream is not None else stream_ptr())
+    qs, ks, a_s = scratch(T, H, D), scratch(T, H, D), scratch(T, H, D)
+    call("fx_chunk_scan_general", _ptr(r), _rows(r), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(a_pre), _rows(a_pre), _ptr(low),
+         _rows(low), _ptr(w2), code(w2), _ptr(w0), code(w0), _ptr(a_bias), code(a_bias), float(rate), w2.shape[1], _ptr(p),
+         _ptr(gam), _ptr(wr), _ptr(qs), _ptr(ks), _ptr(a_s), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0],
+         _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, D, stream if stream is not None else stream_ptr())
     return out
 
 

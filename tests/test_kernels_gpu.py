@@ -1382,25 +1382,3 @@ def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
 
     for a, b in zip(run(True), run(False)):
         assert rel(a, b) < 1e-6
-
-
-@pytest.mark.parametrize("lens,G,D,H,V", [([128], 1, 128, 1, 4), ([1, 2, 3, 200], 1, 64, 2, 36), ([17, 130, 16, 4], 2, 128, 4, 128),
-                                          ([300], 2, 64, 2, 62)])
-def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
-    """What the delta rule needs before its recurrence, in runs of tokens: entries that begin and end inside a run and
-    beside its edges, against the kernel that takes a token a block (the same order of the convolution's sums)."""
-    o = ops()
-    T, C, n = sum(lens), 2 * G * D + H * V, len(lens)
-    seq, slot, _ = scan_setup(lens, 0)
-    proj = rnd(T, C + 2 * H + 4 + (-(C + 2 * H)) % 4)
-    ba, conv, tail = proj[:, C:], rnd(C, 4, seed=1), rnd(n + 2, 3, C, seed=2)
-    a_log, dt = rnd(H, seed=3), rnd(H, seed=4)
-
-    def run(runs):
-        monkeypatch.setattr(o, "DELTA_PREP_RUNS_MIN_TOKENS", 1 if runs else 1 << 30)
-        got = torch.empty(T, C, device=DEV), torch.empty(T, H, device=DEV), torch.empty(T, H, device=DEV)
-        o.delta_prep(proj, conv, 4, tail, ba, a_log, dt, seq, slot, *got, G, D, H, V)
-        return got
-
-    for a, b in zip(run(True), run(False)):
-        assert rel(a, b) < 1e-6
