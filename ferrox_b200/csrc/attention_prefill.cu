@@ -178,20 +178,29 @@ __global__ void __launch_bounds__(NTHREADS) prefill_attention_kernel(
 #pragma unroll
                 for (int j = 0; j < BKEY / 8; ++j)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) s[j][e] = cap * tanhf(s[j][e] * cap_mul);
+                    for (int e = 0; e < 4; ++e) s[j][e] = cap * fx_tanh_fast(s[j][e] * cap_mul);
             }
             // ---- mask by absolute position, online softmax ---------------------------
             const int lo0 = window > 0 ? p_row0 - window + 1 : 0, lo1 = window > 0 ? p_row1 - window + 1 : 0;
             float mx0 = -INFINITY, mx1 = -INFINITY;
+            // (most blocks are seen whole by all of the warp's rows)
+            if (kb + BKEY - 1 <= w_first && (window <= 0 || kb >= w_last - window + 1)) {
 #pragma unroll
-            for (int j = 0; j < BKEY / 8; ++j) {
+                for (int j = 0; j < BKEY / 8; ++j) {
+                    mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
+                    mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
+                }
+            } else {
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int key = kb + j * 8 + 2 * t4 + e;
-                    if (key > p_row0 || key < lo0) s[j][e] = -INFINITY;
-                    if (key > p_row1 || key < lo1) s[j][2 + e] = -INFINITY;
-                    mx0 = fmaxf(mx0, s[j][e]);
-                    mx1 = fmaxf(mx1, s[j][2 + e]);
+                for (int j = 0; j < BKEY / 8; ++j) {
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int key = kb + j * 8 + 2 * t4 + e;
+                        if (key > p_row0 || key < lo0) s[j][e] = -INFINITY;
+                        if (key > p_row1 || key < lo1) s[j][2 + e] = -INFINITY;
+                        mx0 = fmaxf(mx0, s[j][e]);
+                        mx1 = fmaxf(mx1, s[j][2 + e]);
+                    }
                 }
             }
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
@@ -199,14 +208,14 @@ __global__ void __launch_bounds__(NTHREADS) prefill_attention_kernel(
             const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
             // a row that sees no key yet keeps m = -inf: use 0 as the reference so that exp2 stays finite
             const float ref0 = mn0 == -INFINITY ? 0.f : mn0 * scale_log2e, ref1 = mn1 == -INFINITY ? 0.f : mn1 * scale_log2e;
-            const float al0 = m0 == -INFINITY ? 0.f : exp2f(m0 * scale_log2e - ref0);
-            const float al1 = m1 == -INFINITY ? 0.f : exp2f(m1 * scale_log2e - ref1);
+            const float al0 = m0 == -INFINITY ? 0.f : fx_ex2(m0 * scale_log2e - ref0);
+            const float al1 = m1 == -INFINITY ? 0.f : fx_ex2(m1 * scale_log2e - ref1);
             float sum0 = 0.f, sum1 = 0.f;
             uint32_t p[BKEY / 8][2];
 #pragma unroll
             for (int j = 0; j < BKEY / 8; ++j) {
-                const float e0 = exp2f(s[j][0] * scale_log2e - ref0), e1 = exp2f(s[j][1] * scale_log2e - ref0);
-                const float e2 = exp2f(s[j][2] * scale_log2e - ref1), e3 = exp2f(s[j][3] * scale_log2e - ref1);
+                const float e0 = fx_ex2(s[j][0] * scale_log2e - ref0), e1 = fx_ex2(s[j][1] * scale_log2e - ref0);
+                const float e2 = fx_ex2(s[j][2] * scale_log2e - ref1), e3 = fx_ex2(s[j][3] * scale_log2e - ref1);
                 sum0 += e0 + e1; sum1 += e2 + e3;
                 p[j][0] = pack_bf16(e0, e1);
                 p[j][1] = pack_bf16(e2, e3);
