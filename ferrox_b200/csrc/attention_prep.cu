@@ -48,12 +48,14 @@ __global__ void qk_norm_store_kernel(T* __restrict__ qkv, long ld, const int* __
             r = sqrtf(ss / (float)D + eps);
         }
         const float mult = is_q ? temp : 1.f;
+        const bool as_is = !w && mult == 1.f;       // nothing changes: a query row is left alone, a key row only copied
+        if (as_is && (is_q || place < 0)) continue;
         T* kp = (!is_q && place >= 0) ? k_pages + (place + (long)(u - H) * page_size) * D : nullptr;
         for (int i = lane; i < D; i += 32) {
             float v = to_f32(x[i]);
             if (w) v = v / r * load_any(w, w_dtype, i);
             const T o = from_f32<T>(v * mult);
-            x[i] = o;
+            if (!as_is) x[i] = o;
             if (kp) kp[i] = o;
         }
     }

@@ -273,13 +273,41 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
     for (int rc = 0; rc < a.rank; rc += RANK) {
         const int nr = min(RANK, a.rank - rc);
         __syncthreads();
-        for (int i = tid; i < D * RANK; i += PREP_THREADS) {
-            const int d = i / RANK, r = i - d * RANK;
-            w2_s[d * RP + r] = r < nr && d < a.D ? load_any(a.w2, a.w2_dtype, ((long)h * a.D + d) * a.rank + rc + r) : 0.f;
+        if (a.rank % 4 == 0 && (uintptr_t)a.w2 % 16 == 0) {     // four columns a load
+#pragma unroll
+            for (int n = 0; n < D * RANK / 4 / PREP_THREADS; ++n) {
+                const int i = tid + n * PREP_THREADS, d = i / (RANK / 4), r = (i % (RANK / 4)) * 4;
+                const long at = ((long)h * a.D + d) * a.rank + rc + r;
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < nr && d < a.D) {
+                    if (a.w2_dtype == FX_F32) {
+                        x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.w2) + at);
+                    } else {
+                        const uint2 b = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.w2) + at);
+                        x.x = __uint_as_float(b.x << 16); x.y = __uint_as_float(b.x & 0xffff0000u);
+                        x.z = __uint_as_float(b.y << 16); x.w = __uint_as_float(b.y & 0xffff0000u);
+                    }
+                }
+                *reinterpret_cast<float4*>(w2_s + d * RP + r) = x;
+            }
+        } else {
+            for (int i = tid; i < D * RANK; i += PREP_THREADS) {
+                const int d = i / RANK, r = i - d * RANK;
+                w2_s[d * RP + r] = r < nr && d < a.D ? load_any(a.w2, a.w2_dtype, ((long)h * a.D + d) * a.rank + rc + r) : 0.f;
+            }
         }
-        for (int i = tid; i < CHUNK * RANK; i += PREP_THREADS) {
-            const int t = i / RANK, r = i - t * RANK;
-            th_s[t * RP + r] = r < nr && t < rows ? tanhf(a.low[(long)(tok0 + t) * a.ldl + rc + r]) : 0.f;
+        {
+            float x[CHUNK * RANK / PREP_THREADS];       // (all loads before the first tanh)
+#pragma unroll
+            for (int n = 0; n < CHUNK * RANK / PREP_THREADS; ++n) {
+                const int i = tid + n * PREP_THREADS, t = i / RANK, r = i % RANK;
+                x[n] = r < nr && t < rows ? a.low[(long)(tok0 + t) * a.ldl + rc + r] : 0.f;
+            }
+#pragma unroll
+            for (int n = 0; n < CHUNK * RANK / PREP_THREADS; ++n) {
+                const int i = tid + n * PREP_THREADS;
+                th_s[i / RANK * RP + i % RANK] = tanhf(x[n]);
+            }
         }
         __syncthreads();
 #pragma unroll 4

@@ -1382,3 +1382,29 @@ def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
 
     for a, b in zip(run(True), run(False)):
         assert rel(a, b) < 1e-6
+
+
+@pytest.mark.parametrize("hidden", [4, 100, 1028, 2048, 4100, 8192, 8196, 2046])
+@pytest.mark.parametrize("n_rows", [1, 3, 300])
+def test_layer_norms_with_the_row_in_registers(n_rows, hidden):
+    """Layer norm, and layer norm with the residual addition and the next norm, at the edges of a block's pieces (and
+    beyond what the vector form takes), in place, with picked rows, 16- and 32-bit operands; against 64 bits."""
+    o, eps = ops(), 1e-5
+    ln = lambda x, w, b=0.0: (x - x.mean(-1, keepdim=True)) / torch.sqrt(x.var(-1, unbiased=False, keepdim=True) + eps) * w + b
+    x, w, b = rnd(n_rows, hidden) * 3 + 1, rnd(hidden, dtype=torch.bfloat16) + 1, rnd(hidden, seed=4)
+    rows = torch.arange(n_rows - 1, -1, -1, dtype=torch.int32, device=DEV)
+    for dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 1e-2)):
+        out = torch.empty(n_rows, hidden, dtype=dtype, device=DEV)
+        o.layernorm(x, w, eps, out, rows=rows, bias=b)
+        assert rel(out.double(), ln(x.double(), w.double(), b.double()).flip(0)) < tol
+    same = x.clone()
+    o.layernorm(same, w, eps, same)
+    assert rel(same.double(), ln(x.double(), w.double())) < 2e-6
+    for dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 1e-2)):
+        h, y1, y2 = rnd(n_rows, hidden, seed=5), rnd(n_rows, hidden, dtype=dtype, seed=6), rnd(n_rows, hidden, seed=7)
+        for second in (None, y2):
+            z = 0.5 * y1.double() + (0.25 * y2.double() if second is not None else 0.0)
+            want = h.double() + ln(z, w.double())
+            got, nxt = h.clone(), torch.empty(n_rows, hidden, dtype=dtype, device=DEV)
+            o.layernorm_residual(got, y1, w, eps, scale=0.5, y2=second, scale2=0.25, then=(b, eps, nxt))
+            assert rel(got.double(), want) < 2e-6 and rel(nxt.double(), ln(want, b.double())) < 2 * tol
