@@ -490,8 +490,12 @@ __global__ void __launch_bounds__(128) gated_group_norm_warp_kernel(
     }
 }
 
-// The same for groups of whole 16-byte pieces: TPG threads a group (a warp, or the block), four elements each at a time,
-// the group's row in registers between the sum of its squares and the result.
+// The same for groups of whole 16-byte pieces: TPG threads a group (half a warp, a warp, or the block), four elements each at
+// a time, the group's row in registers between the sum of its squares and the result.  It is bound by loads in flight, so a
+// thread holds GN_CH pieces whatever the width: one group of up to GN_CH pieces a thread, or, where a group is one piece a
+// thread (64 elements on half a warp, 128 on a warp), GN_CH groups side by side.  (3,001 tokens of 32 groups of 64, gate in 32
+// bits: a group a warp, half of its lanes idle and every weight a load of its own, 34.6 us; so 17.5.  2,048 tokens of 16
+// groups of 128: 13.0 and 12.3.)
 constexpr int GN_CH = 4;      // pieces a thread holds at most
 
 template <typename GT> __device__ __forceinline__ void load_gate4(const GT* p, float* g);
@@ -502,48 +506,77 @@ template <> __device__ __forceinline__ void load_gate4<bf16>(const bf16* p, floa
     g[2] = __uint_as_float(v.y << 16); g[3] = __uint_as_float(v.y & 0xffff0000u);
 }
 
-template <typename GT, typename OT, int TPG>
+// Four weights from element `at` on; vec: they lie on a boundary of four.
+__device__ __forceinline__ void load_weight4(const void* w, int dtype, long at, bool vec, float* r)
+{
+    if (!vec) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = load_any(w, dtype, at + e);
+    } else if (dtype == FX_F32) {
+        Pack<float>::load(reinterpret_cast<const float*>(w) + at, r);
+    } else {
+        load_gate4<bf16>(reinterpret_cast<const bf16*>(w) + at, r);
+    }
+}
+
+template <typename GT, typename OT, int TPG, int PIECES>
 __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(
-    const float* __restrict__ x, const GT* __restrict__ gate, long ldg, const void* __restrict__ w, int w_dtype,
+    const float* __restrict__ x, const GT* __restrict__ gate, long ldg, const void* __restrict__ w, int w_dtype, int w_vec,
     float eps, int act, OT* __restrict__ out, int groups, int width, long w_stride, long n_groups)
 {
+    constexpr int GROUPS = GN_CH / PIECES;      // of a thread, 256 / TPG apart
     __shared__ float scratch[33];
     fx_pdl_wait();
-    const int own = TPG == 32 ? threadIdx.x & 31 : threadIdx.x;
-    const long at = TPG == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;     // (token, group)
-    if (at >= n_groups) return;      // (whole warps; a block of its own group never)
-    const long t = at / groups;
-    const int grp = (int)(at - t * groups);
-    const float* xr = x + at * width;
-    const GT* gr = gate + t * ldg + (long)grp * width;
+    const int own = threadIdx.x % TPG;
+    const long at0 = (long)blockIdx.x * GROUPS * (256 / TPG) + threadIdx.x / TPG;      // (token, group)
     float v[GN_CH][4], g[GN_CH][4];
-    float ss = 0.f;
+    auto place = [&](int c, long& at, int& i) {
+        at = at0 + (c / PIECES) * (256 / TPG);
+        i = ((c % PIECES) * TPG + own) * 4;
+        return at < n_groups && i < width;
+    };
 #pragma unroll
     for (int c = 0; c < GN_CH; ++c) {
-        const int i = (c * TPG + own) * 4;
-        if (i < width) { Pack<float>::load(xr + i, v[c]); load_gate4<GT>(gr + i, g[c]); }
-    }
+        long at; int i;
+        if (place(c, at, i)) {
+            const long t = at / groups;
+            Pack<float>::load(x + at * width + i, v[c]);
+            load_gate4<GT>(gate + t * ldg + (at - t * groups) * width + i, g[c]);
+        } else {
 #pragma unroll
-    for (int c = 0; c < GN_CH; ++c)
-        if ((c * TPG + own) * 4 < width) {
+            for (int e = 0; e < 4; ++e) { v[c][e] = 0.f; g[c][e] = 0.f; }
+        }
+    }
+    float inv[GROUPS];
+#pragma unroll
+    for (int n = 0; n < GROUPS; ++n) {
+        float ss = 0.f;
+#pragma unroll
+        for (int c = n * PIECES; c < (n + 1) * PIECES; ++c)
 #pragma unroll
             for (int e = 0; e < 4; ++e) ss = fmaf(v[c][e], v[c][e], ss);
+        if (TPG == 256) {
+            ss = block_sum(ss, scratch);
+        } else {
+#pragma unroll
+            for (int o = TPG / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         }
-    ss = TPG == 32 ? warp_sum(ss) : block_sum(ss, scratch);
-    const float inv = 1.0f / sqrtf(ss / (float)width + eps);
-    OT* o = out + at * width;
+        inv[n] = 1.0f / sqrtf(ss / (float)width + eps);
+    }
 #pragma unroll
     for (int c = 0; c < GN_CH; ++c) {
-        const int i = (c * TPG + own) * 4;
-        if (i >= width) continue;
+        long at; int i;
+        if (!place(c, at, i)) continue;
         float r[4];
+        load_weight4(w, w_dtype, (at % groups) * w_stride + i, w_vec, r);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float gv = g[c][e];
-            r[e] = v[c][e] * inv * load_any(w, w_dtype, (long)grp * w_stride + i + e);
+            r[e] = v[c][e] * inv[c / PIECES] * r[e];
             if (sizeof(OT) == 2) r[e] *= act ? fx_sigmoid_fast(gv) : gv * fx_sigmoid_fast(gv);
             else r[e] *= act ? sigmoid_f(gv) : silu_f(gv);
         }
+        OT* o = out + at * width;
         if (sizeof(OT) == 4) Pack<float>::store(reinterpret_cast<float*>(o) + i, r);
         else {
             __nv_bfloat162 p = __floats2bfloat162_rn(r[0], r[1]), q = __floats2bfloat162_rn(r[2], r[3]);
@@ -656,19 +689,22 @@ extern "C" int fx_gated_group_norm(const float* x, const void* gate, int gate_dt
     if (groups <= 0 || width <= 0) return FX_ERR_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const int gb = gate_dtype == FX_F32 ? 16 : 8, ob = out_dtype == FX_F32 ? 16 : 8;     // bytes of four elements
-    const bool vec = width >= 64 && width % 4 == 0 && width <= 4 * GN_CH * 256 && ldg % 4 == 0 && (uintptr_t)x % 16 == 0 &&
+    const bool vec = width % 4 == 0 && width <= 4 * GN_CH * 256 && ldg % 4 == 0 && (uintptr_t)x % 16 == 0 &&
                      (uintptr_t)gate % gb == 0 && (uintptr_t)out % ob == 0;
-    const bool warp_group = width <= 4 * GN_CH * 32;
     const long n_groups = (long)n_tokens * groups;
-    const unsigned vec_blocks = (unsigned)(warp_group ? fx_cdiv(n_groups, 8) : n_groups);
+    const int w_vec = w_stride % 4 == 0 && (uintptr_t)w % (w_dtype == FX_F32 ? 16 : 8) == 0;
     const bool narrow = width <= 64;
     dim3 grid(n_tokens, narrow ? (unsigned)fx_cdiv(groups, 4) : groups);
+#define FX_VEC(GT, OT, TPG, PIECES)                                                                                       \
+    fx_launch_pdl(gated_group_norm_vec_kernel<GT, OT, TPG, PIECES>,                                                       \
+                  (unsigned)fx_cdiv(n_groups, (long)(GN_CH / PIECES) * (256 / TPG)), 256, 0, s, x, (const GT*)gate, ldg,  \
+                  w, w_dtype, w_vec, eps, act, (OT*)out, groups, width, w_stride, n_groups)
 #define FX_GO(GT, OT)                                                                                                     \
     do {                                                                                                                  \
-        if (vec && warp_group) fx_launch_pdl(gated_group_norm_vec_kernel<GT, OT, 32>, vec_blocks, 256, 0, s, x, (const GT*)gate, ldg, w, \
-                                             w_dtype, eps, act, (OT*)out, groups, width, w_stride, n_groups);               \
-        else if (vec) fx_launch_pdl(gated_group_norm_vec_kernel<GT, OT, 256>, vec_blocks, 256, 0, s, x, (const GT*)gate, ldg, w,        \
-                                    w_dtype, eps, act, (OT*)out, groups, width, w_stride, n_groups);                        \
+        if (vec && width <= 64) FX_VEC(GT, OT, 16, 1);                                                                     \
+        else if (vec && width <= 128) FX_VEC(GT, OT, 32, 1);                                                               \
+        else if (vec && width <= 4 * GN_CH * 32) FX_VEC(GT, OT, 32, GN_CH);                                                \
+        else if (vec) FX_VEC(GT, OT, 256, GN_CH);                                                                          \
         else if (narrow) fx_launch_pdl(gated_group_norm_warp_kernel<GT, OT>, grid, 128, 0, s, x, (const GT*)gate, ldg, w, w_dtype, \
                                   eps, act, (OT*)out, groups, width, w_stride);                                         \
         else fx_launch_pdl(gated_group_norm_kernel<GT, OT>, grid, 128, 0, s, x, (const GT*)gate, ldg, w, w_dtype, eps, act, \
@@ -679,5 +715,6 @@ extern "C" int fx_gated_group_norm(const float* x, const void* gate, int gate_dt
     else if (gate_dtype == FX_BF16 && out_dtype == FX_BF16) FX_GO(bf16, bf16);
     else return FX_ERR_DTYPE;
 #undef FX_GO
+#undef FX_VEC
     return fx_launch_status();
 }

@@ -1408,3 +1408,26 @@ def test_layer_norms_with_the_row_in_registers(n_rows, hidden):
             got, nxt = h.clone(), torch.empty(n_rows, hidden, dtype=dtype, device=DEV)
             o.layernorm_residual(got, y1, w, eps, scale=0.5, y2=second, scale2=0.25, then=(b, eps, nxt))
             assert rel(got.double(), want) < 2e-6 and rel(nxt.double(), ln(want, b.double())) < 2 * tol
+
+
+@pytest.mark.parametrize("width", [4, 60, 64, 68, 128, 132, 512, 516, 2048])
+@pytest.mark.parametrize("gate_dtype,out_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16),
+                                                  (torch.bfloat16, torch.bfloat16)])
+def test_gated_group_norm_over_its_forms(width, gate_dtype, out_dtype):
+    """Half a warp, a warp or a block a group, one group or four a thread; numbers of groups that leave a block's last places
+    empty; weights shared, an element each, in 16 bits and off a 16-byte boundary.  Tolerance: the row's sum and the products
+    in 32 bits (1e-5 with the exponential's 1e-6), and the rounding of the result to its type."""
+    g = torch.Generator(device="cuda").manual_seed(width)
+    for T, groups, shared, wdt, off in ((1, 1, True, torch.float32, 0), (7, 5, False, torch.bfloat16, 0), (33, 3, True, torch.float32, 1)):
+        x = torch.randn(T, groups * width, generator=g, device="cuda")
+        rows = torch.randn(T, groups * width + 8, generator=g, device="cuda").to(gate_dtype)
+        gate = rows[:, 8:]
+        w = torch.randn((width if shared else groups * width) + off, generator=g, device="cuda").to(wdt)[off:]
+        for act in ("silu", "sigmoid"):
+            out = torch.full((T, groups * width), float("nan"), device="cuda", dtype=out_dtype)
+            ops().gated_group_norm(x, gate, w, 1e-5, act, out, groups, width)
+            xd, gd = x.double().view(T, groups, width), gate.double().view(T, groups, width)
+            want = xd / (xd.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double().view(1, 1 if shared else groups, width)
+            want = (want * torch.sigmoid(gd) * (gd if act == "silu" else 1)).reshape(T, -1)
+            tol = 1e-5 + (0 if out_dtype == torch.float32 else 2.0 ** -8)
+            assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
