@@ -41,7 +41,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
-from ..kernels.ops import upload
+from ..kernels.ops import SlotZeroer, upload
 from .specs import CacheSpec
 
 
@@ -179,6 +179,10 @@ class CacheManager:
             self._group_of.append(g)
             self._pages.append(pages)
             self._state.append(st)
+        self._states = [st for st in self._state if st is not None]
+        self._states += [st for named in self._named_state for st in (named or {}).values()]
+        self._states = [st for st in self._states if st.numel()]
+        self._zero_slots = SlotZeroer(self._states) if self._states and self.device.type == "cuda" else None
         order = sorted(self.groups.values(), key=lambda g: g.index)
         windows = (ctypes.c_int * max(1, len(order)))(*[-1 if g.window is None else int(g.window) for g in order])
         pages = (ctypes.c_int * max(1, len(order)))(*[g.pool.n_pages for g in order])
@@ -215,11 +219,10 @@ class CacheManager:
         slot = self._lib.fxh_open(self._h)
         if slot < 0:
             return None
-        for st in self._state:
-            if st is not None:
-                st[slot].zero_()
-        for named in self._named_state:
-            for st in (named or {}).values():
+        if self._zero_slots is not None:
+            self._zero_slots(slot)
+        else:
+            for st in self._states:
                 st[slot].zero_()
         return slot
 

@@ -17,8 +17,10 @@ int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long 
                 void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
                 long w_group_stride, int form, int splits, void* part, void* stream);
 
+// Zeros at a slot of every tensor of a table (elementwise.cu).
+int fx_zero_slots(const long* table, int n, long most, long slot, void* stream);
+
 // The recurrences of matrix-state mixers in chunks of tokens (chunk_scan.cu).
-int fx_chunk_size();
 int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const float* v, long ldv, const float* g, const float* beta,
                   const float* take, float q_scale, float* p, float* gam, float* e, float* wr, const float* norm_in, float* norm,
                   int copies, const float* floor_m, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,

@@ -864,8 +864,6 @@ bool off_grid(const void* p, long ld) { return (uintptr_t)p % 16 || ld % 4; }
 
 }  // namespace
 
-extern "C" int fx_chunk_size() { return CHUNK; }
-
 // The delta rule (beta [T, H]) or, with take [T, H] (a factor on k v^T), norm_in, norm and floor_m, an mLSTM's recurrence.
 // q, k [T, G * D], v [T, H * V] 32-bit rows; g [T, H] the decays.  Scratch: p [T, H, CHUNK], gam and e [T, H]; delta rule: wr
 // [T, H, D].  norm_in: the normaliser before the step [entries, H, D], norm its copies in the state [slots, H, copies, D],

@@ -479,6 +479,21 @@ __global__ void gather_rows_scaled_kernel(const T* __restrict__ x, long ldx, con
     for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = from_f32<T>(w * to_f32(src[i]));
 }
 
+// A new request's state: zeros at its slot of every tensor of `table` (address, bytes a slot).  One launch instead of one a
+// tensor (18 of 1.5 us and the gaps between them in front of a prompt of eight layers with states).
+__global__ void __launch_bounds__(256) zero_slots_kernel(const long* __restrict__ table, long slot)
+{
+    fx_pdl_wait();
+    const long bytes = table[2 * blockIdx.y + 1];
+    unsigned char* p = reinterpret_cast<unsigned char*>(table[2 * blockIdx.y]) + slot * bytes;
+    const long first = (long)blockIdx.x * 256 + threadIdx.x, step = (long)gridDim.x * 256;
+    if (((uintptr_t)p | (uintptr_t)bytes) % 16 == 0) {
+        for (long i = first; i < bytes / 16; i += step) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+        for (long i = first; i < bytes; i += step) p[i] = 0;
+    }
+}
+
 }  // namespace
 
 extern "C" int fx_embed(const void* table, int dtype, const int* ids, float* out, int n_tokens, int hidden,
@@ -753,5 +768,15 @@ extern "C" int fx_residual_add(float* h, const void* y, int dtype, long n, void*
     if (dtype == FX_F32) residual_add_kernel<float><<<(unsigned)blocks, 256, 0, s>>>(h, (const float*)y, n);
     else if (dtype == FX_BF16) residual_add_kernel<bf16><<<(unsigned)blocks, 256, 0, s>>>(h, (const bf16*)y, n);
     else return FX_ERR_DTYPE;
+    return fx_launch_status();
+}
+
+// table [n][2] on the device: a tensor's address and its bytes a slot; most: the largest of those.
+extern "C" int fx_zero_slots(const long* table, int n, long most, long slot, void* stream)
+{
+    if (n <= 0 || most <= 0) return FX_OK;
+    if (n > 65535 || slot < 0) return FX_ERR_SIZE;
+    const long blocks = fx_cdiv(most, 256 * 16 * 2);
+    fx_launch_pdl(zero_slots_kernel, dim3((unsigned)(blocks > 128 ? 128 : blocks), (unsigned)n), 256, 0, (cudaStream_t)stream, table, slot);
     return fx_launch_status();
 }

@@ -39,6 +39,7 @@ _SIGNATURES = {
     "fx_gemm": [_P, _I, _L, _P, _P, _I, _L, _P, _I, _P, _I, _L, _I, _I, _I, _I, _P, _I, _L, _P],
     "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
+    "fx_zero_slots": [_P, _I, _L, _L, _P],
     "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
                       _I, _I, _I, _I, _I, _I, _P],
     "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _F, _I, _P, _P, _P, _P, _P, _P, _P,
@@ -300,6 +301,25 @@ def upload(values, device) -> torch.Tensor:
     if device.type != "cuda" or t.numel() == 0:
         return t.to(device)
     return t.pin_memory().to(device, non_blocking=True)
+
+
+class SlotZeroer:
+    """Zeros at one slot of every tensor of ``tensors`` ([slots, ...], contiguous, not empty, on one CUDA device), in one launch."""
+
+    def __init__(self, tensors):
+        for t in tensors:
+            if not t.is_contiguous() or t.numel() == 0:
+                raise KernelError("SlotZeroer: contiguous tensors with elements")
+        self.tensors = list(tensors)      # (held: the table has their addresses)
+        self.device = self.tensors[0].device
+        sizes = [t.stride(0) * t.element_size() for t in self.tensors]
+        self.most = max(sizes)
+        self.table = torch.tensor([[t.data_ptr(), n] for t, n in zip(self.tensors, sizes)], dtype=torch.int64, device=self.device)
+
+    def __call__(self, slot: int) -> None:
+        with torch.cuda.device(self.device):
+            call("fx_zero_slots", _ptr(self.table), len(self.tensors), self.most, int(slot),
+                 torch.cuda.current_stream().cuda_stream)
 
 
 # ---------------------------------------------------------------------------

@@ -1431,3 +1431,13 @@ def test_gated_group_norm_over_its_forms(width, gate_dtype, out_dtype):
             want = (want * torch.sigmoid(gd) * (gd if act == "silu" else 1)).reshape(T, -1)
             tol = 1e-5 + (0 if out_dtype == torch.float32 else 2.0 ** -8)
             assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
+
+
+def test_a_slot_of_every_state_is_zeroed_and_no_other():
+    from ferrox_b200.kernels.ops import SlotZeroer
+
+    shapes = [((4, 3), torch.float32), ((4, 64, 64), torch.float32), ((4, 5), torch.bfloat16), ((4, 8, 1031), torch.float32)]
+    ts = [torch.ones(s, device="cuda", dtype=d) for s, d in shapes]
+    SlotZeroer(ts)(2)
+    for t in ts:
+        assert (t[2] == 0).all() and (t[[0, 1, 3]] == 1).all()
