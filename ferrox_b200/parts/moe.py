@@ -167,6 +167,8 @@ class SoftmaxTopkMoe(FeedForward):
             self._side = rt.groups.get("side stream")
             if self._side is None:
                 self._side = rt.groups["side stream"] = torch.cuda.Stream(device=rt.device)
+            # (a capture would make a layer's second branch wait for the branch of the layer before as well: a stream each)
+            self._side_in_graph = torch.cuda.Stream(device=rt.device)
             self._fork, self._join = torch.cuda.Event(), torch.cuda.Event()
 
     def _load_table(self, src, rt):
@@ -219,10 +221,11 @@ class SoftmaxTopkMoe(FeedForward):
 
     def _shared_on_side(self, x, batch):
         """The shared expert's two products on the second stream, from the point the fork event marks."""
-        self._side.wait_event(self._fork)
-        with torch.cuda.stream(self._side):
-            out = self._shared_expert(x, batch, self._side.cuda_stream)
-            self._join.record(self._side)
+        side = self._side_in_graph if torch.cuda.is_current_stream_capturing() else self._side
+        side.wait_event(self._fork)
+        with torch.cuda.stream(side):
+            out = self._shared_expert(x, batch, side.cuda_stream)
+            self._join.record(side)
         return out
 
     def forward_add(self, x, h, batch, then_norm=None):
