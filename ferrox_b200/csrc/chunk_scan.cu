@@ -25,10 +25,12 @@
 //
 // Kernels: *_chunks make what a chunk needs (a block a chunk and head); walk_kernel goes through an entry's chunks in
 // order (a block 16 columns of a head's state).  A walk's chunk is bound by the chain of its three products and two
-// barriers, at 4 warps an SM: the block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
-// columns: 128 blocks), the next chunk's rows travel by cp.async meanwhile
-// (by untiled bulk copies, one a row, 160 a chunk: 8 us a chunk instead of 3.7).
-#include "common.cuh"
+// barriers, at 8 warps an SM: the block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
+// columns: 128 blocks).  The next chunk's rows travel meanwhile, a TMA box a tensor where the heads fill the tile and the
+// chunk is whole, else by cp.async, whose writes to shared memory cost as much of it as a fifth of the products' reads (2,048
+// tokens of 16 heads of 128: 239 us by cp.async, 215 by boxes; 3,001 of 32 heads of 64, generalized: 325 and 297; by untiled
+// bulk copies, one a row, 160 a chunk: twice as long).
+#include "tc_common.cuh"
 #include "api.h"
 
 namespace {
@@ -524,15 +526,20 @@ struct WalkArgs {
     const int *token_seq, *seq_slot;
     const int* tiles; int n_tiles;             // general: as for the chunks' kernel
     int n_tokens, H, D, V;
+    int tma;                                   // whole chunks by the boxes of WalkMaps
+    int* status;                               // raised where a wait for them runs out
 };
+// [heads][tokens][D] of W, Q, K and (general) the third's rows, a box a chunk's rows of a head
+struct WalkMaps { CUtensorMap w, q, k, a; };
 
 enum { DELTA_RULE = 1, GENERAL = 2, MLSTM = 3 };
 
-template <int D, int KIND> struct Stage {
+template <int D, int KIND> struct alignas(128) Stage {
     static constexpr bool HASW = KIND == DELTA_RULE || KIND == GENERAL;
     static constexpr int C2 = KIND == GENERAL ? 2 * CHUNK : CHUNK;      // rows that update the state
     static constexpr int PITCH = D + 4, PP = C2 + 4;
-    float w[HASW ? CHUNK * PITCH : 4], q[CHUNK * PITCH], k[C2 * D], p[CHUNK * PP];
+    // (eight lanes read a row's neighbouring pieces, so that rows without padding meet no bank twice)
+    float q[CHUNK * D], k[C2 * D], w[HASW ? CHUNK * D : 4], p[CHUNK * PP];
     float v[CHUNK * COLS], y[KIND == GENERAL ? CHUNK * COLS : 4];
     float gam[KIND == GENERAL ? D : CHUNK], e[CHUNK], fl[CHUNK];
 };
@@ -543,6 +550,8 @@ template <int D, int KIND> struct WalkSmem {
     float2 un[Stage<D, KIND>::C2 * COLS];                        // and along the columns, each twice (an FFMA pair's operand)
     float part[(WALK_THREADS / D - 1) * COLS * D];               // partial updates of the state
     float z[D], den[CHUNK];
+    uint64_t bars[2];
+    int abort;
 };
 
 // Partial sums of 4 tokens x 4 columns, spread over eight neighbouring lanes (kg), added up: lane kg gets column
@@ -568,14 +577,14 @@ __device__ __forceinline__ void over_lanes(const float (&x)[4][4], int kg, float
 // parts of the block.  (Heads of 128 x 128, a chunk: 2 x 2 tiles with the whole inner index a thread, 4 warps: 4.1 us;
 // 4 x 4 tiles, 4 warps: 3.7 us, 2,500 instructions a warp at three cycles each.)
 template <int D, int KIND>
-__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
+__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __grid_constant__ WalkMaps maps)
 {
     using St = Stage<D, KIND>;
     constexpr bool HASW = St::HASW;
     constexpr int C2 = St::C2, PITCH = St::PITCH, PP = St::PP;
     constexpr int DG = D / 4;                                    // a thread holds four keys of four columns of the state
     constexpr int PARTS = WALK_THREADS / D;                      // parts of the block, each with its share of the update's rows
-    extern __shared__ __align__(16) unsigned char raw[];
+    extern __shared__ __align__(128) unsigned char raw[];
     WalkSmem<D, KIND>& sm = *reinterpret_cast<WalkSmem<D, KIND>*>(raw);
     const int tid = threadIdx.x, b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
     fx_pdl_wait_only();
@@ -594,12 +603,32 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
             if (a.tiles[mid * 4 + 2] < b) tile0 = mid + 1; else hi = mid;
         }
     }
-    auto fetch = [&](int c0, St& st) {
+    const uint32_t bar0 = fxtc::smem_u32(sm.bars);
+    const bool tma = a.tma && fxtc::smem_u32(raw) % 128 == 0;
+    if (tid == 0) {
+        fxtc::mbar_init(bar0, 1);
+        fxtc::mbar_init(bar0 + 8, 1);
+        sm.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    auto fetch = [&](int c0, St& st, uint32_t bar) {
         const int rows = min(CHUNK, r1 - c0);
-        if (HASW) load_rows<D, WALK_THREADS>(st.w, PITCH, a.w + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
-        load_rows<D, WALK_THREADS>(st.q, PITCH, a.q + (long)c0 * a.ldq + (long)(h / a.q_share) * a.D, a.ldq, rows, a.D);
-        load_rows<D, WALK_THREADS>(st.k, D, a.k + (long)c0 * a.ldk + (long)(h / a.q_share) * a.D, a.ldk, rows, a.D);
-        if (KIND == GENERAL) load_rows<D, WALK_THREADS>(st.k + CHUNK * D, D, a.a + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
+        if (tma && rows == CHUNK) {
+            if (tid == 0) {
+                constexpr uint32_t BOX = CHUNK * D * 4;
+                const int kvh = h / a.q_share;
+                fxtc::mbar_expect_tx(bar, BOX * (2 + (HASW ? 1 : 0) + (KIND == GENERAL ? 1 : 0)));
+                fxtc::tma_load_3d(fxtc::smem_u32(st.q), &maps.q, 0, kvh, c0, bar);
+                if (HASW) fxtc::tma_load_3d(fxtc::smem_u32(st.w), &maps.w, 0, h, c0, bar);
+                fxtc::tma_load_3d(fxtc::smem_u32(st.k), &maps.k, 0, kvh, c0, bar);
+                if (KIND == GENERAL) fxtc::tma_load_3d(fxtc::smem_u32(st.k + CHUNK * D), &maps.a, 0, h, c0, bar);
+            }
+        } else {
+            if (HASW) load_rows<D, WALK_THREADS>(st.w, D, a.w + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
+            load_rows<D, WALK_THREADS>(st.q, D, a.q + (long)c0 * a.ldq + (long)(h / a.q_share) * a.D, a.ldq, rows, a.D);
+            load_rows<D, WALK_THREADS>(st.k, D, a.k + (long)c0 * a.ldk + (long)(h / a.q_share) * a.D, a.ldk, rows, a.D);
+            if (KIND == GENERAL) load_rows<D, WALK_THREADS>(st.k + CHUNK * D, D, a.a + (long)c0 * HD + (long)h * a.D, HD, rows, a.D);
+        }
         for (int i = tid; i < CHUNK * (C2 / 4); i += WALK_THREADS) {
             const int t = i / (C2 / 4), s = (i - t * (C2 / 4)) * 4;
             cp16(st.p + t * PP + s, a.p + (t < rows ? ((long)(c0 + t) * a.H + h) * C2 + s : 0), t < rows);
@@ -639,17 +668,27 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
         z = tid < a.D ? a.norm_in[((long)b * a.H + h) * a.D + tid] : 0.f;
         sm.z[tid] = z;
     }
-    fetch(r0, sm.st[0]);
+    __syncthreads();
+    fetch(r0, sm.st[0], bar0);
     // products: tokens t0 .. t0 + 3 and columns w4 .. w4 + 3, of which this lane ends up with tokens tl, tl + 1 of column c
     const int kg = tid & 7, t0 = (tid >> 7) * 16 + ((tid >> 3) & 3) * 4, w4 = ((tid >> 5) & 3) * 4;
     const int tl = t0 + 2 * (kg >> 2), c = w4 + 2 * (kg & 1) + ((kg >> 1) & 1);
     int buf = 0;
-    for (int c0 = r0; c0 < r1; c0 += CHUNK, buf ^= 1) {
+    for (int c0 = r0, chunk = 0; c0 < r1; c0 += CHUNK, ++chunk, buf ^= 1) {
         const int rows = min(CHUNK, r1 - c0);
         St& st = sm.st[buf];
+        if (tma && rows == CHUNK) fxtc::mbar_wait(bar0 + 8 * buf, (chunk >> 1) & 1, &sm.abort);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();             // this chunk's rows are there, the state is up to date, the other place is free
-        if (c0 + CHUNK < r1) fetch(c0 + CHUNK, sm.st[buf ^ 1]);
+        if (*(volatile int*)&sm.abort) {        // (the boxes waited for are the only ones in flight: once more for them)
+            if (tid == 0) {
+                int again = 0;
+                fxtc::mbar_wait(bar0 + 8 * buf, (chunk >> 1) & 1, &again);
+                if (a.status) atomicExch(a.status, fxtc::STATUS_TC_TIMEOUT);
+            }
+            return;
+        }
+        if (c0 + CHUNK < r1) fetch(c0 + CHUNK, sm.st[buf ^ 1], bar0 + 8 * (buf ^ 1));
 
         // W S_0 and Q S_0
         float xq[4][4], xw[4][4];
@@ -666,13 +705,13 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
                 for (int j = 0; j < 4; ++j) s[j] = *reinterpret_cast<const ulonglong2*>(sm.s + (w4 + j) * PITCH + d);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(st.q + (t0 + i) * PITCH + d);
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(st.q + (t0 + i) * D + d);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) { fma2(pq[i][j], q.x, s[j].x); }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) { fma2(pq[i][j], q.y, s[j].y); }
                     if (HASW) {
-                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(st.w + (t0 + i) * PITCH + d);
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(st.w + (t0 + i) * D + d);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) { fma2(pw[i][j], w.x, s[j].x); }
 #pragma unroll
@@ -708,7 +747,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
             const int t = tid >> 3;
             float acc = 0.f;
             for (int d = kg * 4; d < D; d += 32) {
-                const float4 q = *reinterpret_cast<const float4*>(st.q + t * PITCH + d);
+                const float4 q = *reinterpret_cast<const float4*>(st.q + t * D + d);
                 const float4 n = *reinterpret_cast<const float4*>(sm.z + d);
                 acc = fmaf(q.x, n.x, acc); acc = fmaf(q.y, n.y, acc); acc = fmaf(q.z, n.z, acc); acc = fmaf(q.w, n.w, acc);
             }
@@ -835,14 +874,33 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a)
         for (int i = 0; i < a.copies; ++i) a.norm[((slot * a.H + h) * a.copies + i) * a.D + tid] = z;
 }
 
-template <int D, int KIND> int go_walk(const WalkArgs& a, int n_entries, cudaStream_t s)
+// A map of rows [tokens][heads][d], `ld` floats apart, a box a chunk's rows of a head.
+bool row_map(CUtensorMap* m, const float* p, long ld, int heads, int d, int tokens)
 {
+    const fxtc::EncodeTiledFn fn = fxtc::encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)tokens};
+    cuuint64_t strides[2] = {(cuuint64_t)d * 4, (cuuint64_t)ld * 4};
+    cuuint32_t box[3] = {(cuuint32_t)d, 1, CHUNK}, steps[3] = {1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(p), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int D, int KIND> int go_walk(WalkArgs a, int n_entries, cudaStream_t s)
+{
+    // Boxes need heads as wide as the tile (a narrower head's rows would lie closer together than the kernel reads them) and
+    // as many tokens as a box has rows.  Where a map cannot be made the rows go by cp.async.
+    WalkMaps maps = {};
+    a.tma = a.D == D && a.n_tokens >= CHUNK && row_map(&maps.q, a.q, a.ldq, a.H / a.q_share, D, a.n_tokens) &&
+            row_map(&maps.k, a.k, a.ldk, a.H / a.q_share, D, a.n_tokens) &&
+            (!Stage<D, KIND>::HASW || row_map(&maps.w, a.w, (long)a.H * D, a.H, D, a.n_tokens)) &&
+            (KIND != GENERAL || row_map(&maps.a, a.a, (long)a.H * D, a.H, D, a.n_tokens));
     const int smem = (int)sizeof(WalkSmem<D, KIND>);
     static const cudaError_t set = cudaFuncSetAttribute(walk_kernel<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (set != cudaSuccess) return (int)set;
     // (not set up early: its blocks stay for the whole prompt, see fx_launch_pdl_if)
     fx_launch_pdl_if(false, walk_kernel<D, KIND>, dim3((unsigned)fx_cdiv(a.V, COLS), (unsigned)a.H, (unsigned)n_entries), WALK_THREADS,
-                     (size_t)smem, s, a);
+                     (size_t)smem, s, a, maps);
     return fx_launch_status();
 }
 
@@ -873,7 +931,7 @@ extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk,
                              const float* beta, const float* take, float q_scale, float* p, float* gam, float* e, float* wr,
                              const float* norm_in, float* norm, int copies, const float* floor_m, float* state, float* out,
                              const int* tiles, int n_tiles, const int* token_seq, const int* seq_slot, int n_tokens, int n_entries,
-                             int H, int G, int D, int V, void* stream)
+                             int H, int G, int D, int V, int* status, void* stream)
 {
     if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
     int st = check(H, G, D, V, n_entries);
@@ -893,7 +951,7 @@ extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk,
     WalkArgs a = {};
     a.w = wr; a.q = q; a.ldq = ldq; a.q_share = H / G; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.x0 = out; a.p = p; a.gam = gam; a.e = e;
     a.floor_m = floor_m; a.norm_in = norm_in; a.norm = norm; a.copies = copies; a.q_scale = q_scale; a.state = state; a.out = out;
-    a.ldo = (long)H * V; a.token_seq = token_seq; a.seq_slot = seq_slot; a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = V;
+    a.ldo = (long)H * V; a.token_seq = token_seq; a.seq_slot = seq_slot; a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = V; a.status = status;
     if (beta) return D <= 64 ? go_walk<64, DELTA_RULE>(a, n_entries, s) : go_walk<128, DELTA_RULE>(a, n_entries, s);
     return D <= 64 ? go_walk<64, MLSTM>(a, n_entries, s) : go_walk<128, MLSTM>(a, n_entries, s);
 }
@@ -905,7 +963,8 @@ extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, l
                                      long lda, const float* low, long ldl, const void* w2, int w2_dtype, const void* w0, int w0_dtype,
                                      const void* a_bias, int ab_dtype, float rate, int rank, float* p, float* gam, float* wr, float* qs,
                                      float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles,
-                                     const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, void* stream)
+                                     const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, int* status,
+                                     void* stream)
 {
     if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
     int st = check(H, H, D, D, n_entries);
@@ -926,7 +985,7 @@ extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, l
     WalkArgs a = {};
     a.w = wr; a.q = qs; a.ldq = (long)H * D; a.q_share = 1; a.k = ks; a.ldk = (long)H * D; a.a = as; a.v = v; a.ldv = ldv; a.x0 = out;
     a.p = p; a.gam = gam; a.q_scale = 1.f; a.state = state; a.out = out; a.ldo = (long)H * D; a.token_seq = token_seq; a.seq_slot = seq_slot;
-    a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles;
+    a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles; a.status = status;
     return D <= 64 ? go_walk<64, GENERAL>(a, n_entries, s) : go_walk<128, GENERAL>(a, n_entries, s);
 }
 

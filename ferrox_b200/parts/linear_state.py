@@ -33,8 +33,9 @@ with q = Wq x head_dim^(-1/2); each head's o is RMS-normed, the concatenated hea
 each head's o is RMS-normed, weighted by one vector that the heads share and gated by SiLU(Wg x).
 
 The states live in the cache manager's slots as 32-bit tensors; the recurrences, the gates and the norms are
-32-bit (``csrc/linear_state.cu``); the projections run in the engine's dtype.  Tokens of a request are taken in
-order whatever the step looks like, so a position's output does not depend on how the request was cut.
+32-bit (``csrc/linear_state.cu``, prompts in chunks of tokens: ``csrc/chunk_scan.cu``); the projections run in the
+engine's dtype.  Tokens of a request are taken in order whatever the step looks like, so a position's output does not
+depend on how the request was cut, beyond rounding.
 """
 from __future__ import annotations
 
@@ -58,7 +59,7 @@ def _chunk_tiles(batch, H, V):
     In microseconds on a B200, 16 heads of 128 x 128 (32 of 64 x 64 likewise): token by token 0.33 to 0.43 a token of the
     longest entry, and at least 0.13 a token of the step; in chunks 10 and 4.2 a chunk of the longest entry, or of all
     entries where their blocks (16 columns of a head each) need more than the device's SMs (one prompt of 64 tokens: 31
-    against 19, of 2,048: 868 against 282; 40 tokens beside 16 decoded ones: 39 against 94; four prompts of 500: 267
+    against 19, of 2,048: 868 against 258; 40 tokens beside 16 decoded ones: 39 against 94; four prompts of 500: 267
     against 289)."""
     chunk, most, T = ops.SCAN_CHUNK, batch.max_new, batch.n_tokens
     if most < chunk:
@@ -153,7 +154,7 @@ class GatedDeltaRule(_StateMixer):
         tiles = _chunk_tiles(batch, H, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
         if tiles is not None:
             ops.chunk_scan(q, k, v, g, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
-                           beta=beta, scratch=self._scratch, stream=batch.stream)
+                           beta=beta, scratch=self._scratch, status=batch.status, stream=batch.stream)
         else:
             ops.state_scan(q, k, v, g, H, beta, state, read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
                            stream=batch.stream)
@@ -272,7 +273,7 @@ class GeneralDeltaRule(_StateMixer):
         if tiles is not None:
             ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, tiles,
                                    batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, scratch=self._scratch,
-                                   stream=batch.stream)
+                                   status=batch.status, stream=batch.stream)
         else:
             u, au, w = rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32)
             ops.general_delta_prep(k, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, u, au, w, H, D,
@@ -354,7 +355,7 @@ class Mlstm(_StateMixer):
                             batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, stream=batch.stream)
             ops.chunk_scan(q, k, v, keep, matrix, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, H, D, V,
                            take=take, q_scale=float(D) ** -0.5, scratch=self._scratch, normalizer=(before, norm, floor),
-                           stream=batch.stream)
+                           status=batch.status, stream=batch.stream)
         else:
             ops.mlstm_scan(q, k, v, gates, self.i_bias, self.f_bias, s.gate_cap, float(D) ** -0.5, matrix, norm, log_max,
                            read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, V, stream=batch.stream)

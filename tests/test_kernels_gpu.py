@@ -1239,7 +1239,7 @@ def scan_scratch(*shape):
 
 # (entries' lengths, heads, key heads, D, V)
 SCANS = [([1], 2, 1, 64, 16), ([31, 32, 33], 4, 2, 128, 128), ([100], 3, 3, 20, 36), ([65, 1, 64], 2, 2, 68, 4),
-         ([200, 7], 2, 1, 128, 100)]
+         ([200, 7], 2, 1, 128, 100), ([64, 5, 97], 4, 2, 64, 48)]
 
 
 @pytest.mark.parametrize("case", SCANS)
