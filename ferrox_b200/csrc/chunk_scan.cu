@@ -27,9 +27,9 @@
 // order (a block 16 columns of a head's state).  A walk's chunk is bound by the chain of its three products and two
 // barriers, at 8 warps an SM: the block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
 // columns: 128 blocks).  The next chunk's rows travel meanwhile, a TMA box a tensor where the heads fill the tile and the
-// chunk is whole, else by cp.async, whose writes to shared memory cost as much of it as a fifth of the products' reads (2,048
-// tokens of 16 heads of 128: 239 us by cp.async, 215 by boxes; 3,001 of 32 heads of 64, generalized: 325 and 297; by untiled
-// bulk copies, one a row, 160 a chunk: twice as long).
+// chunk is whole, else by cp.async, whose writes take 1,500 of a chunk's 7,800 cycles of shared memory (2,048 tokens of 16
+// heads of 128: 239 us by cp.async, 215 by boxes; 3,001 of 32 heads of 64, generalized: 325 and 297; by untiled bulk copies,
+// one a row, 160 a chunk: twice as long).
 #include "tc_common.cuh"
 #include "api.h"
 

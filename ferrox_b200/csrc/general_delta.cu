@@ -16,7 +16,7 @@
 //   w = exp(-rate * sigmoid(W2 tanh(w1_out) + w0)),  a = sigmoid(a_pre + a_bias).
 // fx_general_delta_scan runs the recurrence: grid (entries, heads, column groups), 128 threads; the tokens' rows
 // (r, k, u, a u, w and the values of the block's columns) travel into shared memory eight tokens at a time by
-// cp.async, the next chunk while this one is worked on.
+// cp.async, the next chunk while this one is worked on.  (Prompts: chunk_scan.cu, which also makes u, a u and w.)
 #include "common.cuh"
 #include "api.h"
 

@@ -12,7 +12,8 @@
 // Kernels: fx_delta_prep (short causal convolution + SiLU of the projected q, k, v rows with the convolution's tail
 // from the state slot, unit length per head, the gates beta and g), fx_conv_tail_update (the last taps - 1 inputs of
 // every request of the step become its new tail), fx_state_scan (the recurrences above), fx_gated_group_norm (RMS
-// norm over groups of the read-out, times a weight, times an activation of a gate row).
+// norm over groups of the read-out, times a weight, times an activation of a gate row).  Prompts through the delta rule go in
+// chunks of tokens instead (chunk_scan.cu).
 //
 // A step's tokens are flat rows sorted by entry (token_seq ascending); an entry's rows are found by binary search.
 #include "common.cuh"

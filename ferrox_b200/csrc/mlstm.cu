@@ -1,4 +1,4 @@
-// The matrix memory of an mLSTM mixer: per (request, head) a state S [dim, vdim], a normaliser n [dim] and the
+// The matrix memory of an mLSTM mixer, for decoding and short portions (prompts: chunk_scan.cu): per (request, head) a state S [dim, vdim], a normaliser n [dim] and the
 // running maximum m of the gates' logarithms,
 //
 //   i_t = cap tanh((i~_t + b_i) / cap)                     log input gate
