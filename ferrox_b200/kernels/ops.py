@@ -253,20 +253,26 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+_beside_step = False     # inside a scope within a step's own: work that runs on another stream beside the step
+
+
 class stream_scope:
-    """While a step runs, its stream is known: asking torch for the current stream costs more than a launch."""
+    """While a step runs, its stream is known: asking torch for the current stream costs more than a launch.  A scope inside
+    another is a part of the step on a stream of its own."""
 
     def __init__(self, ptr: int):
         self.ptr = ptr
 
     def __enter__(self):
-        global _scoped_stream
-        self.prev, _scoped_stream = _scoped_stream, self.ptr
+        global _scoped_stream, _beside_step
+        self.prev, self.prev_beside = _scoped_stream, _beside_step
+        _beside_step = _beside_step or _scoped_stream is not None
+        _scoped_stream = self.ptr
         return self
 
     def __exit__(self, *exc):
-        global _scoped_stream
-        _scoped_stream = self.prev
+        global _scoped_stream, _beside_step
+        _scoped_stream, _beside_step = self.prev, self.prev_beside
         return False
 
 
@@ -295,11 +301,21 @@ def _rows(t: torch.Tensor) -> int:
 def upload(values, device) -> torch.Tensor:
     """A numpy array's copy on ``device``, ordered on the current stream without waiting for it: by way of pinned memory,
     which torch's allocator hands out again only when the copy is done.  (A pageable copy waits for everything the
-    stream holds: the host then prepares a step while the device stands still, 0.3 ms of every prompt.)"""
+    stream holds: the host then prepares a step while the device stands still, 0.3 ms of every prompt.)
+
+    On a stream beside the step's own it does wait: what a step uploads is shared by its parts, and one that finds it on
+    another stream is not ordered behind this one's copy."""
     t = torch.from_numpy(values)
     device = torch.device(device)
     if device.type != "cuda" or t.numel() == 0:
         return t.to(device)
+    out = _copied_behind(t, device)
+    if _beside_step:
+        torch.cuda.current_stream(device).synchronize()
+    return out
+
+
+def _copied_behind(t: torch.Tensor, device) -> torch.Tensor:
     return t.pin_memory().to(device, non_blocking=True)
 
 

@@ -111,3 +111,33 @@ def test_prompt_attention_items_cover_every_key_block_once():
     # forced runs of four key blocks
     items, merges, parts = ops.prefill_tc_plan([(2048, 0)], None, 16, sms=148, run_blocks=4)
     assert len(items) == 20 and max(int(it[5] - it[4]) for it in items) == 4 and len(merges) == 6
+
+
+def test_uploads_on_a_stream_beside_the_step_are_complete_when_they_return(monkeypatch):
+    """A work list that a mixer beside the step's stream uploads is found by the others in ``batch.shared``, on streams that do
+    not wait for that one: there the upload waits for its copy.  On the step's own stream it does not."""
+    import numpy as np
+    import torch
+
+    waits = []
+
+    class Stream:
+        def synchronize(self):
+            waits.append("copied" if copied else "too early")
+
+    copied = []
+    monkeypatch.setattr(ops, "_copied_behind", lambda t, device: copied.append(t) or t)      # (no device here)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    values = np.arange(4, dtype=np.int32)
+    ops.upload(values, "cuda:0")
+    with ops.stream_scope(11):
+        ops.upload(values, "cuda:0")
+        assert not waits
+        with ops.stream_scope(22):
+            ops.upload(values, "cuda:0")
+            with ops.stream_scope(11):
+                ops.upload(values, "cuda:0")
+        assert waits == ["copied", "copied"]
+        ops.upload(values, "cuda:0")
+    ops.upload(values, "cuda:0")
+    assert len(waits) == 2
