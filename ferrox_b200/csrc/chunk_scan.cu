@@ -499,9 +499,11 @@ __global__ void __launch_bounds__(32) mlstm_gates_kernel(const float* __restrict
         if (lane == 0) before = m;
         if (t < r1) {
             const long at = (long)t * H + h;
-            // (rounding may leave f + before a last place above the maximum that it is one of)
-            keep[at] = expf(fminf(gf + before - after, 0.f));
-            take[at] = expf(fminf(gi - after, 0.f));
+            // (rounding may leave f + before a last place above the maximum that it is one of; what is no number stays none,
+            // though the maxima pass over it)
+            const float dk = gf + before - after, dt = gi - after;
+            keep[at] = expf(dk > 0.f ? 0.f : dk);
+            take[at] = expf(dt > 0.f ? 0.f : dt);
             floor_out[at] = expf(-after);
         }
         m = __shfl_sync(0xffffffffu, after, min(31, r1 - 1 - c0));

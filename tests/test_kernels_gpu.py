@@ -1324,6 +1324,38 @@ def test_chunk_scan(case, kind):
     assert torch.equal(out[keep], got[0][keep]) and bool(out[t].isnan().any())
 
 
+@pytest.mark.parametrize("gate", [0, 1])
+def test_mlstm_gate_that_is_no_number(gate):
+    """A head's input or forget gate that is not a number: its read-outs and states are not from that token on, as token by
+    token; the tokens before it, the other head and the other request keep theirs."""
+    o = ops()
+    lens, H, D, V, cap = [70, 40], 2, 64, 32, 15.0
+    T, (seq, slot, tiles) = sum(lens), scan_setup(lens, 0)
+    q, k, v, gates = rnd(T, H * D, seed=1), rnd(T, H * D, seed=2), rnd(T, H * V, seed=3), rnd(T, 2 * H, seed=4)
+    ib, fb, copies = rnd(H, seed=5), rnd(H, seed=6) + 2, o.mlstm_column_blocks(D, V)
+    gates[45, gate * H + 1] = float("nan")
+
+    def run(chunked):
+        st, out = torch.zeros(4, H, V, D, device=DEV), torch.empty(T, H * V, device=DEV)
+        nm, mx = torch.zeros(4, H, copies, D, device=DEV), torch.zeros(4, H, copies, device=DEV)
+        if chunked:
+            keep, take, floor = (torch.empty(T, H, device=DEV) for _ in range(3))
+            before = torch.empty(2, H, D, device=DEV)
+            o.mlstm_gates(gates, ib, fb, cap, mx, nm, before, keep, take, floor, seq, slot, 2, H, D)
+            o.chunk_scan(q, k, v, keep, st, out, tiles, seq, slot, 2, H, H, D, V, take=take, q_scale=D ** -0.5,
+                         scratch=scan_scratch, normalizer=(before, nm, floor))
+        else:
+            o.mlstm_scan(q, k, v, gates, ib, fb, cap, D ** -0.5, st, nm, mx, out, seq, slot, 2, H, D, V)
+        return [t.isnan() for t in (out, st, nm)]
+
+    got, old = run(True), run(False)
+    want = torch.zeros(T, H, V, dtype=torch.bool, device=DEV)
+    want[45:70, 1] = True
+    assert torch.equal(old[0].view(T, H, V), want)
+    for a, b in zip(got, old):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("lens,H,D,rank", [([1], 2, 64, 64), ([31, 32, 33], 3, 64, 8), ([100, 5], 2, 20, 3), ([65], 2, 128, 96),
                                            ([130, 1, 64], 1, 100, 65)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
