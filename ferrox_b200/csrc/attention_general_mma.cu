@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(128 * NSPLIT) general_attention_kernel(GArgs a
     }
     // A thread copies pieces t, t + NTHREADS, ... of a block's rows: the row and the place in it move on by the same steps
     // each time, so that no quotient is taken in the loop; where a block of keys lies in one page, one look at the table
-    // serves all of it.  (With quotients in the loop, one look a piece and tanhf below, 198 us for 1,531 tokens with 32 query
-    // rows of 64 a token.)
+    // serves all of it.
     const bool one_page = a.page_size % BKEY == 0;
     const int k_r0 = threadIdx.x / kchunks, k_c0 = threadIdx.x - k_r0 * kchunks;
     const int k_dr = NTHREADS / kchunks, k_dc = NTHREADS - k_dr * kchunks;
@@ -272,14 +271,14 @@ __global__ void __launch_bounds__(128 * NSPLIT) general_attention_kernel(GArgs a
             const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
             // a row that sees no key yet keeps m = -inf: use 0 as the reference so that exp2 stays finite
             const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
-            const float al0 = m0 == -INFINITY ? 0.f : fx_ex2(m0 - ref0);
-            const float al1 = m1 == -INFINITY ? 0.f : fx_ex2(m1 - ref1);
+            const float al0 = m0 == -INFINITY ? 0.f : exp2f(m0 - ref0);
+            const float al1 = m1 == -INFINITY ? 0.f : exp2f(m1 - ref1);
             float sum0 = 0.f, sum1 = 0.f;
             uint32_t p[BKEY / 8][2];
 #pragma unroll
             for (int j = 0; j < BKEY / 8; ++j) {
-                const float e0 = fx_ex2(s[j][0] - ref0), e1 = fx_ex2(s[j][1] - ref0);
-                const float e2 = fx_ex2(s[j][2] - ref1), e3 = fx_ex2(s[j][3] - ref1);
+                const float e0 = exp2f(s[j][0] - ref0), e1 = exp2f(s[j][1] - ref0);
+                const float e2 = exp2f(s[j][2] - ref1), e3 = exp2f(s[j][3] - ref1);
                 sum0 += e0 + e1; sum1 += e2 + e3;
                 p[j][0] = pack_bf16(e0, e1);
                 p[j][1] = pack_bf16(e2, e3);
@@ -334,8 +333,8 @@ __global__ void __launch_bounds__(128 * NSPLIT) general_attention_kernel(GArgs a
         // the head's sink in the denominator, once: sums and maximum brought to the larger of the two references
         const float k0 = a.sinks[head0 + min(r0, rows - 1) % n_h] * 1.4426950408889634f;
         const float k1 = a.sinks[head0 + min(r1, rows - 1) % n_h] * 1.4426950408889634f;
-        if (l0 > 0.f) { const float mm = fmaxf(m0, k0), f = fx_ex2(m0 - mm); inv0 = f / (l0 * f + fx_ex2(k0 - mm)); }
-        if (l1 > 0.f) { const float mm = fmaxf(m1, k1), f = fx_ex2(m1 - mm); inv1 = f / (l1 * f + fx_ex2(k1 - mm)); }
+        if (l0 > 0.f) { const float mm = fmaxf(m0, k0), f = exp2f(m0 - mm); inv0 = f / (l0 * f + exp2f(k0 - mm)); }
+        if (l1 > 0.f) { const float mm = fmaxf(m1, k1), f = exp2f(m1 - mm); inv1 = f / (l1 * f + exp2f(k1 - mm)); }
     }
     const bf16* g0 = a.gate ? a.gate + (long)(tok0 + min(r0, rows - 1) / n_h) * a.ldg + (long)(head0 + min(r0, rows - 1) % n_h) * a.value_dim + col0 : nullptr;
     const bf16* g1 = a.gate ? a.gate + (long)(tok0 + min(r1, rows - 1) / n_h) * a.ldg + (long)(head0 + min(r1, rows - 1) % n_h) * a.value_dim + col0 : nullptr;
@@ -381,7 +380,7 @@ __global__ void general_merge_kernel(const float* __restrict__ part_o, const flo
     if (sinks && mm != -INFINITY) {
         const float sk = sinks[h] * 1.4426950408889634f;
         mm = fmaxf(mm, sk);
-        sunk = fx_ex2(sk - mm);
+        sunk = exp2f(sk - mm);
     }
     for (int e0 = 0; e0 < value_dim; e0 += blockDim.x) {      // (every lane takes every trip: partners of a pair meet)
         const int e = e0 + threadIdx.x;
@@ -391,7 +390,7 @@ __global__ void general_merge_kernel(const float* __restrict__ part_o, const flo
             if (!has_keys(s)) continue;
             const float ms = part_ml[(base + s) * 2];
             if (ms == -INFINITY) continue;
-            const float w = fx_ex2(ms - mm);
+            const float w = exp2f(ms - mm);
             ll += part_ml[(base + s) * 2 + 1] * w;
             acc += part_o[(base + s) * value_dim + e] * w;
         }

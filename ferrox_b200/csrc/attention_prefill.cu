@@ -208,14 +208,14 @@ __global__ void __launch_bounds__(NTHREADS) prefill_attention_kernel(
             const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
             // a row that sees no key yet keeps m = -inf: use 0 as the reference so that exp2 stays finite
             const float ref0 = mn0 == -INFINITY ? 0.f : mn0 * scale_log2e, ref1 = mn1 == -INFINITY ? 0.f : mn1 * scale_log2e;
-            const float al0 = m0 == -INFINITY ? 0.f : fx_ex2(m0 * scale_log2e - ref0);
-            const float al1 = m1 == -INFINITY ? 0.f : fx_ex2(m1 * scale_log2e - ref1);
+            const float al0 = m0 == -INFINITY ? 0.f : exp2f(m0 * scale_log2e - ref0);
+            const float al1 = m1 == -INFINITY ? 0.f : exp2f(m1 * scale_log2e - ref1);
             float sum0 = 0.f, sum1 = 0.f;
             uint32_t p[BKEY / 8][2];
 #pragma unroll
             for (int j = 0; j < BKEY / 8; ++j) {
-                const float e0 = fx_ex2(s[j][0] * scale_log2e - ref0), e1 = fx_ex2(s[j][1] * scale_log2e - ref0);
-                const float e2 = fx_ex2(s[j][2] * scale_log2e - ref1), e3 = fx_ex2(s[j][3] * scale_log2e - ref1);
+                const float e0 = exp2f(s[j][0] * scale_log2e - ref0), e1 = exp2f(s[j][1] * scale_log2e - ref0);
+                const float e2 = exp2f(s[j][2] * scale_log2e - ref1), e3 = exp2f(s[j][3] * scale_log2e - ref1);
                 sum0 += e0 + e1; sum1 += e2 + e3;
                 p[j][0] = pack_bf16(e0, e1);
                 p[j][1] = pack_bf16(e2, e3);

@@ -899,6 +899,40 @@ def test_prefill_attention_tiles(case):
         assert rel(out[i].float().cpu().reshape(nh, d), want) < 1.5e-2, (i, s, pos)
 
 
+def mma_attention(kernel, q, kp, vp, table, page, portions, nh, nkv, window=0, scale=1.0, **options):
+    """The mma.sync prompt attention ("prefill") or that of the general form ("general", options as it takes them) over
+    portions of (slot, first position, tokens); q [tokens, nh * d] bfloat16."""
+    o = ops()
+    as_int = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    d, dv = kp.shape[-1], vp.shape[-1]
+    out = torch.full((q.shape[0], nh * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
+    slots = as_int([s for s, _, _ in portions])
+    if kernel == "prefill":
+        tiles, flat = [], 0
+        for b, (_, start, n) in enumerate(portions):
+            tiles += [(flat + i, min(64, n - i), b, start + i) for i in range(0, n, 64)]
+            flat += n
+        return o.prefill_attention(q, kp, vp, table, page, as_int(tiles), slots, out, nh, nkv, d, window, scale, **options)
+    positions = as_int([p for _, start, n in portions for p in range(start, start + n)])
+    seq = as_int([b for b, (_, _, n) in enumerate(portions) for _ in range(n)])
+    items = torch.from_numpy(o.general_attention_items([n for _, _, n in portions], nh, nkv)).to(DEV)
+    return o.general_attention(q, q.stride(0), d, kp, vp, d, dv, table, page, positions, seq, slots, items, out, nh * dv, dv,
+                               nh, nkv, d, dv, window, scale, **options)
+
+
+@pytest.mark.parametrize("kernel", ["prefill", "general"])
+def test_prompt_attention_on_mma_keeps_32_bit_scores_and_weights(kernel):
+    """A weight below the smallest normal number still counts (it is rounded to 16 bits: 2^-130 to three bits)."""
+    lens, nh, nkv, d, page = [70], 2, 1, 64, 32
+    kp, vp, table, ks, vs = build_cache(torch.bfloat16, lens, nkv, d, page, n_pages=4)
+    run = lambda q, kp, vp, **kw: mma_attention(kernel, q, kp, vp, table, page, [(1, 0, q.shape[0])], nh, nkv, **kw)
+    q, kp, vp = torch.zeros(2, nh * d, dtype=torch.bfloat16, device=DEV), torch.zeros_like(kp), torch.zeros_like(vp)
+    first = int(table[1, 0])
+    q[:, ::d], kp[first, 0, 1, 0], vp[first, 0, 1] = 1.0, -90.0, 1e38
+    got, want = run(q, kp, vp).double(), math.exp(-90.0) * float(vp[first, 0, 1, 0])
+    assert bool((got[0] == 0).all()) and bool(((got[1] - want).abs() < want / 8).all())
+
+
 TC_ATT_CASES = [
     # nh, nkv, d, page, window, lengths
     (16, 16, 128, 64, 0, [300, 64, 65]),
