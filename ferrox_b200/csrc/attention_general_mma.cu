@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128 * NSPLIT) general_attention_kernel(GArgs a
 #pragma unroll
                 for (int j = 0; j < BKEY / 8; ++j) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) s[j][e] = back * fx_tanh_fast(s[j][e] * a.scale_over_cap);
+                    for (int e = 0; e < 4; ++e) s[j][e] = back * tanhf(s[j][e] * a.scale_over_cap);
                 }
             }
             // (most blocks are seen whole by all of the warp's rows)

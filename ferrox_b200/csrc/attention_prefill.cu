@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(NTHREADS) prefill_attention_kernel(
 #pragma unroll
                 for (int j = 0; j < BKEY / 8; ++j)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) s[j][e] = cap * fx_tanh_fast(s[j][e] * cap_mul);
+                    for (int e = 0; e < 4; ++e) s[j][e] = cap * tanhf(s[j][e] * cap_mul);
             }
             // ---- mask by absolute position, online softmax ---------------------------
             const int lo0 = window > 0 ? p_row0 - window + 1 : 0, lo1 = window > 0 ? p_row1 - window + 1 : 0;

@@ -148,21 +148,6 @@ __device__ __forceinline__ void fx_gate_32(float* x, const uint32_t* u, int act,
     }
 }
 
-// 2^x by the hardware's unit alone (2 units in the last place; results below 2^-126 become 0).
-__device__ __forceinline__ float fx_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// tanh(x) = 1 - 2 / (e^2x + 1) with the hardware's exponential and quotient, for scores whose softmax weights are rounded
-// to 16 bits: within 3e-7 of tanh(x), that is 1e-5 of a weight at a cap of 30, a two hundredth of that rounding.  (tanhf is
-// some 25 instructions with a branch; a block of 64 keys asks a thread for 32 of them.)  Right at both ends: the quotient
-// is 0 for e^2x beyond range and 2 for 0.
-__device__ __forceinline__ float fx_tanh_fast(float x) {
-    return 1.0f + __fdividef(-2.0f, fx_ex2(x * 2.8853900817779268f) + 1.0f);
-}
-
 // log(1 + e^x) = max(x, 0) + log(1 + e) with e = e^-|x| in (0, 1]; log(1 + e) = 2 artanh(s), s = e / (2 + e) <= 1/3, by
 // its series 2 (s + s^3/3 + s^5/5 + ...), the first term left out below 2e-8 of the sum.
 __device__ __forceinline__ float fx_softplus(float x)

@@ -922,10 +922,16 @@ def mma_attention(kernel, q, kp, vp, table, page, portions, nh, nkv, window=0, s
 
 @pytest.mark.parametrize("kernel", ["prefill", "general"])
 def test_prompt_attention_on_mma_keeps_32_bit_scores_and_weights(kernel):
-    """A weight below the smallest normal number still counts (it is rounded to 16 bits: 2^-130 to three bits)."""
+    """A cap far above the scores leaves them as they are (a tanh whose error is absolute would not: 3e-7 of 1e7), and a weight
+    below the smallest normal number still counts (it is rounded to 16 bits: 2^-130 to three bits)."""
     lens, nh, nkv, d, page = [70], 2, 1, 64, 32
     kp, vp, table, ks, vs = build_cache(torch.bfloat16, lens, nkv, d, page, n_pages=4)
+    q = rnd(70, nh * d, dtype=torch.bfloat16)
     run = lambda q, kp, vp, **kw: mma_attention(kernel, q, kp, vp, table, page, [(1, 0, q.shape[0])], nh, nkv, **kw)
+    out = run(q, kp, vp, scale=d ** -0.5, softcap=1e7)
+    for t in range(70):
+        want = plain_attention(q[t].float().cpu().view(nh, d), ks[0], vs[0], t, 0, d ** -0.5)
+        assert rel(out[t].float().cpu().view(nh, d), want) < 1.5e-2, t
     q, kp, vp = torch.zeros(2, nh * d, dtype=torch.bfloat16, device=DEV), torch.zeros_like(kp), torch.zeros_like(vp)
     first = int(table[1, 0])
     q[:, ::d], kp[first, 0, 1, 0], vp[first, 0, 1] = 1.0, -90.0, 1e38
