@@ -496,7 +496,8 @@ __global__ void __launch_bounds__(128) gated_group_norm_warp_kernel(
 // thread holds GN_CH pieces whatever the width: one group of up to GN_CH pieces a thread, or, where a group is one piece a
 // thread (64 elements on half a warp, 128 on a warp), GN_CH groups side by side.  (3,001 tokens of 32 groups of 64, gate in 32
 // bits: a group a warp, half of its lanes idle and every weight a load of its own, 34.6 us; so 17.5.  2,048 tokens of 16
-// groups of 128: 13.0 and 12.3.)
+// groups of 128: 13.0 and 12.3.)  16-bit results take the sigmoid by the hardware's quotient, but not those of groups below 64,
+// which never did.
 constexpr int GN_CH = 4;      // pieces a thread holds at most
 
 template <typename GT> __device__ __forceinline__ void load_gate4(const GT* p, float* g);
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(
         for (int e = 0; e < 4; ++e) {
             const float gv = g[c][e];
             r[e] = v[c][e] * inv[c / PIECES] * r[e];
-            if (sizeof(OT) == 2) r[e] *= act ? fx_sigmoid_fast(gv) : gv * fx_sigmoid_fast(gv);
+            if (sizeof(OT) == 2 && width >= 64) r[e] *= act ? fx_sigmoid_fast(gv) : gv * fx_sigmoid_fast(gv);
             else r[e] *= act ? sigmoid_f(gv) : silu_f(gv);
         }
         OT* o = out + at * width;

@@ -1505,6 +1505,19 @@ def test_gated_group_norm_over_its_forms(width, gate_dtype, out_dtype):
             assert ((out.double() - want).abs() <= tol * want.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("width", [4, 32, 60])
+def test_gated_group_norm_of_narrow_groups_takes_gates_that_hardly_open(width):
+    """sigmoid(-88) is below the smallest normal number, and with large weights it still counts (the quotient of the hardware
+    alone answers 0 where its divisor passes 2^126)."""
+    x, w = torch.ones(3, 2 * width, device="cuda"), torch.full((2 * width,), 1e30, device="cuda")
+    gate = torch.full((3, 2 * width), -88.0, device="cuda")
+    for act in ("silu", "sigmoid"):
+        out = torch.empty(3, 2 * width, device="cuda", dtype=torch.bfloat16)
+        ops().gated_group_norm(x, gate, w, 1e-5, act, out, 2, width)
+        want = 1e30 / (1.0 + math.exp(88.0)) * (-88.0 if act == "silu" else 1.0)
+        assert ((out.double() - want).abs() < 2.0 ** -7 * abs(want)).all()
+
+
 def test_a_slot_of_every_state_is_zeroed_and_no_other():
     from ferrox_b200.kernels.ops import SlotZeroer
 
