@@ -22,6 +22,11 @@
 //
 // Everything is 32-bit FFMA arithmetic; products of decays are taken in 64 bits and rounded once, because one of a
 // chunk's is raised to the power of the chunks that a memory travels through.  State [slots, H, V, D], as before.
+// Error against a 64-bit evaluation, as a multiple of that of the kernels that take the tokens one by one (read-outs and
+// states; seven shapes, twelve seeds): delta 0.99 and 0.89, general 0.87 and 0.72, mLSTM's states 0.97.  It takes short chains
+// in the products of a chunk's rows (in one chain of pairs a row: 1.14 for delta, 1.16 for general), a token's product with
+// itself from the rows as they are, decays after a token as products of their own instead of G_C / G_t, a chunk's sum made
+// before the state is added to it, and the mLSTM's maxima in 64 bits (states 1.1).
 //
 // Kernels: *_chunks make what a chunk needs (a block a chunk and head); walk_kernel goes through an entry's chunks in
 // order (a block 16 columns of a head's state).  A walk's chunk is bound by the chain of its three products and two
@@ -43,6 +48,16 @@ typedef unsigned long long u64;
 
 __device__ __forceinline__ void fma2(u64& d, u64 a, u64 b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ u64 fma2_of(u64 a, u64 b, u64 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 __device__ __forceinline__ u64 pair(float x, float y) {
     return (u64)__float_as_uint(x) | ((u64)__float_as_uint(y) << 32);
@@ -123,10 +138,45 @@ __device__ __forceinline__ float decay_product(const double (*win)[CHUNK], int t
     return (float)r;
 }
 
-template <int D, bool DELTA>
-__global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
+// One product of two rows as N chains of pairs: what a chunk's tokens are to each other enters every later sum whole.
+template <int N> struct Sums {
+    u64 c[N];
+    __device__ __forceinline__ Sums() {
+#pragma unroll
+        for (int n = 0; n < N; ++n) c[n] = 0ull;
+    }
+    __device__ __forceinline__ void add(int n, const ulonglong2& a, const ulonglong2& b) { fma2(c[n], a.x, b.x); fma2(c[n + 1], a.y, b.y); }
+    __device__ __forceinline__ float sum() const {
+        float s[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) s[n] = sum_of(c[n]);
+#pragma unroll
+        for (int w = N / 2; w > 0; w >>= 1)
+#pragma unroll
+            for (int n = 0; n < w; ++n) s[n] += s[n + w];
+        return s[0];
+    }
+};
+
+// sum of l[s] x[s] over the tokens s < t (t known when compiled: x stays in registers)
+__device__ __forceinline__ float before(const float* l, const float (&x)[CHUNK], int t)
 {
-    constexpr int PITCH = D + 4, LP = CHUNK + 4;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int s = 0; s < t; s += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(l + s);
+        s0 = fmaf(a.x, x[s], s0);
+        if (s + 1 < t) s1 = fmaf(a.y, x[s + 1], s1);
+        if (s + 2 < t) s0 = fmaf(a.z, x[s + 2], s0);
+        if (s + 3 < t) s1 = fmaf(a.w, x[s + 3], s1);
+    }
+    return s0 + s1;
+}
+
+template <int D, bool DELTA>
+__global__ void __launch_bounds__(PREP_THREADS, 2) scalar_chunks(ChunkArgs a)
+{
+    constexpr int PITCH = D + 4, LP = CHUNK + 4, CHAINS = 4;
     extern __shared__ __align__(16) float sm[];
     float* k_s = sm;                                  // [CHUNK][PITCH]
     float* q_s = k_s + CHUNK * PITCH;
@@ -158,23 +208,27 @@ __global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
 
     // thread (ty, tx): tokens t = ty, ty + 16 against s = tx, tx + 16
     const int ty = tid >> 4, tx = tid & 15;
-    u64 qk[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, kk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
-#pragma unroll 4
-    for (int d = 0; d < D; d += 4) {
-        ulonglong2 ks[2], qt[2], kt[2];
+    Sums<CHAINS> qk[2][2], kk[2][2];
+#pragma unroll 2
+    for (int d0 = 0; d0 < D; d0 += 2 * CHAINS) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
-            qt[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * PITCH + d);
-            if (DELTA) kt[i] = *reinterpret_cast<const ulonglong2*>(k_s + (ty + 16 * i) * PITCH + d);
-        }
+        for (int n = 0; n < CHAINS; n += 2) {
+            const int d = d0 + 2 * n;
+            ulonglong2 ks[2], qt[2], kt[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                fma2(qk[i][j], qt[i].x, ks[j].x); fma2(qk[i][j], qt[i].y, ks[j].y);
-                if (DELTA) { fma2(kk[i][j], kt[i].x, ks[j].x); fma2(kk[i][j], kt[i].y, ks[j].y); }
+            for (int i = 0; i < 2; ++i) {
+                ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
+                qt[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * PITCH + d);
+                if (DELTA) kt[i] = *reinterpret_cast<const ulonglong2*>(k_s + (ty + 16 * i) * PITCH + d);
             }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    qk[i][j].add(n, qt[i], ks[j]);
+                    if (DELTA) kk[i][j].add(n, kt[i], ks[j]);
+                }
+        }
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -182,10 +236,10 @@ __global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
         for (int j = 0; j < 2; ++j) {
             const int t = ty + 16 * i, s = tx + 16 * j;
             const float r = s < t ? decay_product(win, t, t - s) : 1.f;
-            if (DELTA) l_s[t * LP + s] = s < t ? gate_s[t] * (r * sum_of(kk[i][j])) : 0.f;
+            if (DELTA) l_s[t * LP + s] = s < t ? gate_s[t] * (r * kk[i][j].sum()) : 0.f;
             if (t < rows)
                 a.p[((long)(tok0 + t) * a.H + h) * CHUNK + s] =
-                    s <= t ? r * sum_of(qk[i][j]) * (DELTA ? 1.f : a.scale * gate_s[s]) : 0.f;
+                    s <= t ? r * qk[i][j].sum() * (DELTA ? 1.f : a.scale * gate_s[s]) : 0.f;
         }
     if (tid < rows) {
         a.gam[(long)(tok0 + tid) * a.H + h] = gam[tid];
@@ -208,16 +262,7 @@ __global__ void __launch_bounds__(PREP_THREADS) scalar_chunks(ChunkArgs a)
         for (int t = 0; t < CHUNK; ++t) x[t] *= gate_s[t];
 #pragma unroll
         for (int t = 1; t < CHUNK; ++t) {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int s = 0; s < t; s += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(l_s + t * LP + s);     // (zeros from t on)
-                s0 = fmaf(l.x, x[s], s0);
-                if (s + 1 < t) s1 = fmaf(l.y, x[s + 1], s1);
-                if (s + 2 < t) s0 = fmaf(l.z, x[s + 2], s0);
-                if (s + 3 < t) s1 = fmaf(l.w, x[s + 3], s1);
-            }
-            x[t] -= s0 + s1;
+            x[t] -= before(l_s + t * LP, x, t);
         }
         float* to = val ? a.x0 + ((long)tok0 * a.H + h) * a.V + c : a.wr + ((long)tok0 * a.H + h) * a.D + (c - a.V);
         const long ld = (long)a.H * (val ? a.V : a.D);
@@ -236,9 +281,9 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf
 // memory for 32 tokens, and u, a u and w never go to memory.  (The kernel that makes them for the token-by-token form,
 // eight tokens a block, took 249 us for 3,001 tokens of 32 heads of 64.)
 template <int D>
-__global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
+__global__ void __launch_bounds__(PREP_THREADS, D <= 64 ? 2 : 1) general_chunks(ChunkArgs a)
 {
-    constexpr int PITCH = D + 4, LP = CHUNK + 4, RP = RANK + 4;
+    constexpr int PITCH = D + 4, LP = CHUNK + 4, RP = RANK + 4, CHAINS = D <= 64 ? 2 : 4;
     extern __shared__ __align__(16) float sm[];
     float* u_s = sm;                                  // [CHUNK][PITCH] each
     float* r_s = u_s + CHUNK * PITCH;
@@ -249,7 +294,8 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
     float* B_s = A_s + CHUNK * LP;
     float* w2_s = B_s + CHUNK * LP;                   // [D][RP]
     float* th_s = w2_s + D * RP;                      // [CHUNK][RP]
-    __shared__ float len_s[CHUNK];
+    float* e_s = w2_s;                                // (when W2 has been read) products of the decays after each token
+    __shared__ float len_s[CHUNK], rk_s[CHUNK], ra_s[CHUNK];
     fx_pdl_wait();
     const int4 tile = reinterpret_cast<const int4*>(a.tiles)[blockIdx.x];
     const int tok0 = tile.x, rows = tile.y, h = blockIdx.y, tid = threadIdx.x;
@@ -349,73 +395,94 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
             g_s[t * PITCH + d] = expf(-a.rate * sigmoid_f(sum_of(zacc[i][j]) + load_any(a.w0, a.w0_dtype, c)));
         }
     __syncthreads();
-    // a channel's products: runs of RUN tokens a thread, then the runs before it
+    {
+        // what a token reads of itself, from the rows as they are: in most read-outs the largest term
+        const int t = tid >> 3;
+        float rk = 0.f, ra = 0.f;
+        for (int d = (tid & 7) * 4; d < D; d += 32) {
+            const float4 r = *reinterpret_cast<const float4*>(r_s + t * PITCH + d), k = *reinterpret_cast<const float4*>(k_s + t * PITCH + d);
+            const float4 x = *reinterpret_cast<const float4*>(a_s + t * PITCH + d);
+            rk = fmaf(r.x, k.x, rk); rk = fmaf(r.y, k.y, rk); rk = fmaf(r.z, k.z, rk); rk = fmaf(r.w, k.w, rk);
+            ra = fmaf(r.x, x.x, ra); ra = fmaf(r.y, x.y, ra); ra = fmaf(r.z, x.z, ra); ra = fmaf(r.w, x.w, ra);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) { rk += __shfl_xor_sync(0xffffffffu, rk, o); ra += __shfl_xor_sync(0xffffffffu, ra, o); }
+        if ((tid & 7) == 0) { rk_s[t] = rk; ra_s[t] = ra; }
+    }
+    // a channel's products of decays up to each token and after it: runs of RUN tokens a thread, then the runs on either side
     constexpr int RUNS = PREP_THREADS / D, RUN = CHUNK / RUNS;
     __shared__ double total[RUNS][D];
     {
         const int d = tid % D, run = tid / D;
-        double r[RUN], p = 1.0;
+        float g[RUN];
+        double p = 1.0, q = 1.0;
 #pragma unroll
         for (int i = 0; i < RUN; ++i) {
             const int t = run * RUN + i;
-            if (t < rows && d < a.D) p *= (double)g_s[t * PITCH + d];
-            r[i] = p;
+            g[i] = t < rows && d < a.D ? g_s[t * PITCH + d] : 1.f;
+            p *= (double)g[i];
         }
         total[run][d] = p;
         __syncthreads();
         p = 1.0;
         for (int i = 0; i < run; ++i) p *= total[i][d];
+        for (int i = run + 1; i < RUNS; ++i) q *= total[i][d];
 #pragma unroll
-        for (int i = 0; i < RUN; ++i) g_s[(run * RUN + i) * PITCH + d] = (float)(p * r[i]);
-        if (run == RUNS - 1 && d < a.D) a.gam[((long)blockIdx.x * a.H + h) * a.D + d] = (float)(p * r[RUN - 1]);
+        for (int i = 0; i < RUN; ++i) {
+            p *= (double)g[i];
+            g_s[(run * RUN + i) * PITCH + d] = (float)p;
+            e_s[(run * RUN + RUN - 1 - i) * PITCH + d] = (float)q;
+            q *= (double)g[RUN - 1 - i];
+        }
+        if (run == RUNS - 1 && d < a.D) a.gam[((long)blockIdx.x * a.H + h) * a.D + d] = (float)p;
     }
     __syncthreads();
     for (int i = tid; i < CHUNK * D; i += PREP_THREADS) {
         const int t = i / D, d = i - t * D, at = t * PITCH + d;
-        const float g = g_s[at], inv = 1.0f / g, last = g_s[(CHUNK - 1) * PITCH + d];
-        const float kk = k_s[at] * inv, aa = a_s[at] * inv, rr = r_s[at] * g;
+        const float g = g_s[at], e = e_s[at], k = k_s[at], x = a_s[at], rr = r_s[at] * g;
         u_s[at] *= t ? g_s[at - PITCH] : 1.f;
-        k_s[at] = kk; a_s[at] = aa; r_s[at] = rr;
+        k_s[at] = k / g; a_s[at] = x / g; r_s[at] = rr;
         if (t < rows && d < a.D) {
             const long to = at0 + (long)t * hd + d;
-            a.qs[to] = rr; a.ks[to] = kk * last; a.as[to] = -aa * last;
+            a.qs[to] = rr; a.ks[to] = k * e; a.as[to] = -x * e;
         }
     }
     __syncthreads();
     const int ty = tid >> 4, tx = tid & 15;
-    u64 ua[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, uk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
-    u64 ra[2][2] = {{0ull, 0ull}, {0ull, 0ull}}, rk[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+    Sums<CHAINS> ua[2][2], uk[2][2], ra[2][2], rk[2][2];
 #pragma unroll 2
-    for (int d = 0; d < D; d += 4) {
-        ulonglong2 ks[2], as[2], ut[2], rt[2];
+    for (int d0 = 0; d0 < D; d0 += 2 * CHAINS) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
-            as[i] = *reinterpret_cast<const ulonglong2*>(a_s + (tx + 16 * i) * PITCH + d);
-            ut[i] = *reinterpret_cast<const ulonglong2*>(u_s + (ty + 16 * i) * PITCH + d);
-            rt[i] = *reinterpret_cast<const ulonglong2*>(r_s + (ty + 16 * i) * PITCH + d);
-        }
+        for (int n = 0; n < CHAINS; n += 2) {
+            const int d = d0 + 2 * n;
+            ulonglong2 ks[2], as[2], ut[2], rt[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                fma2(ua[i][j], ut[i].x, as[j].x); fma2(ua[i][j], ut[i].y, as[j].y);
-                fma2(uk[i][j], ut[i].x, ks[j].x); fma2(uk[i][j], ut[i].y, ks[j].y);
-                fma2(ra[i][j], rt[i].x, as[j].x); fma2(ra[i][j], rt[i].y, as[j].y);
-                fma2(rk[i][j], rt[i].x, ks[j].x); fma2(rk[i][j], rt[i].y, ks[j].y);
+            for (int i = 0; i < 2; ++i) {
+                ks[i] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * i) * PITCH + d);
+                as[i] = *reinterpret_cast<const ulonglong2*>(a_s + (tx + 16 * i) * PITCH + d);
+                ut[i] = *reinterpret_cast<const ulonglong2*>(u_s + (ty + 16 * i) * PITCH + d);
+                rt[i] = *reinterpret_cast<const ulonglong2*>(r_s + (ty + 16 * i) * PITCH + d);
             }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    ua[i][j].add(n, ut[i], as[j]); uk[i][j].add(n, ut[i], ks[j]);
+                    ra[i][j].add(n, rt[i], as[j]); rk[i][j].add(n, rt[i], ks[j]);
+                }
+        }
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int t = ty + 16 * i, s = tx + 16 * j;
-            A_s[t * LP + s] = s < t ? sum_of(ua[i][j]) : 0.f;
-            B_s[t * LP + s] = s < t ? sum_of(uk[i][j]) : 0.f;
+            A_s[t * LP + s] = s < t ? ua[i][j].sum() : 0.f;
+            B_s[t * LP + s] = s < t ? uk[i][j].sum() : 0.f;
             if (t < rows) {
                 float* p = a.p + ((long)(tok0 + t) * a.H + h) * (2 * CHUNK);
-                p[s] = s <= t ? sum_of(rk[i][j]) : 0.f;
-                p[CHUNK + s] = s <= t ? -sum_of(ra[i][j]) : 0.f;
+                p[s] = s < t ? rk[i][j].sum() : s == t ? rk_s[t] : 0.f;
+                p[CHUNK + s] = s < t ? -ra[i][j].sum() : s == t ? -ra_s[t] : 0.f;
             }
         }
     __syncthreads();
@@ -426,16 +493,7 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
             x[0] = 0.f;      // (V <= PREP_THREADS: its values are here)
 #pragma unroll
             for (int t = 1; t < CHUNK; ++t) {
-                float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-                for (int s = 0; s < t; s += 4) {
-                    const float4 b = *reinterpret_cast<const float4*>(B_s + t * LP + s);
-                    s0 = fmaf(b.x, v[s], s0);
-                    if (s + 1 < t) s1 = fmaf(b.y, v[s + 1], s1);
-                    if (s + 2 < t) s0 = fmaf(b.z, v[s + 2], s0);
-                    if (s + 3 < t) s1 = fmaf(b.w, v[s + 3], s1);
-                }
-                x[t] = s0 + s1;
+                x[t] = before(B_s + t * LP, v, t);
             }
         } else {
 #pragma unroll
@@ -443,16 +501,7 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
         }
 #pragma unroll
         for (int t = 1; t < CHUNK; ++t) {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int s = 0; s < t; s += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(A_s + t * LP + s);
-                s0 = fmaf(l.x, x[s], s0);
-                if (s + 1 < t) s1 = fmaf(l.y, x[s + 1], s1);
-                if (s + 2 < t) s0 = fmaf(l.z, x[s + 2], s0);
-                if (s + 3 < t) s1 = fmaf(l.w, x[s + 3], s1);
-            }
-            x[t] -= s0 + s1;
+            x[t] -= before(A_s + t * LP, x, t);
         }
         float* to = val ? a.x0 + ((long)tok0 * a.H + h) * a.V + c : a.wr + ((long)tok0 * a.H + h) * a.D + (c - a.V);
         const long ld = (long)a.H * (val ? a.V : a.D);
@@ -463,7 +512,9 @@ __global__ void __launch_bounds__(PREP_THREADS) general_chunks(ChunkArgs a)
 }
 
 // The gates of an mLSTM and its running maximum of their logarithms (mlstm.cu states them): a warp an (entry, head), a lane
-// a token.  m_t = max(f_t + m_(t-1), i_t) is a scan under (f, i) o (f', i') = (f + f', max(i + f', i')).
+// a token.  m_t = max(f_t + m_(t-1), i_t) is a scan under (f, i) o (f', i') = (f + f', max(i + f', i')).  The scan's sums are of
+// other numbers than the chain's, and a state (S, n, m) is off by what its maximum is off: so it runs in 64 bits up to the step's
+// last token (2,048 tokens of 16 heads: 24 us in 32 bits, 31 us).
 __device__ __forceinline__ float logsigmoid_f(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
 __global__ void __launch_bounds__(32) mlstm_gates_kernel(const float* __restrict__ gates, long ldg, const void* i_bias,
@@ -480,35 +531,33 @@ __global__ void __launch_bounds__(32) mlstm_gates_kernel(const float* __restrict
     // (the walk's blocks start from a copy: the first of them moves the state's own on while others may not have begun)
     for (int d = lane; d < D; d += 32) norm_in[((long)b * H + h) * D + d] = norm[((long)seq_slot[b] * H + h) * copies * D + d];
     const float bi = load_any(i_bias, bias_dtype, h), bf = load_any(f_bias, bias_dtype, h), inv_cap = 1.0f / cap;
-    float m = mp[0];
+    double m = mp[0];
     float in_i = gates[(long)min(r0 + lane, r1 - 1) * ldg + h], in_f = gates[(long)min(r0 + lane, r1 - 1) * ldg + H + h];
     for (int c0 = r0; c0 < r1; c0 += 32) {
         const int t = c0 + lane;
-        const float gi = cap * tanhf((in_i + bi) * inv_cap);
-        const float gf = logsigmoid_f(cap * tanhf((in_f + bf) * inv_cap));
+        const double gi = cap * tanhf((in_i + bi) * inv_cap);
+        const double gf = logsigmoid_f(cap * tanhf((in_f + bf) * inv_cap));
         const float* g = gates + (long)min(t + 32, r1 - 1) * ldg;      // (the next tokens' inputs travel meanwhile)
         in_i = g[h]; in_f = g[H + h];
-        float f = gf, i = gi;
+        double f = gf, i = gi;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const float pf = __shfl_up_sync(0xffffffffu, f, o), pi = __shfl_up_sync(0xffffffffu, i, o);
-            if (lane >= o) { i = fmaxf(pi + f, i); f = pf + f; }
+            const double pf = __shfl_up_sync(0xffffffffu, f, o), pi = __shfl_up_sync(0xffffffffu, i, o);
+            if (lane >= o) { i = fmax(pi + f, i); f = pf + f; }
         }
-        const float after = fmaxf(f + m, i);
-        float before = __shfl_up_sync(0xffffffffu, after, 1);
+        double after = fmax(f + m, i);
+        if (t == r1 - 1) after = (float)after;                         // as the state keeps it
+        double before = __shfl_up_sync(0xffffffffu, after, 1);
         if (lane == 0) before = m;
         if (t < r1) {
             const long at = (long)t * H + h;
-            // (rounding may leave f + before a last place above the maximum that it is one of; what is no number stays none,
-            // though the maxima pass over it)
-            const float dk = gf + before - after, dt = gi - after;
-            keep[at] = expf(dk > 0.f ? 0.f : dk);
-            take[at] = expf(dt > 0.f ? 0.f : dt);
-            floor_out[at] = expf(-after);
+            keep[at] = expf((float)(gf + before - after));
+            take[at] = expf((float)(gi - after));
+            floor_out[at] = expf((float)-after);
         }
         m = __shfl_sync(0xffffffffu, after, min(31, r1 - 1 - c0));
     }
-    for (int i = lane; i < copies; i += 32) mp[i] = m;
+    for (int i = lane; i < copies; i += 32) mp[i] = (float)m;
 }
 
 // ------------------------------------------------------------------------------------------------------ the walk
@@ -809,21 +858,15 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
             }
         }
 
-        // the state
+        // the state: the chunk's own sum first, then once the state before it, times the chunk's decay, on top (added to the
+        // state one by one the tokens' shares would each be rounded at its size)
+        u64 decay[2];
         if (KIND == GENERAL) {
             const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(st.gam + dg * 4);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                S[j][0] = pair(lo_of(S[j][0]) * lo_of(g.x), hi_of(S[j][0]) * hi_of(g.x));
-                S[j][1] = pair(lo_of(S[j][1]) * lo_of(g.y), hi_of(S[j][1]) * hi_of(g.y));
-            }
+            decay[0] = g.x; decay[1] = g.y;
         } else {
             const float g = st.gam[rows - 1];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                S[j][0] = pair(lo_of(S[j][0]) * g, hi_of(S[j][0]) * g);
-                S[j][1] = pair(lo_of(S[j][1]) * g, hi_of(S[j][1]) * g);
-            }
+            decay[0] = decay[1] = pair(g, g);
             if (KIND == MLSTM && tid < D) {
                 float acc = 0.f;
 #pragma unroll 8
@@ -831,21 +874,22 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
                 z = fmaf(g, z, acc);
             }
         }
+        u64 U[4][2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) U[j][0] = U[j][1] = 0ull;
 #pragma unroll 8
         for (int i = 0; i < C2 / PARTS; ++i) {
             const int s = part * (C2 / PARTS) + i;
             const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(st.k + s * D + dg * 4);
             const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4);
             const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4 + 2);
-            fma2(S[0][0], k.x, u.x); fma2(S[0][1], k.y, u.x); fma2(S[1][0], k.x, u.y); fma2(S[1][1], k.y, u.y);
-            fma2(S[2][0], k.x, v.x); fma2(S[2][1], k.y, v.x); fma2(S[3][0], k.x, v.y); fma2(S[3][1], k.y, v.y);
+            fma2(U[0][0], k.x, u.x); fma2(U[0][1], k.y, u.x); fma2(U[1][0], k.x, u.y); fma2(U[1][1], k.y, u.y);
+            fma2(U[2][0], k.x, v.x); fma2(U[2][1], k.y, v.x); fma2(U[3][0], k.x, v.y); fma2(U[3][1], k.y, v.y);
         }
         if (part > 0) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                *reinterpret_cast<ulonglong2*>(sm.part + ((part - 1) * COLS + cg * 4 + j) * D + dg * 4) = make_ulonglong2(S[j][0], S[j][1]);
-                S[j][0] = 0ull; S[j][1] = 0ull;
-            }
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<ulonglong2*>(sm.part + ((part - 1) * COLS + cg * 4 + j) * D + dg * 4) = make_ulonglong2(U[j][0], U[j][1]);
         }
         __syncthreads();
         if (part == 0) {
@@ -854,9 +898,11 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
 #pragma unroll
                 for (int i = 0; i < PARTS - 1; ++i) {
                     const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sm.part + (i * COLS + cg * 4 + j) * D + dg * 4);
-                    S[j][0] = pair(lo_of(S[j][0]) + lo_of(x.x), hi_of(S[j][0]) + hi_of(x.x));
-                    S[j][1] = pair(lo_of(S[j][1]) + lo_of(x.y), hi_of(S[j][1]) + hi_of(x.y));
+                    U[j][0] = add2(U[j][0], x.x);
+                    U[j][1] = add2(U[j][1], x.y);
                 }
+                S[j][0] = fma2_of(S[j][0], decay[0], U[j][0]);
+                S[j][1] = fma2_of(S[j][1], decay[1], U[j][1]);
                 *reinterpret_cast<ulonglong2*>(sm.s + (cg * 4 + j) * PITCH + dg * 4) = make_ulonglong2(S[j][0], S[j][1]);
             }
         }

@@ -1434,6 +1434,83 @@ def test_chunk_scan_general(dtype, lens, H, D, rank):
     assert far(out, want) < max(2e-6, 1.5 * far(old, want)) and far(st, S_want) < max(1e-6, 1.5 * far(st_old, S_want))
 
 
+@pytest.mark.parametrize("kind,rate", [("delta", 0), ("mlstm", 0), ("general", math.exp(-0.5)), ("general", 1.0)])
+def test_chunked_recurrences_are_as_near_to_64_bits_as_token_by_token(kind, rate):
+    """The chunked recurrences' error against the loop in 64 bits, beside that of the kernels that take the tokens one by one:
+    summed over shapes and seeds, so that chance evens out, it is no larger (5 % for what chance is left).  An mLSTM's state
+    stands for S e^m (its read-outs are quotients, and what their nearly vanishing denominators do to an error is chance)."""
+    o = ops()
+    d = lambda t: t.double()
+    far = lambda a, b: float((d(a) - b).norm() / b.norm())
+    new, old = [0.0, 0.0], [0.0, 0.0]
+    for lens, H, G, D, V in (([1], 2, 1, 64, 16), ([31, 32, 33], 4, 2, 128, 128), ([100], 3, 3, 20, 36), ([65, 1, 64], 2, 2, 68, 4),
+                             ([200, 7], 2, 1, 128, 100), ([64, 5, 97], 4, 2, 64, 48), ([600], 2, 2, 128, 128)):
+        G, V = (G if kind == "delta" else H), (D if kind == "general" else V)
+        T, n, (seq, slot, tiles) = sum(lens), len(lens), scan_setup(lens, 0)
+        at, copies = (seq, slot, n), o.mlstm_column_blocks(D, V)
+        for seed in range(12 if kind == "mlstm" else 4):
+            gen = torch.Generator(device=DEV).manual_seed(seed)
+            rand = lambda *shape: torch.randn(*shape, generator=gen, device=DEV)
+            q, k, v, state = rand(T, G * D), rand(T, G * D), rand(T, H * V), rand(n + 2, H, V, D)
+            outs, states = [torch.empty(T, H * V, device=DEV) for _ in range(2)], [state.clone(), state.clone()]
+            if kind == "delta":
+                k = torch.nn.functional.normalize(k.view(T, G, D), dim=-1).view(T, -1).contiguous()
+                g, beta = torch.sigmoid(rand(T, H) * 3 + 2), torch.sigmoid(rand(T, H))
+                o.chunk_scan(q, k, v, g, states[0], outs[0], tiles, *at, H, G, D, V, beta=beta, scratch=scan_scratch)
+                o.state_scan(q, k, v, g, H, beta, states[1], outs[1], *at, H, G, D, V)
+            elif kind == "mlstm":
+                gates, ib, fb, cap = rand(T, 2 * H) * 4, rand(H), rand(H) + 2, 15.0
+                n0 = rand(n + 2, H, 1, D).expand(n + 2, H, copies, D).contiguous()
+                m0 = rand(n + 2, H, 1).expand(n + 2, H, copies).contiguous()
+                norm, top = [n0.clone(), n0.clone()], [m0.clone(), m0.clone()]
+                keep, take, floor = (torch.empty(T, H, device=DEV) for _ in range(3))
+                was = torch.empty(n, H, D, device=DEV)
+                o.mlstm_gates(gates, ib, fb, cap, top[0], norm[0], was, keep, take, floor, *at, H, D)
+                o.chunk_scan(q, k, v, keep, states[0], outs[0], tiles, *at, H, H, D, V, take=take, q_scale=D ** -0.5,
+                             scratch=scan_scratch, normalizer=(was, norm[0], floor))
+                o.mlstm_scan(q, k, v, gates, ib, fb, cap, D ** -0.5, states[1], norm[1], top[1], outs[1], *at, H, D, V)
+            else:
+                a_pre, low, w2, w0, ab = rand(T, H * D), rand(T, 64), rand(H * D, 64) * 0.3, rand(H * D) * 2, rand(H * D)
+                w0[::7], w0[1::7] = 30.0, -30.0
+                o.chunk_scan_general(q, k, v, a_pre, low, w2, w0, ab, rate, states[0], outs[0], tiles, *at, H, D, scratch=scan_scratch)
+                u, au, w = (torch.empty(T, H * D, device=DEV) for _ in range(3))
+                o.general_delta_prep(k, a_pre, low, w2, w0, ab, rate, u, au, w, H, D)
+                o.general_delta_scan(q, k, v, u, au, w, states[1], outs[1], *at, H, D)
+                U = d(k).view(T, H, D)
+                U = U / torch.sqrt((U * U).sum(-1, keepdim=True) + 1e-6)
+                A = torch.sigmoid(d(a_pre) + d(ab)).view(T, H, D) * U
+                W = torch.exp(-rate * torch.sigmoid(torch.tanh(d(low)) @ d(w2).T + d(w0))).view(T, H, D)
+            Q, K = (d(x).view(T, G, D).repeat_interleave(H // G, 1) for x in (q, k))
+            X, want, S_want, t = d(v).view(T, H, V), torch.zeros(T, H, V, dtype=torch.float64, device=DEV), d(state), 0
+            for b, L in enumerate(lens):
+                S = S_want[int(slot[b])].transpose(1, 2)
+                m = d(m0)[int(slot[b]), :, 0] if kind == "mlstm" else None
+                for t in range(t, t + L):
+                    if kind == "delta":
+                        S = S * d(g)[t][:, None, None]
+                        S = S + K[t][:, :, None] * (d(beta)[t][:, None] * (X[t] - torch.einsum("hdv,hd->hv", S, K[t])))[:, None]
+                    elif kind == "general":
+                        y = torch.einsum("hi,hij->hj", U[t], S)
+                        S = W[t][:, :, None] * S - A[t][:, :, None] * y[:, None] + K[t][:, :, None] * X[t][:, None]
+                    else:
+                        gi = cap * torch.tanh((d(gates)[t, :H] + d(ib)) / cap)
+                        gf = torch.nn.functional.logsigmoid(cap * torch.tanh((d(gates)[t, H:] + d(fb)) / cap))
+                        mn = torch.maximum(gf + m, gi)
+                        S = torch.exp(gf + m - mn)[:, None, None] * S + torch.exp(gi - mn)[:, None, None] * K[t][:, :, None] * X[t][:, None]
+                        m = mn
+                    want[t] = torch.einsum("hdv,hd->hv", S, Q[t])
+                t += 1
+                S_want[int(slot[b])] = S.transpose(1, 2)
+                if kind == "mlstm":
+                    for i in range(2):
+                        states[i] = d(states[i])
+                        states[i][int(slot[b])] *= torch.exp(d(top[i])[int(slot[b]), :, 0] - m)[:, None, None]
+            for e, i in ((new, 0), (old, 1)):
+                e[0] += far(outs[i], want.view(T, -1)) if kind != "mlstm" else 0.0
+                e[1] += far(states[i], S_want)
+    assert new[0] <= 1.05 * old[0] and new[1] <= 1.05 * old[1], (new, old)
+
+
 @pytest.mark.parametrize("lens,G,D,H,V", [([128], 1, 128, 1, 4), ([1, 2, 3, 200], 1, 64, 2, 36), ([17, 130, 16, 4], 2, 128, 4, 128),
                                           ([300], 2, 64, 2, 62)])
 def test_delta_prep_by_runs(lens, G, D, H, V, monkeypatch):
