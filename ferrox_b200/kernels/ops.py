@@ -727,7 +727,7 @@ def chunk_scan_general(r, k, v, a_pre, low, w2, w0, a_bias, rate, state, out, ti
                        scratch, status=None, stream=None):
     """:func:`general_delta_prep` and :func:`general_delta_scan` over a prompt's chunks (see :func:`chunk_scan`): ``r``,
     ``k``, ``v``, ``a_pre`` 32-bit row views [T, H*D], ``low`` [T, rank], ``w2`` contiguous [H*D, rank]; a ``rate`` of at
-    most 1, so that a chunk's products of decays stay inside 32-bit numbers' range."""
+    most 1: a chunk's products of decays then stay above 1e-14."""
     T = r.shape[0]
     if not (out.is_contiguous() and w2.is_contiguous()) or low.dtype != torch.float32:
         raise KernelError("chunk_scan_general: 32-bit low-rank rows, a contiguous matrix and read-outs")

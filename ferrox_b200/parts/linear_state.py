@@ -268,7 +268,7 @@ class GeneralDeltaRule(_StateMixer):
         r, k, v, gate = (proj[:, i * hd:(i + 1) * hd] for i in range(4))
         a_pre, low = proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:]
         read, state = rt.empty(T, hd, dtype=f32), cache.states["matrix"]
-        # (a rate of at most 1: over a chunk the products of stronger decays would leave 32-bit numbers' range)
+        # (a rate of at most 1: a chunk's products of decays stay above 1e-14, far from the end of 32-bit numbers)
         tiles = _chunk_tiles(batch, H, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
         if tiles is not None:
             ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, tiles,

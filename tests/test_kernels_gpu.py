@@ -1398,8 +1398,8 @@ def test_mlstm_gate_that_is_no_number(gate):
 
 @pytest.mark.parametrize("lens,H,D,rank", [([1], 2, 64, 64), ([31, 32, 33], 3, 64, 8), ([100, 5], 2, 20, 3), ([65], 2, 128, 96),
                                            ([130, 1, 64], 1, 100, 65)])
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_chunk_scan_general(dtype, lens, H, D, rank):
+@pytest.mark.parametrize("dtype,rate", [("float32", math.exp(-0.5)), ("bfloat16", math.exp(-0.5)), ("float32", 1.0), ("float32", 0.0)])
+def test_chunk_scan_general(dtype, rate, lens, H, D, rank):
     """The generalized delta rule in chunks, from its projections, against the loop in 64 bits, with decays over their whole
     range."""
     o = ops()
@@ -1408,7 +1408,7 @@ def test_chunk_scan_general(dtype, lens, H, D, rank):
     r, k, v, a_pre = (wide[:, i * H * D:(i + 1) * H * D] for i in range(4))
     low, w2, w0 = wide[:, 4 * H * D:4 * H * D + rank], rnd(H * D, rank, dtype=DT[dtype], scale=0.3), rnd(H * D, dtype=DT[dtype], scale=2.0)
     w0[::7], w0[1::7] = 30.0, -30.0            # channels that forget as fast as they can, and that never do
-    a_bias, rate = rnd(H * D, dtype=DT[dtype], seed=2), math.exp(-0.5)
+    a_bias = rnd(H * D, dtype=DT[dtype], seed=2)
     state = rnd(len(lens) + 2, H, D, D, seed=3)
     st, st_old = state.clone(), state.clone()
     out, old = torch.empty(T, H * D, device=DEV), torch.empty(T, H * D, device=DEV)
