@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(NT, 2) attention_f32_kernel(AttArgs a)
 
 template <int D> int go(const AttArgs& a, int n_tiles, cudaStream_t s)
 {
-    static const cudaError_t set = cudaFuncSetAttribute(attention_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        (int)sizeof(Smem<D>));
+    const cudaError_t set = cudaFuncSetAttribute(attention_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)sizeof(Smem<D>));      // (of the current device: asked for each time)
     if (set != cudaSuccess) return (int)set;
     fx_launch_pdl(attention_f32_kernel<D>, dim3((unsigned)n_tiles, (unsigned)a.n_heads), NT, sizeof(Smem<D>), s, a);
     return fx_launch_status();

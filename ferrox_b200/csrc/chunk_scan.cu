@@ -945,7 +945,8 @@ template <int D, int KIND> int go_walk(WalkArgs a, int n_entries, cudaStream_t s
             (!Stage<D, KIND>::HASW || row_map(&maps.w, a.w, (long)a.H * D, a.H, D, a.n_tokens)) &&
             (KIND != GENERAL || row_map(&maps.a, a.a, (long)a.H * D, a.H, D, a.n_tokens));
     const int smem = (int)sizeof(WalkSmem<D, KIND>);
-    static const cudaError_t set = cudaFuncSetAttribute(walk_kernel<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // (of the current device: asked for each time)
+    const cudaError_t set = cudaFuncSetAttribute(walk_kernel<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (set != cudaSuccess) return (int)set;
     // (not set up early: its blocks stay for the whole prompt, see fx_launch_pdl_if)
     fx_launch_pdl_if(false, walk_kernel<D, KIND>, dim3((unsigned)fx_cdiv(a.V, COLS), (unsigned)a.H, (unsigned)n_entries), WALK_THREADS,

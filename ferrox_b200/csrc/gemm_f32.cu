@@ -373,7 +373,8 @@ template <int MT, int R> int go_stream(const Args& a, cudaStream_t s)
 template <int BM> int go_tile(const Args& a, cudaStream_t s)
 {
     const size_t smem = sizeof(float) * STAGES * (BM + BN) * PITCH;
-    static const cudaError_t set = cudaFuncSetAttribute(tile_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (of the current device: asked for each time)
+    const cudaError_t set = cudaFuncSetAttribute(tile_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (set != cudaSuccess) return (int)set;
     const long rows = fx_cdiv(a.M, BM) + (a.offsets ? a.G : 0);
     if (rows > 65535) return FX_ERR_SIZE;

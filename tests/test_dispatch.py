@@ -141,3 +141,16 @@ def test_uploads_on_a_stream_beside_the_step_are_complete_when_they_return(monke
         ops.upload(values, "cuda:0")
     ops.upload(values, "cuda:0")
     assert len(waits) == 2
+
+
+def test_shared_memory_limits_are_not_asked_for_on_one_device_only():
+    """The limit belongs to a function on the device that is current: an answer kept from the process's first call (which may
+    also have been an error that passed) says nothing of a second device."""
+    import os
+    import re
+
+    from ferrox_b200.kernels import lib
+
+    for name in lib.sources():
+        with open(os.path.join(lib.CSRC, name)) as f:
+            assert not re.search(r"static\s+(const\s+)?\w+\s+\w+\s*=\s*cudaFuncSetAttribute", f.read()), name
