@@ -372,6 +372,9 @@ def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=N
     return out
 
 
+F32_WORKSPACE_MAX = 1 << 27      # bytes of partial sums a 32-bit product may ask for beside its operands
+
+
 @functools.lru_cache(maxsize=4096)
 def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
     """(form, runs of K) of the 32-bit product's kernel (gemm_f32.cu): minus the rows a pass of the weight-streaming
@@ -381,7 +384,9 @@ def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
     microseconds as measured on a B200: a pass of 8 rows streams the weights at 3.1 TB/s; a round of the tiled kernel
     (four warps an SM: one 64-row tile, two 32-row tiles or half a 128-row one) takes 0.0555 us an element of K, and a
     product cut into runs of K writes and reads its partial sums (16 x 6144 x 2048: 30.6 us streamed, 28.2 us in 32-row
-    tiles and 6 runs; 16 x 2048 x 2048: 12.3 against 20.2 us; 60 x 2048 x 5632: 46 us in 8 runs, 312 us in one).
+    tiles and 6 runs; 16 x 2048 x 2048: 12.3 against 20.2 us; 60 x 2048 x 5632: 46 us in 8 runs, 312 us in one).  The partial
+    sums stay within F32_WORKSPACE_MAX: where there are many tiles, runs of K save a part of one round of them, and an engine
+    whose pages fill the device has no room for a gigabyte (597 x 151936 x 16384 in 3 runs).
     Of groups, the mean number of rows decides: 4 rows a pass up to 6 rows a group (60 experts of 2816 x 2048, 4 rows
     each: 332 us against 532 us in 32-row tiles; 13 rows each: 922 against 536 us)."""
     if groups is not None:
@@ -397,6 +402,8 @@ def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
         if tiles // n_tiles > 65535:     # (rows of blocks in a grid)
             continue
         for splits in range(1, max(1, min(16, K // 128)) + 1):
+            if splits > 1 and 4 * splits * M * N > F32_WORKSPACE_MAX:
+                break
             rounds = -(-tiles * splits * (bm // 16) // (4 * sms))
             t = rounds * 0.0555 * K / splits + 4.0
             if splits > 1:

@@ -154,3 +154,18 @@ def test_shared_memory_limits_are_not_asked_for_on_one_device_only():
     for name in lib.sources():
         with open(os.path.join(lib.CSRC, name)) as f:
             assert not re.search(r"static\s+(const\s+)?\w+\s+\w+\s*=\s*cudaFuncSetAttribute", f.read()), name
+
+
+def test_32_bit_product_plans_by_size():
+    """Up to 4 rows the weights are streamed; beyond, tiles, in runs of K where they are few, whose partial sums stay within the
+    workspace's limit; grids stay within their limits."""
+    assert ops.F32_WORKSPACE_MAX <= 128 << 20
+    assert [ops.gemm_f32_plan(m, 6144, 2048) for m in (1, 2, 3, 4)] == [(-1, 1), (-2, 1), (-4, 1), (-4, 1)]
+    for m in (5, 16, 60, 129, 412, 517, 597, 2048, 2780, 70000, 3000000):
+        for n in (1, 61, 2048, 15616, 151936):
+            for k in (4, 128, 2048, 16384):
+                form, splits = ops.gemm_f32_plan(m, n, k)
+                assert form in (-8, 32, 64, 128) and 1 <= splits <= 16 and (form > 0 or splits == 1)
+                assert splits == 1 or (4 * splits * m * n <= ops.F32_WORKSPACE_MAX and splits * 128 <= k)
+                assert form < 0 or -(-m // form) <= 65535
+    assert ops.gemm_f32_plan(60, 2048, 5632)[1] > 1 and ops.gemm_f32_plan(517, 15616, 2048)[1] > 1
