@@ -12,7 +12,8 @@ int fx_gemm(const void* A, int a_dtype, long lda, const int* a_rows, const void*
             const int* group_offsets, int n_groups, long w_group_stride, void* stream);
 
 // The same in 32 bits throughout, for rows of 4 n elements on the 16-byte grid (gemm_f32.cu).  form > 0: rows a tile
-// (128, 64, 32), K in `splits` runs with their partial sums in `part`; form < 0: W streamed once for -form rows a pass.
+// (128, 64, 32), K in `splits` runs with their partial sums in `part`; form < 0: W streamed once for -form rows a pass
+// (groups, splits 2: or tiles, by the groups' sizes).
 int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long ldw, const void* bias, int bias_dtype,
                 void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
                 long w_group_stride, int form, int splits, void* part, void* stream);

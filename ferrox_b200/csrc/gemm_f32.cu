@@ -18,7 +18,8 @@
 //    partial sums a second kernel adds in order.  A thread's 8 x 4 outputs on twice the warps were 8 % slower.
 //
 // Error against 64-bit sums at K = 2048: 1.0e-7 (stream), 5.7e-7 (tile); one thread summing K in order: 8.1e-7.
-// Grouped mode (`group_offsets`): rows [off[g], off[g+1]) use matrix g of W; `a_rows` gathers rows of A.
+// Grouped mode (`group_offsets`): rows [off[g], off[g+1]) use matrix g of W; `a_rows` gathers rows of A.  The host knows
+// how many rows there are, not how they lie: tiles_better().
 // The element-at-a-time kernel of gemm_generic.cu takes what is refused here (K or strides no multiple of 4, operands
 // off the 16-byte grid, mixed element types).
 #include "common.cuh"
@@ -38,6 +39,37 @@ struct Args {
     float* part; int splits; int split_len;
 };
 
+// For groups where tiles_better() decides, for so many rows a pass.  (A struct of its own: with these in Args the compiler made tiles
+// of 64 and 32 rows that took 3 % longer.)
+struct PickArgs : Args {
+    int pass, sms, tiles_y;          // (rows of tiles)
+    int* picked;                     // the tiles' kernel, which runs first, leaves its answer here
+};
+
+// Groups whose rows are few on average may hide some that have most of them: the stream kernel takes `pass` rows of a group
+// at a time, and the blocks that hold a large group's rows of W go through its passes one after the other.  In microseconds
+// on a B200: 3.3 a pass of 4 rows (2.2 of 2) of a block's 8 rows of W and 2,048 elements of K, two blocks an SM, but no less
+// than the largest group's passes; 0.0555 an element of K a round of 32-row tiles, three in flight on two SMs, and 3.  Both
+// kernels are launched and one of the two has nothing to do.  60 experts of 2816 x 2048: 240 rows spread evenly 276 us
+// streamed (527 in tiles), a quarter of them on each of four 130 in tiles (262 streamed), 360 rows on one 227 (574).
+__device__ __forceinline__ bool tiles_better(const PickArgs& a, int lane)
+{
+    int passes = 0, most = 0, tiles = 0;
+    for (int g = lane; g < a.G; g += 32) {
+        const int rows = a.offsets[g + 1] - a.offsets[g], n = (rows + a.pass - 1) / a.pass;
+        passes += n;
+        most = max(most, n);
+        tiles += (rows + 31) / 32;
+    }
+    passes = __reduce_add_sync(0xffffffffu, passes);
+    most = __reduce_max_sync(0xffffffffu, most);
+    tiles = __reduce_add_sync(0xffffffffu, tiles);
+    const long blocks = (a.N + 7) / 8, slots = 2 * a.sms;
+    const long turns = max((passes * blocks + slots - 1) / slots, most * ((blocks + slots - 1) / slots));
+    const long rounds = (2L * tiles * ((a.N + 127) / 128) + 3 * a.sms - 1) / (3 * a.sms);
+    return turns * ((a.K + 2047) / 2048) * (a.pass <= 2 ? 22000 : 33000) > rounds * a.K * 555 + 30000;
+}
+
 __device__ __forceinline__ float4 ld_stream(const float* p) {
     float4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
@@ -52,8 +84,8 @@ constexpr int CHUNK = 128;           // elements of K a warp takes at a time
 // R: rows of W a block holds; two chunks of each are in flight.  Eight rows, and four where eight tokens' sums leave no
 // registers for more: two blocks an SM are worth more than rows (8 tokens x 6144 x 2048: R = 8 with one block an SM 24.0
 // us, R = 4 with two 16.9 us).
-template <int MT, int R>
-__global__ void __launch_bounds__(SW * 32, 2) stream_kernel(Args a)
+template <int MT, int R, typename A>
+__global__ void __launch_bounds__(SW * 32, 2) stream_kernel(A a)
 {
     constexpr int U = 2;
     __shared__ float red[SW][MT * R];
@@ -90,6 +122,7 @@ __global__ void __launch_bounds__(SW * 32, 2) stream_kernel(Args a)
                 if (has) act[n + __popc(m & ((1u << lane) - 1))] = g;
                 n += __popc(m);
             }
+            if constexpr (sizeof(A) != sizeof(Args)) n = *a.picked ? 0 : n;
             if (lane == 0) n_act = n;
         }
         __syncthreads();
@@ -193,9 +226,11 @@ __device__ __forceinline__ void cp16(uint32_t dst, const float* src, bool valid)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(n));
 }
 
-template <int BM>
-__global__ void __launch_bounds__(BM * 2) tile_kernel(Args a)
+// With PickArgs it may have nothing to do, and takes no more blocks than go at once (1,500 that ask and leave take 7 us).
+template <int BM, typename A>
+__global__ void __launch_bounds__(BM * 2) tile_kernel(A a)
 {
+    constexpr bool PICK = sizeof(A) != sizeof(Args);
     constexpr int NT = BM * 2;                       // threads
     constexpr int CA = BM * (BK / 4) / NT, CB = BN * (BK / 4) / NT;   // 16-byte copies of a thread a stage
     constexpr int STAGE = (BM + BN) * PITCH;         // floats
@@ -203,136 +238,150 @@ __global__ void __launch_bounds__(BM * 2) tile_kernel(Args a)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     fx_pdl_wait();
-    int row0 = blockIdx.y * BM, row_end = a.M;
-    const float* W = a.W;
-    if (a.offsets) {
-        // block row y is the y-th tile of rows of the groups laid one after the other (every warp finds it for itself)
-        int left = blockIdx.y, found = -1;
-        for (int g0 = 0; g0 < a.G && found < 0; g0 += 32) {
-            const int g = g0 + lane;
-            const int rows = g < a.G ? a.offsets[g + 1] - a.offsets[g] : 0;
-            const int t = (rows + BM - 1) / BM;
-            int sum = t;                              // tiles of the groups up to this lane's
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, sum, o);
-                if (lane >= o) sum += v;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, sum > left);
-            if (m) {
-                const int l = __ffs(m) - 1;
-                found = g0 + l;
-                left -= __shfl_sync(0xffffffffu, sum - t, l);
-            } else {
-                left -= __shfl_sync(0xffffffffu, sum, 31);
-            }
-        }
-        if (found < 0) return;
-        row0 = a.offsets[found] + left * BM;
-        row_end = a.offsets[found + 1];
-        W += (long)found * a.w_gs;
+    if constexpr (PICK) {
+        const bool mine = tiles_better(a, lane);      // (the same answer in every warp)
+        if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *a.picked = mine;
+        if (!mine) return;
     }
-    const int n0 = blockIdx.x * BN;
-    const int k_begin = blockIdx.z * a.split_len, k_end = min(a.K, k_begin + a.split_len);
-    const int n_stages = (k_end - k_begin + BK - 1) / BK;
-
-    // what this thread copies of every stage: piece `kc` of rows lr, lr + NT / 4, ...
-    const int lr = tid >> 2, kc = (tid & 3) * 4;
-    const float* a_src[CA];
-    bool a_ok[CA];
+    int y = blockIdx.y;
+    do {
+        int row0 = y * BM, row_end = a.M;
+        const float* W = a.W;
+        if (a.offsets) {
+            // block row y is the y-th tile of rows of the groups laid one after the other (every warp finds it for itself)
+            int left = y, found = -1;
+            for (int g0 = 0; g0 < a.G && found < 0; g0 += 32) {
+                const int g = g0 + lane;
+                const int rows = g < a.G ? a.offsets[g + 1] - a.offsets[g] : 0;
+                const int t = (rows + BM - 1) / BM;
+                int sum = t;                              // tiles of the groups up to this lane's
 #pragma unroll
-    for (int i = 0; i < CA; ++i) {
-        const int r = row0 + lr + i * (NT / 4);
-        a_ok[i] = r < row_end;
-        a_src[i] = a.A + (a_ok[i] ? (long)(a.a_rows ? a.a_rows[r] : r) * a.lda : 0) + kc;
-    }
-    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(sm);
-    const uint32_t dst = smem + (uint32_t)(lr * PITCH + kc) * 4;
-    auto fetch = [&](int s) {
-        if (s < n_stages) {
-            const int k = k_begin + s * BK;
-            const bool in_k = k + kc < k_end;
-            const uint32_t d = dst + (uint32_t)((s % STAGES) * STAGE) * 4;
-#pragma unroll
-            for (int i = 0; i < CA; ++i)
-                cp16(d + i * (NT / 4) * PITCH * 4, a_src[i] + (in_k ? k : 0), a_ok[i] && in_k);
-#pragma unroll
-            for (int i = 0; i < CB; ++i) {
-                const int n = n0 + lr + i * (NT / 4);
-                const bool ok = n < a.N && in_k;
-                cp16(d + (BM + i * (NT / 4)) * PITCH * 4, W + (ok ? (long)n * a.ldw + k + kc : 0), ok);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += v;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, sum > left);
+                if (m) {
+                    const int l = __ffs(m) - 1;
+                    found = g0 + l;
+                    left -= __shfl_sync(0xffffffffu, sum - t, l);
+                } else {
+                    left -= __shfl_sync(0xffffffffu, sum, 31);
+                }
             }
+            if (found < 0) return;
+            row0 = a.offsets[found] + left * BM;
+            row_end = a.offsets[found + 1];
+            W += (long)found * a.w_gs;
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+        const int n0 = blockIdx.x * BN;
+        const int k_begin = blockIdx.z * a.split_len, k_end = min(a.K, k_begin + a.split_len);
+        const int n_stages = (k_end - k_begin + BK - 1) / BK;
 
-    // a warp owns 32 x 64 outputs, a lane rows ty + 4 i and columns tx + 8 j of them
-    const int wm = warp >> 1, wn = warp & 1;
-    const int ty = lane >> 3, tx = lane & 7;
-    const uint32_t a_at = smem + (uint32_t)((wm * 32 + ty) * PITCH) * 4;
-    const uint32_t b_at = smem + (uint32_t)((BM + wn * 64 + tx) * PITCH) * 4;
-    u64 acc[8][8];
+        // what this thread copies of every stage: piece `kc` of rows lr, lr + NT / 4, ...
+        const int lr = tid >> 2, kc = (tid & 3) * 4;
+        const float* a_src[CA];
+        bool a_ok[CA];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < CA; ++i) {
+            const int r = row0 + lr + i * (NT / 4);
+            a_ok[i] = r < row_end;
+            a_src[i] = a.A + (a_ok[i] ? (long)(a.a_rows ? a.a_rows[r] : r) * a.lda : 0) + kc;
+        }
+        const uint32_t smem = (uint32_t)__cvta_generic_to_shared(sm);
+        const uint32_t dst = smem + (uint32_t)(lr * PITCH + kc) * 4;
+        auto fetch = [&](int s) {
+            if (s < n_stages) {
+                const int k = k_begin + s * BK;
+                const bool in_k = k + kc < k_end;
+                const uint32_t d = dst + (uint32_t)((s % STAGES) * STAGE) * 4;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
-
-    // Four elements of K a step.  The next step's rows of A and the next column's of W are read while this one's
-    // products run; the last step of a stage reads the next stage's, after the block has met.  By then everyone is done
-    // with the stage before this one, and its place is filled again.
-    u64 av[2][8][2], bv[2][2];
-    auto lds = [](u64* v, uint32_t at) {
-        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(at));
-    };
+                for (int i = 0; i < CA; ++i)
+                    cp16(d + i * (NT / 4) * PITCH * 4, a_src[i] + (in_k ? k : 0), a_ok[i] && in_k);
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
-    asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2) : "memory");
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) lds(av[0][i], a_at + i * 4 * PITCH * 4);
-    lds(bv[0], b_at);
-    uint32_t base = 0;                                // this stage's place
-    for (int s = 0; s < n_stages; ++s) {
-        const uint32_t next = s % STAGES == STAGES - 1 ? 0 : base + STAGE * 4;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q == 3) {
-                asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 3) : "memory");
-                __syncthreads();
-                fetch(s + STAGES - 1);
+                for (int i = 0; i < CB; ++i) {
+                    const int n = n0 + lr + i * (NT / 4);
+                    const bool ok = n < a.N && in_k;
+                    cp16(d + (BM + i * (NT / 4)) * PITCH * 4, W + (ok ? (long)n * a.ldw + k + kc : 0), ok);
+                }
             }
-            const uint32_t off = q == 3 ? next : base + (q + 1) * 16;
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+
+        // a warp owns 32 x 64 outputs, a lane rows ty + 4 i and columns tx + 8 j of them
+        const int wm = warp >> 1, wn = warp & 1;
+        const int ty = lane >> 3, tx = lane & 7;
+        const uint32_t a_at = smem + (uint32_t)((wm * 32 + ty) * PITCH) * 4;
+        const uint32_t b_at = smem + (uint32_t)((BM + wn * 64 + tx) * PITCH) * 4;
+        u64 acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+
+        // Four elements of K a step.  The next step's rows of A and the next column's of W are read while this one's
+        // products run; the last step of a stage reads the next stage's, after the block has met.  By then everyone is done
+        // with the stage before this one, and its place is filled again.
+        u64 av[2][8][2], bv[2][2];
+        auto lds = [](u64* v, uint32_t at) {
+            asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(at));
+        };
+#pragma unroll
+        for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+        asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2) : "memory");
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) lds(av[0][i], a_at + i * 4 * PITCH * 4);
+        lds(bv[0], b_at);
+        uint32_t base = 0;                                // this stage's place
+        for (int s = 0; s < n_stages; ++s) {
+            const uint32_t next = s % STAGES == STAGES - 1 ? 0 : base + STAGE * 4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q == 3) {
+                    asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 3) : "memory");
+                    __syncthreads();
+                    fetch(s + STAGES - 1);
+                }
+                const uint32_t off = q == 3 ? next : base + (q + 1) * 16;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    lds(bv[(j + 1) & 1], j == 7 ? b_at + off : b_at + base + (j + 1) * 8 * PITCH * 4 + q * 16);
+                    lds(av[(q + 1) & 1][j], a_at + off + j * 4 * PITCH * 4);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[q & 1][i][0], bv[j & 1][0]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[q & 1][i][1], bv[j & 1][1]);
+                }
+            }
+            base = next;
+        }
+
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = row0 + wm * 32 + ty + 4 * i;
+            if (r >= row_end) continue;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                lds(bv[(j + 1) & 1], j == 7 ? b_at + off : b_at + base + (j + 1) * 8 * PITCH * 4 + q * 16);
-                lds(av[(q + 1) & 1][j], a_at + off + j * 4 * PITCH * 4);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[q & 1][i][0], bv[j & 1][0]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[q & 1][i][1], bv[j & 1][1]);
+                const int n = n0 + wn * 64 + tx + 8 * j;
+                if (n >= a.N) continue;
+                float v = __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+                if (a.part) {
+                    a.part[((long)blockIdx.z * a.M + r) * a.N + n] = v;
+                    continue;
+                }
+                if (a.bias) v += load_any(a.bias, a.bias_dtype, n);
+                float* c = a.C + (long)r * a.ldc + n;
+                *c = a.accumulate ? *c + v : v;
             }
         }
-        base = next;
-    }
-
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = row0 + wm * 32 + ty + 4 * i;
-        if (r >= row_end) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int n = n0 + wn * 64 + tx + 8 * j;
-            if (n >= a.N) continue;
-            float v = __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
-            if (a.part) {
-                a.part[((long)blockIdx.z * a.M + r) * a.N + n] = v;
-                continue;
-            }
-            if (a.bias) v += load_any(a.bias, a.bias_dtype, n);
-            float* c = a.C + (long)r * a.ldc + n;
-            *c = a.accumulate ? *c + v : v;
+        if constexpr (PICK) {
+            __syncthreads();             // (everyone is done with the places in shared memory)
+            y += gridDim.y;
+            if (y < a.tiles_y) continue;
         }
-    }
+        break;
+    } while (true);
 }
 
 // The runs' partial sums, added in order; V neighbouring outputs of a row a thread.
@@ -363,22 +412,25 @@ __global__ void __launch_bounds__(128) add_runs_kernel(Args a)
     }
 }
 
-template <int MT, int R> int go_stream(const Args& a, cudaStream_t s)
+template <int MT, int R, typename A> int go_stream(const A& a, bool early, cudaStream_t s)
 {
     const long tiles = fx_cdiv(a.N, R) * (long)(a.offsets ? a.G : 1), resident = 2L * fx_sm_count();
-    fx_launch_pdl(stream_kernel<MT, R>, dim3((unsigned)(tiles < resident ? tiles : resident)), SW * 32, 0, s, a);
+    fx_launch_pdl_if(early, stream_kernel<MT, R, A>, dim3((unsigned)(tiles < resident ? tiles : resident)), SW * 32, 0, s, a);
     return fx_launch_status();
 }
 
+template <typename K> int allow_smem(K kernel, size_t bytes)       // of the current device: asked for each time
+{
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+constexpr size_t tile_smem(int bm) { return sizeof(float) * STAGES * (bm + BN) * PITCH; }
+
 template <int BM> int go_tile(const Args& a, cudaStream_t s)
 {
-    const size_t smem = sizeof(float) * STAGES * (BM + BN) * PITCH;
-    // (of the current device: asked for each time)
-    const cudaError_t set = cudaFuncSetAttribute(tile_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (set != cudaSuccess) return (int)set;
     const long rows = fx_cdiv(a.M, BM) + (a.offsets ? a.G : 0);
     if (rows > 65535) return FX_ERR_SIZE;
-    fx_launch_pdl(tile_kernel<BM>, dim3((unsigned)fx_cdiv(a.N, BN), (unsigned)rows, (unsigned)a.splits), BM * 2, smem, s, a);
+    if (const int e = allow_smem(tile_kernel<BM, Args>, tile_smem(BM))) return e;
+    fx_launch_pdl(tile_kernel<BM, Args>, dim3((unsigned)fx_cdiv(a.N, BN), (unsigned)rows, (unsigned)a.splits), BM * 2, tile_smem(BM), s, a);
     if (a.splits > 1) {
         const int st = fx_launch_status();
         if (st != FX_OK) return st;
@@ -390,23 +442,42 @@ template <int BM> int go_tile(const Args& a, cudaStream_t s)
     return fx_launch_status();
 }
 
+// The stream kernel, and where the groups' sizes are to decide the tiles before it: neither set up early beside the other, whose
+// registers and L1 it would sit on while it has nothing to do (281 us became 400).
+template <int MT, int R> int go_few(const Args& a, int* picked, cudaStream_t s)
+{
+    if (!picked) return go_stream<MT, R>(a, true, s);
+    constexpr int BM = 32;
+    PickArgs p;
+    static_cast<Args&>(p) = a;
+    p.pass = MT; p.sms = fx_sm_count(); p.tiles_y = (int)(fx_cdiv(a.M, BM) + a.G); p.picked = picked;
+    const long cols = fx_cdiv(a.N, BN), at_once = fx_cdiv(4L * p.sms, cols), y = at_once < p.tiles_y ? at_once : p.tiles_y;
+    if (const int e = allow_smem(tile_kernel<BM, PickArgs>, tile_smem(BM))) return e;
+    fx_launch_pdl_if(false, tile_kernel<BM, PickArgs>, dim3((unsigned)cols, (unsigned)y), BM * 2, tile_smem(BM), s, p);
+    if (const int e = fx_launch_status()) return e;
+    return go_stream<MT, R>(p, false, s);
+}
+
 }  // namespace
 
 // `form` > 0: the tile kernel with that many rows a tile (128, 64, 32) and K cut into `splits` runs (partial sums in
-// `part`, splits * M * N floats; not with groups).  `form` < 0: the stream kernel with -form rows a pass (1, 2, 4, 8).
+// `part`, splits * M * N floats; not with groups).  `form` < 0: the stream kernel with -form rows a pass (1, 2, 4, 8); with
+// groups and `splits` 2 that or tiles of 32 rows, as the groups' sizes say (two launches; `part` holds an int).
 extern "C" int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long ldw, const void* bias,
                            int bias_dtype, void* C, long ldc, int accumulate, int M, int N, int K,
                            const int* group_offsets, int n_groups, long w_group_stride, int form, int splits, void* part,
                            void* stream)
 {
     if (M <= 0 || N <= 0) return FX_OK;
-    if (K <= 0 || splits < 1 || (splits > 1 && (group_offsets || !part))) return FX_ERR_SIZE;
+    if (K <= 0 || splits < 1 || (splits > 1 && (!part || (group_offsets ? form >= 0 || splits > 2 : form < 0)))) return FX_ERR_SIZE;
     if (K % 4 || lda % 4 || ldw % 4 || w_group_stride % 4 || (uintptr_t)A % 16 || (uintptr_t)W % 16) return FX_ERR_ALIGN;
     if (form < 0 && group_offsets && n_groups > MAX_ACTIVE) return FX_ERR_SIZE;
     Args a;
     a.A = (const float*)A; a.lda = lda; a.a_rows = a_rows; a.W = (const float*)W; a.ldw = ldw; a.w_gs = w_group_stride;
     a.bias = bias; a.bias_dtype = bias_dtype; a.C = (float*)C; a.ldc = ldc; a.accumulate = accumulate;
-    a.M = M; a.N = N; a.K = K; a.offsets = group_offsets; a.G = n_groups; a.part = splits > 1 ? (float*)part : nullptr;
+    a.M = M; a.N = N; a.K = K; a.offsets = group_offsets; a.G = n_groups; a.part = splits > 1 && !group_offsets ? (float*)part : nullptr;
+    int* picked = group_offsets && splits > 1 ? (int*)part : nullptr;
+    if (picked) splits = 1;
     a.split_len = (int)(fx_cdiv(fx_cdiv(K, splits), BK) * BK);
     a.splits = splits;
     cudaStream_t s = (cudaStream_t)stream;
@@ -414,10 +485,10 @@ extern "C" int fx_gemm_f32(const void* A, long lda, const int* a_rows, const voi
         case 128: return go_tile<128>(a, s);
         case 64: return go_tile<64>(a, s);
         case 32: return go_tile<32>(a, s);
-        case -1: return go_stream<1, 8>(a, s);
-        case -2: return go_stream<2, 8>(a, s);
-        case -4: return go_stream<4, 8>(a, s);
-        case -8: return go_stream<8, 4>(a, s);
+        case -1: return go_few<1, 8>(a, picked, s);
+        case -2: return go_few<2, 8>(a, picked, s);
+        case -4: return go_few<4, 8>(a, picked, s);
+        case -8: return go_few<8, 4>(a, picked, s);
     }
     return FX_ERR_SIZE;
 }

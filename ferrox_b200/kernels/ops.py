@@ -359,10 +359,13 @@ def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=N
     if (a.dtype == w.dtype == out.dtype == torch.float32 and M > 0 and N > 0 and K > 0 and K % 4 == 0 and _rows(a) % 4 == 0
             and ldw % 4 == 0 and wstride % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and a.is_cuda):
         form, splits = gemm_f32_plan(M, N, K, G if group_offsets is not None else None)
-        part = torch.empty(splits * M * N, dtype=torch.float32, device=out.device) if splits > 1 else None
+        part = None
+        if splits > 1:       # the runs' partial sums; of groups which of the two kernels it is
+            part = torch.empty(splits * M * N if group_offsets is None else 1, dtype=torch.float32, device=out.device)
         call("fx_gemm_f32", _ptr(a), _rows(a), _ptr(a_rows), _ptr(w), ldw, _ptr(bias), code(bias) if bias is not None else 0,
              _ptr(out), _rows(out), int(accumulate), M, N, K, _ptr(group_offsets), G, wstride, form, splits, _ptr(part),
              stream if stream is not None else stream_ptr())
+        count_launches(int(splits > 1))      # (the runs' sums; the second of two kernels)
         return out
     call(
         "fx_gemm", _ptr(a), code(a), _rows(a), _ptr(a_rows), _ptr(w), code(w), ldw,
@@ -387,12 +390,13 @@ def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
     tiles and 6 runs; 16 x 2048 x 2048: 12.3 against 20.2 us; 60 x 2048 x 5632: 46 us in 8 runs, 312 us in one).  The partial
     sums stay within F32_WORKSPACE_MAX: where there are many tiles, runs of K save a part of one round of them, and an engine
     whose pages fill the device has no room for a gigabyte (597 x 151936 x 16384 in 3 runs).
-    Of groups, the mean number of rows decides: 4 rows a pass up to 6 rows a group (60 experts of 2816 x 2048, 4 rows
-    each: 332 us against 532 us in 32-row tiles; 13 rows each: 922 against 536 us)."""
+    Of groups, the mean number of rows decides: 2 or 4 rows a pass up to 6 rows a group (60 experts of 2816 x 2048, 4 rows
+    each: 281 us against 527 us in 32-row tiles; 6.7 rows each: 465 against 529 us), the latter number then being 1 where no
+    distribution of so few rows (64) is better off in tiles, and 2 where the kernels decide by the groups' sizes."""
     if groups is not None:
         if M > 6 * groups or groups > 1024:
             return (32 if M <= 1 << 20 else 128), 1
-        return (-2 if M <= groups else -4), 1
+        return (-2 if M <= groups else -4), (1 if M <= 64 else 2)
     if M <= 4:
         return -(1 if M == 1 else 2 if M == 2 else 4), 1
     sms, n_tiles = sm_count(), -(-N // 128)

@@ -168,4 +168,8 @@ def test_32_bit_product_plans_by_size():
                 assert form in (-8, 32, 64, 128) and 1 <= splits <= 16 and (form > 0 or splits == 1)
                 assert splits == 1 or (4 * splits * m * n <= ops.F32_WORKSPACE_MAX and splits * 128 <= k)
                 assert form < 0 or -(-m // form) <= 65535
+    # groups: 2 or 4 rows a pass, from 65 rows on with a second kernel beside it, tiles above 6 rows a group
+    assert [ops.gemm_f32_plan(m, 2816, 2048, 60) for m in (8, 60, 64, 65, 360, 361)] == [
+        (-2, 1), (-2, 1), (-4, 1), (-4, 2), (-4, 2), (32, 1)]
+    assert ops.gemm_f32_plan(100, 2816, 2048, 128) == (-2, 2) and ops.gemm_f32_plan(3000, 64, 64, 1025) == (32, 1)
     assert ops.gemm_f32_plan(60, 2048, 5632)[1] > 1 and ops.gemm_f32_plan(517, 15616, 2048)[1] > 1

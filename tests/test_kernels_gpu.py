@@ -89,6 +89,34 @@ def test_gemm_f32_groups(form, monkeypatch):
     assert rel(out, want) < 3e-6
 
 
+@pytest.mark.parametrize("counts,tiles", [([6] * 40, False), ([1] * 39 + [100], False), ([0] * 39 + [240], True),
+                                          ([0] * 17 + [60, 60, 60, 60] + [0] * 19, True), ([0] * 40, False)])
+def test_gemm_f32_groups_go_by_their_sizes(counts, tiles, monkeypatch):
+    """Up to 6 rows a group on average: weights streamed, unless a few groups have most rows; the results are those of the one
+    kernel or of the other, bit for bit, and all there."""
+    o = ops()
+    M, G, N, K = 240, len(counts), 2048, 2048
+    w = torch.randn(G, N, K, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+    x, off = rnd(M, K), [0]
+    for c in counts:
+        off.append(off[-1] + c)
+    offsets = torch.tensor(off, dtype=torch.int32, device=DEV)
+    out = torch.full((M, N), 3.0, device=DEV)
+    o.gemm(x, w, out, group_offsets=offsets)
+    plan = o.gemm_f32_plan(M, N, K, G)
+    alone = {}
+    for name, form in (("stream", plan[0]), ("tiles", 32)):
+        monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (form, 1))
+        alone[name] = torch.full((M, N), 3.0, device=DEV)
+        o.gemm(x, w, alone[name], group_offsets=offsets)
+    assert torch.equal(out, alone["tiles" if tiles else "stream"])
+    if off[-1]:
+        assert not torch.equal(alone["tiles"], alone["stream"])
+        want = torch.cat([x[off[g]:off[g + 1]].double() @ w[g].double().T for g in range(G)])
+        assert rel(out[:off[-1]], want) < 3e-6
+    assert bool((out[off[-1]:] == 3).all())
+
+
 def test_gemm_mixed_precision_weights_stay_32_bit():
     o = ops()
     a, w = rnd(5, 96, dtype=torch.bfloat16), rnd(40, 96, dtype=torch.float32)
