@@ -162,8 +162,7 @@ class SoftmaxTopkMoe(FeedForward):
             self.w_route = torch.cat([self.w_router.to(dtr), self.w_shared_gate.to(dtr)], dim=0).contiguous()
         self._scratch = torch.zeros(2 * E, dtype=torch.int32, device=rt.device)
         if self.w_shared_gu is not None and rt.device.type == "cuda":
-            # one second stream for all such layers of a model (they run one after the other): its buffers are the
-            # same in every layer, and a new model's first step asks the device for them once
+            # one second stream for all such layers of a model: they run one after the other
             self._side = rt.groups.get("side stream")
             if self._side is None:
                 self._side = rt.groups["side stream"] = torch.cuda.Stream(device=rt.device)
@@ -206,27 +205,19 @@ class SoftmaxTopkMoe(FeedForward):
         l = self._table_index
         return w, offsets[l], src_token[l], inv_perm[l], active[l] if small else None
 
-    def _shared_expert(self, x, batch, st):
-        """silu(gate) * up, then down, of the expert that every token visits: [T, H]."""
-        s, rt = self.spec, self.rt
-        T, Is = x.shape[0], s.shared_intermediate
-        sact = rt.empty(T, Is)
-        if self.plain:
-            ops.linear(x, self.w_shared_gu, sact, status=batch.status, stream=st, activation=self.plain)
-        else:
-            ops.gated_linear(x, self.w_shared_gu, sact, status=batch.status, stream=st, activation=self.shared_activation)
-        shared = rt.empty(T, s.hidden)
-        ops.linear(sact, self.w_shared_down, shared, status=batch.status, stream=st)
-        return shared
-
-    def _shared_on_side(self, x, batch):
-        """The shared expert's two products on the second stream, from the point the fork event marks."""
+    def _shared_on_side(self, x, batch, sact, shared):
+        """The shared expert's two products, silu(gate) * up (``sact``), then down (``shared``), on the second stream, from
+        the point the fork event marks."""
         side = self._side_in_graph if torch.cuda.is_current_stream_capturing() else self._side
         side.wait_event(self._fork)
         with torch.cuda.stream(side):
-            out = self._shared_expert(x, batch, side.cuda_stream)
+            st = side.cuda_stream
+            if self.plain:
+                ops.linear(x, self.w_shared_gu, sact, status=batch.status, stream=st, activation=self.plain)
+            else:
+                ops.gated_linear(x, self.w_shared_gu, sact, status=batch.status, stream=st, activation=self.shared_activation)
+            ops.linear(sact, self.w_shared_down, shared, status=batch.status, stream=st)
             self._join.record(side)
-        return out
 
     def forward_add(self, x, h, batch, then_norm=None):
         st = batch.stream
@@ -253,6 +244,24 @@ class SoftmaxTopkMoe(FeedForward):
     def expert_rows(self, x, batch):
         """The experts' results: (rows in expert order [T * K, H], each (token, rank) pair's row, the weights they are
         added up with (None: as they are), the shared expert's rows or None, its gate's logits or None)."""
+        if self.w_shared_gu is None:
+            return self._expert_rows(x, batch, None)
+        # The shared expert's two products run on a second stream beside the routing and the routed experts; both
+        # meet again at the combination.  In a decode step the routed experts' kernels leave most of the machine
+        # idle; in a prompt the router's short kernels hide under the shared expert's products.  Measured on a
+        # B200: 3 to 10 % of a decode step of 8 to 64 tokens, 14 % of a prompt portion of 256 tokens, 4 % at 2,048.
+        # Their buffers are this stream's, asked for before the fork and held until it has waited for the join: memory
+        # that another stream asked for is found again by that stream only, and a new model's first prompt, on a
+        # stream nobody had used, waited for the device's allocations (2,048 tokens, 4 layers: 3.5 to 150 ms; 2.7 so).
+        main = torch.cuda.current_stream()
+        held = self.rt.empty(x.shape[0], self.spec.shared_intermediate), self.rt.empty(x.shape[0], self.spec.hidden)
+        self._fork.record(main)          # the shared expert may start from here on
+        try:
+            return self._expert_rows(x, batch, held)
+        finally:
+            main.wait_event(self._join)
+
+    def _expert_rows(self, x, batch, held):
         s, rt, st = self.spec, self.rt, batch.stream
         T, E, K, I, H = x.shape[0], s.n_experts, s.top_k, s.expert_intermediate, s.hidden
         i32 = torch.int32
@@ -266,18 +275,8 @@ class SoftmaxTopkMoe(FeedForward):
         tiles = expert_tile_tokens(T, K, E) if tc and T >= SWAP_MIN_TOKENS and E <= ops.TC_SWAP_MAX_GROUPS else None
         small = tiles is None and T <= ops.SKINNY_MAX_TOKENS and ops.skinny_ok(x, self.w_gu) and I % 32 == 0
         big = T > ops.SKINNY_MAX_TOKENS and tc
-        # The shared expert's two products run on a second stream beside the routing and the routed experts; both
-        # meet again at the combination.  In a decode step the routed experts' kernels leave most of the machine
-        # idle; in a prompt the router's short kernels hide under the shared expert's products.  Measured on a
-        # B200: 3 to 10 % of a decode step of 8 to 64 tokens, 14 % of a prompt portion of 256 tokens, 4 % at 2,048.
-        shared = None
-        overlap = self.w_shared_gu is not None
-
-        if overlap:
-            main = torch.cuda.current_stream()
-            self._fork.record(main)          # the shared expert may start from here on
-            if not fused:
-                shared = self._shared_on_side(x, batch)
+        if held is not None and not fused:
+            self._shared_on_side(x, batch, *held)
         if table:
             weights, offsets, src_token, inv_perm, active = self._route_by_table(batch, T, small)
         else:
@@ -299,8 +298,8 @@ class SoftmaxTopkMoe(FeedForward):
             xp = rt.empty(T * K, H) if tiles is not None or scaled else None
             ops.route_fused(x, self.w_route, logits, K, mode | (4 if scaled else 0), ids, weights, offsets, src_token, inv_perm, active,
                             n_experts=E, xp_out=xp, stream=st, extra=extra)
-            if overlap:
-                shared = self._shared_on_side(x, batch)
+            if held is not None:
+                self._shared_on_side(x, batch, *held)
         elif T <= ops.ROUTE_SMALL_MAX_TOKENS and E <= ops.ROUTE_SMALL_MAX_EXPERTS:
             ops.linear(x, self.w_route, logits, status=batch.status, stream=st)
             ops.route_small(logits, K, mode, ids, weights, offsets, src_token, inv_perm, active,
@@ -351,15 +350,9 @@ class SoftmaxTopkMoe(FeedForward):
                 ops.silu_mul(gu, act, stream=st, activation=self.activation)
             ops.gemm(act, self.w_down, y, group_offsets=offsets, stream=st)
 
-        gate_logit = None
-        if self.w_shared_gu is not None:
-            if overlap:
-                main.wait_event(self._join)
-            else:
-                shared = self._shared_expert(x, batch, st)
-            if self.w_shared_gate is not None:
-                gate_logit = logits[:, E:]      # [T, 1] view with the logits' row stride
-        return y, inv_perm, None if scaled else weights, shared, gate_logit
+        # [T, 1] view with the logits' row stride
+        gate_logit = logits[:, E:] if self.w_shared_gate is not None else None
+        return y, inv_perm, None if scaled else weights, held[1] if held is not None else None, gate_logit
 
 
 register_part("softmax_topk_moe", SoftmaxTopkMoe, replace=True)

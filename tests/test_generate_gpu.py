@@ -44,6 +44,25 @@ def test_greedy_generation_matches_plain(folders, name):
     assert eng.cache.n_free_slots == 4
 
 
+def test_a_new_engine_finds_the_buffers_that_an_earlier_one_left(folders):
+    """The first prompt of a process's third engine asks the device for no memory: what its shared experts need beside the
+    step's stream is found where the engines before it left it."""
+    import gc
+
+    from ferrox_b200 import StepEntry
+
+    for n in range(4):
+        eng = engine(folders["A"], dtype="bfloat16")
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["num_device_alloc"]
+        eng.step([StepEntry(eng.open_request(), list(range(1, 90)), want=[88])])
+        torch.cuda.synchronize()
+        asked = torch.cuda.memory_stats()["num_device_alloc"] - before
+        assert n < 2 or asked == 0, (n, asked)
+        del eng
+        gc.collect()
+
+
 def test_generation_with_preemption_gives_the_same_tokens(folders):
     cfg, w = plain.load_model(folders["A"])
     prompts = [[i + 1, i + 3, i + 7, 99, 4, 8, 15, 16] for i in range(4)]
