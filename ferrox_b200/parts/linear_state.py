@@ -52,23 +52,38 @@ from .base import Mixer, register_part
 FIXED_DECAY_MIN_TOKENS = 32
 
 
-def _chunk_tiles(batch, H, V):
-    """The step's entries cut into chunks of tokens (the work list of ``ops.chunk_scan``) where that form of a recurrence
-    is the faster one, else None.
+# Both forms of a recurrence in microseconds on a B200, by (heads x columns x (rows of a tile + 64)) in millions, w:
+#   in chunks         c0 + max(c1 a chunk of the longest entry, c2 w a chunk of all entries and 0.45 chunks' worth an entry)
+#   token by token    t0 + max(t1 a token of the longest entry, t2 w a token of all entries)
+# Fitted to 286 measurements: 2 to 64 heads of 32, 64 and 128 rows, 32 to 256 columns; single prompts of 32 to 2,048 tokens, 4 of
+# 500, 8 of 64, 16 of 32, and 40, 53 and 200 tokens beside 7 or 16 decoded ones.  Chosen by it a recurrence takes 1.01 times the
+# faster form's time on average, and nowhere more than 1.05 times that of token by token.  (16 heads of 128 x 128, delta: 64
+# tokens 31 against 19, 2,048 870 against 247; 16 prompts of 32 85 against 93; 64 heads, 2,048 tokens: 1,132 against 983, mLSTM
+# 1,858 against 732.)
+_CHUNK_COSTS = {          # c0, c1, c2, t0, t1, t2
+    "delta": (8.0, 3.6, 10.0, 2.0, 0.37, 0.36),
+    "mlstm": (9.0, 3.4, 7.0, 2.0, 0.325, 0.47),
+    "general": (13.0, 4.7, 17.5, 4.0, 0.42, 0.7),
+}
 
-    In microseconds on a B200, 16 heads of 128 x 128 (32 of 64 x 64 likewise): token by token 0.33 to 0.43 a token of the
-    longest entry, and at least 0.13 a token of the step; in chunks 10 and 4.2 a chunk of the longest entry, or of all
-    entries where their blocks (16 columns of a head each) need more than the device's SMs (one prompt of 64 tokens: 31
-    against 19, of 2,048: 868 against 258; 40 tokens beside 16 decoded ones: 39 against 94; four prompts of 500: 267
-    against 289)."""
-    chunk, most, T = ops.SCAN_CHUNK, batch.max_new, batch.n_tokens
+
+def chunks_better(kind, lens, H, D, V) -> bool:
+    """Whether the recurrence ``kind`` of H heads of D rows and V columns over entries of ``lens`` tokens goes in chunks."""
+    c0, c1, c2, t0, t1, t2 = _CHUNK_COSTS[kind]
+    chunk, most = ops.SCAN_CHUNK, max(lens)
     if most < chunk:
+        return False
+    w = H * V * ((64 if D <= 64 else 128) + 64) / 1e6
+    chunks = sum(-(-n // chunk) for n in lens) + 0.45 * len(lens)
+    return c0 + max(c1 * -(-most // chunk), c2 * chunks * w) < t0 + max(t1 * most, t2 * sum(lens) * w)
+
+
+def _chunk_tiles(batch, kind, H, D, V):
+    """The step's entries cut into chunks of tokens (the work list of ``ops.chunk_scan``) where that form of a recurrence
+    is the faster one, else None."""
+    if batch.max_new < ops.SCAN_CHUNK or not chunks_better(kind, [len(e.tokens) for e in batch.entries], H, D, V):
         return None
-    chunks = sum(-(-len(e.tokens) // chunk) for e in batch.entries)
-    rounds = max(-(-most // chunk), chunks * H * -(-V // 16) / ops.sm_count())
-    if 10 + 4.2 * rounds >= max(0.38 * most, 0.13 * T):
-        return None
-    return query_tiles(batch, chunk)
+    return query_tiles(batch, ops.SCAN_CHUNK)
 
 
 def _cat_rows(tensors):
@@ -151,7 +166,7 @@ class GatedDeltaRule(_StateMixer):
                                  stream=batch.stream)
         read = rt.empty(T, self.vv, dtype=f32)
         q, k, v = qkv[:, :self.qk], qkv[:, self.qk:2 * self.qk], qkv[:, 2 * self.qk:]
-        tiles = _chunk_tiles(batch, H, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
+        tiles = _chunk_tiles(batch, "delta", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
         if tiles is not None:
             ops.chunk_scan(q, k, v, g, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
                            beta=beta, scratch=self._scratch, status=batch.status, stream=batch.stream)
@@ -269,7 +284,7 @@ class GeneralDeltaRule(_StateMixer):
         a_pre, low = proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:]
         read, state = rt.empty(T, hd, dtype=f32), cache.states["matrix"]
         # (a rate of at most 1: a chunk's products of decays stay above 1e-14, far from the end of 32-bit numbers)
-        tiles = _chunk_tiles(batch, H, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
+        tiles = _chunk_tiles(batch, "general", H, D, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
         if tiles is not None:
             ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, tiles,
                                    batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, scratch=self._scratch,
@@ -347,7 +362,7 @@ class Mlstm(_StateMixer):
         gates = proj[:, 2 * self.qk + 2 * self.vv:]       # [i | f] as projected
         read = rt.empty(T, self.vv, dtype=f32)
         matrix, norm, log_max = (cache.states[n] for n in ("matrix", "normalizer", "log_max"))
-        tiles = _chunk_tiles(batch, H, V) if ops.chunk_scan_ok((q, k, v), D, V, matrix) else None
+        tiles = _chunk_tiles(batch, "mlstm", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, matrix) else None
         if tiles is not None:
             keep, take, floor = rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32)
             before = rt.empty(batch.n_seqs, H, D, dtype=f32)

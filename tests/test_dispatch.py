@@ -173,3 +173,19 @@ def test_32_bit_product_plans_by_size():
         (-2, 1), (-2, 1), (-4, 1), (-4, 2), (-4, 2), (32, 1)]
     assert ops.gemm_f32_plan(100, 2816, 2048, 128) == (-2, 2) and ops.gemm_f32_plan(3000, 64, 64, 1025) == (32, 1)
     assert ops.gemm_f32_plan(60, 2048, 5632)[1] > 1 and ops.gemm_f32_plan(517, 15616, 2048)[1] > 1
+
+
+def test_which_steps_take_a_recurrence_in_chunks():
+    """Decisions where the two forms were measured more than a tenth apart."""
+    from ferrox_b200.parts.linear_state import chunks_better
+
+    for kind in ("delta", "mlstm", "general"):
+        assert not chunks_better(kind, [31], 16, 128, 128) and not chunks_better(kind, [1] * 16 + [40], 16, 128, 128)
+        for heads, d in ((2, 64), (4, 32), (16, 128), (32, 64), (64, 128), (64, 64)):
+            assert chunks_better(kind, [2048], heads, d, d) and chunks_better(kind, [512], heads, d, d) or (kind, heads) == ("delta", 64)
+        assert chunks_better(kind, [64], 2, 64, 64) and chunks_better(kind, [128], 16, 128, 128)
+    # many short entries: a state is read and written for every chunk
+    assert not chunks_better("delta", [32] * 16, 4, 128, 128) and not chunks_better("delta", [32] * 16, 64, 128, 128)
+    assert not chunks_better("general", [32] * 16, 4, 128, 128) and not chunks_better("general", [32] * 16, 64, 64, 64)
+    assert chunks_better("mlstm", [32] * 16, 16, 128, 128) and chunks_better("mlstm", [500] * 4, 64, 128, 128)
+    assert chunks_better("delta", [500] * 4, 64, 128, 128) and chunks_better("delta", [500] * 4, 64, 64, 64)
