@@ -967,6 +967,56 @@ def test_prompt_attention_on_mma_keeps_32_bit_scores_and_weights(kernel):
     assert bool((got[0] == 0).all()) and bool(((got[1] - want).abs() < want / 8).all())
 
 
+EDGES = [     # kernel, head widths of keys and values, page, options
+    ("prefill", 64, 64, 32, {}), ("prefill", 48, 48, 96, dict(window=33)), ("prefill", 128, 128, 64, dict(window=64)),
+    ("prefill", 64, 64, 4, dict(window=97)), ("general", 64, 64, 64, {}), ("general", 64, 128, 96, dict(window=65)),
+    ("general", 48, 80, 32, dict(window=64, keep_first=4)), ("general", 64, 64, 64, dict(window=32, keep_first=70)),
+    ("general", 192, 128, 32, dict(window=31, keep_first=33)), ("general", 64, 64, 64, dict(chunk=64)),
+    ("general", 80, 48, 20, dict(chunk=100)), ("general", 128, 128, 128, dict(window=128, softcap=5.0)),
+]
+
+
+@pytest.mark.parametrize("kernel,d,dv,page,options", EDGES)
+def test_every_query_sees_its_keys_and_no_other(kernel, d, dv, page, options):
+    """Queries of zeros weigh all keys that they see alike, and key j's value is the unit vector j mod width: the result counts the
+    keys seen, one by one.  Portions that begin and end at and beside the edges of blocks of 32 and 64 keys, windows, kept first
+    positions, chunks and pages; and, one token a request, keys cut into runs."""
+    o = ops()
+    nh, nkv = 4, 2
+    portions = [(1, 0, 200), (2, 31, 34), (3, 64, 65), (4, 127, 1), (5, 189, 4), (6, 95, 97)]
+    lens = [a + n for _, a, n in portions]
+    kp, _, table, _, _ = build_cache(torch.bfloat16, lens, nkv, d, page, n_pages=sum(-(-L // page) for L in lens) + 2)
+    # (rows of no request and positions behind a request's last hold what must not be seen)
+    vp = torch.full((kp.shape[0], nkv, page, dv), 1e4, dtype=torch.bfloat16, device=DEV)
+    for slot, L in enumerate(lens, 1):
+        for j in range(L):
+            vp[int(table[slot, j // page]), :, j % page] = torch.nn.functional.one_hot(torch.tensor(j % dv), dv).to(DEV)
+    window, keep, chunk = (options.get(x) or 0 for x in ("window", "keep_first", "chunk"))
+
+    def seen(pos):
+        return [j for j in range(pos + 1) if (not window or j > pos - window or j < keep) and (not chunk or j // chunk == pos // chunk)]
+
+    def check(out, tokens):
+        for row, pos in zip(out.double().cpu().view(len(tokens), nh, dv), tokens):
+            keys = seen(pos)
+            want = torch.bincount(torch.tensor(keys) % dv, minlength=dv).double() / len(keys)
+            assert ((row - want).abs() <= 2.0 ** -8 * want).all(), pos
+
+    tokens = [p for _, a, n in portions for p in range(a, a + n)]
+    q = torch.zeros(len(tokens), nh * d, dtype=torch.bfloat16, device=DEV)
+    check(mma_attention(kernel, q, kp, vp, table, page, portions, nh, nkv, **options), tokens)
+    if kernel == "general":
+        as_int = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        last, n = [L - 1 for L in lens], len(lens)
+        for splits in (1, 3):
+            out = torch.empty(n, nh * dv, dtype=torch.bfloat16, device=DEV)
+            part_o, part_ml = torch.empty(n, nh, splits, dv, device=DEV), torch.empty(n, nh, splits, 2, device=DEV)
+            o.general_attention(q[:n], q.stride(0), d, kp, vp, d, dv, table, page, as_int(last), as_int(list(range(n))),
+                                as_int(list(range(1, n + 1))), None, out, nh * dv, dv, nh, nkv, d, dv, scale=1.0, n_splits=splits,
+                                part_o=part_o, part_ml=part_ml, **dict(dict(window=0), **options))
+            check(out, last)
+
+
 TC_ATT_CASES = [
     # nh, nkv, d, page, window, lengths
     (16, 16, 128, 64, 0, [300, 64, 65]),
