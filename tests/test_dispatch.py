@@ -189,3 +189,28 @@ def test_which_steps_take_a_recurrence_in_chunks():
     assert not chunks_better("general", [32] * 16, 4, 128, 128) and not chunks_better("general", [32] * 16, 64, 64, 64)
     assert chunks_better("mlstm", [32] * 16, 16, 128, 128) and chunks_better("mlstm", [500] * 4, 64, 128, 128)
     assert chunks_better("delta", [500] * 4, 64, 128, 128) and chunks_better("delta", [500] * 4, 64, 64, 64)
+
+
+def test_what_the_delta_rule_needs_first_by_runs_of_tokens_or_a_token_a_block(monkeypatch):
+    """Runs of tokens take prompts from 128 tokens on, 32-bit rows on the 16-byte grid, heads of 64 and 128, four taps; the rest,
+    and steps that move the tail on, a block a token."""
+    import torch
+
+    called = []
+    monkeypatch.setattr(ops, "call", lambda name, *args: called.append(name))
+    monkeypatch.setattr(ops, "_ptr", lambda t: 0)      # (no device here)
+
+    def kernel(T=128, G=2, D=64, H=2, V=64, taps=4, cols=0, at=0, dtype=torch.float32, **more):
+        C = 2 * G * D + H * V
+        proj = torch.empty(T, C + cols + at, dtype=dtype)[:, at:]
+        rows = lambda n: torch.empty(T, n)
+        ops.delta_prep(proj, torch.empty(C, taps), taps, torch.empty(1, taps - 1, C), rows(2 * H), rows(1), rows(1),
+                       torch.empty(T, dtype=torch.int32), torch.empty(1, dtype=torch.int32), rows(C), rows(H), rows(H), G, D, H, V,
+                       stream=0, **more)
+        return called.pop()
+
+    for taken in (dict(), dict(T=3001), dict(D=128, G=1), dict(V=62), dict(cols=4), dict(H=3, V=4)):
+        assert kernel(**taken) == "fx_delta_prep_runs", taken
+    for refused in (dict(T=127), dict(T=1), dict(update_tail=True), dict(taps=3), dict(D=96), dict(G=1, D=32), dict(V=61), dict(cols=2),
+                    dict(at=1, cols=3), dict(dtype=torch.bfloat16)):
+        assert kernel(**refused) == "fx_delta_prep", refused
