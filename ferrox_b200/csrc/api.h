@@ -18,6 +18,11 @@ int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long 
                 void* C, long ldc, int accumulate, int M, int N, int K, const int* group_offsets, int n_groups,
                 long w_group_stride, int form, int splits, void* part, void* stream);
 
+// The same for many rows on the tensor cores, each operand as three bfloat16 parts (gemm_f32_tc.cu); n_tile: rows of X a tile
+// (16 .. 208, steps of 16); `work`: see there.
+int fx_gemm_f32_tc(const void* X, long ldx, const void* W, long ldw, const void* bias, int bias_dtype, void* C, long ldc,
+                   int accumulate, int M, int N, int K, int n_tile, void* work, long work_bytes, int* status, void* stream);
+
 // Zeros at a slot of every tensor of a table (elementwise.cu).
 int fx_zero_slots(const long* table, int n, long most, long slot, void* stream);
 

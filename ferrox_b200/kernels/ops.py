@@ -38,6 +38,7 @@ _SIGNATURES = {
     "fx_set_scan_lanes": [_I],
     "fx_gemm": [_P, _I, _L, _P, _P, _I, _L, _P, _I, _P, _I, _L, _I, _I, _I, _I, _P, _I, _L, _P],
     "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
+    "fx_gemm_f32_tc": [_P, _L, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
     "fx_zero_slots": [_P, _I, _L, _L, _P],
     "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
@@ -339,10 +340,10 @@ class SlotZeroer:
 
 
 # ---------------------------------------------------------------------------
-def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=None, stream=None):
+def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=None, status=None, stream=None):
     """out[M,N] (+)= a[M,K] . w[N,K]^T (+ bias).  With ``group_offsets`` ([G+1],
     int32) ``w`` is [G,N,K] and rows off[g]..off[g+1] use matrix g; ``a_rows``
-    gathers rows of ``a``."""
+    gathers rows of ``a``.  ``status``: the step's word for a kernel that gives up waiting."""
     M, N = out.shape
     if group_offsets is not None:
         G, Nw, K = w.shape
@@ -359,6 +360,10 @@ def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=N
     if (a.dtype == w.dtype == out.dtype == torch.float32 and M > 0 and N > 0 and K > 0 and K % 4 == 0 and _rows(a) % 4 == 0
             and ldw % 4 == 0 and wstride % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and a.is_cuda):
         form, splits = gemm_f32_plan(M, N, K, G if group_offsets is not None else None)
+        if form > 0 and group_offsets is None and a_rows is None:
+            tile = gemm_f32_tc_tile(M, N, K)
+            if tile:
+                return _gemm_f32_tc(a, w, out, tile, bias, accumulate, status, stream)
         part = None
         if splits > 1:       # the runs' partial sums; of groups which of the two kernels it is
             part = torch.empty(splits * M * N if group_offsets is None else 1, dtype=torch.float32, device=out.device)
@@ -376,6 +381,55 @@ def gemm(a, w, out, *, bias=None, accumulate=False, a_rows=None, group_offsets=N
 
 
 F32_WORKSPACE_MAX = 1 << 27      # bytes of partial sums a 32-bit product may ask for beside its operands
+F32_TC_MIN_K = 1024
+F32_TC_MAX_TILE = 208
+
+
+def _f32_tc_rows(K: int) -> int:
+    """Rows of the tensor-core kernel's first operand whose parts (6 bytes an element) fit the workspace beside the shares of the
+    tiles that it cuts along K."""
+    return (F32_WORKSPACE_MAX - sm_count() * F32_TC_MAX_TILE * 1024) // (6 * (-(-K // 8) * 8))
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_f32_tc_tile(M: int, N: int, K: int) -> int:
+    """Rows a tile if a 32-bit product that would go to the FFMA tiles is to go to the tensor cores in three parts
+    (gemm_f32_tc.cu), or 0.
+
+    Times in microseconds, as measured on a B200: a stage of 32 elements of K takes 0.70 and 0.0018 a row of the tile, the three
+    kernels 11 beside that, the shares of the tiles that are cut are written and read at 6 TB/s.  12 x 3072 x 2048: 18 against 25;
+    517 x 15616 x 2048: 172 against 805; 64 x 60 x 2048: 16 against 21; 16 x 2048 x 2048 stays with the weight-streaming kernel
+    (13).  Errors against 64-bit sums there: 1.3e-7 to 2.9e-7 (a relative 2-norm), of the FFMA tiles 1.6e-7 to 7.9e-7; with
+    fewer than 1,024 elements of K their chains are as short as this kernel's and their errors no larger, so those stay."""
+    rows = min(M, _f32_tc_rows(K))
+    if K < F32_TC_MIN_K or rows < min(M, F32_TC_MAX_TILE):
+        return 0
+    sms = sm_count()
+    m = -(-M // -(-M // rows))           # rows a call
+    per = -(-m // F32_TC_MAX_TILE)
+    tile = 16 * -(-m // (16 * per))
+    tiles, stages = per * -(-N // 128), -(-K // 32)
+    cut = tiles % sms
+    shares = min(sms, max(cut, cut * stages // 4))
+    t = 11.0 + (tiles // sms * stages + (-(-cut * stages // shares) if cut else 0)) * (0.70 + 0.0018 * tile)
+    t += (shares + cut) * tile * 1024.0 / 6e6
+    return tile if t * -(-M // m) < _gemm_f32_best(M, N, K)[0] else 0
+
+
+def _gemm_f32_tc(a, w, out, tile, bias, accumulate, status, stream):
+    M, N = out.shape
+    K = w.shape[1]
+    kp = -(-K // 8) * 8
+    m = -(-M // -(-M // _f32_tc_rows(K)))
+    work = torch.empty(6 * min(m, M) * kp + sm_count() * tile * 1024, dtype=torch.uint8, device=out.device)
+    for r in range(0, M, m):
+        n = min(m, M - r)
+        x, c = a[r:r + n], out[r:r + n]
+        call("fx_gemm_f32_tc", _ptr(x), _rows(a), _ptr(w), _rows(w), _ptr(bias), code(bias) if bias is not None else 0, _ptr(c),
+             _rows(out), int(accumulate), n, N, K, tile, _ptr(work), work.numel(), _ptr(status),
+             stream if stream is not None else stream_ptr())
+        count_launches(1 + int(-(-n // tile) * -(-N // 128) % sm_count() > 0))      # (the parts of a; the shares' sums)
+    return out
 
 
 @functools.lru_cache(maxsize=4096)
@@ -397,8 +451,13 @@ def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
         if M > 6 * groups or groups > 1024:
             return (32 if M <= 1 << 20 else 128), 1
         return (-2 if M <= groups else -4), (1 if M <= 64 else 2)
+    return _gemm_f32_best(M, N, K)[1:]
+
+
+def _gemm_f32_best(M: int, N: int, K: int):
+    """(microseconds, form, runs of K) of :func:`gemm_f32_plan` without groups."""
     if M <= 4:
-        return -(1 if M == 1 else 2 if M == 2 else 4), 1
+        return 2.0 + 4.0 * N * K / 6.2e6, -(1 if M == 1 else 2 if M == 2 else 4), 1
     sms, n_tiles = sm_count(), -(-N // 128)
     best = (-(-M // 8) * (2.0 + 4.0 * N * K / 3.1e6), -8, 1)
     for bm in (128, 64, 32):
@@ -414,7 +473,7 @@ def gemm_f32_plan(M: int, N: int, K: int, groups: Optional[int] = None):
                 t += 3.0 + splits * 8.0 * M * N / 5e6
             if t < best[0]:
                 best = (t, bm, splits)
-    return best[1], best[2]
+    return best
 
 
 def embed(table, ids, out, status=None, stream=None, scale=1.0):
@@ -1814,7 +1873,7 @@ def linear(x, w, out, *, bias=None, accumulate=False, status=None, stream=None, 
         if w.dim() == 2 and pairs_better(T, w.shape[0]):
             return gemm_tc2(x, w, out, bias=bias, accumulate=accumulate, unary=act, status=status, stream=stream)
         return gemm_tc(x, w, out, bias=bias, accumulate=accumulate, unary=act, status=status, stream=stream)
-    gemm(x, w, out, bias=bias, accumulate=accumulate, stream=stream)
+    gemm(x, w, out, bias=bias, accumulate=accumulate, status=status, stream=stream)
     return _apply_unary_(out, act, stream) if act else out
 
 
@@ -1835,7 +1894,7 @@ def gated_linear(x, w_gu, out, *, status=None, stream=None, activation="silu", b
             return gemm_tc2(x, w_gu, out, bias=bias, gated=gated, status=status, stream=stream)
         return gemm_tc(x, w_gu, out, bias=bias, gated=gated, status=status, stream=stream)
     gu = torch.empty(T, 2 * I, dtype=out.dtype, device=out.device)
-    gemm(x, w_gu, gu, bias=bias, stream=stream)
+    gemm(x, w_gu, gu, bias=bias, status=status, stream=stream)
     return silu_mul(gu, out, stream=stream, activation=activation)
 
 

@@ -214,3 +214,18 @@ def test_what_the_delta_rule_needs_first_by_runs_of_tokens_or_a_token_a_block(mo
     for refused in (dict(T=127), dict(T=1), dict(update_tail=True), dict(taps=3), dict(D=96), dict(G=1, D=32), dict(V=61), dict(cols=2),
                     dict(at=1, cols=3), dict(dtype=torch.bfloat16)):
         assert kernel(**refused) == "fx_delta_prep", refused
+
+
+def test_32_bit_products_that_go_to_the_tensor_cores():
+    """Many rows, 1,024 elements of K and more; workspaces within the limit; what the FFMA kernels are faster or nearer at stays."""
+    assert [ops.gemm_f32_tc_tile(m, 15616, 2048) for m in (12, 64, 208, 209, 517)] == [16, 64, 208, 112, 176]
+    assert ops.gemm_f32_tc_tile(517, 60, 2048) == 0 and ops.gemm_f32_tc_tile(517, 15616, 1020) == 0
+    assert ops.gemm_f32_tc_tile(65, 257, 2048) == 0 and ops.gemm_f32_tc_tile(16, 2048, 2048) == 0
+    for m in (9, 60, 209, 517, 2780, 70000):
+        for n in (61, 2048, 151936):
+            for k in (1024, 7808, 16384, 1 << 20):
+                tile = ops.gemm_f32_tc_tile(m, n, k)
+                assert tile % 16 == 0 and 0 <= tile <= ops.F32_TC_MAX_TILE
+                if tile:
+                    rows = min(m, ops._f32_tc_rows(k))
+                    assert rows >= min(m, 208) and 6 * rows * k + 148 * 1024 * tile <= ops.F32_WORKSPACE_MAX

@@ -68,6 +68,62 @@ def test_gemm_f32_forms(form, splits, M, N, K, monkeypatch):
     assert rel(acc, base + want) < 3e-6
 
 
+@pytest.mark.parametrize("M,N,K,tile", [(1, 1, 4, 16), (16, 128, 32, 16), (17, 129, 36, 32), (40, 61, 132, 48), (81, 300, 1028, 96),
+                                        (208, 257, 516, 208), (209, 2048, 2048, 112), (517, 130, 7808, 176), (130, 19000, 100, 144)])
+def test_gemm_f32_on_tensor_cores(M, N, K, tile, monkeypatch):
+    """The 32-bit product in three parts at the edges of its tiles, stages and shares of K: with a bias, added to what is there,
+    rows wider than K.  Against 64-bit sums: what the parts leave out (2^-24 of a product) and a chain of K / 32 additions."""
+    o = ops()
+    monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *a: tile)
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (32, 1))
+    a, w, bias = rnd(M, K + 4)[:, :K], rnd(N, K + 8)[:, :K], rnd(N)
+    want = a.double() @ w.double().T
+    out = torch.full((M, N + 3), 7.0, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    o.gemm(a, w, out[:, :N], bias=bias, status=status)
+    assert rel(out[:, :N], want + bias) < 5e-7 and bool((out[:, N:] == 7).all()) and int(status) == 0
+    acc = rnd(M, N, seed=5)
+    base = acc.clone()
+    o.gemm(a, w, acc, accumulate=True)
+    assert rel(acc, base + want) < 5e-7
+
+
+def test_gemm_f32_on_tensor_cores_in_slices_of_rows(monkeypatch):
+    o = ops()
+    monkeypatch.setattr(o, "_f32_tc_rows", lambda k: 100)
+    a, w = rnd(250, 1024), rnd(300, 1024)
+    out = torch.empty(250, 300, device=DEV)
+    o._gemm_f32_tc(a, w, out, 96, None, False, None, None)
+    assert rel(out, a.double() @ w.double().T) < 5e-7
+
+
+@pytest.mark.parametrize("cut", [False, True])
+def test_gemm_f32_on_tensor_cores_beyond_finite_numbers(cut, monkeypatch):
+    """Infinite operands, no numbers, overflows and values whose lower parts are subnormal: what the FFMA kernels give."""
+    o = ops()
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (32, 1))
+    M, N, K = 20, 128 * (5 if cut else 148), 256
+    a, w = rnd(M, K), rnd(N, K)
+    a[3, 200], a[4, 7], a[5] = float("inf"), float("nan"), 0.0
+    a[6:8] = 0.0         # (one product each: where sums overflow on the way depends on their order)
+    a[6, 10], a[7, 0] = 3e38, torch.finfo(torch.float32).max
+    a[8] *= 1e-30
+    w[9, 100], w[10, 5], w[11, 2] = float("-inf"), float("nan"), 0.0
+    w[12] *= 1e-3
+    a[9, 64] = float("inf")
+    w[9, 65] = float("inf")
+    want, out = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *x: 0)
+    o.gemm(a, w, want)
+    monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *x: 32)
+    o.gemm(a, w, out)
+    assert bool(((out == want) | (out.isnan() == want.isnan()))[~want.isfinite()].all())
+    assert torch.equal(out.isfinite(), want.isfinite()) and torch.equal(out[out.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    exact, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - exact).abs() <= 2e-6 * size)[ok].all())
+
+
 @pytest.mark.parametrize("form", [-1, -4, -8, 32, 64, 128])
 def test_gemm_f32_groups(form, monkeypatch):
     """Groups without rows, of one row, of a tile's rows and one more, with gathered rows, more groups than a warp."""
