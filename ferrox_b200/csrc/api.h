@@ -127,15 +127,15 @@ int fx_moe_align(const int* ids, int n_tokens, int top_k, int n_experts, int* sc
 // rows' at [gate_up_offset, gate_up_offset + N): C = act(gate + b_gate) * (up + b_up).
 int fx_gemm_tc(const void* X, long ldx, const void* W, long ldw, long w_group_stride, int w_rows, const void* bias,
                int bias_dtype, void* C, int c_dtype, long ldc, int accumulate, int M, int N, int K, int gated,
-               int gate_up_offset, float act_limit, float act_alpha, const int* group_offsets, int n_groups, int* status,
-               void* stream);
+               int gate_up_offset, float act_limit, float act_alpha, const int* group_offsets, int n_groups, int n_tile,
+               int* status, void* stream);
 int fx_gemm_tc_swap(const void* X, long ldx, const void* W, long ldw, long w_group_stride, int w_rows, const void* bias,
                     int bias_dtype, void* C, int c_dtype, long ldc, int accumulate, int M, int N, int K, int gated,
                     int gate_up_offset, float act_limit, float act_alpha, const int* group_offsets, int n_groups, int tokens_per_tile, int weights_first,
                     int k_splits, float* partials, int* status, void* stream);
 int fx_gemm_tc2(const void* X, long ldx, const void* W, long ldw, int w_rows, const void* bias, int bias_dtype, void* C,
                 int c_dtype, long ldc, int accumulate, int M, int N, int K, int gated, int gate_up_offset, float act_limit,
-                float act_alpha, int* status, void* stream);
+                float act_alpha, int n_tile, int* status, void* stream);
 int fx_moe_combine_norm(float* h, const void* y, int dtype, const int* inv_perm, const float* topk_w, int top_k,
                         const void* shared, const float* shared_gate_logit, long gate_ld, int n_tokens, int hidden,
                         const void* norm_w, int norm_w_dtype, float eps, void* x_out, void* stream);

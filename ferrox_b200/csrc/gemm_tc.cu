@@ -37,7 +37,8 @@ constexpr int UMMA_K = 16;
 constexpr int NTHREADS = 192;    // producer warp, mma warp, four epilogue warps
 
 template <int BN> struct Cfg {
-    static constexpr int STAGES = BN <= 128 ? 6 : 4;
+    static constexpr int STAGES = BN <= 128 ? 6 : BN <= 192 ? 5 : 4;
+    static constexpr int TMEM = BN <= 128 ? 256 : 512;       // two accumulators, a power of two
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc_kernel(const __grid_const
     }
     if (warp == 1) {   // tensor memory: two accumulators of BN columns (128 lanes x 32 bit each)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_base_s)), "r"((uint32_t)(2 * BN)) : "memory");
+                     ::"r"(smem_u32(&tmem_base_s)), "r"((uint32_t)C::TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -262,6 +263,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc_kernel(const __grid_const
             const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
 #pragma unroll 1
             for (int c = 0; c < OUT_N / 32; ++c) {
+                // (a bfloat16 tile's last chunk has no partner to fill a line with where their number is odd)
+                const bool lines = fast && !(OUT_N % 64 && c == OUT_N / 32 - 1 && a.c_dtype != FX_F32);
                 uint32_t r[32], u[32];
                 tc_ld32(lane_addr + c * 32, r);
                 if (GATED) tc_ld32(lane_addr + BN / 2 + c * 32, u);
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc_kernel(const __grid_const
                     if (lane == 0) mbar_arrive(acc_empty_bar(buf));
                 }
                 const int nb = tc.n0 + c * 32;
-                if (!fast && (!row_ok || nb >= a.N)) continue;
+                if (!lines && (!row_ok || nb >= a.N)) continue;
                 float v[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc_kernel(const __grid_const
                     v[j] = x;
                 }
                 if (GATED) fx_gate_32(v, u, a.act, a.act_limit, a.act_alpha);
-                if (fast) {
+                if (lines) {
                     const long row0 = tc.m0 + quad * 32;
                     if (a.c_dtype == FX_F32) {
                         epi_stage_f32(stage, lane, v);
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc_kernel(const __grid_const
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * BN)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::TMEM) : "memory");
     }
     if (threadIdx.x == 0 && abort_flag_s && a.status) atomicExch(a.status, STATUS_TC_TIMEOUT);
 }
@@ -399,18 +402,21 @@ int run_bn(const void* X, long ldx, const void* W, long ldw, long w_group_stride
         return FX_ERR_SIZE;
     const long m_tiles = a.group_offsets ? fx_cdiv(a.M, BM) + a.n_groups : fx_cdiv(a.M, BM);   // an upper bound when grouped
     const long max_tiles = m_tiles * fx_cdiv(a.N, out_n);
-    return gated ? launch<BN, true>(ma, mb, a, max_tiles, s) : launch<BN, false>(ma, mb, a, max_tiles, s);
+    if constexpr (BN % 128 == 0)
+        if (gated) return launch<BN, true>(ma, mb, a, max_tiles, s);
+    return launch<BN, false>(ma, mb, a, max_tiles, s);
 }
 
 }  // namespace
 
 // X [M, K] and W [G, w_rows, K] bfloat16; C bfloat16 or float32.  gated: W holds gate rows [0, N) and up rows
 // [gate_up_offset, gate_up_offset + N), C = act(gate) * up (gated 1: SiLU, 2: ReLU).  grouped: group_offsets [n_groups + 1] on the device,
-// rows of X (and of C) sorted by group; M is then the total number of rows.
+// rows of X (and of C) sorted by group; M is then the total number of rows.  n_tile: rows of W a tile, 128 or 256, of plain products
+// also 160, 192 or 224 (kernels/ops.py: dense_tile).
 extern "C" int fx_gemm_tc(const void* X, long ldx, const void* W, long ldw, long w_group_stride, int w_rows,
                           const void* bias, int bias_dtype, void* C, int c_dtype, long ldc, int accumulate,
                           int M, int N, int K, int gated, int gate_up_offset, float act_limit, float act_alpha,
-                          const int* group_offsets, int n_groups,
+                          const int* group_offsets, int n_groups, int n_tile,
                           int* status, void* stream)
 {
     // gated < 0: a plain product whose result passes through the activation -gated (fx_unary) before it is stored
@@ -420,16 +426,19 @@ extern "C" int fx_gemm_tc(const void* X, long ldx, const void* W, long ldw, long
     if (K <= 0 || K % 8) return FX_ERR_SIZE;
     if (ldx % 8 || ldw % 8 || w_group_stride % 8 || (uintptr_t)X % 16 || (uintptr_t)W % 16) return FX_ERR_ALIGN;
     if (c_dtype != FX_F32 && c_dtype != FX_BF16) return FX_ERR_DTYPE;
-    if (group_offsets && n_groups > MAX_GROUPS) return FX_ERR_SIZE;
+    if ((group_offsets && n_groups > MAX_GROUPS) || (gated && n_tile % 128)) return FX_ERR_SIZE;
     TcArgs a;
     a.C = C; a.ldc = ldc; a.c_dtype = c_dtype; a.accumulate = accumulate;
     a.bias = bias; a.bias_dtype = bias_dtype;
     a.M = M; a.N = N; a.K = K; a.gate_up_offset = gate_up_offset; a.act = gated > 0 ? gated - 1 : unary; a.act_limit = act_limit; a.act_alpha = act_alpha;
     a.group_offsets = group_offsets; a.n_groups = n_groups; a.status = status;
     cudaStream_t s = (cudaStream_t)stream;
-    // wide outputs take 128 x 256 tiles (fewer bytes fetched per flop; measured faster even when they give
-    // every SM a single tile); narrow ones 128 x 128
-    const int wide = gated ? N >= 256 : N >= 512;
-    if (wide) return run_bn<256>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
-    return run_bn<128>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+    switch (n_tile) {
+        case 256: return run_bn<256>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+        case 224: return run_bn<224>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+        case 192: return run_bn<192>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+        case 160: return run_bn<160>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+        case 128: return run_bn<128>(X, ldx, W, ldw, w_group_stride, w_rows, a, gated, s);
+    }
+    return FX_ERR_SIZE;
 }

@@ -27,13 +27,16 @@ namespace {
 using namespace fxtc;
 
 constexpr int BM = 128;          // rows of X per CTA (256 per pair)
-constexpr int BNH = 128;         // rows of W per CTA (256 per pair)
 constexpr int BK = 64;
 constexpr int NTHREADS = 192;
 constexpr int STAGES = 6;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BNH * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + 4 * EPI_WARP_BYTES;   // ring, alignment slack, barriers, the epilogue warps' staging tiles
-constexpr int ACC_COLS = 2 * BNH;            // columns of one accumulator: both halves of W
+constexpr int A_BYTES = BM * BK * 2;
+template <int BNH> struct Cfg {              // BNH: rows of W per CTA (twice that per pair)
+    static constexpr int B_BYTES = BNH * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + 4 * EPI_WARP_BYTES;   // ring, alignment slack, barriers, the epilogue warps' staging tiles
+    static constexpr int ACC_COLS = 2 * BNH;     // columns of one accumulator: both halves of W
+    static constexpr int TMEM = 512;             // two accumulators, a power of two
+};
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;  // a shared::cluster address with this bit cleared names the pair's first CTA
 
 struct Tc2Args {
@@ -80,10 +83,11 @@ __device__ __forceinline__ void arrive_on_first_cta(uint32_t bar) {
 
 // GATED as a template argument: with a run-time flag the compiler evaluates the gate's exponential and division for
 // every element of plain products too (a select instead of a branch).
-template <bool GATED>
+template <int BNH, bool GATED>
 __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                const __grid_constant__ CUtensorMap map_b, Tc2Args a)
 {
+    constexpr int STAGE_BYTES = Cfg<BNH>::STAGE_BYTES, ACC_COLS = Cfg<BNH>::ACC_COLS;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int abort_flag_s;
     __shared__ uint32_t tmem_base_s;
@@ -116,7 +120,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc2_kernel(const __grid_cons
     }
     if (warp == 1) {   // the same warp in both CTAs, the same destination
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_base_s)), "r"((uint32_t)(2 * ACC_COLS)) : "memory");
+                     ::"r"(smem_u32(&tmem_base_s)), "r"((uint32_t)Cfg<BNH>::TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_tc2_kernel(const __grid_cons
     cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * ACC_COLS)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)Cfg<BNH>::TMEM) : "memory");
     }
     if (threadIdx.x == 0 && abort_flag_s && a.status) atomicExch(a.status, STATUS_TC_TIMEOUT);
 }
@@ -332,13 +336,45 @@ bool make_map(CUtensorMap* map, const void* ptr, uint64_t K, uint64_t rows, uint
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int BNH, bool GATED> int launch(const void* X, long ldx, const void* W, long ldw, int w_rows, const Tc2Args& a, cudaStream_t stream)
+{
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, X, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)ldx, BM)) return FX_ERR_SIZE;
+    if (!make_map(&mb, W, (uint64_t)a.K, (uint64_t)w_rows, (uint64_t)ldw, BNH)) return FX_ERR_SIZE;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<BNH, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BNH>::SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int sms = fx_sm_count();
+    const long tiles = fx_cdiv(a.M, 2 * BM) * fx_cdiv(a.N, GATED ? BNH : 2 * BNH);
+    const long pairs = tiles < sms / 2 ? tiles : sms / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * pairs));
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = Cfg<BNH>::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_fx_pdl_enabled ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<BNH, GATED>, ma, mb, a);
+    if (e != cudaSuccess) return (int)e;
+    return fx_launch_status();
+}
+
 }  // namespace
 
 // X [M, K] and W [w_rows, K] bfloat16; C bfloat16 or float32.  gated: W holds gate rows [0, N) and up rows
 // [gate_up_offset, gate_up_offset + N), C = act(gate) * up (gated 1: SiLU, 2: ReLU).  Dense products only (no groups).
+// n_tile: rows of W a pair's tile, 256, of plain products also 192 (kernels/ops.py: dense_tile).
 extern "C" int fx_gemm_tc2(const void* X, long ldx, const void* W, long ldw, int w_rows, const void* bias, int bias_dtype,
                            void* C, int c_dtype, long ldc, int accumulate, int M, int N, int K, int gated,
-                           int gate_up_offset, float act_limit, float act_alpha, int* status, void* stream)
+                           int gate_up_offset, float act_limit, float act_alpha, int n_tile, int* status, void* stream)
 {
     // gated < 0: a plain product whose result passes through the activation -gated (fx_unary) before it is stored
     const int unary = gated < 0 ? -gated : 0;
@@ -351,33 +387,11 @@ extern "C" int fx_gemm_tc2(const void* X, long ldx, const void* W, long ldw, int
     a.C = C; a.ldc = ldc; a.c_dtype = c_dtype; a.accumulate = accumulate;
     a.bias = bias; a.bias_dtype = bias_dtype;
     a.M = M; a.N = N; a.K = K; a.gate_up_offset = gate_up_offset; a.gated = gated; a.act = gated > 0 ? gated - 1 : unary; a.act_limit = act_limit; a.act_alpha = act_alpha; a.status = status;
-    CUtensorMap ma, mb;
-    if (!make_map(&ma, X, (uint64_t)K, (uint64_t)M, (uint64_t)ldx, BM)) return FX_ERR_SIZE;
-    if (!make_map(&mb, W, (uint64_t)K, (uint64_t)w_rows, (uint64_t)ldw, BNH)) return FX_ERR_SIZE;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (gated) return launch<128, true>(X, ldx, W, ldw, w_rows, a, s);
+    switch (n_tile) {
+        case 256: return launch<128, false>(X, ldx, W, ldw, w_rows, a, s);
+        case 192: return launch<96, false>(X, ldx, W, ldw, w_rows, a, s);
     }
-    const int sms = fx_sm_count();
-    const int out_n = gated ? BNH : 2 * BNH;
-    const long tiles = fx_cdiv(M, 2 * BM) * fx_cdiv(N, out_n);
-    long pairs = tiles < sms / 2 ? tiles : sms / 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * pairs));
-    cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = SMEM;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = g_fx_pdl_enabled ? 2 : 1;
-    cudaError_t e = gated ? cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<true>, ma, mb, a) : cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<false>, ma, mb, a);
-    if (e != cudaSuccess) return (int)e;
-    return fx_launch_status();
+    return FX_ERR_SIZE;
 }

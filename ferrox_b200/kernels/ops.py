@@ -54,10 +54,10 @@ _SIGNATURES = {
     "fx_silu_mul": [_P, _L, _P, _L, _I, _P, _I, _I, _P],
     "fx_rope_kv_write": [_P, _I, _L, _P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "fx_rope_table": [_P, _P, _I, _I, _P, _F, _P],
-    "fx_gemm_tc": [_P, _L, _P, _L, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _F, _P, _I, _P, _P],
+    "fx_gemm_tc": [_P, _L, _P, _L, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _F, _P, _I, _I, _P, _P],
     "fx_gemm_tc_swap": [_P, _L, _P, _L, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _F, _P, _I, _I, _I, _I, _P, _P,
                         _P],
-    "fx_gemm_tc2": [_P, _L, _P, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
+    "fx_gemm_tc2": [_P, _L, _P, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P, _P],
     "fx_gather_rows": [_P, _L, _P, _P, _L, _I, _I, _I, _P],
     "fx_gather_rows_scaled": [_P, _L, _P, _P, _P, _I, _P, _L, _I, _I, _I, _P],
     "fx_paged_attention_ex": [_P, _L, _L, _P, _P, _L, _L, _I, _P, _I, _I, _P, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _I, _F,
@@ -1731,9 +1731,11 @@ def tc_ok(x, w) -> bool:
             and w.data_ptr() % 16 == 0 and x.stride(1) == 1 and w.stride(-1) == 1)
 
 
-def gemm_tc(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None, group_offsets=None, status=None, stream=None):
+def gemm_tc(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None, group_offsets=None, tile=None, status=None,
+            stream=None):
     """out[M, N] (+)= x . w^T on the tcgen05 tensor cores.  ``gated``: ``w`` is [gate rows ; up rows] and
-    out = silu(gate) * up.  Grouped: ``w`` is [G, rows, K] and the rows of ``x``/``out`` are sorted by group."""
+    out = silu(gate) * up.  Grouped: ``w`` is [G, rows, K] and the rows of ``x``/``out`` are sorted by group.
+    ``tile``: rows of ``w`` a tile (None: by the sizes)."""
     M, N = out.shape
     K = x.shape[1]
     if group_offsets is not None:
@@ -1743,9 +1745,14 @@ def gemm_tc(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None, 
     gated, lim, alpha = _gate_args(gated)
     if wrows != (2 * N if gated else N) or w.shape[-1] != K or x.shape[0] != M:
         raise KernelError(f"gemm_tc shapes do not agree: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
+    if tile is None:
+        if gated:
+            tile = 256 if N >= 256 else 128
+        else:
+            tile = dense_tile(M, N, False)[1] if group_offsets is None else 256 if N >= 512 else 128
     call("fx_gemm_tc", _ptr(x), _rows(x), _ptr(w), ldw, wstride, wrows, _ptr(bias), code(bias) if bias is not None else 0,
          _ptr(out), code(out), _rows(out), int(accumulate), M, N, K, int(_gated_or_unary(gated, unary)), N if gated else 0, lim, alpha,
-         _ptr(group_offsets), G, _ptr(status), stream if stream is not None else stream_ptr())
+         _ptr(group_offsets), G, int(tile), _ptr(status), stream if stream is not None else stream_ptr())
     return out
 
 
@@ -1776,9 +1783,10 @@ def gemm_tc_swap(x, w, out, *, bias=None, accumulate=False, gated=False, unary=N
     return out
 
 
-def gemm_tc2(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None, status=None, stream=None):
+def gemm_tc2(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None, tile=256, status=None, stream=None):
     """The dense product of :func:`gemm_tc` on pairs of SMs (tcgen05 cta_group::2: 256 x 256 tiles shared by the two
-    CTAs of a cluster, each fetching half of the tile's operands).  For prompt-sized dense products."""
+    CTAs of a cluster, each fetching half of the tile's operands).  For prompt-sized dense products.  ``tile``: rows of
+    ``w`` a tile (plain products: 256 or 192)."""
     M, N = out.shape
     K = x.shape[1]
     gated, lim, alpha = _gate_args(gated)
@@ -1786,7 +1794,7 @@ def gemm_tc2(x, w, out, *, bias=None, accumulate=False, gated=False, unary=None,
         raise KernelError(f"gemm_tc2 shapes do not agree: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
     call("fx_gemm_tc2", _ptr(x), _rows(x), _ptr(w), w.stride(0), w.shape[0], _ptr(bias), code(bias) if bias is not None else 0,
          _ptr(out), code(out), _rows(out), int(accumulate), M, N, K, int(_gated_or_unary(gated, unary)), N if gated else 0, lim, alpha,
-         _ptr(status), stream if stream is not None else stream_ptr())
+         int(tile), _ptr(status), stream if stream is not None else stream_ptr())
     return out
 
 
@@ -1818,6 +1826,32 @@ def pairs_better(M: int, N: int, gated: bool = False) -> bool:
     rows); with fewer tiles than SMs the pairs leave SMs idle."""
     tiles = -(-M // 256) * -(-N // (128 if gated else 256))
     return M >= 1024 and tiles >= sm_count()
+
+
+# Time of a tile of 128 rows of x on one SM, of 256 on a pair, by its rows of w: 1 = 1 us a 64 elements of K.
+_TILE_TIMES = ((256, 0.445), (224, 0.42), (192, 0.385), (160, 0.365), (128, 0.35))
+_PAIR_TIMES = ((256, 0.41), (192, 0.365))
+
+
+@functools.lru_cache(maxsize=4096)
+def dense_tile(M: int, N: int, pairs: bool = True):
+    """(on pairs of SMs, rows of w a tile) of a plain dense product of M rows on the tensor cores.
+
+    What counts is how the tiles go into rounds of the SMs: the times of one tile are those measured on a B200 (176 slices of 64
+    elements of K with 100 to 140 tiles in flight), and the least sum over the rounds is taken.  A narrow tile is nowhere near as
+    much faster as it is narrower (a slice's operands arrive at 60 bytes a cycle of an SM at most), so that it pays only where
+    it saves a round or the SMs are idle anyway.  Weights from memory, 32-bit output added to, us: 1531 x 2048 x 11264 78.8 in
+    tiles of 256, 67.9 in 192; 3001 x 2048 x 5632 77.4 and 69.8; 517 x 3072 x 2048 22.7 and 18.3 in 128; 400 x 2048 x 5632 42.9
+    and 35.2; 2600 x 3584 x 20480 372 on pairs in 256, 275 on single SMs."""
+    if N < 512:
+        return False, 128
+    sms = sm_count()
+    best = min((-(-(-(-M // 128) * -(-N // bn)) // sms) * t, i, bn) for i, (bn, t) in enumerate(_TILE_TIMES))
+    if pairs and pairs_better(M, N):
+        on_pairs = min((-(-(-(-M // 256) * -(-N // bn)) // (sms // 2)) * t, i, bn) for i, (bn, t) in enumerate(_PAIR_TIMES))
+        if on_pairs[0] < best[0]:
+            return True, on_pairs[2]
+    return False, best[2]
 
 
 def swap_k_splits(T: int, N: int, K: int) -> int:
@@ -1870,8 +1904,9 @@ def linear(x, w, out, *, bias=None, accumulate=False, status=None, stream=None, 
     if T <= SKINNY_MAX_TOKENS and skinny_ok(x, w):
         return gemm_skinny(x, w, out, bias=bias, accumulate=accumulate, unary=act, stream=stream)
     if T > SKINNY_MAX_TOKENS and tc_ok(x, w):
-        if w.dim() == 2 and pairs_better(T, w.shape[0]):
-            return gemm_tc2(x, w, out, bias=bias, accumulate=accumulate, unary=act, status=status, stream=stream)
+        pairs, tile = dense_tile(T, w.shape[0]) if w.dim() == 2 else (False, None)
+        if pairs:
+            return gemm_tc2(x, w, out, bias=bias, accumulate=accumulate, unary=act, tile=tile, status=status, stream=stream)
         return gemm_tc(x, w, out, bias=bias, accumulate=accumulate, unary=act, status=status, stream=stream)
     gemm(x, w, out, bias=bias, accumulate=accumulate, status=status, stream=stream)
     return _apply_unary_(out, act, stream) if act else out

@@ -229,3 +229,14 @@ def test_32_bit_products_that_go_to_the_tensor_cores():
                 if tile:
                     rows = min(m, ops._f32_tc_rows(k))
                     assert rows >= min(m, 208) and 6 * rows * k + 148 * 1024 * tile <= ops.F32_WORKSPACE_MAX
+
+
+def test_tiles_of_dense_products_by_rounds():
+    """Tiles that save a round of the SMs, narrow ones where the SMs are idle anyway, pairs where they need no more rounds."""
+    assert [ops.dense_tile(m, 2048) for m in (96, 1531, 2048, 3001)] == [(False, 128), (False, 192), (False, 256), (False, 192)]
+    assert [ops.dense_tile(m, 6144) for m in (517, 2048)] == [(False, 224), (True, 256)]
+    assert ops.dense_tile(2600, 3584) == (False, 256) and ops.dense_tile(4096, 3584) == (True, 256) and ops.dense_tile(3000, 60) == (False, 128)
+    for m in range(65, 5000, 97):
+        for n in (512, 1000, 2048, 3584, 20480):
+            pairs, tile = ops.dense_tile(m, n)
+            assert tile in ((192, 256) if pairs else (128, 160, 192, 224, 256)) and (not pairs or ops.pairs_better(m, n))

@@ -741,6 +741,23 @@ def test_gemm_tc_dense(M, N, K):
     assert rel(out32, wide[:, :K].float() @ w.float().T) < 2e-5
 
 
+@pytest.mark.parametrize("pairs,tile", [(False, 160), (False, 192), (False, 224), (True, 192)])
+@pytest.mark.parametrize("M,N,K", [(65, 64, 72), (129, 512, 136), (300, 1344, 2048), (1000, 1001, 520)])
+def test_dense_tiles_of_other_widths(pairs, tile, M, N, K):
+    """Tiles narrower than 256 rows of w, whose last 32 columns may have no partner to fill a line with: bit for bit what the
+    widest tiles give (each element's sum runs over K in one order), with a bias, in both types, added to what is there."""
+    o = ops()
+    x, w, bias = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, scale=0.1), rnd(N)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kern = o.gemm_tc2 if pairs else o.gemm_tc
+    for dt, acc in ((torch.bfloat16, False), (torch.float32, False), (torch.float32, True)):
+        got, want = (torch.full((M, N + 8), 7.0, dtype=dt, device=DEV) for _ in range(2))
+        for t, out in ((tile, got), (256, want)):
+            kern(x, w, out[:, :N], bias=bias, accumulate=acc, tile=t, status=status)
+        assert int(status) == 0 and torch.equal(got, want) and bool((got[:, N:] == 7).all())
+        assert rel(got[:, :N], x.float() @ w.float().T + bias + (7 if acc else 0)) < (TOL["bfloat16"] if dt == torch.bfloat16 else 2e-5)
+
+
 @pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 520, 136), (2048, 2048, 2048), (70, 100, 96), (1000, 6144, 264)])
 def test_gemm_tc2_pairs_of_sms(M, N, K):
     """The dense product on pairs of SMs (cta_group::2): plain with bias, accumulating, into a strided view."""
