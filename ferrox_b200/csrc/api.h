@@ -105,11 +105,12 @@ int fx_general_attention(const void* q, long ldq, long ldqh, const void* k_pages
                          const float* sinks, int value_share, int chunk, const void* gate, long ldg,
                          const float* turn, void* stream);
 
-int fx_prefill_attention_tc(const void* q, long ldq, int n_tokens, const void* k_pages, const void* v_pages, int n_pages,
+int fx_prefill_attention_tc(const void* q, long ldq, long ldqh, int n_tokens, const void* k_pages, const void* v_pages, int n_pages,
                             const int* block_table, int table_width, int page_size, const int* items, int n_items,
                             const int* seq_slot, void* out, long ldo, int n_heads, int n_kv_heads, int head_dim, int value_dim,
                             int window, int chunk, float scale, const float* sinks, const void* gate, long ldg, const float* turn,
-                            int* status, float* part_o, float* part_ml, const int* merges, int n_merges, void* stream);
+                            const long* kv_strides, int keep_first, float softcap, int value_share, int general, int* status,
+                            float* part_o, float* part_ml, const int* merges, int n_merges, void* stream);
 int fx_prefill_attention(const void* q, long ldq, const void* k_pages, const void* v_pages, const int* block_table,
                          int table_width, int page_size, const int* tiles, int n_tiles, const int* seq_slot, void* out,
                          long ldo, int n_heads, int n_kv_heads, int head_dim, int window, float scale, float softcap,

@@ -1,6 +1,6 @@
-// Attention for prompt portions on the 5th-generation tensor cores (bfloat16, keys and values of up to 128
-// elements a head in steps of 8, pages of 64 positions or a multiple).  Key and value widths may differ; in shared
-// and tensor memory both are rounded up to 64 or 128 (D and V below), the rest filled with zeros by the TMA.
+// Attention for prompt portions on the 5th-generation tensor cores (bfloat16, keys of up to 192 and values of up to
+// 128 elements a head in steps of 8, pages of 64 positions or a multiple).  Key and value widths may differ; in shared
+// and tensor memory both are rounded up to 64, 128 or 192 (D and V below), the rest filled with zeros by the TMA.
 //
 // One CTA takes up to 256 query tokens of one request and one head, as two sub-tiles of 128 rows, and
 // walks that request's keys in blocks of 128 positions (earlier steps' keys and the portion's own alike,
@@ -37,10 +37,21 @@
 // it has (the unnormalised sums in 32 bits, and each row's reference maximum and sum of weights) into
 // scratch memory, and a second kernel (prefill_merge_kernel) adds a tile's runs up in their order.
 //
-// Options: `chunk` (a query sees the keys of its own chunk of that many positions only, counted from the request's
+// Queries, keys and values are reached through strides of their own (rows that hold all heads side by side, or pages);
+// `value_share` consecutive key heads may read one value head.
+//
+// Options: `keep_first` (with a window: the request's first positions stay visible; the key blocks that hold them and lie
+// before a tile's own are walked first, by its first run), `softcap` (scores pass through c tanh(s / c); the row's maximum
+// is taken before, tanh keeps the order), `chunk` (a query sees the keys of its own chunk of that many positions only, counted from the request's
 // start), `sinks` (one number per head: exp(sink_h) joins the softmax's denominator once, at the end or in the merge),
 // `gate` (token rows of n_heads * value_dim: the result is multiplied by sigmoid(gate) before it is rounded), `turn`
 // ([tokens][value_dim / 2] (cos, sin): pair (2m, 2m + 1) of the result is turned by minus that angle before the gate).
+//
+// What bounds it: the softmax threads' instructions a score (4.5 plain, 12 capped) beside the two products; an item costs 13 us
+// before its first key block.  The general forms against the mma.sync kernels that took them before (16 heads of 128, 2,048
+// tokens in a window of 1,024): with kept first keys 111 -> 61 us, capped 127 -> 83; 16 heads of 192 and 128, 2,048 tokens: 220
+// -> 76; 32 maps of 64 on values of 128, capped, 1,531 tokens: 130 -> 100.  A warp none of whose rows exists leaves its block to
+// the others (300 tokens beside 15 single ones, capped: 176 -> 124).
 //
 // Reference: crates/ferrox-core/src/attention.rs:531-563 (query t over keys 0..=t), :146-175 (online
 // softmax), :484-524 (window), :572-610 (pages), :432-449 (grouped heads).  The mma.sync kernel of
@@ -61,7 +72,49 @@ __device__ __forceinline__ float fast_exp2(float x) {   // 2^x, approximate; -in
     return y;
 }
 
-constexpr int ITEM_INTS = 8;   // a work item: first flat token, rows, entry, first position, kb_begin, kb_end, part, -
+// How a score becomes a weight: the plain kernel's exponential is the hardware's (weights below 2^-126 are 0), the general
+// forms' is exp2f, and their denominators add up the weights as the second product has them (rounded to bfloat16: a row with
+// one large weight then has none of its rounding).
+enum { FAST = 0, GENERAL = 1, CAPPED = 2 };
+
+// A capped score in powers of two, c log2(e) tanh(k s) with k = scale / c.  Up to k s = 1/2, tanh(x) = x + x z p(z), z = x^2, p
+// fitted (weighted least squares towards the smallest largest error, 1.5e-8 of tanh(x); in 32 bits 7.5e-8): a cubic in s^2
+// whose coefficients hold k and the unit, two scores an instruction, no special function.  Beyond, tanhf.  The caps taken here (up
+// to CAP_MAX) keep every weight above 2^-126, where exp2f is the hardware's exponential.
+constexpr float CAP_MAX = 40.f, CAP_SMALL = 0.5f;
+struct Cap {
+    float k, unit, cap, c[4];        // c: of s^3, s^5, s^7, s^9
+};
+
+__device__ __forceinline__ uint64_t pair_of(float x, float y) { return (uint64_t)__float_as_uint(x) | ((uint64_t)__float_as_uint(y) << 32); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// 32 scores <- capped, less ref
+__device__ __forceinline__ void cap_small(const Cap& cap, uint32_t* s, float ref) {
+    const uint64_t c0 = pair_of(cap.c[0], cap.c[0]), c1 = pair_of(cap.c[1], cap.c[1]), c2 = pair_of(cap.c[2], cap.c[2]),
+                   c3 = pair_of(cap.c[3], cap.c[3]), u = pair_of(cap.unit, cap.unit), r = pair_of(-ref, -ref);
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        const uint64_t x = (uint64_t)s[i] | ((uint64_t)s[i + 1] << 32), x2 = mul2(x, x);
+        const uint64_t q = fma2(fma2(fma2(c3, x2, c2), x2, c1), x2, c0);
+        const uint64_t y = fma2(mul2(x, x2), q, fma2(x, u, r));
+        s[i] = (uint32_t)y; s[i + 1] = (uint32_t)(y >> 32);
+    }
+}
+__device__ __forceinline__ void cap_any(const Cap& cap, uint32_t* s, float ref) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) s[i] = __float_as_uint(fmaf(cap.cap, tanhf(cap.k * __uint_as_float(s[i])), -ref));
+}
+
+constexpr int ITEM_INTS = 8;   // a work item: first flat token, rows, entry, first position, kb_begin, kb_end, part, kept blocks
 
 struct AttnArgs {
     const int* block_table; int table_width; int page_size;
@@ -69,6 +122,8 @@ struct AttnArgs {
     bf16* out; long ldo;
     float* part_o; float* part_ml;   // partial results of items that hold a run of their tile's key blocks only
     int n_heads, n_kv_heads, window, chunk;
+    int keep_first, value_share;
+    Cap cap;                         // CAPPED
     int value_dim;                   // elements of a value head (V: rounded up)
     const float* sinks;              // (optional) one per head
     const bf16* gate; long ldg;      // (optional) token rows of n_heads * value_dim
@@ -90,12 +145,14 @@ struct Smem {
     static constexpr int HALVES = D / 64, V_HALVES = V / 64;   // 64-element (128-byte) slices of a key's, a value's row
     static constexpr int SUB = 128 * 128;                  // bytes of a [128 rows x 128 bytes] piece
     static constexpr int Q_BYTES = HALVES * SUB, K_BYTES = HALVES * SUB, V_BYTES = V_HALVES * SUB;
+    static constexpr int V_PLACES = D > 128 ? 1 : 2;       // (wider keys leave room for one block of values)
     static constexpr int Q_OFF = 0, K_OFF = 2 * Q_BYTES, V_OFF = K_OFF + 2 * K_BYTES;
-    static constexpr int BAR_OFF = V_OFF + 2 * V_BYTES;
+    static constexpr int BAR_OFF = V_OFF + V_PLACES * V_BYTES;
     static constexpr int TOTAL = BAR_OFF + 128 + 1024;     // barriers, alignment slack
+    static_assert(TOTAL <= 232448 - 64, "shared memory of a block");
 };
 
-template <int D, int V>
+template <int D, int V, int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                            const __grid_constant__ CUtensorMap map_k,
                                                                            const __grid_constant__ CUtensorMap map_v,
@@ -111,7 +168,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
     // heaviest item, then every head's next one, so that the light items fill the gaps at the end.
     const int* item = a.tiles + (long)blockIdx.y * ITEM_INTS;
     const int tok0 = item[0], rows = item[1], entry = item[2], pos0 = item[3];
-    const int kb_begin = item[4], kb_end = item[5], part = item[6];
+    const int kb_begin = item[4], kb_end = item[5], part = item[6], n_kept = item[7];
     const int head = blockIdx.x;
     const int kvh = head / (a.n_heads / a.n_kv_heads);
     const int last_pos = pos0 + rows - 1;
@@ -130,7 +187,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
     const bool act0 = lo0 <= hi0, act1 = lo1 <= hi1;
     const int first_blk = act0 && act1 ? min(lo0, lo1) : act0 ? lo0 : lo1;
     const int last_blk = act0 && act1 ? max(hi0, hi1) : act0 ? hi0 : hi1;
-    auto active = [&](int t, int j) { return t < 2 && j >= lo_of(t) && j <= hi_of(t); };
+    // what the item walks: the kept blocks 0 .. n_kept - 1, then first_blk .. last_blk
+    const int n_walk = n_kept + max(0, last_blk - first_blk + 1), kept_end = (a.keep_first + BKEY - 1) / BKEY;
+    auto block_of = [&](int i) { return i < n_kept ? i : first_blk + i - n_kept; };
+    auto active = [&](int t, int i) {
+        if (t >= nt || i >= n_walk) return false;
+        const int j = block_of(i);
+        return (j >= lo_of(t) && j <= hi_of(t)) || (j < kept_end && j < blk_lo(t));
+    };
+    auto last_of = [&](int t) {                            // the last walked block that sub-tile t needs (none: -1)
+        int i = n_walk - 1;
+        while (i >= 0 && !active(t, i)) --i;
+        return i;
+    };
 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar0 = base + L::BAR_OFF;
@@ -174,9 +243,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 for (int h = 0; h < L::HALVES; ++h)
                     tma_load_3d(base + L::Q_OFF + t * L::Q_BYTES + h * L::SUB, &map_q, h * 64, head, tok0 + t * BQ, q_full);
             const int* table = a.block_table + (long)a.seq_slot[entry] * a.table_width;
-            int issued = 0;
-            for (int j = first_blk; j <= last_blk; ++j) {
-                const int i = j - first_blk, b = i & 1;
+            int issued = 0, v_issued = 0;
+            for (int i = 0; i < n_walk; ++i) {
+                const int j = block_of(i), b = i & 1, vb = L::V_PLACES == 2 ? b : 0;
                 if (!mbar_wait(kv_empty(b), (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag)) break;
                 int page[2], off[2];
                 for (int hk = 0; hk < 2; ++hk) {   // the two runs of 64 keys of the block
@@ -190,17 +259,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                     for (int hk = 0; hk < 2; ++hk)
                         tma_load_4d(base + L::K_OFF + b * L::K_BYTES + h * L::SUB + hk * 8192, &map_k, h * 64, off[hk], kvh,
                                     page[hk], k_full(b));
-                mbar_expect_tx(v_full(b), L::V_BYTES);
+                issued = i + 1;
+                // (one place of values: free when the block before this one has been multiplied)
+                if (L::V_PLACES == 1 && i > 0 && !mbar_wait(kv_empty((i - 1) & 1), (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) break;
+                mbar_expect_tx(v_full(vb), L::V_BYTES);
                 for (int h = 0; h < L::V_HALVES; ++h)
                     for (int hk = 0; hk < 2; ++hk)
-                        tma_load_4d(base + L::V_OFF + b * L::V_BYTES + h * L::SUB + hk * 8192, &map_v, h * 64, off[hk], kvh,
-                                    page[hk], v_full(b));
-                issued = i + 1;
+                        tma_load_4d(base + L::V_OFF + vb * L::V_BYTES + h * L::SUB + hk * 8192, &map_v, h * 64, off[hk],
+                                    kvh / a.value_share, page[hk], v_full(vb));
+                v_issued = i + 1;
             }
             if (*abort_flag) {   // loads already issued must land before the shared memory is released
                 for (int i = max(0, issued - 2); i < issued; ++i)
                     for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
-                        if (mbar_try_wait(k_full(i & 1), (uint32_t)((i >> 1) & 1)) && mbar_try_wait(v_full(i & 1), (uint32_t)((i >> 1) & 1))) break;
+                        if (mbar_try_wait(k_full(i & 1), (uint32_t)((i >> 1) & 1))) break;
+                for (int i = max(0, v_issued - L::V_PLACES); i < v_issued; ++i)
+                    for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
+                        if (mbar_try_wait(v_full(i % L::V_PLACES), (uint32_t)((i / L::V_PLACES) & 1))) break;
             }
         }
     } else if (warp == 1) {
@@ -208,13 +283,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
         if (lane == 0) {
             constexpr uint32_t idesc_s = instr_desc_ex(BQ, BKEY, 0);   // S: B = K tile, K-major
             constexpr uint32_t idesc_o = instr_desc_ex(BQ, V, 1);      // O: B = V tile, N-major
-            int k_ready = first_blk - 1;   // the last block whose K is known to have landed
+            int k_ready = -1;              // the last walked block whose K is known to have landed
+            const int last0 = last_of(0), last1 = last_of(1);
             bool ok = mbar_wait(q_full, 0, abort_flag);
-            auto issue_s = [&](int t, int j) {
-                const int i = j - first_blk, b = i & 1;
-                if (k_ready < j) {
+            auto issue_s = [&](int t, int i) {
+                const int b = i & 1;
+                if (k_ready < i) {
                     if (!mbar_wait(k_full(b), (uint32_t)((i >> 1) & 1), abort_flag)) return false;
-                    k_ready = j;
+                    k_ready = i;
                     tc_fence_after();
                 }
 #pragma unroll
@@ -228,15 +304,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 return true;
             };
             for (int t = 0; t < nt && ok; ++t)
-                if (active(t, first_blk)) ok = issue_s(t, first_blk);
+                if (active(t, 0)) ok = issue_s(t, 0);
             int n_p[2] = {0, 0};   // blocks of each sub-tile whose P has been taken
-            for (int j = first_blk; j <= last_blk && ok; ++j) {
-                const int i = j - first_blk, b = i & 1;
+            for (int i = 0; i < n_walk && ok; ++i) {
+                const int b = i & 1, vb = L::V_PLACES == 2 ? b : 0;
                 bool v_ready = false;
                 for (int t = 0; t < nt && ok; ++t) {
-                    if (active(t, j)) {
+                    if (active(t, i)) {
                         ok = mbar_wait(p_full(t), (uint32_t)(n_p[t] & 1), abort_flag);
-                        if (ok && !v_ready) { ok = mbar_wait(v_full(b), (uint32_t)((i >> 1) & 1), abort_flag); v_ready = true; }
+                        if (ok && !v_ready) { ok = mbar_wait(v_full(vb), (uint32_t)((i / L::V_PLACES) & 1), abort_flag); v_ready = true; }
                         if (!ok) break;
                         tc_fence_after();
                         // O_t += P V: 8 steps of 16 keys.  A = P from tensor memory, 8 columns a step.  B = V,
@@ -244,14 +320,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                         // 64-element slices of the head dimension lie SUB bytes apart (the leading operand).
 #pragma unroll
                         for (int ks = 0; ks < BKEY / 16; ++ks) {
-                            const uint64_t dv = smem_desc_lbo_sbo(base + L::V_OFF + b * L::V_BYTES + ks * 2048, L::SUB, 1024);
+                            const uint64_t dv = smem_desc_lbo_sbo(base + L::V_OFF + vb * L::V_BYTES + ks * 2048, L::SUB, 1024);
                             tc_mma_ts(tmem_o(t), tmem_s(t) + 8u * ks, dv, idesc_o, (n_p[t] | ks) != 0);
                         }
                         ++n_p[t];
-                        if (j == hi_of(t)) tc_commit(o_done(t));
+                        if (i == (t ? last1 : last0)) tc_commit(o_done(t));
                     }
                     if (t == nt - 1) tc_commit(kv_empty(b));   // every product that reads this stage has been issued
-                    if (active(t, j + 1)) ok = issue_s(t, j + 1);
+                    if (active(t, i + 1)) ok = issue_s(t, i + 1);
                 }
             }
         }
@@ -268,18 +344,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
             const int lo_last = fx_first_key(pos0_t + BQ - 1, a.window, a.chunk);     // the largest of the sub-tile's rows
             const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
             const uint32_t ts = tmem_s(t) + lane_off, to = tmem_o(t) + lane_off;
-            const float sl2 = a.scale_log2e;
+            const float sl2 = MODE == CAPPED ? 1.f : a.scale_log2e;   // (a capped score is one of 2's powers already)
             float m = -INFINITY, l = 0.f;
             bool ok = true;
             int cnt = 0;
-            const int hi = hi_of(t);
-            for (int j = lo_of(t); j <= hi; ++j, ++cnt) {
+            for (int i = 0; i < n_walk; ++i) {
+                if (!active(t, i)) continue;
+                const int j = block_of(i);
                 ok = __all_sync(0xffffffffu, mbar_wait(s_full(t), (uint32_t)(cnt & 1), abort_flag));
                 if (!ok) break;
                 tc_fence_after();
+                if (quad * 32 >= rows_t) {           // none of the warp's rows exists: what its rows of P hold reaches no others
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(p_full(t));
+                    ++cnt;
+                    continue;
+                }
                 const int kb = j * BKEY;
                 // every key of the block visible to every row of the sub-tile: no masking (most blocks)
-                const bool interior = kb + BKEY - 1 <= pos0_t && kb >= lo_last;
+                const bool interior = kb + BKEY - 1 <= pos0_t && (kb >= lo_last || kb + BKEY <= a.keep_first);
                 // The row of S is read in chunks of 32 columns into two register buffers in turn: the load of the
                 // next chunk is in flight while the current one is worked on.
                 uint32_t ca[32], cb[32], pk[32];
@@ -288,12 +372,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
 #pragma unroll
                     for (int k = 0; k < 32; ++k) {
                         const int key = kb + chunk * 32 + k;
-                        if (key > p_r || key < lo_r) c[k] = 0xff800000u;   // -inf
+                        if (key > p_r || (key < lo_r && key >= a.keep_first)) c[k] = 0xff800000u;   // -inf
                     }
                 };
                 // first pass: the row's maximum
-                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY, size0 = 0.f, size1 = 0.f;
                 auto take_max = [&](uint32_t* c, int chunk) {
+                    if (MODE == CAPPED) {
+#pragma unroll
+                        for (int k = 0; k < 32; k += 2) {
+                            size0 = fmaxf(size0, fabsf(__uint_as_float(c[k]))); size1 = fmaxf(size1, fabsf(__uint_as_float(c[k + 1])));
+                        }
+                    }
                     mask(c, chunk);
 #pragma unroll
                     for (int k = 0; k < 32; k += 4) {
@@ -307,7 +397,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 tc_ld32(ts + 64, ca); take_max(cb, 1); tc_ld_wait_for(ca);
                 tc_ld32(ts + 96, cb); take_max(ca, 2); tc_ld_wait_for(cb);
                 tc_ld32(ts, ca);      take_max(cb, 3);   // chunk 0 again, for the second pass
-                const float mn = fmaxf(fmaxf(m, fmaxf(mx0, mx1)), fmaxf(mx2, mx3));
+                float top = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+                const bool all_small = MODE == CAPPED && __all_sync(0xffffffffu, fmaxf(size0, size1) * a.cap.k <= CAP_SMALL);
+                if (MODE == CAPPED && top != -INFINITY) {
+                    // (as its weight will be worked out, but for the last place)
+                    const float x2 = top * top, q = fmaf(fmaf(fmaf(a.cap.c[3], x2, a.cap.c[2]), x2, a.cap.c[1]), x2, a.cap.c[0]);
+                    top = all_small ? fmaf(top * x2, q, top * a.cap.unit) : a.cap.cap * tanhf(a.cap.k * top);
+                }
+                const float mn = fmaxf(m, top);
                 const bool raise = mn > m && (m == -INFINITY || (mn - m) * sl2 > RAISE_MAX_BY);
                 if (__any_sync(0xffffffffu, raise)) {
                     const float alpha = m == -INFINITY ? 0.f : fast_exp2((m - mn) * sl2);
@@ -328,14 +425,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 // (columns 0-31 are written after columns 0-63 were read, columns 32-63 after all were)
                 const float ref = m == -INFINITY ? 0.f : m * sl2;
                 float sum0 = 0.f, sum1 = 0.f;
+                auto weight = [&](uint32_t c) {
+                    if (MODE == CAPPED) return fast_exp2(__uint_as_float(c));
+                    const float x = fmaf(__uint_as_float(c), sl2, -ref);
+                    return MODE == FAST ? fast_exp2(x) : exp2f(x);
+                };
                 auto take_exp = [&](uint32_t* c, int chunk, uint32_t* out) {
+                    if (MODE == CAPPED) {
+                        if (all_small) cap_small(a.cap, c, ref); else cap_any(a.cap, c, ref);
+                    }
                     mask(c, chunk);
 #pragma unroll
                     for (int k = 0; k < 32; k += 2) {
-                        const float e0 = fast_exp2(fmaf(__uint_as_float(c[k]), sl2, -ref));
-                        const float e1 = fast_exp2(fmaf(__uint_as_float(c[k + 1]), sl2, -ref));
-                        sum0 += e0; sum1 += e1;
+                        float e0 = weight(c[k]), e1 = weight(c[k + 1]);
                         __nv_bfloat162 pr = __floats2bfloat162_rn(e0, e1);
+                        if (MODE != FAST) {
+                            const uint32_t w = *reinterpret_cast<uint32_t*>(&pr);
+                            e0 = __uint_as_float(w << 16); e1 = __uint_as_float(w & 0xffff0000u);
+                        }
+                        sum0 += e0; sum1 += e1;
                         out[k >> 1] = *reinterpret_cast<uint32_t*>(&pr);
                     }
                 };
@@ -353,8 +461,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full(t));
+                ++cnt;
             }
-            const bool has_blocks = lo_of(t) <= hi_of(t);
+            const bool has_blocks = last_of(t) >= 0;
             if (ok && has_blocks) ok = __all_sync(0xffffffffu, mbar_wait(o_done(t), 0, abort_flag));
             if (ok && part >= 0) {
                 // a run of the tile's key blocks: the sums as they are, each row's reference and sum of weights
@@ -494,11 +603,11 @@ bool encode(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t* dims,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int D, int V>
+template <int D, int V, int MODE>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnArgs& a, dim3 grid, const int* merges,
            int n_merges, cudaStream_t s)
 {
-    auto kern = prefill_attention_tc_kernel<D, V>;
+    auto kern = prefill_attention_tc_kernel<D, V, MODE>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D, V>::TOTAL);
@@ -506,51 +615,74 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
         configured = true;
     }
     fx_launch_pdl(kern, grid, NTHREADS, Smem<D, V>::TOTAL, s, mq, mk, mv, a);
+    const float unit = MODE == CAPPED ? 1.f : a.scale_log2e;
     if (n_merges > 0)
         fx_launch_pdl(prefill_merge_kernel<V>, dim3(n_merges, a.n_heads, 2 * BQ / 4), 128, 0, s, merges, (const float*)a.part_o,
-                      (const float*)a.part_ml, a.out, a.ldo, a.n_heads, a.scale_log2e, a.value_dim, a.sinks, a.gate, a.ldg, a.turn);
+                      (const float*)a.part_ml, a.out, a.ldo, a.n_heads, unit, a.value_dim, a.sinks, a.gate, a.ldg, a.turn);
     return fx_launch_status();
+}
+
+template <int MODE>
+int pick(int head_dim, int value_dim, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnArgs& a, dim3 grid,
+         const int* merges, int n_merges, cudaStream_t s)
+{
+    const bool narrow = value_dim <= 64;
+    if (head_dim <= 64) return narrow ? launch<64, 64, MODE>(mq, mk, mv, a, grid, merges, n_merges, s) : launch<64, 128, MODE>(mq, mk, mv, a, grid, merges, n_merges, s);
+    if (head_dim <= 128) return narrow ? launch<128, 64, MODE>(mq, mk, mv, a, grid, merges, n_merges, s) : launch<128, 128, MODE>(mq, mk, mv, a, grid, merges, n_merges, s);
+    if constexpr (MODE == GENERAL)
+        return narrow ? launch<192, 64, MODE>(mq, mk, mv, a, grid, merges, n_merges, s) : launch<192, 128, MODE>(mq, mk, mv, a, grid, merges, n_merges, s);
+    return FX_ERR_SIZE;
 }
 
 }  // namespace
 
 // items: int32 [n_items, 8] = (first flat token, rows <= 256, entry index, absolute position of the first row, first
-// key block of 128 positions, end of the key blocks, part or -1, unused), the heavy ones first.  An item with part -1
+// key block of 128 positions, end of the key blocks, part or -1, kept blocks: blocks 0 .. that - 1 before the first, for keep_first), the heavy ones first.  An item with part -1
 // holds every key block its tile sees and writes the tile's output; the items of a tile that was cut write their
 // partial results to part_o [parts, n_heads, 256, value_dim rounded up to 64 or 128] and part_ml [parts, n_heads, 256, 2] (32-bit), and
 // merges: int32 [n_merges, 4] = (first flat token, rows, first part, runs) tells the second kernel which to add up
 // (a tile's runs have consecutive parts, in the order of their keys).
-// q is the fused [tokens, ldq] buffer whose rows start with the query heads; n_tokens its number of rows.
+// q: rows `ldq` elements apart, heads `ldqh`; n_tokens its number of rows.  kv_strides (elements; null: pages [page][kv head]
+// [position][width]): of a page, a head and a position of the keys, then of the values.  general: exp2f for the weights, as every
+// softcap, keep_first, value_share or key width above 128 has it (those refuse 0).
 // Refuses (FX_ERR_SIZE / FX_ERR_ALIGN) what it does not take; the caller then uses the mma.sync kernel.
-extern "C" int fx_prefill_attention_tc(const void* q, long ldq, int n_tokens, const void* k_pages, const void* v_pages,
+extern "C" int fx_prefill_attention_tc(const void* q, long ldq, long ldqh, int n_tokens, const void* k_pages, const void* v_pages,
                                        int n_pages, const int* block_table, int table_width, int page_size,
                                        const int* tiles, int n_tiles, const int* seq_slot, void* out, long ldo,
                                        int n_heads, int n_kv_heads, int head_dim, int value_dim, int window, int chunk,
                                        float scale, const float* sinks, const void* gate, long ldg, const float* turn,
-                                       int* status,
+                                       const long* kv_strides, int keep_first, float softcap, int value_share, int general, int* status,
                                        float* part_o, float* part_ml, const int* merges, int n_merges, void* stream)
 {
     if (n_tiles <= 0) return FX_OK;
     if (n_merges > 0 && (!part_o || !part_ml || !merges || (uintptr_t)part_o % 16)) return FX_ERR_ALIGN;
-    if (head_dim <= 0 || head_dim > 128 || head_dim % 8 || value_dim <= 0 || value_dim > 128 || value_dim % 8 ||
+    if (keep_first < 0 || value_share < 1 || n_kv_heads % value_share || !(softcap >= 0.f) || softcap > CAP_MAX) return FX_ERR_SIZE;
+    if (softcap > 0.f && !(scale / softcap >= 1e-4f && scale / softcap <= 1e4f)) return FX_ERR_SIZE;      // (the coefficients' range)
+    if (!general && (softcap > 0.f || keep_first || value_share > 1 || head_dim > 128)) return FX_ERR_SIZE;
+    if (head_dim <= 0 || head_dim > (softcap > 0.f ? 128 : 192) || head_dim % 8 || value_dim <= 0 || value_dim > 128 || value_dim % 8 ||
         page_size < 64 || page_size % 64 || n_kv_heads <= 0 || n_heads % n_kv_heads || chunk < 0 || !(scale > 0.f))
         return FX_ERR_SIZE;
-    if (ldq % 8 || ldo % 8 || (uintptr_t)q % 16 || (uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16 || (uintptr_t)out % 16)
+    if (ldqh % 8 || ldq % 8 || ldo % 8 || (uintptr_t)q % 16 || (uintptr_t)k_pages % 16 || (uintptr_t)v_pages % 16 || (uintptr_t)out % 16)
         return FX_ERR_ALIGN;
     if ((gate && (ldg % 8 || (uintptr_t)gate % 16)) || (uintptr_t)turn % 16) return FX_ERR_ALIGN;
     if (n_tiles > 65535) return FX_ERR_SIZE;
     CUtensorMap mq, mk, mv;
     {
         cuuint64_t dims[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_heads, (cuuint64_t)n_tokens};
-        cuuint64_t strides[2] = {(cuuint64_t)head_dim * 2, (cuuint64_t)ldq * 2};
+        cuuint64_t strides[2] = {(cuuint64_t)ldqh * 2, (cuuint64_t)ldq * 2};
         cuuint32_t box[3] = {64, 1, 128};
         if (!encode(&mq, q, 3, dims, strides, box)) return FX_ERR_SIZE;
     }
     for (int v = 0; v < 2; ++v) {
         const int width = v ? value_dim : head_dim;
-        cuuint64_t dims[4] = {(cuuint64_t)width, (cuuint64_t)page_size, (cuuint64_t)n_kv_heads, (cuuint64_t)n_pages};
-        cuuint64_t strides[3] = {(cuuint64_t)width * 2, (cuuint64_t)page_size * width * 2,
-                                 (cuuint64_t)n_kv_heads * page_size * width * 2};
+        const int heads = v ? n_kv_heads / value_share : n_kv_heads;
+        long at[3] = {(long)heads * page_size * width, (long)page_size * width, width};      // of a page, a head, a position
+        for (int i = 0; i < 3; ++i) {
+            if (kv_strides) at[i] = kv_strides[3 * v + i];
+            if (at[i] % 8) return FX_ERR_ALIGN;
+        }
+        cuuint64_t dims[4] = {(cuuint64_t)width, (cuuint64_t)page_size, (cuuint64_t)heads, (cuuint64_t)n_pages};
+        cuuint64_t strides[3] = {(cuuint64_t)at[2] * 2, (cuuint64_t)at[1] * 2, (cuuint64_t)at[0] * 2};
         cuuint32_t box[4] = {64, 64, 1, 1};
         if (!encode(v ? &mv : &mk, v ? v_pages : k_pages, 4, dims, strides, box)) return FX_ERR_SIZE;
     }
@@ -560,12 +692,16 @@ extern "C" int fx_prefill_attention_tc(const void* q, long ldq, int n_tokens, co
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.window = window; a.chunk = chunk; a.value_dim = value_dim;
     a.sinks = sinks; a.gate = (const bf16*)gate; a.ldg = ldg; a.turn = turn;
     a.scale_log2e = scale * 1.4426950408889634f; a.status = status;
-    a.part_o = part_o; a.part_ml = part_ml;
+    a.part_o = part_o; a.part_ml = part_ml; a.keep_first = window > 0 ? keep_first : 0; a.value_share = value_share;
+    if (softcap > 0.f) {
+        const double k = (double)scale / softcap, u = (double)scale * 1.4426950408889634, p[4] = {-0.33333140612, 0.13325783610, -0.05303649604, 0.01721787080};
+        double kk = k * k;
+        for (int i = 0; i < 4; ++i, kk *= k * k) a.cap.c[i] = (float)(u * kk * p[i]);
+        a.cap.k = (float)k; a.cap.unit = (float)u; a.cap.cap = softcap * 1.4426950408889634f;
+    }
     dim3 grid(n_heads, n_tiles);
     cudaStream_t s = (cudaStream_t)stream;
-    if (head_dim <= 64)
-        return value_dim <= 64 ? launch<64, 64>(mq, mk, mv, a, grid, merges, n_merges, s)
-                               : launch<64, 128>(mq, mk, mv, a, grid, merges, n_merges, s);
-    return value_dim <= 64 ? launch<128, 64>(mq, mk, mv, a, grid, merges, n_merges, s)
-                           : launch<128, 128>(mq, mk, mv, a, grid, merges, n_merges, s);
+    if (softcap > 0.f) return pick<CAPPED>(head_dim, value_dim, mq, mk, mv, a, grid, merges, n_merges, s);
+    if (general) return pick<GENERAL>(head_dim, value_dim, mq, mk, mv, a, grid, merges, n_merges, s);
+    return pick<FAST>(head_dim, value_dim, mq, mk, mv, a, grid, merges, n_merges, s);
 }

@@ -111,8 +111,8 @@ _SIGNATURES = {
     "fx_softcap": [_P, _L, _F, _P],
     "fx_relu_square": [_P, _I, _L, _I, _I, _P],
     "fx_prefill_attention": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
-    "fx_prefill_attention_tc": [_P, _L, _I, _P, _P, _I, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I, _I, _F, _P, _P, _L,
-                                _P, _P, _P, _P, _P, _I, _P],
+    "fx_prefill_attention_tc": [_P, _L, _L, _I, _P, _P, _I, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _I, _I, _F, _P, _P, _L,
+                                _P, _P, _I, _F, _I, _I, _P, _P, _P, _P, _I, _P],
     "fx_router_topk": [_P, _L, _I, _I, _I, _I, _P, _P, _P, _F, _F, _P],
     "fx_moe_align": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _P],
     "fx_gemm_slab_ok": [_I, _I, _I],
@@ -1422,6 +1422,18 @@ def prefill_tc_ok(q, out, k_pages, page_size, head_dim, value_dim=None, scale=1.
             and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
 
 
+def prefill_tc_general_ok(q, ldq, ldqh, k_pages, v_pages, page_size, out, ldo, ldoh, key_dim, value_dim, scale, softcap=None,
+                          kv_strides=None) -> bool:
+    """Whether that kernel takes these operands of :func:`general_attention` (no distance bias): keys of up to 192 elements
+    (capped scores: 128, and a cap of up to 40), values of up to 128, a head's results side by side."""
+    return (q.dtype == torch.bfloat16 and k_pages.dtype == torch.bfloat16 and v_pages.dtype == torch.bfloat16
+            and out.dtype == torch.bfloat16 and 0 < key_dim <= (128 if softcap else 192) and 0 < value_dim <= 128
+            and key_dim % 8 == 0 and value_dim % 8 == 0 and scale > 0 and (softcap is None or 0 < softcap <= 40 and 1e-4 <= scale / softcap <= 1e4) and page_size >= 64
+            and page_size % 64 == 0 and ldq % 8 == 0 and ldqh % 8 == 0 and ldo % 8 == 0 and ldoh == value_dim
+            and (kv_strides is None or all(int(x) > 0 and int(x) % 8 == 0 for x in kv_strides))
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_pages, v_pages, out)))
+
+
 PREFILL_KEY_BLOCK = 128          # positions per key block of the tcgen05 prompt attention kernel
 PREFILL_MAX_RUNS = 32            # runs of key blocks a tile may be cut into (a lane of the merging warp each)
 # The planner's cost model, in units of the time a block of 128 keys takes a tile (measured on a B200, 16 heads of
@@ -1433,19 +1445,19 @@ PREFILL_RUN_CHOICES = (0, 16, 12, 8, 6, 4)   # key blocks a run (0: tiles stay w
 
 def _prefill_items(tiles, run: int):
     items, merges, parts = [], [], 0
-    for tok0, rows, b, pos0, first, end in tiles:
+    for tok0, rows, b, pos0, first, end, kept in tiles:
         n_blk = end - first
         runs = min(PREFILL_MAX_RUNS, -(-n_blk // run)) if run > 0 else 1
         if runs <= 1:
-            items.append((tok0, rows, b, pos0, first, end, -1, 0))
+            items.append((tok0, rows, b, pos0, first, end, -1, kept))
             continue
         per = -(-n_blk // runs)
         first_part = parts
         for kb in range(first, end, per):
-            items.append((tok0, rows, b, pos0, kb, min(end, kb + per), parts, 0))
+            items.append((tok0, rows, b, pos0, kb, min(end, kb + per), parts, kept if kb == first else 0))
             parts += 1
         merges.append((tok0, rows, first_part, parts - first_part))
-    items.sort(key=lambda it: it[4] - it[5])      # most key blocks first (stable: ties stay in order)
+    items.sort(key=lambda it: it[4] - it[5] - it[7])      # most key blocks first (stable: ties stay in order)
     return items, merges, parts
 
 
@@ -1453,7 +1465,7 @@ def _prefill_makespan(items, parts: int, n_heads: int, sms: int) -> float:
     """How long the items take on ``sms`` SMs that take them heaviest first, each head its own copy of every item:
     no less than the heaviest item, than an even share of all work, and than the two items that must share an SM once
     there are more items than SMs; plus the adding up of the parts."""
-    costs = [it[5] - it[4] + PREFILL_ITEM_OVERHEAD for it in items]           # descending already
+    costs = [it[5] - it[4] + it[7] + PREFILL_ITEM_OVERHEAD for it in items]           # descending already
     n = len(costs) * n_heads
     est = max(costs[0], sum(costs) * n_heads / sms)
     if n > sms:
@@ -1472,7 +1484,49 @@ def first_key(pos: int, window=None, chunk=None) -> int:
     return max(lo, pos // int(chunk) * int(chunk)) if chunk else lo
 
 
-def prefill_tc_plan(entries, window, n_heads: int, sms: int = 0, run_blocks: int = -1, chunk=None):
+def prefill_tc_better(entries, window, n_heads: int, key_dim: int, value_dim: int, *, chunk=None, keep_first: int = 0,
+                      capped: bool = False, sms: int = 0) -> bool:
+    """Whether the tcgen05 prompt attention kernel is clearly ahead of the mma.sync ones on a step that either takes (``entries`` as
+    for :func:`prefill_tc_plan`), in microseconds as measured on a B200.
+
+    A tile of the mma.sync kernels holds 64 (token, head) pairs of one request and goes through its keys 32 at a time, 0.058 a key
+    for rows of 256 elements (keys and values together) and longer for wider ones; all pairs of a query and a key together run at 55e6
+    elements a microsecond.  An item of this kernel (a request's tokens of one head) costs 2.2 a block of 128 keys on an empty device
+    and 3.6 on a full one, a third more with capped scores, and five blocks beside: many requests of one token each are better off in
+    the others.  16 heads of 128, keys from 0: 16 tokens 6.8 against 9.5, 256 22 against 15, 2,048 in a window of 1,024 111 against 61
+    (capped 127 against 83); 16 tokens after 700 keys 54 against 25; 15 single tokens beside 300 52 against 51, capped, 32 heads 52
+    against 124."""
+    sms = sms or sm_count()
+    window, chunk, tile, block = int(window or 0), int(chunk or 0), WIDE_PREFILL_TILE, PREFILL_KEY_BLOCK
+    kept_blocks = -(-keep_first // block) if window else 0
+    width, pairs, most, items, work, longest = key_dim + value_dim, 0.0, 0, 0, 0, 0
+    for n, start in entries:          # (every step without a graph asks: no calls in here)
+        reach = start + n
+        if window and window + keep_first < reach:
+            reach = window + keep_first
+        if chunk and chunk < reach:
+            reach = chunk
+        if reach > most:
+            most = reach
+        mean = start + 0.5 * n
+        pairs += n * (reach if reach < mean else mean)
+        for pos0 in range(start, start + n, tile):
+            last = pos0 + tile - 1 if pos0 + tile < start + n else start + n - 1
+            first = pos0 - window + 1 if window and pos0 >= window else 0
+            if chunk and pos0 - pos0 % chunk > first:
+                first = pos0 - pos0 % chunk
+            first //= block
+            cost = last // block + 1 - first + (kept_blocks if kept_blocks < first else first) + PREFILL_ITEM_OVERHEAD
+            items += 1
+            work += cost
+            if cost > longest:
+                longest = cost
+    mma = max(5.0 + 0.058 * most * max(1.0, width / 256), pairs * n_heads * width / 55e6)
+    unit = (2.2 + 1.4 * min(1.0, items * n_heads / sms)) * (1.3 if capped else 1.0)
+    return unit * max(longest, work * n_heads / sms) < 0.85 * mma
+
+
+def prefill_tc_plan(entries, window, n_heads: int, sms: int = 0, run_blocks: int = -1, chunk=None, keep_first: int = 0):
     """The work items of the tcgen05 prompt attention kernel for a step.  ``entries``: (tokens, first position) of
     each entry, in the order of the flattened batch.  A tile is up to 256 queries of one entry; it sees the key blocks
     (of 128 positions) from its first query's first visible key to its last query's own.  Tiles with many key blocks
@@ -1481,7 +1535,8 @@ def prefill_tc_plan(entries, window, n_heads: int, sms: int = 0, run_blocks: int
     (PREFILL_ITEM_OVERHEAD), so the run length is the one of PREFILL_RUN_CHOICES whose items finish first by
     :func:`_prefill_makespan`, and whole tiles stay unless a cut is 15 % faster by that estimate.  Returns (items int32 [n, 8], merges int32 [m, 4], parts) as
     ``fx_prefill_attention_tc`` takes them: heavy items first; a tile's runs have consecutive parts in the order of
-    their keys.  ``run_blocks`` >= 0: this many key blocks a run instead of the choice (0: no cut; tests)."""
+    their keys.  ``keep_first`` (with a window): the positions below it stay visible; their blocks before a tile's own go to
+    its first run.  ``run_blocks`` >= 0: this many key blocks a run instead of the choice (0: no cut; tests)."""
     import numpy as np
 
     sms = sms or sm_count()
@@ -1491,7 +1546,8 @@ def prefill_tc_plan(entries, window, n_heads: int, sms: int = 0, run_blocks: int
             rows, pos0 = min(WIDE_PREFILL_TILE, n - i), start + i
             first = first_key(pos0, window, chunk) // PREFILL_KEY_BLOCK
             end = (pos0 + rows - 1) // PREFILL_KEY_BLOCK + 1
-            tiles.append((flat + i, rows, b, pos0, first, end))
+            kept = min(first, -(-keep_first // PREFILL_KEY_BLOCK)) if window else 0
+            tiles.append((flat + i, rows, b, pos0, first, end, kept))
         flat += n
     best = first = None
     whole = 0.0
@@ -1511,20 +1567,28 @@ def prefill_tc_plan(entries, window, n_heads: int, sms: int = 0, run_blocks: int
 
 def prefill_attention_tc(q, k_pages, v_pages, block_table, page_size, items, seq_slot, out, n_heads, n_kv_heads,
                          head_dim, window, scale, status=None, stream=None, merges=None, part_o=None, part_ml=None,
-                         value_dim=None, chunk=None, sinks=None, gate=None, turn=None):
+                         value_dim=None, chunk=None, sinks=None, gate=None, turn=None, q_strides=None, kv_strides=None,
+                         keep_first=0, softcap=None, value_share=1, general=False, n_pages=None):
     """Flash attention of prompt portions on the tcgen05 tensor cores (bfloat16, keys and values of up to 128 elements
     in steps of 8, pages of a multiple of 64 positions).  ``value_dim``, ``chunk``, ``sinks``, ``gate``,
-    ``turn``: as :func:`paged_attention_ex`.  ``items``, ``merges``: device copies of what :func:`prefill_tc_plan` returns;
+    ``turn``: as :func:`paged_attention_ex`.  ``general``: with exp2f for the softmax's weights, and then also what
+    :func:`prefill_tc_general_ok` takes: ``keep_first`` (``items`` made with it), ``softcap``, ``value_share``, keys of up to
+    192 elements, ``q_strides`` = (row, head) and ``kv_strides`` = (page, head, position of the keys, of the values) in
+    elements, with ``n_pages`` pages.  ``items``, ``merges``: device copies of what :func:`prefill_tc_plan` returns;
     ``part_o`` float32 [parts, n_heads, 256, :func:`prefill_value_width`] and ``part_ml`` float32 [parts, n_heads, 256, 2]: scratch for the
     tiles that were cut into runs of key blocks (a second kernel adds the runs up)."""
     global _launches
     n_merges = merges.shape[0] if merges is not None else 0
     if n_merges:
         _launches += 1
-    call("fx_prefill_attention_tc", _ptr(q), _rows(q), q.shape[0], _ptr(k_pages), _ptr(v_pages), k_pages.shape[0],
-         _ptr(block_table), block_table.shape[1], page_size, _ptr(items), items.shape[0], _ptr(seq_slot), _ptr(out),
-         _rows(out), n_heads, n_kv_heads, head_dim, int(value_dim or head_dim), int(window or 0), int(chunk or 0), float(scale),
-         _ptr(sinks), _ptr(gate), _rows(gate) if gate is not None else 0, _ptr(turn), _ptr(status),
+    ldq, ldqh = q_strides if q_strides is not None else (_rows(q), head_dim)
+    strides = (ctypes.c_long * 6)(*[int(x) for x in kv_strides]) if kv_strides is not None else None
+    call("fx_prefill_attention_tc", _ptr(q), int(ldq), int(ldqh), q.shape[0], _ptr(k_pages), _ptr(v_pages),
+         int(n_pages or k_pages.shape[0]), _ptr(block_table), block_table.shape[1], page_size, _ptr(items), items.shape[0],
+         _ptr(seq_slot), _ptr(out), _rows(out), n_heads, n_kv_heads, head_dim, int(value_dim or head_dim), int(window or 0), int(chunk or 0), float(scale),
+         _ptr(sinks), _ptr(gate), _rows(gate) if gate is not None else 0, _ptr(turn),
+         ctypes.cast(strides, c_void_p) if strides is not None else None, int(keep_first or 0), float(softcap or 0.0),
+         int(value_share), int(general), _ptr(status),
          _ptr(part_o) if n_merges else None, _ptr(part_ml) if n_merges else None, _ptr(merges) if n_merges else None,
          n_merges, stream if stream is not None else stream_ptr())
     return out

@@ -53,18 +53,37 @@ def query_tiles(batch, rows: int) -> torch.Tensor:
     return t
 
 
-def prefill_tc_plan(batch, window, n_heads: int, chunk=None):
+def prefill_tc_plan(batch, window, n_heads: int, chunk=None, keep_first: int = 0):
     """This step's work items for the tcgen05 prompt attention kernel (``ops.prefill_tc_plan``) on the device: made
     once a step for each window and chunk and shared by the layers that have it."""
-    key = ("attention tcgen05 items", window, n_heads, chunk)
+    key = ("attention tcgen05 items", window, n_heads, chunk, keep_first)
     plan = batch.shared.get(key)
     if plan is None:
         items, merges, parts = ops.prefill_tc_plan([(len(e.tokens), e.start) for e in batch.entries], window, n_heads,
-                                                   chunk=chunk)
+                                                   chunk=chunk, keep_first=keep_first)
         both = ops.upload(np.concatenate([items.reshape(-1), merges.reshape(-1)]), batch.token_ids.device)
         plan = (both[:items.size].view(-1, 8), both[items.size:].view(-1, 4) if merges.size else None, parts)
         batch.shared[key] = plan
     return plan
+
+
+def prefill_tc_better(batch, window, n_heads, key_dim, value_dim, chunk=None, keep_first=0, capped=False) -> bool:
+    """``ops.prefill_tc_better`` for this step, asked once for the layers that share it."""
+    key = ("attention tcgen05 better", window, n_heads, key_dim, value_dim, chunk, keep_first, capped)
+    better = batch.shared.get(key)
+    if better is None:
+        better = batch.shared[key] = ops.prefill_tc_better(
+            [(len(e.tokens), e.start) for e in batch.entries], window, n_heads, key_dim, value_dim, chunk=chunk,
+            keep_first=keep_first, capped=capped)
+    return better
+
+
+def prefill_tc_scratch(rt, parts, n_heads, value_dim):
+    """Where the tiles that were cut into runs leave their results (None, None: there are none)."""
+    if not parts:
+        return None, None
+    return (rt.empty(parts, n_heads, ops.WIDE_PREFILL_TILE, ops.prefill_value_width(value_dim), dtype=torch.float32),
+            rt.empty(parts, n_heads, ops.WIDE_PREFILL_TILE, 2, dtype=torch.float32))
 
 
 class GqaAttention(Mixer):
@@ -297,17 +316,17 @@ class GqaAttention(Mixer):
                 store_new=in_kernel is not None, write_pages=cache.writes, cos_sin=in_kernel[0] if in_kernel else None,
                 softcap=self.softcap,
             )
-        elif not capped and ops.prefill_tc_ok(qkv, attn, cache.k, cache.page_size, s.head_dim):
+        elif (prefill_tc_better(batch, s.window, s.n_heads, s.head_dim, s.head_dim, capped=True)
+              and ops.prefill_tc_general_ok(qkv, qkv.stride(0), s.head_dim, cache.k, cache.v, cache.page_size, attn, attn.stride(0),
+                                            s.head_dim, s.head_dim, s.head_dim, self.scale, self.softcap) if capped else
+              ops.prefill_tc_ok(qkv, attn, cache.k, cache.page_size, s.head_dim)):
             # prompt portions: tiles of 256 queries (long ones cut into runs of key blocks), tcgen05
             items, merges, parts = prefill_tc_plan(batch, s.window, s.n_heads)
-            part_o = part_ml = None
-            if parts:
-                part_o = self.rt.empty(parts, s.n_heads, ops.WIDE_PREFILL_TILE, s.head_dim, dtype=torch.float32)
-                part_ml = self.rt.empty(parts, s.n_heads, ops.WIDE_PREFILL_TILE, 2, dtype=torch.float32)
+            part_o, part_ml = prefill_tc_scratch(self.rt, parts, s.n_heads, s.head_dim)
             ops.prefill_attention_tc(
                 qkv, cache.k, cache.v, cache.block_table, cache.page_size, items, batch.seq_slot, attn,
                 s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, status=batch.status, stream=batch.stream,
-                merges=merges, part_o=part_o, part_ml=part_ml,
+                merges=merges, part_o=part_o, part_ml=part_ml, softcap=self.softcap, general=capped,
             )
         elif ops.prefill_ok(qkv, attn, cache.k, s.head_dim):
             # prompt portions, other head and page sizes: tiles of 64 queries, mma.sync
@@ -386,10 +405,7 @@ class GqaAttention(Mixer):
         elif (not few and not self.slopes_spec and not self.keep_first
               and ops.prefill_tc_ok(qkv, attn, cache.k, cache.page_size, D, V, self.scale)):
             items, merges, parts = prefill_tc_plan(batch, s.window, s.n_heads, self.chunk)
-            part_o = part_ml = None
-            if parts:
-                part_o = self.rt.empty(parts, s.n_heads, ops.WIDE_PREFILL_TILE, ops.prefill_value_width(V), dtype=torch.float32)
-                part_ml = self.rt.empty(parts, s.n_heads, ops.WIDE_PREFILL_TILE, 2, dtype=torch.float32)
+            part_o, part_ml = prefill_tc_scratch(self.rt, parts, s.n_heads, V)
             ops.prefill_attention_tc(qkv, cache.k, cache.v, cache.block_table, cache.page_size, items, batch.seq_slot, attn,
                                      s.n_heads, s.n_kv_heads, D, s.window, self.scale, status=batch.status,
                                      stream=batch.stream, merges=merges, part_o=part_o, part_ml=part_ml, value_dim=V,
@@ -441,8 +457,21 @@ def general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldoh, 
     """Attention over pages in its general form (keys and values of different widths, strided queries and outputs, an
     optional distance bias, a window that may keep the request's first positions visible, chunks, capped scores, a
     learned number per head in the softmax's denominator, key heads that share value heads, a result turned back by
-    the query's position, a result multiplied by the sigmoid of a gate), by the kernel that fits the step: tiles of (token, head) pairs on the tensor cores
-    in bfloat16, a warp per (token, head) on the CUDA cores in 32-bit and for widths that are no multiple of 16."""
+    the query's position, a result multiplied by the sigmoid of a gate), by the kernel that fits the step: in bfloat16 tiles of
+    256 queries of a head by tcgen05 or of (token, head) pairs by mma.sync, a warp per (token, head) on the CUDA cores in 32-bit and
+    for widths that are no multiple of 16."""
+    if (batch.max_new > DECODE_ATTENTION_MAX_NEW and slopes is None and ldk == key_dim and ldv == value_dim
+            and prefill_tc_better(batch, window, n_heads, key_dim, value_dim, chunk, keep_first, bool(softcap))
+            and ops.prefill_tc_general_ok(q, ldq, ldqh, k_pages, v_pages, cache.page_size, out, ldo, ldoh, key_dim, value_dim, scale,
+                                          softcap)
+            and k_pages.is_contiguous() and v_pages.is_contiguous()):
+        items, merges, parts = prefill_tc_plan(batch, window, n_heads, chunk, keep_first)
+        part_o, part_ml = prefill_tc_scratch(rt, parts, n_heads, value_dim)
+        return ops.prefill_attention_tc(q, k_pages, v_pages, cache.block_table, cache.page_size, items, batch.seq_slot, out, n_heads,
+                                        n_kv_heads, key_dim, window, scale, status=batch.status, stream=batch.stream, merges=merges,
+                                        part_o=part_o, part_ml=part_ml, value_dim=value_dim, chunk=chunk, sinks=sinks, gate=gate,
+                                        turn=turn, q_strides=(ldq, ldqh), keep_first=keep_first, softcap=softcap,
+                                        value_share=value_share, general=True)
     per_sm = ops.general_attention_ok(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldoh, key_dim, value_dim)
     if per_sm:
         items, n_splits, part_o, part_ml = None, 1, None, None

@@ -34,7 +34,8 @@ import torch
 from ..cache.specs import CacheSpec, PagedSpec, PagedTensorSpec
 from ..kernels import ops
 from ..weights.loader import TensorDecl
-from .attention import _common_dtype, general_attention
+from .attention import (DECODE_ATTENTION_MAX_NEW, _common_dtype, general_attention, prefill_tc_better, prefill_tc_plan,
+                        prefill_tc_scratch)
 from .base import Mixer, build_part, register_part
 from .specs import AdjacentRotarySpec, ScaledRotarySpec
 
@@ -235,9 +236,20 @@ class LatentAttention(Mixer):
         ops.linear(seen.view(n_copies * ps, row), self.w_exp, kv, status=batch.status, stream=st)
         attn = rt.empty(T, self.o_size)
         k_view, v_view = kv, kv[:, H * (D + R):]
-        ops.general_attention(q, q.stride(0), D + R, k_view, v_view, wide, wide, table, ps, batch.positions, batch.token_seq,
-                              rows_of, items, attn, attn.stride(0), V, H, H, D + R, V, s.window, s.scale, stream=st,
-                              kv_strides=(ps * wide, D + R, ps * wide, V), sinks=self.sink)
+        strides = (ps * wide, D + R, wide, ps * wide, V, wide)       # of a page, a head, a position: keys, values
+        if (batch.max_new > DECODE_ATTENTION_MAX_NEW and prefill_tc_better(batch, s.window, H, D + R, V)
+                and ops.prefill_tc_general_ok(q, q.stride(0), D + R, k_view, v_view, ps, attn, attn.stride(0), V, D + R, V, s.scale,
+                                              kv_strides=strides)):
+            tc_items, merges, parts = prefill_tc_plan(batch, s.window, H)
+            part_o, part_ml = prefill_tc_scratch(rt, parts, H, V)
+            ops.prefill_attention_tc(q, k_view, v_view, table, ps, tc_items, rows_of, attn, H, H, D + R, s.window, s.scale,
+                                     status=batch.status, stream=st, merges=merges, part_o=part_o, part_ml=part_ml, value_dim=V,
+                                     sinks=self.sink, q_strides=(q.stride(0), D + R), kv_strides=strides, n_pages=n_copies,
+                                     general=True)
+        else:
+            ops.general_attention(q, q.stride(0), D + R, k_view, v_view, wide, wide, table, ps, batch.positions, batch.token_seq,
+                                  rows_of, items, attn, attn.stride(0), V, H, H, D + R, V, s.window, s.scale, stream=st,
+                                  kv_strides=(ps * wide, D + R, ps * wide, V), sinks=self.sink)
         if gate is not None:
             ops.gate_heads_(attn, gate, H, stream=st, gate_per_head=self.gate_per_head)
         ops.linear(attn, self.w_o, out, accumulate=accumulate, status=batch.status, stream=st, after_short_kernel=True)

@@ -240,3 +240,18 @@ def test_tiles_of_dense_products_by_rounds():
         for n in (512, 1000, 2048, 3584, 20480):
             pairs, tile = ops.dense_tile(m, n)
             assert tile in ((192, 256) if pairs else (128, 160, 192, 224, 256)) and (not pairs or ops.pairs_better(m, n))
+
+
+def test_which_prompts_the_general_forms_take_to_tcgen05():
+    """Where the two kernels were measured more than a tenth apart; kept blocks are an item's, of its first run only."""
+    better = lambda e, window=None, heads=16, d=128, v=128, **k: ops.prefill_tc_better(e, window, heads, d, v, sms=148, **k)
+    assert better([(2048, 0)], 1024, keep_first=4) and better([(256, 0)], 1024) and better([(16, 700)]) and better([(1531, 0)], d=192)
+    assert better([(2048, 0)], 1024, capped=True) and better([(1531, 0)], heads=32, d=64, capped=True)
+    assert not better([(9, 0)]) and not better([(40, 0)], capped=True)
+    singles = [(1, 700)] * 15 + [(300, 0)]
+    assert not better(singles, heads=32, d=64, capped=True) and not better(singles, 1024, capped=True)
+    items, merges, parts = ops.prefill_tc_plan([(700, 0)], 150, 4, run_blocks=2, keep_first=200)
+    for tok0, rows, entry, pos0, first, end, part, kept in items.tolist():
+        blk = max(0, pos0 - 149) // 128
+        assert kept == (min(2, blk) if first == blk else 0)
+    assert all(k == 0 for *_, k in ops.prefill_tc_plan([(700, 0)], None, 4, keep_first=200)[0].tolist())

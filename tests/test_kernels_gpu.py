@@ -1158,6 +1158,105 @@ def test_prefill_attention_tcgen05(case, run_blocks):
     assert rel(got, vs[0][far, 0]) < 5e-2
 
 
+def general_attention_in_64_bits(q, kp, vp, table, lens, starts, H, G, share, window, keep, chunk, cap, scale, sinks):
+    """[tokens, H, V] of the general forms, from the pages; q [tokens, H, D]."""
+    outs, flat = [], 0
+    for b, (n, start) in enumerate(zip(lens, starts)):
+        L = start + n
+        pages = table[b, :-(-L // kp.shape[2])].long().clamp(min=0)
+        K, V = (t[pages].transpose(0, 1).flatten(1, 2)[:, :L].double() for t in (kp, vp))
+        i, j = torch.arange(start, L, device=DEV)[:, None], torch.arange(L, device=DEV)[None]
+        seen = j <= i
+        if window:
+            seen &= (j > i - window) | (j < keep)
+        if chunk:
+            seen &= j // chunk == i // chunk
+        out = []
+        for h in range(H):
+            s = q[flat:flat + n, h].double() @ K[h * G // H].T * scale
+            s = (cap * torch.tanh(s / cap) if cap else s).masked_fill(~seen, -math.inf)
+            if sinks is not None:
+                s = torch.cat([s, sinks[h].double().expand(n, 1)], 1)
+            out.append(torch.softmax(s, -1)[:, :L] @ V[h * G // H // share])
+        outs.append(torch.stack(out, 1))
+        flat += n
+    return torch.cat(outs)
+
+
+# heads, key heads, key heads a value head, D, V, window, keep_first, chunk, cap, sinks, query size, (lengths, starts)
+TC_GENERAL = [
+    (8, 4, 2, 64, 128, 0, 0, None, 30.0, False, 3.0, ([300, 9], [0, 500])),     # scores up to a sixth of the cap: all by the cubic
+    (4, 2, 1, 128, 128, 200, 0, None, 5.0, True, 8.0, ([600], [100])),           # scores beyond the cap: tanhf
+    (4, 2, 2, 128, 64, 0, 0, None, 40.0, False, 1.0, ([130, 1], [0, 0])),
+    (4, 1, 1, 128, 128, 150, 5, None, None, False, 1.0, ([700, 20], [0, 900])),
+    (2, 2, 1, 64, 64, 129, 300, None, None, True, 1.0, ([900], [0])),            # kept blocks that the first tile's own range holds
+    (2, 1, 1, 64, 128, 130, 128, None, 20.0, False, 2.0, ([513, 64], [300, 0])),
+    (3, 3, 1, 192, 128, 0, 0, None, None, True, 1.0, ([700, 40], [0, 300])),
+    (2, 2, 1, 136, 64, 300, 0, None, None, False, 1.0, ([400], [600])),
+    (2, 2, 1, 192, 64, 256, 7, None, None, False, 1.0, ([1000], [0])),
+    (2, 1, 1, 96, 40, 0, 0, 300, None, False, 1.0, ([700], [50])),
+]
+
+
+@pytest.mark.parametrize("run_blocks", [-1, 0, 1, 2])
+@pytest.mark.parametrize("case", TC_GENERAL)
+def test_prefill_attention_tcgen05_general(case, run_blocks):
+    """The general forms on the tcgen05 kernel: capped scores, kept first positions, shared value heads, wide keys, sinks,
+    chunks; tiles whole and cut, strided queries, pages behind a window given back.  Against 64 bits: P and the result are
+    rounded to bfloat16 (2^-9 each, a row's P weighted), as in the mma.sync kernels' test."""
+    o = ops()
+    H, G, share, D, V, window, keep, chunk, cap, with_sinks, size, (lens, starts) = case
+    ps, T, n = 64, sum(lens), len(lens)
+    width = max(-(-(s + l) // ps) for s, l in zip(starts, lens))
+    perm = torch.randperm(n * width + 1, generator=torch.Generator().manual_seed(7))[:n * width].view(n, width)
+    table = perm.to(torch.int32).to(DEV)
+    kp, vp = rnd(n * width + 1, G, ps, D, dtype=torch.bfloat16, seed=1), rnd(n * width + 1, G // share, ps, V, dtype=torch.bfloat16, seed=2)
+    rows = rnd(T, H * D + 16, dtype=torch.bfloat16, seed=3, scale=size)
+    q = rows[:, :H * D]
+    sinks = rnd(H, seed=4) if with_sinks else None
+    scale = D ** -0.5
+    want = general_attention_in_64_bits(q.reshape(T, H, D), kp, vp, table, lens, starts, H, G, share, window, keep, chunk, cap, scale, sinks)
+    if window:      # pages that no query of the step sees: given back
+        for b, s in enumerate(starts):
+            table[b, -(-keep // ps):max(-(-keep // ps), (s - window + 1) // ps)] = -1
+    items, merges, parts = o.prefill_tc_plan(list(zip(lens, starts)), window, H, run_blocks=run_blocks, chunk=chunk, keep_first=keep)
+    part_o = torch.full((max(parts, 1), H, 256, o.prefill_value_width(V)), float("nan"), device=DEV)
+    part_ml = torch.full((max(parts, 1), H, 256, 2), float("nan"), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = torch.full((T, H * V + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    assert o.prefill_tc_general_ok(q, q.stride(0), D, kp, vp, ps, out, out.stride(0), V, D, V, scale, cap)
+    o.prefill_attention_tc(q, kp, vp, table, ps, torch.from_numpy(items).to(DEV), torch.arange(n, dtype=torch.int32, device=DEV),
+                           out[:, :H * V], H, G, D, window, scale, status=status, merges=torch.from_numpy(merges).to(DEV) if parts else None,
+                           part_o=part_o, part_ml=part_ml, value_dim=V, chunk=chunk, sinks=sinks, q_strides=(q.stride(0), D),
+                           keep_first=keep, softcap=cap, value_share=share, general=True)
+    assert int(status) == 0 and bool((out[:, H * V:] == 7).all())
+    got = out[:, :H * V].reshape(T, H, V).double()
+    assert rel(got, want) < 4e-3
+    err = (got - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+    assert float(err.max()) < 1.2e-2
+
+
+def test_prefill_attention_tcgen05_keys_and_values_side_by_side():
+    """Rows that hold all heads' keys and values next to each other, reached by strides, are what pages of their own are."""
+    o = ops()
+    H, D, V, ps, n_pages, T = 3, 192, 128, 128, 4, 300
+    wide = H * (D + V)
+    kv = rnd(n_pages * ps, wide, dtype=torch.bfloat16, seed=1)
+    kp = kv[:, :H * D].reshape(n_pages, ps, H, D).transpose(1, 2).contiguous()
+    vp = kv[:, H * D:].reshape(n_pages, ps, H, V).transpose(1, 2).contiguous()
+    q = rnd(T, H * D, dtype=torch.bfloat16, seed=2)
+    table = torch.tensor([[2, 0, 3, 1]], dtype=torch.int32, device=DEV)
+    items, merges, parts = o.prefill_tc_plan([(T, 150)], None, H, run_blocks=0)
+    slot = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for k, v, strides in ((kp, vp, None), (kv, kv[:, H * D:], (ps * wide, D, wide, ps * wide, V, wide))):
+        out = torch.empty(T, H * V, dtype=torch.bfloat16, device=DEV)
+        o.prefill_attention_tc(q, k, v, table, ps, torch.from_numpy(items).to(DEV), slot, out, H, H, D, None, D ** -0.5, value_dim=V,
+                               kv_strides=strides, n_pages=n_pages, general=True)
+        outs.append(out)
+    assert torch.equal(*outs)
+
+
 def test_prefill_attention_tcgen05_refuses_other_sizes():
     o = ops()
     q = rnd(4, 3 * 136, dtype=torch.bfloat16)
@@ -1169,6 +1268,11 @@ def test_prefill_attention_tcgen05_refuses_other_sizes():
     slots = torch.zeros(1, dtype=torch.int32, device=DEV)
     with pytest.raises(o.KernelError):
         o.prefill_attention_tc(q, kp, kp, table, 64, tiles, slots, out, 1, 1, 136, 0, 1.0)
+    for bad in (dict(softcap=50.0), dict(softcap=-1.0), dict(softcap=30.0, scale=1e-6), dict(value_share=2), dict(keep_first=-1)):
+        with pytest.raises(o.KernelError):
+            o.prefill_attention_tc(q, kp, kp, table, 64, tiles, slots, out[:, :128], 1, 1, 128, 10, **dict(dict(scale=1.0, general=True), **bad))
+    with pytest.raises(o.KernelError):       # the plain kernel has none of the general forms
+        o.prefill_attention_tc(q, kp, kp, table, 64, tiles, slots, out[:, :128], 1, 1, 128, 10, 1.0, keep_first=3)
 
 
 def test_gemm_skinny_transposed_store_and_linear_picks_it_for_narrow_outputs():
