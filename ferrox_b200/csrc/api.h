@@ -29,13 +29,14 @@ int fx_zero_slots(const long* table, int n, long most, long slot, void* stream);
 // The recurrences of matrix-state mixers in chunks of tokens (chunk_scan.cu).
 int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const float* v, long ldv, const float* g, const float* beta,
                   const float* take, float q_scale, float* p, float* gam, float* e, float* wr, const float* norm_in, float* norm,
-                  int copies, const float* floor_m, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,
-                  const int* seq_slot, int n_tokens, int n_entries, int H, int G, int D, int V, int* status, void* stream);
+                  int copies, const float* floor_m, float* state, float* out, const int* tiles, int n_tiles, const int* walks,
+                  const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int G, int D, int V, int* status,
+                  void* stream);
 int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, const float* a_pre, long lda,
                           const float* low, long ldl, const void* w2, int w2_dtype, const void* w0, int w0_dtype,
                           const void* a_bias, int ab_dtype, float rate, int rank, float* p, float* gam, float* wr, float* qs,
-                          float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles, const int* token_seq,
-                          const int* seq_slot, int n_tokens, int n_entries, int H, int D, int* status, void* stream);
+                          float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles, const int* walks,
+                          const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, int* status, void* stream);
 int fx_mlstm_gates(const float* gates, long ldg, const void* i_bias, const void* f_bias, int bias_dtype, float cap, float* m,
                    int copies, const float* norm, float* norm_in, int D, float* keep, float* take, float* floor_m,
                    const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, void* stream);

@@ -30,12 +30,19 @@
 // before the state is added to it, and the mLSTM's maxima in 64 bits (states 1.1).
 //
 // Kernels: *_chunks make what a chunk needs (a block a chunk and head); walk_kernel goes through an entry's chunks in
-// order (a block 16 columns of a head's state).  A walk's chunk is bound by the chain of its three products and two
-// barriers, at 8 warps an SM: the block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
-// columns: 128 blocks).  The next chunk's rows travel meanwhile, a TMA box a tensor where the heads fill the tile and the
-// chunk is whole, else by cp.async, whose writes take 1,500 of a chunk's 7,800 cycles of shared memory (2,048 tokens of 16
-// heads of 128: 239 us by cp.async, 215 by boxes; 3,001 of 32 heads of 64, generalized: 325 and 297; by untiled bulk copies,
+// order (a block 16 columns of a head's state).  A walk's chunk is bound by what shared memory delivers to registers (128 bytes
+// a cycle, broadcasts counted whole: 4,300 of a chunk's 5,900 cycles for heads of 128 under the delta rule, before the update's
+// values were read once and doubled in registers), at 8 warps an SM; twice the warps, one half reading out while the other
+// updates, took as long.  The block's tiles are as many columns as one prompt's heads leave SMs for (16 heads of 128
+// columns: 128 blocks).  Where the host says which entry is how long, the longest is walked first (3,001 tokens in three
+// prompts of 32 heads of 64, generalized: 297 us one block an SM in the batch's order, 246 two an SM and the longest first,
+// 226 with the values read once; 2,048 of 16 heads of 128, delta: 202, 199, 186).
+// The next chunk's rows travel meanwhile, a TMA box a tensor where the heads fill the tile and the
+// chunk is whole, else by cp.async, whose writes take 1,500 of a chunk's cycles of shared memory (2,048 tokens of 16
+// heads of 128: 239 us by cp.async where boxes took 215; by untiled bulk copies,
 // one a row, 160 a chunk: twice as long).
+#include <stddef.h>
+
 #include "tc_common.cuh"
 #include "api.h"
 
@@ -577,6 +584,7 @@ struct WalkArgs {
     float* state; float* out; long ldo;
     const int *token_seq, *seq_slot;
     const int* tiles; int n_tiles;             // general: as for the chunks' kernel
+    const int* walks;                          // (or null) per entry (index, first token, one past the last, first chunk), longest first
     int n_tokens, H, D, V;
     int tma;                                   // whole chunks by the boxes of WalkMaps
     int* status;                               // raised where a wait for them runs out
@@ -591,16 +599,21 @@ template <int D, int KIND> struct alignas(128) Stage {
     static constexpr int C2 = KIND == GENERAL ? 2 * CHUNK : CHUNK;      // rows that update the state
     static constexpr int PITCH = D + 4, PP = C2 + 4;
     // (eight lanes read a row's neighbouring pieces, so that rows without padding meet no bank twice)
-    float q[CHUNK * D], k[C2 * D], w[HASW ? CHUNK * D : 4], p[CHUNK * PP];
+    // (boxes land on 128-byte boundaries; without W its place is one such piece)
+    float q[CHUNK * D], w[HASW ? CHUNK * D : 32], k[C2 * D], p[CHUNK * PP];
     float v[CHUNK * COLS], y[KIND == GENERAL ? CHUNK * COLS : 4];
     float gam[KIND == GENERAL ? D : CHUNK], e[CHUNK], fl[CHUNK];
 };
+// Partial updates of the state lie over the chunk's rows of Q (and W), which have been used by then: with the generalized rule's 120
+// KB at D = 64 an SM held one block, so it holds two.
 template <int D, int KIND> struct WalkSmem {
+    static constexpr int PART = (WALK_THREADS / D - 1) * COLS * D;
+    static constexpr bool PART_OVER_ROWS = PART <= CHUNK * D * (Stage<D, KIND>::HASW ? 2 : 1);
     Stage<D, KIND> st[2];
     float s[COLS * (D + 4)];                                     // the state's columns, along the keys
     float ut[COLS * Stage<D, KIND>::PP];                         // the update's values along the tokens,
-    float2 un[Stage<D, KIND>::C2 * COLS];                        // and along the columns, each twice (an FFMA pair's operand)
-    float part[(WALK_THREADS / D - 1) * COLS * D];               // partial updates of the state
+    float un[Stage<D, KIND>::C2 * COLS];                         // and along the columns
+    float part[PART_OVER_ROWS ? 4 : PART];
     float z[D], den[CHUNK];
     uint64_t bars[2];
     int abort;
@@ -638,17 +651,23 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
     constexpr int PARTS = WALK_THREADS / D;                      // parts of the block, each with its share of the update's rows
     extern __shared__ __align__(128) unsigned char raw[];
     WalkSmem<D, KIND>& sm = *reinterpret_cast<WalkSmem<D, KIND>*>(raw);
-    const int tid = threadIdx.x, b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
+    const int tid = threadIdx.x, h = blockIdx.y, col0 = blockIdx.x * COLS;
     fx_pdl_wait_only();
-    const int r0 = first_row_of(a.token_seq, a.n_tokens, b), r1 = first_row_of(a.token_seq, a.n_tokens, b + 1);
+    int b = blockIdx.z, r0, r1, tile0 = 0;           // (tile0: the entry's first chunk)
+    if (a.walks) {
+        const int4 w = reinterpret_cast<const int4*>(a.walks)[blockIdx.z];
+        b = w.x; r0 = w.y; r1 = w.z; tile0 = w.w;
+    } else {
+        r0 = first_row_of(a.token_seq, a.n_tokens, b);
+        r1 = first_row_of(a.token_seq, a.n_tokens, b + 1);
+    }
     if (r1 <= r0) return;
     const int nc = min(COLS, a.V - col0);
     const long slot = a.seq_slot[b];
     float* state = a.state + ((slot * a.H + h) * a.V + col0) * a.D;
 
     const long HD = (long)a.H * a.D, HV = (long)a.H * a.V;
-    int tile0 = 0;                   // general: the entry's first chunk
-    if (KIND == GENERAL) {
+    if (KIND == GENERAL && !a.walks) {
         int hi = a.n_tiles;
         while (tile0 < hi) {
             const int mid = (tile0 + hi) >> 1;
@@ -785,10 +804,10 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
                 u[i] = st.v[t * COLS + c];
                 if (KIND == DELTA_RULE) u[i] -= x[i];
                 const float ue = KIND == GENERAL ? u[i] : u[i] * st.e[t];
-                sm.un[t * COLS + c] = make_float2(ue, ue);
+                sm.un[t * COLS + c] = ue;
                 if (KIND == GENERAL) {
                     y[i] = st.y[t * COLS + c] + x[i];
-                    sm.un[(CHUNK + t) * COLS + c] = make_float2(y[i], y[i]);
+                    sm.un[(CHUNK + t) * COLS + c] = y[i];
                 }
             }
             *reinterpret_cast<float2*>(sm.ut + c * PP + tl) = make_float2(u[0], u[1]);
@@ -882,15 +901,16 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
         for (int i = 0; i < C2 / PARTS; ++i) {
             const int s = part * (C2 / PARTS) + i;
             const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(st.k + s * D + dg * 4);
-            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4);
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sm.un + s * COLS + cg * 4 + 2);
-            fma2(U[0][0], k.x, u.x); fma2(U[0][1], k.y, u.x); fma2(U[1][0], k.x, u.y); fma2(U[1][1], k.y, u.y);
-            fma2(U[2][0], k.x, v.x); fma2(U[2][1], k.y, v.x); fma2(U[3][0], k.x, v.y); fma2(U[3][1], k.y, v.y);
+            const float4 u4 = *reinterpret_cast<const float4*>(sm.un + s * COLS + cg * 4);
+            const float u[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { const u64 uu = pair(u[j], u[j]); fma2(U[j][0], k.x, uu); fma2(U[j][1], k.y, uu); }
         }
+        float* const parts = WalkSmem<D, KIND>::PART_OVER_ROWS ? st.q : sm.part;       // (everyone is behind the barrier after the products with Q and W)
         if (part > 0) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<ulonglong2*>(sm.part + ((part - 1) * COLS + cg * 4 + j) * D + dg * 4) = make_ulonglong2(U[j][0], U[j][1]);
+                *reinterpret_cast<ulonglong2*>(parts + ((part - 1) * COLS + cg * 4 + j) * D + dg * 4) = make_ulonglong2(U[j][0], U[j][1]);
         }
         __syncthreads();
         if (part == 0) {
@@ -898,7 +918,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
             for (int j = 0; j < 4; ++j) {
 #pragma unroll
                 for (int i = 0; i < PARTS - 1; ++i) {
-                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sm.part + (i * COLS + cg * 4 + j) * D + dg * 4);
+                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(parts + (i * COLS + cg * 4 + j) * D + dg * 4);
                     U[j][0] = add2(U[j][0], x.x);
                     U[j][1] = add2(U[j][1], x.y);
                 }
@@ -908,6 +928,7 @@ __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(WalkArgs a, const __
             }
         }
         if (KIND == MLSTM && tid < D) sm.z[tid] = z;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // (boxes will be written where partial updates were)
     }
     fx_pdl_trigger();
     if (part == 0) {
@@ -935,10 +956,18 @@ bool row_map(CUtensorMap* m, const float* p, long ld, int heads, int d, int toke
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+static_assert(2 * (sizeof(WalkSmem<64, GENERAL>) + 1024) <= 233472, "two blocks an SM");
+
+template <int D, int KIND> constexpr bool on_boundaries() {
+    using S = Stage<D, KIND>;
+    return offsetof(S, q) % 128 == 0 && offsetof(S, w) % 128 == 0 && offsetof(S, k) % 128 == 0 && sizeof(S) % 128 == 0;
+}
+
 template <int D, int KIND> int go_walk(WalkArgs a, int n_entries, cudaStream_t s)
 {
     // Boxes need heads as wide as the tile (a narrower head's rows would lie closer together than the kernel reads them) and
     // as many tokens as a box has rows.  Where a map cannot be made the rows go by cp.async.
+    static_assert(on_boundaries<D, KIND>(), "where boxes land");
     WalkMaps maps = {};
     a.tma = a.D == D && a.n_tokens >= CHUNK && row_map(&maps.q, a.q, a.ldq, a.H / a.q_share, D, a.n_tokens) &&
             row_map(&maps.k, a.k, a.ldk, a.H / a.q_share, D, a.n_tokens) &&
@@ -980,15 +1009,15 @@ bool off_grid(const void* p, long ld) { return (uintptr_t)p % 16 || ld % 4; }
 extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk, const float* v, long ldv, const float* g,
                              const float* beta, const float* take, float q_scale, float* p, float* gam, float* e, float* wr,
                              const float* norm_in, float* norm, int copies, const float* floor_m, float* state, float* out,
-                             const int* tiles, int n_tiles, const int* token_seq, const int* seq_slot, int n_tokens, int n_entries,
-                             int H, int G, int D, int V, int* status, void* stream)
+                             const int* tiles, int n_tiles, const int* walks, const int* token_seq, const int* seq_slot, int n_tokens,
+                             int n_entries, int H, int G, int D, int V, int* status, void* stream)
 {
     if (n_tokens <= 0 || n_entries <= 0 || n_tiles <= 0) return FX_OK;
     int st = check(H, G, D, V, n_entries);
     if (st != FX_OK) return st;
     if (beta ? !wr || take || norm : !take || !norm || !norm_in || !floor_m || copies < 1) return FX_ERR_SIZE;
     if (off_grid(q, ldq) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(p, 0) || off_grid(state, 0) || off_grid(out, 0) ||
-        off_grid(wr, 0) || off_grid(tiles, 0))
+        off_grid(wr, 0) || off_grid(tiles, 0) || off_grid(walks, 0))
         return FX_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     ChunkArgs c = {};
@@ -1001,7 +1030,7 @@ extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk,
     WalkArgs a = {};
     a.w = wr; a.q = q; a.ldq = ldq; a.q_share = H / G; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.x0 = out; a.p = p; a.gam = gam; a.e = e;
     a.floor_m = floor_m; a.norm_in = norm_in; a.norm = norm; a.copies = copies; a.q_scale = q_scale; a.state = state; a.out = out;
-    a.ldo = (long)H * V; a.token_seq = token_seq; a.seq_slot = seq_slot; a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = V; a.status = status;
+    a.ldo = (long)H * V; a.token_seq = token_seq; a.seq_slot = seq_slot; a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = V; a.walks = walks; a.status = status;
     if (beta) return D <= 64 ? go_walk<64, DELTA_RULE>(a, n_entries, s) : go_walk<128, DELTA_RULE>(a, n_entries, s);
     return D <= 64 ? go_walk<64, MLSTM>(a, n_entries, s) : go_walk<128, MLSTM>(a, n_entries, s);
 }
@@ -1012,7 +1041,7 @@ extern "C" int fx_chunk_scan(const float* q, long ldq, const float* k, long ldk,
 extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, long ldk, const float* v, long ldv, const float* a_pre,
                                      long lda, const float* low, long ldl, const void* w2, int w2_dtype, const void* w0, int w0_dtype,
                                      const void* a_bias, int ab_dtype, float rate, int rank, float* p, float* gam, float* wr, float* qs,
-                                     float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles,
+                                     float* ks, float* as, float* state, float* out, const int* tiles, int n_tiles, const int* walks,
                                      const int* token_seq, const int* seq_slot, int n_tokens, int n_entries, int H, int D, int* status,
                                      void* stream)
 {
@@ -1022,7 +1051,7 @@ extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, l
     if (rank <= 0 || !(rate >= 0.f && rate <= 1.f)) return FX_ERR_SIZE;      // (see the header)
     if (off_grid(r, ldr) || off_grid(k, ldk) || off_grid(v, ldv) || off_grid(a_pre, lda) || off_grid(p, 0) || off_grid(gam, 0) ||
         off_grid(wr, 0) || off_grid(qs, 0) || off_grid(ks, 0) || off_grid(as, 0) || off_grid(out, 0) || off_grid(state, 0) ||
-        off_grid(tiles, 0))
+        off_grid(tiles, 0) || off_grid(walks, 0))
         return FX_ERR_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     ChunkArgs c = {};
@@ -1035,7 +1064,7 @@ extern "C" int fx_chunk_scan_general(const float* r, long ldr, const float* k, l
     WalkArgs a = {};
     a.w = wr; a.q = qs; a.ldq = (long)H * D; a.q_share = 1; a.k = ks; a.ldk = (long)H * D; a.a = as; a.v = v; a.ldv = ldv; a.x0 = out;
     a.p = p; a.gam = gam; a.q_scale = 1.f; a.state = state; a.out = out; a.ldo = (long)H * D; a.token_seq = token_seq; a.seq_slot = seq_slot;
-    a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles; a.status = status;
+    a.n_tokens = n_tokens; a.H = H; a.D = D; a.V = D; a.tiles = tiles; a.n_tiles = n_tiles; a.walks = walks; a.status = status;
     return D <= 64 ? go_walk<64, GENERAL>(a, n_entries, s) : go_walk<128, GENERAL>(a, n_entries, s);
 }
 

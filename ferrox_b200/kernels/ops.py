@@ -41,10 +41,10 @@ _SIGNATURES = {
     "fx_gemm_f32_tc": [_P, _L, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
     "fx_zero_slots": [_P, _I, _L, _L, _P],
-    "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P,
+    "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P,
                       _I, _I, _I, _I, _I, _I, _P, _P],
     "fx_chunk_scan_general": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _F, _I, _P, _P, _P, _P, _P, _P, _P,
-                              _P, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P],
+                              _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P],
     "fx_delta_prep_runs": [_P, _L, _P, _P, _P, _L, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "fx_mlstm_gates": [_P, _L, _P, _P, _I, _F, _P, _I, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "fx_embed": [_P, _I, _P, _P, _I, _I, _I, _P, _F, _P],
@@ -772,13 +772,27 @@ def chunk_scan_ok(rows, D, V, state) -> bool:
             and all(t.dtype == torch.float32 and _rows(t) % 4 == 0 and t.data_ptr() % 16 == 0 for t in rows))
 
 
+def chunk_walks(lens):
+    """The entries of a step as the chunked recurrences walk them: int32 [n, 4] rows of (entry, first token, one past its last,
+    its first chunk), the longest first (its walk is what the others fill the gaps of).  ``lens``: the entries' tokens, in the order
+    of the flattened batch."""
+    import numpy as np
+
+    rows, flat, chunks = [], 0, 0
+    for b, n in enumerate(lens):
+        rows.append((b, flat, flat + n, chunks))
+        flat, chunks = flat + n, chunks - (-n // SCAN_CHUNK)
+    rows.sort(key=lambda r: r[1] - r[2])
+    return np.asarray(rows, dtype=np.int32).reshape(-1, 4)
+
+
 def chunk_scan(q, k, v, g, state, out, tiles, token_seq, seq_slot, n_entries, H, G, D, V, *, beta=None, take=None,
-               q_scale=1.0, normalizer=None, scratch, status=None, stream=None):
+               q_scale=1.0, normalizer=None, walks=None, scratch, status=None, stream=None):
     """Over a prompt's chunks of SCAN_CHUNK tokens, with ``beta`` [T, H] the delta rule of :func:`state_scan`, with ``take``
     [T, H] and ``normalizer`` = (its value before the step, the state's copies, exp(-m)), as :func:`mlstm_gates` makes
     them, the recurrence of :func:`mlstm_scan`.  ``g`` [T, H]: the decays; ``out`` contiguous [T, H * V]; ``tiles``: int32
-    [n, 4] rows of (first token, tokens, entry, position), the entries cut into chunks; ``scratch(*shape)``: 32-bit
-    buffers."""
+    [n, 4] rows of (first token, tokens, entry, position), the entries cut into chunks; ``walks`` (or None): :func:`chunk_walks`
+    on the device; ``scratch(*shape)``: 32-bit buffers."""
     T = q.shape[0]
     if not (g.is_contiguous() and out.is_contiguous()):
         raise KernelError("chunk_scan: contiguous decays and read-outs")
@@ -788,13 +802,13 @@ def chunk_scan(q, k, v, g, state, out, tiles, token_seq, seq_slot, n_entries, H,
     call("fx_chunk_scan", _ptr(q), _rows(q), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(g), _ptr(beta), _ptr(take),
          float(q_scale), _ptr(p), _ptr(gam), _ptr(e), _ptr(wr), _ptr(norm_in), _ptr(norm),
          int(norm.shape[2]) if norm is not None else 0, _ptr(floor_m), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0],
-         _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, G, D, V, _ptr(status),
+         _ptr(walks), _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, G, D, V, _ptr(status),
          stream if stream is not None else stream_ptr())
     return out
 
 
 def chunk_scan_general(r, k, v, a_pre, low, w2, w0, a_bias, rate, state, out, tiles, token_seq, seq_slot, n_entries, H, D, *,
-                       scratch, status=None, stream=None):
+                       walks=None, scratch, status=None, stream=None):
     """:func:`general_delta_prep` and :func:`general_delta_scan` over a prompt's chunks (see :func:`chunk_scan`): ``r``,
     ``k``, ``v``, ``a_pre`` 32-bit row views [T, H*D], ``low`` [T, rank], ``w2`` contiguous [H*D, rank]; a ``rate`` of at
     most 1: a chunk's products of decays then stay above 1e-14."""
@@ -806,7 +820,7 @@ def chunk_scan_general(r, k, v, a_pre, low, w2, w0, a_bias, rate, state, out, ti
     call("fx_chunk_scan_general", _ptr(r), _rows(r), _ptr(k), _rows(k), _ptr(v), _rows(v), _ptr(a_pre), _rows(a_pre), _ptr(low),
          _rows(low), _ptr(w2), code(w2), _ptr(w0), code(w0), _ptr(a_bias), code(a_bias), float(rate), w2.shape[1], _ptr(p),
          _ptr(gam), _ptr(wr), _ptr(qs), _ptr(ks), _ptr(a_s), _ptr(state), _ptr(out), _ptr(tiles), tiles.shape[0],
-         _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, D, _ptr(status), stream if stream is not None else stream_ptr())
+         _ptr(walks), _ptr(token_seq), _ptr(seq_slot), T, int(n_entries), H, D, _ptr(status), stream if stream is not None else stream_ptr())
     return out
 
 

@@ -42,15 +42,19 @@ def query_tiles(batch, rows: int) -> torch.Tensor:
     key = ("attention query tiles", rows)
     t = batch.shared.get(key)
     if t is None:
-        out, flat = [], 0
-        for b, e in enumerate(batch.entries):
-            n = len(e.tokens)
-            for i in range(0, n, rows):
-                out.append((flat + i, min(rows, n - i), b, e.start + i))
-            flat += n
-        t = ops.upload(np.asarray(out, dtype=np.int32).reshape(-1, 4), batch.token_ids.device)
-        batch.shared[key] = t
+        t = batch.shared[key] = ops.upload(tile_rows(batch, rows), batch.token_ids.device)
     return t
+
+
+def tile_rows(batch, rows: int):
+    """:func:`query_tiles` on the host."""
+    out, flat = [], 0
+    for b, e in enumerate(batch.entries):
+        n = len(e.tokens)
+        for i in range(0, n, rows):
+            out.append((flat + i, min(rows, n - i), b, e.start + i))
+        flat += n
+    return np.asarray(out, dtype=np.int32).reshape(-1, 4)
 
 
 def prefill_tc_plan(batch, window, n_heads: int, chunk=None, keep_first: int = 0):
@@ -451,6 +455,16 @@ class GqaAttention(Mixer):
         return batch.shared[key]
 
 
+def general_items(batch, n_heads, n_kv_heads):
+    """This step's work list of the mma.sync kernel of the general form (``ops.general_attention_items``) on the device."""
+    key = ("general attention items", n_heads, n_kv_heads)
+    items = batch.shared.get(key)
+    if items is None:
+        items = batch.shared[key] = ops.upload(
+            ops.general_attention_items([len(e.tokens) for e in batch.entries], n_heads, n_kv_heads), batch.token_ids.device)
+    return items
+
+
 def general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldoh, batch, cache, n_heads, n_kv_heads,
                       key_dim, value_dim, window, scale, slopes, rt, keep_first=0, softcap=None, sinks=None,
                       value_share=1, chunk=None, gate=None, turn=None):
@@ -490,12 +504,7 @@ def general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldoh, 
                 part_o = rt.empty(T, n_heads, n_splits, value_dim, dtype=torch.float32)
                 part_ml = rt.empty(T, n_heads, n_splits, 2, dtype=torch.float32)
         if batch.max_new > 1:
-            key = ("general attention items", n_heads, n_kv_heads)
-            items = batch.shared.get(key)
-            if items is None:
-                items = ops.upload(ops.general_attention_items([len(e.tokens) for e in batch.entries], n_heads, n_kv_heads),
-                                   batch.token_ids.device)
-                batch.shared[key] = items
+            items = general_items(batch, n_heads, n_kv_heads)
         return ops.general_attention(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, cache.block_table, cache.page_size,
                                      batch.positions, batch.token_seq, batch.seq_slot, items, out, ldo, ldoh, n_heads,
                                      n_kv_heads, key_dim, value_dim, window, scale, slopes=slopes, stream=batch.stream,

@@ -34,7 +34,7 @@ import torch
 from ..cache.specs import CacheSpec, PagedSpec, PagedTensorSpec
 from ..kernels import ops
 from ..weights.loader import TensorDecl
-from .attention import (DECODE_ATTENTION_MAX_NEW, _common_dtype, general_attention, prefill_tc_better, prefill_tc_plan,
+from .attention import (DECODE_ATTENTION_MAX_NEW, _common_dtype, general_attention, general_items, prefill_tc_better, prefill_tc_plan,
                         prefill_tc_scratch)
 from .base import Mixer, build_part, register_part
 from .specs import AdjacentRotarySpec, ScaledRotarySpec
@@ -182,8 +182,8 @@ class LatentAttention(Mixer):
 
     def _expanded_plan(self, batch, cache):
         """What the expanded form needs from the host for this step, made once and shared by the layers with the same
-        window: the pages to copy (their ids in the layer's group), a block table over the copies (row = entry), the
-        entries' rows of that table, and the attention's work list (every head its own kv head)."""
+        window: the pages to copy (their ids in the layer's group), a block table over the copies (row = entry) and the
+        entries' rows of that table."""
         key = ("latent attention expanded", self.spec.window, self.spec.n_heads)
         plan = batch.shared.get(key)
         if plan is None:
@@ -196,12 +196,11 @@ class LatentAttention(Mixer):
                 src.append(ids)
                 table[b, p0:p1] = np.arange(n, n + (p1 - p0), dtype=np.int32)
                 n += p1 - p0
-            items = ops.general_attention_items([len(e.tokens) for e in batch.entries], self.spec.n_heads, self.spec.n_heads)
             flat = np.concatenate([np.concatenate(src).astype(np.int32), table.reshape(-1),
-                                   np.arange(len(spans), dtype=np.int32), items.reshape(-1)])
+                                   np.arange(len(spans), dtype=np.int32)])
             dev = ops.upload(flat, self.rt.device)
-            a, b2, c = n, n + table.size, n + table.size + len(spans)
-            plan = (dev[:a], dev[a:b2].view(len(spans), width), dev[b2:c], dev[c:].view(-1, 5), n)
+            a, b2 = n, n + table.size
+            plan = (dev[:a], dev[a:b2].view(len(spans), width), dev[b2:], n)
             batch.shared[key] = plan
         return plan
 
@@ -228,7 +227,7 @@ class LatentAttention(Mixer):
         ops.latent_prep(q, dkv, batch.positions, batch.token_seq, batch.seq_slot, self.c_norm, s.norm_eps, cos_sin,
                         s.rotary_dims, None, None, pages, cache.block_table, ps, H, D, R, C, write_cache=True,
                         status=batch.status, stream=st, pairing=self.pairing)
-        src_pages, table, rows_of, items, n_copies = self._expanded_plan(batch, cache)
+        src_pages, table, rows_of, n_copies = self._expanded_plan(batch, cache)
         seen = rt.empty(n_copies, ps * row)
         ops.gather_rows(pages.view(pages.shape[0], ps * row), src_pages, seen, stream=st)
         wide = H * (D + R) + H * V
@@ -248,7 +247,7 @@ class LatentAttention(Mixer):
                                      general=True)
         else:
             ops.general_attention(q, q.stride(0), D + R, k_view, v_view, wide, wide, table, ps, batch.positions, batch.token_seq,
-                                  rows_of, items, attn, attn.stride(0), V, H, H, D + R, V, s.window, s.scale, stream=st,
+                                  rows_of, general_items(batch, H, H), attn, attn.stride(0), V, H, H, D + R, V, s.window, s.scale, stream=st,
                                   kv_strides=(ps * wide, D + R, ps * wide, V), sinks=self.sink)
         if gate is not None:
             ops.gate_heads_(attn, gate, H, stream=st, gate_per_head=self.gate_per_head)

@@ -39,12 +39,13 @@ depend on how the request was cut, beyond rounding.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..cache.specs import CacheSpec, StateSpec
 from ..kernels import ops
 from ..weights.loader import TensorDecl
-from .attention import query_tiles
+from .attention import tile_rows
 from .base import Mixer, register_part
 
 
@@ -79,11 +80,16 @@ def chunks_better(kind, lens, H, D, V) -> bool:
 
 
 def _chunk_tiles(batch, kind, H, D, V):
-    """The step's entries cut into chunks of tokens (the work list of ``ops.chunk_scan``) where that form of a recurrence
-    is the faster one, else None."""
+    """The step's entries cut into chunks of tokens and the order to walk them in (``tiles`` and ``walks`` of
+    ``ops.chunk_scan``) where that form of a recurrence is the faster one, else None.  Made once a step and shared."""
     if batch.max_new < ops.SCAN_CHUNK or not chunks_better(kind, [len(e.tokens) for e in batch.entries], H, D, V):
         return None
-    return query_tiles(batch, ops.SCAN_CHUNK)
+    lists = batch.shared.get("chunks of tokens")
+    if lists is None:
+        tiles, walks = tile_rows(batch, ops.SCAN_CHUNK), ops.chunk_walks([len(e.tokens) for e in batch.entries])
+        both = ops.upload(np.concatenate([tiles, walks]), batch.token_ids.device)
+        lists = batch.shared["chunks of tokens"] = (both[:len(tiles)], both[len(tiles):])
+    return lists
 
 
 def _cat_rows(tensors):
@@ -166,10 +172,10 @@ class GatedDeltaRule(_StateMixer):
                                  stream=batch.stream)
         read = rt.empty(T, self.vv, dtype=f32)
         q, k, v = qkv[:, :self.qk], qkv[:, self.qk:2 * self.qk], qkv[:, 2 * self.qk:]
-        tiles = _chunk_tiles(batch, "delta", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
-        if tiles is not None:
-            ops.chunk_scan(q, k, v, g, state, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
-                           beta=beta, scratch=self._scratch, status=batch.status, stream=batch.stream)
+        chunks = _chunk_tiles(batch, "delta", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, state) else None
+        if chunks is not None:
+            ops.chunk_scan(q, k, v, g, state, read, chunks[0], batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
+                           beta=beta, walks=chunks[1], scratch=self._scratch, status=batch.status, stream=batch.stream)
         else:
             ops.state_scan(q, k, v, g, H, beta, state, read, batch.token_seq, batch.seq_slot, batch.n_seqs, H, G, D, V,
                            stream=batch.stream)
@@ -284,10 +290,10 @@ class GeneralDeltaRule(_StateMixer):
         a_pre, low = proj[:, 4 * hd:5 * hd], proj[:, 5 * hd:]
         read, state = rt.empty(T, hd, dtype=f32), cache.states["matrix"]
         # (a rate of at most 1: a chunk's products of decays stay above 1e-14, far from the end of 32-bit numbers)
-        tiles = _chunk_tiles(batch, "general", H, D, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
-        if tiles is not None:
-            ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, tiles,
-                                   batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, scratch=self._scratch,
+        chunks = _chunk_tiles(batch, "general", H, D, D) if 0 <= s.decay_rate <= 1 and ops.chunk_scan_ok((r, k, v, a_pre), D, D, state) else None
+        if chunks is not None:
+            ops.chunk_scan_general(r, k, v, a_pre, low, self.w2, self.w0, self.a_bias, s.decay_rate, state, read, chunks[0],
+                                   batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, walks=chunks[1], scratch=self._scratch,
                                    status=batch.status, stream=batch.stream)
         else:
             u, au, w = rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32), rt.empty(T, hd, dtype=f32)
@@ -362,14 +368,14 @@ class Mlstm(_StateMixer):
         gates = proj[:, 2 * self.qk + 2 * self.vv:]       # [i | f] as projected
         read = rt.empty(T, self.vv, dtype=f32)
         matrix, norm, log_max = (cache.states[n] for n in ("matrix", "normalizer", "log_max"))
-        tiles = _chunk_tiles(batch, "mlstm", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, matrix) else None
-        if tiles is not None:
+        chunks = _chunk_tiles(batch, "mlstm", H, D, V) if ops.chunk_scan_ok((q, k, v), D, V, matrix) else None
+        if chunks is not None:
             keep, take, floor = rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32), rt.empty(T, H, dtype=f32)
             before = rt.empty(batch.n_seqs, H, D, dtype=f32)
             ops.mlstm_gates(gates, self.i_bias, self.f_bias, s.gate_cap, log_max, norm, before, keep, take, floor,
                             batch.token_seq, batch.seq_slot, batch.n_seqs, H, D, stream=batch.stream)
-            ops.chunk_scan(q, k, v, keep, matrix, read, tiles, batch.token_seq, batch.seq_slot, batch.n_seqs, H, H, D, V,
-                           take=take, q_scale=float(D) ** -0.5, scratch=self._scratch, normalizer=(before, norm, floor),
+            ops.chunk_scan(q, k, v, keep, matrix, read, chunks[0], batch.token_seq, batch.seq_slot, batch.n_seqs, H, H, D, V,
+                           take=take, q_scale=float(D) ** -0.5, walks=chunks[1], scratch=self._scratch, normalizer=(before, norm, floor),
                            status=batch.status, stream=batch.stream)
         else:
             ops.mlstm_scan(q, k, v, gates, self.i_bias, self.f_bias, s.gate_cap, float(D) ** -0.5, matrix, norm, log_max,

@@ -255,3 +255,8 @@ def test_which_prompts_the_general_forms_take_to_tcgen05():
         blk = max(0, pos0 - 149) // 128
         assert kept == (min(2, blk) if first == blk else 0)
     assert all(k == 0 for *_, k in ops.prefill_tc_plan([(700, 0)], None, 4, keep_first=200)[0].tolist())
+
+
+def test_walks_of_chunked_recurrences():
+    """Longest entry first, each with its rows and its first chunk in the order of the batch."""
+    assert ops.chunk_walks([33, 1, 100, 64]).tolist() == [[2, 34, 134, 3], [3, 134, 198, 7], [0, 0, 33, 0], [1, 33, 34, 2]]

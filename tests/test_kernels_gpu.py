@@ -1859,3 +1859,25 @@ def test_a_slot_of_every_state_is_zeroed_and_no_other():
     SlotZeroer(ts)(2)
     for t in ts:
         assert (t[2] == 0).all() and (t[[0, 1, 3]] == 1).all()
+
+
+@pytest.mark.parametrize("kind,D", [("delta", 64), ("delta", 128), ("general", 64), ("general", 128)])
+def test_chunk_scans_by_a_list_of_walks(kind, D):
+    """Which block walks which entry, from a list (longest first) or found in the tokens' entries: the same bits."""
+    o = ops()
+    lens, H = [33, 1, 100, 64], 3
+    T, (seq, slot, tiles) = sum(lens), scan_setup(lens, 0)
+    q, k, v, a_pre = (rnd(T, H * D, seed=i) for i in range(4))
+    low, w2, w0, ab = rnd(T, 64, seed=5), rnd(H * D, 64, seed=6) * 0.3, rnd(H * D, seed=7), rnd(H * D, seed=8)
+    k = torch.nn.functional.normalize(k.view(T, H, D), dim=-1).view(T, -1).contiguous()
+    g, beta = torch.sigmoid(rnd(T, H, seed=9) * 3 + 2), torch.sigmoid(rnd(T, H, seed=10))
+    got = []
+    for walks in (None, torch.from_numpy(o.chunk_walks(lens)).to(DEV)):
+        st, out = rnd(len(lens) + 2, H, D, D, seed=11), torch.empty(T, H * D, device=DEV)
+        if kind == "delta":
+            o.chunk_scan(q, k, v, g, st, out, tiles, seq, slot, len(lens), H, H, D, D, beta=beta, walks=walks, scratch=scan_scratch)
+        else:
+            o.chunk_scan_general(q, k, v, a_pre, low, w2, w0, ab, 0.6, st, out, tiles, seq, slot, len(lens), H, D, walks=walks,
+                                 scratch=scan_scratch)
+        got.append((out, st))
+    assert all(torch.equal(a, b) and bool(a.isfinite().all()) for a, b in zip(*got))
