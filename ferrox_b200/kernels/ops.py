@@ -14,6 +14,7 @@ from typing import Optional
 
 import torch
 
+from . import fastcall
 from . import lib as _libmod
 
 F32, BF16 = 0, 1
@@ -146,6 +147,7 @@ def count_launches(n: int) -> None:
 
 
 def _get(name: str):
+    """An entry point as ctypes calls it: pointers also as what ctypes takes for them."""
     f = _fn.get(name)
     if f is None:
         lib = _libmod.load()
@@ -153,6 +155,16 @@ def _get(name: str):
         f.argtypes = _SIGNATURES[name]
         f.restype = c_int
         _fn[name] = f
+    return f
+
+
+_fast = {}      # entry points as the extension module calls them: plain ints, floats and None
+
+
+def _get_fast(name: str):
+    f = _fast.get(name)
+    if f is None:
+        f = _fast[name] = fastcall.bind(_get(name), _SIGNATURES[name]) or _get(name)
     return f
 
 
@@ -166,8 +178,12 @@ def call(name: str, *args) -> None:
     _launches += _KERNELS.get(name, 1)
     if _trace is not None:
         return _call_traced(name, args)
-    rc = _get(name)(*args)
+    rc = (_fast.get(name) or _get_fast(name))(*args)
     if rc != 0:
+        if rc is NotImplemented:         # (a structure or an array among the arguments)
+            rc = _get(name)(*args)
+            if rc == 0:
+                return
         if rc > 0:
             raise KernelError(f"{name}: CUDA error {rc} at launch ({torch.cuda.get_device_name()})")
         raise KernelError(f"{name}: refused: {_ERRORS.get(rc, rc)}")
@@ -297,6 +313,18 @@ def _rows(t: torch.Tensor) -> int:
     if t.dim() != 2 or t.stride(1) != 1:
         raise KernelError(f"expected a 2-D tensor with contiguous rows, found shape {tuple(t.shape)} strides {t.stride()}")
     return t.stride(0)
+
+
+def _use_extension():
+    """:func:`_ptr` and :func:`_rows` by the extension module where there is one: it calls these for what it does not take."""
+    global _ptr, _rows
+    m = fastcall.module()
+    if m is not None:
+        m.set_slow(_ptr, _rows)
+        _ptr, _rows = m.ptr, m.rows
+
+
+_use_extension()
 
 
 def upload(values, device) -> torch.Tensor:
@@ -1246,7 +1274,7 @@ def general_attention_ok(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldo
     return int(q.dtype == torch.bfloat16 and k_pages.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
             and ldq % 8 == 0 and ldqh % 8 == 0 and ldk % 8 == 0 and ldv % 8 == 0 and ldo % 2 == 0 and ldoh % 2 == 0
             and q.data_ptr() % 16 == 0 and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0
-            and out.data_ptr() % 4 == 0 and _get("fx_general_attention_ok")(key_dim, value_dim, alias))
+            and out.data_ptr() % 4 == 0 and _get_fast("fx_general_attention_ok")(key_dim, value_dim, alias))
 
 
 def general_attention_fits(key_dim: int, value_dim: int) -> bool:
@@ -1669,7 +1697,7 @@ def slab_ok(x, w) -> bool:
         return False
     if x.stride(0) % 8 or w.stride(0) % 8 or x.data_ptr() % 16 or w.data_ptr() % 16 or x.stride(1) != 1 or w.stride(1) != 1:
         return False
-    return bool(_get("fx_gemm_slab_ok")(w.shape[0], w.shape[1], x.shape[0]))
+    return bool(_get_fast("fx_gemm_slab_ok")(w.shape[0], w.shape[1], x.shape[0]))
 
 
 def gemm_slab(x, w, out, *, bias=None, accumulate=False, status=None, stream=None):

@@ -1,4 +1,7 @@
 """The host-side choices between kernels and launch shapes (pure functions of sizes; no GPU)."""
+import pytest
+import torch
+
 from ferrox_b200.kernels import ops
 from ferrox_b200.parts.moe import expert_tile_tokens
 
@@ -260,3 +263,43 @@ def test_which_prompts_the_general_forms_take_to_tcgen05():
 def test_walks_of_chunked_recurrences():
     """Longest entry first, each with its rows and its first chunk in the order of the batch."""
     assert ops.chunk_walks([33, 1, 100, 64]).tolist() == [[2, 34, 134, 3], [3, 134, 198, 7], [0, 0, 33, 0], [1, 33, 34, 2]]
+
+
+def test_calls_by_the_extension_module_pass_what_ctypes_passes(tmp_path):
+    """Every kind of argument, more integers and floats than registers hold, in mixed order; what is not read there is handed
+    back; addresses and strides of tensors, and the errors of those that are none."""
+    import ctypes
+    import subprocess
+    from ctypes import c_double, c_float, c_int, c_long, c_ulonglong, c_void_p
+
+    from ferrox_b200.kernels import fastcall, hostlib
+
+    if fastcall.module() is None:
+        pytest.skip("no C compiler or no Python headers")
+    kinds = [c_void_p, c_int, c_float, c_long, c_double, c_int, c_ulonglong, c_int, c_float, c_long, c_int, c_void_p, c_float, c_int,
+             c_int, c_float, c_long, c_float, c_int, c_float, c_int, c_void_p, c_int, c_float, c_long]
+    c_of = {c_void_p: "void*", c_int: "int", c_float: "float", c_long: "long", c_double: "double", c_ulonglong: "unsigned long long"}
+    params = ", ".join(f"{c_of[k]} a{i}" for i, k in enumerate(kinds))
+    store = " ".join(f"last[{i}] = (double){'(unsigned long)' if k is c_void_p else ''}a{i};" for i, k in enumerate(kinds))
+    src = tmp_path / "f.cpp"
+    src.write_text(f'extern "C" {{ static double last[99]; int f({params}) {{ {store} return -7; }} double get(int i) {{ return last[i]; }} }}')
+    subprocess.run([hostlib._compiler(), "-O2", "-shared", "-fPIC", "-o", str(tmp_path / "f.so"), str(src)], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "f.so"))
+    lib.f.argtypes, lib.f.restype, lib.get.restype = kinds, c_int, c_double
+    value = {c_void_p: lambda i: None if i % 2 else 2 ** 47 + i, c_int: lambda i: -i if i % 3 else True, c_float: lambda i: i + 0.1,
+             c_long: lambda i: -2 ** 40 - i, c_double: lambda i: i / 7, c_ulonglong: lambda i: 2 ** 63 + i}
+    args = [value[k](i) for i, k in enumerate(kinds)]
+    fast = fastcall.bind(lib.f, kinds)
+    assert fast(*args) == -7
+    got = [lib.get(i) for i in range(len(kinds))]
+    assert lib.f(*args) == -7 and got == [lib.get(i) for i in range(len(kinds))]
+    assert fast(ctypes.c_void_p(3), *args[1:]) is NotImplemented
+    for bad in (args[:-1], args + [1], args[:2] + ["x"] + args[3:]):
+        with pytest.raises(TypeError):
+            fast(*bad)
+    assert fastcall.bind(lib.f, [c_float] * 9) is None
+    t = torch.zeros(3, 8)
+    assert ops._ptr(None) is None and ops._rows(t[:, :5]) == 8
+    for call in (lambda: ops._ptr(t), lambda: ops._rows(t.T), lambda: ops._rows(t[0])):
+        with pytest.raises(ops.KernelError):
+            call()
