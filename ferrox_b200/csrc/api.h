@@ -23,6 +23,12 @@ int fx_gemm_f32(const void* A, long lda, const int* a_rows, const void* W, long 
 int fx_gemm_f32_tc(const void* X, long ldx, const void* W, long ldw, const void* bias, int bias_dtype, void* C, long ldc,
                    int accumulate, int M, int N, int K, int n_tile, void* work, long work_bytes, int* status, void* stream);
 
+// fx_prefill_attention_f32 on the tensor cores, operands in three bfloat16 parts (attention_f32_tc.cu; items, spans, work: there).
+int fx_prefill_attention_f32_tc(const void* q, long ldq, int n_tokens, const void* k_pages, const void* v_pages, const int* block_table,
+                                int table_width, int page_size, const int* items, int n_items, const int* spans, int n_spans, long rows,
+                                const int* seq_slot, void* out, long ldo, int n_heads, int n_kv_heads, int head_dim, int window,
+                                float scale, float softcap, void* work, long work_bytes, int* status, void* stream);
+
 // Zeros at a slot of every tensor of a table (elementwise.cu).
 int fx_zero_slots(const long* table, int n, long most, long slot, void* stream);
 

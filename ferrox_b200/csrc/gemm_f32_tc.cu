@@ -1,9 +1,9 @@
 // C[M,N] (+)= A[M,K] . W[N,K]^T (+ bias) of 32-bit operands on the tensor cores, no further from the 64-bit sums than the
 // FFMA kernels of gemm_f32.cu.
 //
-// A 32-bit value is the sum of three bfloat16 (8 bits of its mantissa each, cut off, not rounded: exact, and no cut can
-// overflow).  Of the nine products of two such sums six are made: hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi; what is
-// left out is below 2^-21 of a product, 2^-24 on average.  Products of two bfloat16 are exact in 32 bits.  The tensor
+// A 32-bit value is the sum of three bfloat16 (split3.cuh).  Of the nine products of two such sums six are made: hi.hi,
+// hi.mid, mid.hi, mid.mid, hi.lo, lo.hi; what is left out is below 2^-21 of a product, 2^-24 on average.  Products of two
+// bfloat16 are exact in 32 bits.  The tensor
 // core adds them up by cutting instead of rounding, which over K = 2,048 would cost 1e-5; so its accumulator holds only 32
 // elements of K (the small products first, then two instructions of large ones), and each thread adds these sums to
 // 32-bit registers of its own, rounding as an FFMA does.  What cannot be had from the parts is done again by a
@@ -22,6 +22,7 @@
 // Every CTA gets the same number of stages: whole tiles as far as they go round, then the rest cut along K into equal
 // shares (`sk_tiles` tiles over `sk_ctas` CTAs), whose sums go to `part`; sum_kernel adds a tile's up in the order of K.
 #include "tc_common.cuh"
+#include "split3.cuh"
 #include "api.h"
 
 namespace {
@@ -136,24 +137,6 @@ __device__ __forceinline__ void tc_ld_wait16(uint32_t* r) {
 __device__ __forceinline__ void tc_st8(uint32_t taddr, uint4 a, uint4 b) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
-}
-
-// x = hi + mid + lo, eight bits of the mantissa each; the upper halves of the words returned are the bfloat16.
-__device__ __forceinline__ void split3(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    hi = __float_as_uint(x) & 0xffff0000u;
-    const float r = x - __uint_as_float(hi);
-    mid = __float_as_uint(r) & 0xffff0000u;
-    lo = __float_as_uint(r - __uint_as_float(mid));
-}
-__device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
-
-__device__ __forceinline__ void split3_8(const float* x, uint4& hi, uint4& mid, uint4& lo) {
-    uint32_t h[8], m[8], l[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) split3(x[i], h[i], m[i], l[i]);
-    hi = make_uint4(upper_halves(h[0], h[1]), upper_halves(h[2], h[3]), upper_halves(h[4], h[5]), upper_halves(h[6], h[7]));
-    mid = make_uint4(upper_halves(m[0], m[1]), upper_halves(m[2], m[3]), upper_halves(m[4], m[5]), upper_halves(m[6], m[7]));
-    lo = make_uint4(upper_halves(l[0], l[1]), upper_halves(l[2], l[3]), upper_halves(l[4], l[5]), upper_halves(l[6], l[7]));
 }
 
 // A's rows in their three parts: planes [3][M][Kp] of bfloat16, Kp = K rounded up to 8; 8 elements a thread.

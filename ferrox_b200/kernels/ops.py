@@ -41,6 +41,8 @@ _SIGNATURES = {
     "fx_gemm_f32": [_P, _L, _P, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _P, _I, _L, _I, _I, _P, _P],
     "fx_gemm_f32_tc": [_P, _L, _P, _L, _P, _I, _P, _L, _I, _I, _I, _I, _I, _P, _L, _P, _P],
     "fx_prefill_attention_f32": [_P, _L, _P, _P, _P, _I, _I, _P, _I, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P],
+    "fx_prefill_attention_f32_tc": [_P, _L, _I, _P, _P, _P, _I, _I, _P, _I, _P, _I, _L, _P, _P, _L, _I, _I, _I, _I, _F, _F, _P, _L,
+                                    _P, _P],
     "fx_zero_slots": [_P, _I, _L, _L, _P],
     "fx_chunk_scan": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P,
                       _I, _I, _I, _I, _I, _I, _P, _P],
@@ -131,7 +133,8 @@ _SIGNATURES = {
 _fn = {}
 
 # kernels launched by one call of an entry point (fx_moe_align: count, scan, place)
-_KERNELS = {"fx_moe_align": 3, "fx_route": 2, "fx_decode_attention": 2}   # (a split-K product adds a second kernel; not counted)
+# (a split-K product adds a second kernel; not counted)
+_KERNELS = {"fx_moe_align": 3, "fx_route": 2, "fx_decode_attention": 2, "fx_prefill_attention_f32_tc": 2}
 _launches = 0
 
 
@@ -1213,9 +1216,66 @@ def prefill_f32_ok(q, out, k_pages, head_dim) -> bool:
             and out.data_ptr() % 16 == 0)
 
 
+F32_TC_TILE, F32_TC_KEYS = 128, 64     # queries a tile and keys a block of attention_f32_tc.cu
+
+
+def prefill_f32_tc_plan(entries, window, head_dim):
+    """The work of :func:`prefill_attention_f32_tc` for a step.  ``entries``: (tokens, first position) of each entry, in the order
+    of the flattened batch.  Returns (items int32 [n, 8], spans int32 [m, 4], plane rows, rest int32 [k, 4]): tiles of up to 128
+    queries, the most key blocks first; the positions of every entry that its queries see, in rows of the planes that begin at
+    multiples of 64; and the entries that the tensor cores do not take, as the tiles of :func:`prefill_attention_f32`.
+
+    They take an entry that sees 64 keys or more (128 with heads of 64 elements or fewer).  Below, their cut sums are further from
+    64 bits than FFMA's rounded ones, and there is little to gain.  B200, one request from position 0, FFMA and tensor cores, error
+    and time: 16 heads of 128, 33 keys: 1.48e-7 and 1.50e-7, 18 and 11 us; 64: 1.74e-7 and 1.71e-7, 18 and 12 us; 517: 2.62e-7 and
+    2.21e-7, 145 and 42 us; 2000: 3.75e-7 and 2.41e-7, 1299 and 135 us.  8 heads of 64, a window of 150, 64 keys: 1.35e-7 and
+    1.44e-7, 13 and 9 us; 128: 1.61e-7 and 1.58e-7, 23 and 12 us; 2000: 2.60e-7 and 2.14e-7, 87 and 24 us."""
+    import numpy as np
+
+    items, spans, rest, flat, row = [], [], [], 0, 0
+    least = 64 if head_dim > 64 else 128
+    for b, (n, start) in enumerate(entries):
+        if min(start + n, window or start + n) < least:
+            rest += [(flat + i, min(F32_PREFILL_TILE, n - i), b, start + i) for i in range(0, n, F32_PREFILL_TILE)]
+        else:
+            p0 = first_key(start, window) // F32_TC_KEYS * F32_TC_KEYS
+            spans.append((b, p0, start + n, row))
+            for i in range(0, n, F32_TC_TILE):
+                m, pos0 = min(F32_TC_TILE, n - i), start + i
+                items.append((flat + i, m, b, pos0, first_key(pos0, window) // F32_TC_KEYS, (pos0 + m - 1) // F32_TC_KEYS + 1, row - p0, 0))
+            row += -(-(start + n - p0) // F32_TC_KEYS) * F32_TC_KEYS
+        flat += n
+    items.sort(key=lambda it: it[4] - it[5])
+    return (np.asarray(items, dtype=np.int32).reshape(-1, 8), np.asarray(spans, dtype=np.int32).reshape(-1, 4), row,
+            np.asarray(rest, dtype=np.int32).reshape(-1, 4))
+
+
+def prefill_f32_tc_ok(q, out, k_pages, page_size, head_dim) -> bool:
+    """Whether :func:`prefill_attention_f32_tc` takes these operands: those of :func:`prefill_attention_f32` with heads of 64 elements
+    or more (shorter ones gain nothing: their products are padded to 64) in steps of 8, and pages of a multiple of 64 positions."""
+    return prefill_f32_ok(q, out, k_pages, head_dim) and head_dim >= 64 and head_dim % 8 == 0 and page_size % 64 == 0
+
+
+def prefill_f32_tc_fits(n_items, n_tokens, rows, n_heads, n_kv_heads, head_dim) -> bool:
+    """Whether a plan's parts are within F32_WORKSPACE_MAX and its tiles within a grid."""
+    return 0 < n_items <= 65535 and 6 * head_dim * (n_tokens * n_heads + 2 * rows * n_kv_heads) <= F32_WORKSPACE_MAX
+
+
+def prefill_attention_f32_tc(q, k_pages, v_pages, block_table, page_size, items, spans, rows, seq_slot, out, n_heads, n_kv_heads,
+                             head_dim, window, scale, status=None, stream=None, softcap=None):
+    """:func:`prefill_attention_f32` on the tensor cores, operands in three bfloat16 parts; ``items`` and ``spans``: device copies of
+    what :func:`prefill_f32_tc_plan` returns, with its ``rows``."""
+    work = torch.empty(6 * head_dim * (q.shape[0] * n_heads + 2 * rows * n_kv_heads), dtype=torch.uint8, device=out.device)
+    call("fx_prefill_attention_f32_tc", _ptr(q), _rows(q), q.shape[0], _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+         block_table.shape[1], page_size, _ptr(items), items.shape[0], _ptr(spans), spans.shape[0], rows, _ptr(seq_slot), _ptr(out),
+         _rows(out), n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), float(softcap or 0.0), _ptr(work), work.numel(),
+         _ptr(status), stream if stream is not None else stream_ptr())
+    return out
+
+
 def prefill_attention_f32(q, k_pages, v_pages, block_table, page_size, tiles, seq_slot, out, n_heads, n_kv_heads, head_dim,
                           window, scale, stream=None, softcap=None):
-    """Prompt attention in 32 bits; ``tiles``: int32 [n, 4] rows of (first token, rows, entry, position of the first
+    """Prompt attention in 32 bits with FFMA; ``tiles``: int32 [n, 4] rows of (first token, rows, entry, position of the first
     row), at most F32_PREFILL_TILE rows each."""
     call("fx_prefill_attention_f32", _ptr(q), _rows(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
          block_table.shape[1], page_size, _ptr(tiles), tiles.shape[0], _ptr(seq_slot), _ptr(out), _rows(out), n_heads,

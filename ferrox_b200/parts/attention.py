@@ -82,6 +82,24 @@ def prefill_tc_better(batch, window, n_heads, key_dim, value_dim, chunk=None, ke
     return better
 
 
+def prefill_f32_plan(batch, window, n_heads, n_kv_heads, head_dim):
+    """This step's work for the 32-bit prompt attention on the device: (items, spans, plane rows) for the tensor cores, or None, and
+    the tiles for FFMA, or None.  Made once a step for each form and shared by the layers that have it."""
+    key = ("attention 32-bit items", window, n_heads, n_kv_heads, head_dim)
+    plan = batch.shared.get(key)
+    if plan is None:
+        entries = [(len(e.tokens), e.start) for e in batch.entries]
+        items, spans, rows, rest = ops.prefill_f32_tc_plan(entries, window, head_dim)
+        if ops.prefill_f32_tc_fits(len(items), sum(n for n, _ in entries), rows, n_heads, n_kv_heads, head_dim):
+            all_ = ops.upload(np.concatenate([items.reshape(-1), spans.reshape(-1), rest.reshape(-1)]), batch.token_ids.device)
+            a, b = items.size, items.size + spans.size
+            plan = (all_[:a].view(-1, 8), all_[a:b].view(-1, 4), rows), all_[b:].view(-1, 4) if rest.size else None
+        else:
+            plan = None, query_tiles(batch, ops.F32_PREFILL_TILE)
+        batch.shared[key] = plan
+    return plan
+
+
 def prefill_tc_scratch(rt, parts, n_heads, value_dim):
     """Where the tiles that were cut into runs leave their results (None, None: there are none)."""
     if not parts:
@@ -340,12 +358,24 @@ class GqaAttention(Mixer):
                 s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream, softcap=self.softcap,
             )
         elif ops.prefill_f32_ok(qkv, attn, cache.k, s.head_dim):
-            # prompt portions in 32 bits: tiles of 32 queries
-            ops.prefill_attention_f32(
-                qkv, cache.k, cache.v, cache.block_table, cache.page_size, query_tiles(batch, ops.F32_PREFILL_TILE),
-                batch.seq_slot, attn,
-                s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream, softcap=self.softcap,
-            )
+            # prompt portions in 32 bits: tiles of 128 queries on the tensor cores; short ones, and head and page sizes that these
+            # do not take, tiles of 32 queries with FFMA
+            if ops.prefill_f32_tc_ok(qkv, attn, cache.k, cache.page_size, s.head_dim):
+                on_tc, tiles = prefill_f32_plan(batch, s.window, s.n_heads, s.n_kv_heads, s.head_dim)
+            else:
+                on_tc, tiles = None, query_tiles(batch, ops.F32_PREFILL_TILE)
+            if on_tc is not None:
+                items, spans, rows = on_tc
+                ops.prefill_attention_f32_tc(
+                    qkv, cache.k, cache.v, cache.block_table, cache.page_size, items, spans, rows, batch.seq_slot, attn,
+                    s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, status=batch.status, stream=batch.stream,
+                    softcap=self.softcap,
+                )
+            if tiles is not None:
+                ops.prefill_attention_f32(
+                    qkv, cache.k, cache.v, cache.block_table, cache.page_size, tiles, batch.seq_slot, attn,
+                    s.n_heads, s.n_kv_heads, s.head_dim, s.window, self.scale, stream=batch.stream, softcap=self.softcap,
+                )
         else:
             # head sizes that no tiled kernel takes: a warp per (token, head)
             ops.paged_attention(

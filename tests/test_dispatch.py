@@ -303,3 +303,26 @@ def test_calls_by_the_extension_module_pass_what_ctypes_passes(tmp_path):
     for call in (lambda: ops._ptr(t), lambda: ops._rows(t.T), lambda: ops._rows(t[0])):
         with pytest.raises(ops.KernelError):
             call()
+
+
+def test_work_of_the_32_bit_prompt_attention():
+    """Each query is in one tile of one kernel, tiles hold no block that no query sees, and the planes' rows hold what they see."""
+    for window in (None, 70, 200):
+        for dim in (64, 128):
+            entries = [(9, 0), (300, 0), (1, 700), (64, 0), (129, 63), (63, 0)]
+            items, spans, rows, rest = ops.prefill_f32_tc_plan(entries, window, dim)
+            taken = sorted((f, n, b, p) for f, n, b, p, *_ in items.tolist()) + sorted(map(tuple, rest.tolist()))
+            seen = sorted(f + i for f, n, *_ in taken for i in range(n))
+            assert seen == list(range(sum(n for n, _ in entries)))
+            least = 64 if dim > 64 else 128
+            assert {b for _, _, b, _ in taken[:len(items)]} == {b for b, (n, s) in enumerate(entries) if min(n + s, window or 9999) >= least}
+            starts = [sum(n for n, _ in entries[:b]) for b in range(len(entries))]
+            at = {b: (p0, end, row) for b, p0, end, row in spans.tolist()}
+            for f, n, b, pos, lo, hi, row0, _ in items.tolist():
+                assert f - starts[b] + entries[b][1] == pos and n <= ops.F32_TC_TILE
+                p0, end, row = at[b]
+                assert lo == ops.first_key(pos, window) // 64 and (hi - 1) * 64 <= pos + n - 1 < hi * 64
+                assert row0 == row - p0 and p0 <= lo * 64 and row % 64 == 0 and row0 + hi * 64 <= rows
+            assert [it[5] - it[4] for it in items.tolist()] == sorted((it[5] - it[4] for it in items.tolist()), reverse=True)
+    assert ops.prefill_f32_tc_fits(3, 517, 576, 16, 16, 128) and not ops.prefill_f32_tc_fits(0, 9, 0, 16, 16, 128)
+    assert not ops.prefill_f32_tc_fits(40, 5000, 5056, 16, 16, 128)

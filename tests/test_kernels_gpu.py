@@ -517,6 +517,78 @@ def test_prefill_attention_f32(case):
     assert torch.equal(out[keep], before[keep])
 
 
+@pytest.mark.parametrize("case", [
+    # heads, kv heads, head_dim, page size, window, cap, [(first position, tokens)], an entry's page that is not there
+    (4, 2, 128, 64, 0, None, [(0, 64), (0, 129), (500, 1), (63, 65)], None),
+    (6, 3, 64, 128, 150, 5.0, [(0, 128), (777, 127), (127, 130), (0, 9)], None),
+    (3, 1, 80, 64, 0, None, [(5, 300), (0, 33)], (0, 1)),
+    (2, 2, 72, 64, 70, None, [(0, 400), (129, 1)], None),
+])
+def test_prefill_attention_f32_on_tensor_cores(case):
+    """32-bit prompt attention from bfloat16 parts, short entries by the FFMA kernel, against 64 bits; then with keys and values that
+    are no finite numbers, where it has to be none where the FFMA kernel's is none."""
+    o = ops()
+    nh, nkv, d, ps, window, cap, portions, hole = case
+    lens = [a + n for a, n in portions]
+    kp, vp, table, ks, vs = build_cache(torch.float32, lens, nkv, d, ps, n_pages=sum(-(-L // ps) for L in lens) + 3)
+    T, scale = sum(n for _, n in portions), d ** -0.5
+    q = rnd(T, nh * d + 8)
+    slots = torch.tensor([b + 1 for b in range(len(lens))], dtype=torch.int32, device=DEV)
+    if hole:
+        table[hole[0] + 1, hole[1]] = -1
+    items, spans, rows, rest = o.prefill_f32_tc_plan([(n, s) for s, n in portions], window, d)
+    ffma, flat = [], 0
+    for b, (start, n) in enumerate(portions):
+        ffma += [(flat + i, min(32, n - i), b, start + i) for i in range(0, n, 32)]
+        flat += n
+    ffma = torch.tensor(ffma, dtype=torch.int32, device=DEV)
+    items, spans, rest = (torch.from_numpy(x).to(DEV) for x in (items, spans, rest))
+    out, plain, status = torch.empty(T, nh * d, device=DEV), torch.empty(T, nh * d, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert o.prefill_f32_tc_ok(q, out, kp, ps, d) and items.shape[0] and not o.prefill_f32_tc_ok(q[:, 2:], out, kp, ps, d)
+
+    def run():
+        out.fill_(7.0)
+        o.prefill_attention_f32_tc(q, kp, vp, table, ps, items, spans, rows, slots, out, nh, nkv, d, window, scale, status=status, softcap=cap)
+        if rest.shape[0]:
+            o.prefill_attention_f32(q, kp, vp, table, ps, rest, slots, out, nh, nkv, d, window, scale, softcap=cap)
+        o.prefill_attention_f32(q, kp, vp, table, ps, ffma, slots, plain, nh, nkv, d, window, scale, softcap=cap)
+        assert int(status) == 0
+
+    run()
+    flat, bound = 0, torch.empty(T, nh, 1)
+    for b, (start, n) in enumerate(portions):
+        pos, key = torch.arange(start, start + n)[:, None], torch.arange(start + n)
+        sees = (key <= pos) & (key > pos - (window or 1 << 30))
+        if hole and hole[0] == b:
+            sees &= key // ps != hole[1]
+        x = q[flat:flat + n, :nh * d].cpu().double().view(n, nh, d)
+        k, v = (t[b].double().repeat_interleave(nh // nkv, 1) for t in (ks, vs))
+        s = torch.einsum("thd,khd->htk", x, k) * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        want = torch.einsum("htk,khd->thd", torch.softmax(s.masked_fill(~sees, float("-inf")), -1), v)
+        # A score's sum is cut once for each 16 elements (by a unit of at most |q| |k| in 24 bits), what the six products leave out is
+        # a few units more, and expf, tanhf and the scale some; a weight is off by that and its sum's, and a block's result, by cuts of
+        # the same kind, by a unit for each 16 keys.
+        unit = 2.0 ** -23
+        es = unit * (d / 16 + 8) * scale * x.norm(dim=-1).max() * k.norm(dim=-1).max()
+        bound[flat:flat + n] = v.abs().max() * (2 * es + unit * (8 + (start + n) / 16))
+        err = (out[flat:flat + n].cpu().double().view(n, nh, d) - want).abs()
+        assert bool((err <= bound[flat:flat + n]).all()), float((err / bound[flat:flat + n]).max())
+        flat += n
+    before = out.clone()
+    for b, L in enumerate(lens):
+        page = int(table[b + 1, (L - 1) // ps])
+        kp[page, :, (L - 1) % ps], vp[page, :, (L - 1) % ps] = float("nan"), float("inf")
+    page = int(table[1, 0])                  # (the first entry sees these, where they are not out of its window)
+    kp[page, 0, 3, 1], vp[page, 0, 5, 2], vp[page, 0, 6, 3] = float("inf"), float("-inf"), float("nan")
+    run()
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    fine = plain.isfinite()
+    for seen, other in ((before, portions[0][1]), (plain, 0)):       # (the other entries as if they were not there, but for their last)
+        off = (out - seen).abs().view(T, nh, d) <= 2 * bound.to(DEV)
+        assert bool((off | ~fine.view(T, nh, d))[other:].all())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("case", ATT_CASES)
 @pytest.mark.parametrize("kernel", ["generic", "decode"])
