@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "api.h"
 #include "no_alloc.h"
+#include "merge_runs.cuh"
 
 namespace {
 
@@ -259,13 +260,12 @@ __global__ void merge_kernel(const float* __restrict__ part_acc, const float* __
     fx_pdl_wait();
     const int tkn = blockIdx.x, h = blockIdx.y;
     const long base = ((long)tkn * n_heads + h) * n_splits;
+    const RunsOfHead runs = {part_acc + base * head_dim, part_ml + base * 2, n_splits, head_dim};
     // the splits that hold visible keys of this token (the others were not written)
     const int pos = positions[tkn];
     const int lo = fx_first_key(pos, window, x.chunk);
     auto has_keys = [&](int s) { int b, e; fx_split_range(pos, lo, s, n_splits, split_len, b, e); return b < e; };
-    float mm = -INFINITY;
-    for (int s = 0; s < n_splits; ++s)
-        if (has_keys(s)) mm = fmaxf(mm, part_ml[(base + s) * 2]);
+    float mm = fx_runs_max(runs, has_keys);
     float sunk = 0.f;        // the head's sink: a term of the denominator that no range holds
     if (x.sinks && mm != -INFINITY) {
         mm = fmaxf(mm, x.sinks[h]);
@@ -274,15 +274,8 @@ __global__ void merge_kernel(const float* __restrict__ part_acc, const float* __
     for (int e0 = 0; e0 < head_dim; e0 += blockDim.x) {      // (every lane takes every trip: partners of a pair meet)
         const int e = e0 + threadIdx.x;
         const bool in = e < head_dim;
-        float ll = sunk, a = 0.f;
-        for (int s = 0; s < n_splits && in; ++s) {
-            if (!has_keys(s)) continue;
-            const float ms = part_ml[(base + s) * 2];
-            if (ms == -INFINITY) continue;
-            const float w = fx_exp<T>(ms - mm);
-            ll += part_ml[(base + s) * 2 + 1] * w;
-            a += part_acc[(base + s) * head_dim + e] * w;
-        }
+        const float2 sum = fx_runs_sum(runs, e, in, mm, sunk, has_keys, [](float d) { return fx_exp<T>(d); });
+        const float a = sum.x, ll = sum.y;
         float v = ll > 0.f ? a / ll : 0.f;
         if (x.turn) {
             const float2 cs = in ? *reinterpret_cast<const float2*>(x.turn + (long)tkn * head_dim + (e & ~1)) : make_float2(1.f, 0.f);
@@ -359,7 +352,7 @@ int run(const void* q, long ldq, const void* k_pages, const void* v_pages, int n
                                          token_seq, seq_slot, part_acc, part_ml, n_tokens, n_heads, n_kv_heads,
                                          head_dim, window, scale, split_len, n_splits, fresh, softcap, (void*)s);
         if (rc_mma == FX_OK) {
-            fx_launch_pdl(merge_kernel<T>, dim3(n_tokens, n_heads), 64, 0, s, part_acc, part_ml, positions, (T*)out, ldo,
+            fx_launch_pdl(merge_kernel<T>, dim3(n_tokens, n_heads), fx_merge_threads(head_dim), 0, s, part_acc, part_ml, positions, (T*)out, ldo,
                           n_heads, head_dim, n_splits, split_len, window, x);
             return fx_launch_status();
         }
@@ -386,7 +379,7 @@ int run(const void* q, long ldq, const void* k_pages, const void* v_pages, int n
     else { FX_GO(16, 4); }
 #undef FX_GO
     if (rc != FX_OK) return rc;
-    fx_launch_pdl(merge_kernel<T>, dim3(n_tokens, n_heads), 64, 0, s, part_acc, part_ml, positions, (T*)out, ldo, n_heads, head_dim,
+    fx_launch_pdl(merge_kernel<T>, dim3(n_tokens, n_heads), fx_merge_threads(head_dim), 0, s, part_acc, part_ml, positions, (T*)out, ldo, n_heads, head_dim,
                                                           n_splits, split_len, window, x);
     return fx_launch_status();
 }

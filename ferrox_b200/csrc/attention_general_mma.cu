@@ -24,6 +24,7 @@
 // window.  The key blocks that hold them and lie wholly before the first window block are taken first (blocks
 // 0 .. n_kept - 1 of the loop), then the window's blocks; of a decoding token's runs, run 0 takes them.
 #include "common.cuh"
+#include "merge_runs.cuh"
 #include "api.h"
 
 namespace {
@@ -370,12 +371,11 @@ __global__ void general_merge_kernel(const float* __restrict__ part_o, const flo
     fx_pdl_wait();
     const int tkn = blockIdx.x, h = blockIdx.y;
     const long base = ((long)tkn * n_heads + h) * n_splits;
+    const RunsOfHead runs = {part_o + base * value_dim, part_ml + base * 2, n_splits, value_dim};
     const int pos = positions[tkn];
     const int lo = fx_first_key(pos, window, chunk);
     auto has_keys = [&](int s) { int b, e; fx_split_range(pos, lo, s, n_splits, 0, b, e); return b < e; };
-    float mm = -INFINITY;
-    for (int s = 0; s < n_splits; ++s)
-        if (has_keys(s)) mm = fmaxf(mm, part_ml[(base + s) * 2]);
+    float mm = fx_runs_max(runs, has_keys);
     float sunk = 0.f;        // the head's sink: a term of the denominator that no run holds
     if (sinks && mm != -INFINITY) {
         const float sk = sinks[h] * 1.4426950408889634f;
@@ -385,15 +385,8 @@ __global__ void general_merge_kernel(const float* __restrict__ part_o, const flo
     for (int e0 = 0; e0 < value_dim; e0 += blockDim.x) {      // (every lane takes every trip: partners of a pair meet)
         const int e = e0 + threadIdx.x;
         const bool in = e < value_dim;
-        float ll = sunk, acc = 0.f;
-        for (int s = 0; s < n_splits && in; ++s) {
-            if (!has_keys(s)) continue;
-            const float ms = part_ml[(base + s) * 2];
-            if (ms == -INFINITY) continue;
-            const float w = exp2f(ms - mm);
-            ll += part_ml[(base + s) * 2 + 1] * w;
-            acc += part_o[(base + s) * value_dim + e] * w;
-        }
+        const float2 sum = fx_runs_sum(runs, e, in, mm, sunk, has_keys, [](float d) { return exp2f(d); });
+        const float acc = sum.x, ll = sum.y;
         float x = ll > 0.f ? acc / ll : 0.f;
         if (turn) {
             const float2 cs = in ? *reinterpret_cast<const float2*>(turn + (long)tkn * value_dim + (e & ~1)) : make_float2(1.f, 0.f);
@@ -415,7 +408,7 @@ int launch(dim3 grid, size_t smem, cudaStream_t s, const GArgs& a)
     }
     fx_launch_pdl(kern, grid, dim3(128 * NSPLIT), smem, s, a);
     if (a.n_splits > 1)
-        fx_launch_pdl(general_merge_kernel, dim3(grid.x, a.n_heads), dim3(64), 0, s, (const float*)a.part_o,
+        fx_launch_pdl(general_merge_kernel, dim3(grid.x, a.n_heads), dim3(fx_merge_threads(a.value_dim)), 0, s, (const float*)a.part_o,
                       (const float*)a.part_ml, a.positions, a.out, a.ldo, a.ldoh, a.n_heads, a.value_dim, a.n_splits,
                       a.window, a.sinks, a.chunk, a.gate, a.ldg, a.turn);
     return fx_launch_status();
