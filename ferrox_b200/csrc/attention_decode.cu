@@ -9,7 +9,7 @@
 //
 // A block reads each key and value of its range once for all query heads that
 // share the kv head (up to 8; more are handled by further head chunks).  Threads
-// form groups of LPK lanes; a group takes every (128/LPK)-th key, each lane
+// form groups of LPK lanes; a group takes every (threads/LPK)-th key, each lane
 // holding 8 (bfloat16) or 4 (float) consecutive elements of the head dimension,
 // scores it with a group-wide sum and keeps a running (m, l, acc) per query head.
 // The groups are merged in fixed order through shared memory, the block writes
@@ -27,8 +27,6 @@
 
 namespace {
 
-constexpr int NTHREADS = 128;
-constexpr int STAGES = 4;    // buffers of the key/value ring
 constexpr int MAXQ = 8;      // query heads per block
 constexpr int MAX_D = 256;
 
@@ -60,16 +58,38 @@ template <> __device__ __forceinline__ float fx_exp<bf16>(float x) { return __ex
 
 // LPK lanes per key; each lane owns VPL vectors of Vec<T>::N elements: element
 // index of vector v of lane ln is (v * LPK + ln) * N.
+//
+// Bound by latency: a key's scores are a chain of sums, shuffles and exponentials that one warp a scheduler does not hide, and a run
+// of 64 keys is all that a block has.  In 32 bits eight warps take it, in two or three tiles that are on their way together; wider
+// groups of query heads and widths over 128, whose sums do not leave the registers for them, and bfloat16 (whose kernels are elsewhere),
+// four.  16 heads of 128 on 4 kv heads, with the merge: 1 token at 700 positions in 11 runs 15.2 us with four warps that score a key
+// at a time, 10.4 so; 8 tokens at 2,000 in 5 runs 73 and 43 (28 in 8).
+template <typename T, int LPK, int VPL, int GQ> struct Shape {
+    static constexpr int N = Vec<T>::N;
+    static constexpr bool EIGHT = sizeof(T) == 4 && VPL <= 2 && GQ * VPL <= 8;
+    static constexpr int THREADS = EIGHT ? 256 : 128, GROUPS = THREADS / LPK;
+    static constexpr int KB = EIGHT && VPL == 2 ? 2 : GQ * VPL <= 2 ? 4 : GQ * VPL * N <= 32 ? 2 : 1;      // keys of a group scored together
+    static constexpr int STAGES = EIGHT ? 3 : 4;                                     // buffers of the key/value ring
+    // keys per tile
+    static __host__ __device__ __forceinline__ int tile(int row_bytes) {
+        if (EIGHT) return GROUPS * KB < 64 ? GROUPS * KB : 64;
+        return row_bytes <= 256 ? 32 : row_bytes <= 512 ? 16 : 8;
+    }
+    static __host__ __device__ __forceinline__ int stage_bytes(int row_bytes) {     // K rows, V rows, validity flags
+        return 2 * tile(row_bytes) * row_bytes + 128;
+    }
+};
+
 template <typename T, int LPK, int VPL, int GQ>
-__global__ void __launch_bounds__(NTHREADS) decode_split_kernel(
+__global__ void __launch_bounds__(Shape<T, LPK, VPL, GQ>::THREADS) decode_split_kernel(
     const T* __restrict__ q, long ldq, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
     const int* __restrict__ block_table, int table_width, int page_size,
     const int* __restrict__ positions, const int* __restrict__ token_seq, const int* __restrict__ seq_slot,
     float* __restrict__ part_acc, float* __restrict__ part_ml,
     int n_heads, int n_kv_heads, int head_dim, int window, float scale, int split_len, int n_splits, float cap)
 {
-    constexpr int N = Vec<T>::N;
-    constexpr int GROUPS = NTHREADS / LPK;
+    using S = Shape<T, LPK, VPL, GQ>;
+    constexpr int N = S::N, NTHREADS = S::THREADS, GROUPS = S::GROUPS, STAGES = S::STAGES, KB = S::KB;
     fx_pdl_wait();
     const int group_size = n_heads / n_kv_heads;
     const int chunks = (group_size + GQ - 1) / GQ;
@@ -104,26 +124,30 @@ __global__ void __launch_bounds__(NTHREADS) decode_split_kernel(
     // of each tile, in key order.
     extern __shared__ __align__(16) uint8_t dyn_smem[];
     const int row_bytes = head_dim * (int)sizeof(T);
-    const int TK = row_bytes <= 256 ? 32 : (row_bytes <= 512 ? 16 : 8);   // keys per tile (multiple of GROUPS)
-    const int stage_bytes = 2 * TK * row_bytes + 128;                     // K rows, V rows, validity flags
+    const int TK = S::tile(row_bytes), stage_bytes = S::stage_bytes(row_bytes);
     const int n_tiles = k_begin < k_end ? (k_end - k_begin + TK - 1) / TK : 0;
-    constexpr int KB = (GQ * VPL <= 2) ? 4 : (GQ * VPL <= 4 ? 2 : 1);    // keys of a group scored together
     if (n_tiles > 0) {
         const int* table = block_table + (long)seq_slot[token_seq[tkn]] * table_width;
         const long head_stride = (long)page_size * head_dim;
         const int cpk = row_bytes / 16;                                   // 16-byte chunks per key row
         const uint32_t smem_u = (uint32_t)__cvta_generic_to_shared(dyn_smem);
+        // a thread's 16-byte chunks of a tile, NTHREADS apart, without a division for each
+        const int r_first = threadIdx.x / cpk, ch_first = threadIdx.x - r_first * cpk, r_step = NTHREADS / cpk, ch_step = NTHREADS - r_step * cpk;
         auto issue = [&](int tile) {
             if (tile < n_tiles) {
                 uint8_t* st = dyn_smem + (tile % STAGES) * stage_bytes;
                 const uint32_t su = smem_u + (tile % STAGES) * stage_bytes;
-                for (int c = threadIdx.x; c < TK * cpk; c += NTHREADS) {
-                    const int r = c / cpk, ch = c - r * cpk;
-                    const int key = k_begin + tile * TK + r;
-                    int page = -1;
-                    if (key < k_end) page = table[key / page_size];
+                const int key0 = k_begin + tile * TK, p0 = key0 / page_size, o0 = key0 - p0 * page_size;
+                for (int r = r_first, ch = ch_first; r < TK; r += r_step, ch += ch_step) {
+                    if (ch >= cpk) {
+                        ch -= cpk;
+                        if (++r >= TK) break;
+                    }
+                    int p = p0, off = o0 + r, page = -1;
+                    if (off >= page_size) { p += off / page_size; off %= page_size; }
+                    if (key0 + r < k_end) page = table[p];
                     const bool ok = page >= 0;
-                    const long base = ok ? ((long)page * n_kv_heads + kvh) * head_stride + (long)(key % page_size) * head_dim : 0;
+                    const long base = ok ? ((long)page * n_kv_heads + kvh) * head_stride + (long)off * head_dim : 0;
                     const uint32_t dst = su + r * row_bytes + ch * 16;
                     const uint8_t* ksrc = reinterpret_cast<const uint8_t*>(k_pages + base) + ch * 16;
                     const uint8_t* vsrc = reinterpret_cast<const uint8_t*>(v_pages + base) + ch * 16;
@@ -234,14 +258,23 @@ __global__ void __launch_bounds__(NTHREADS) decode_split_kernel(
             for (int i = 0; i < N; ++i)
                 sm_acc[((long)grp * GQ + h) * dpad + (v * LPK + ln) * N + i] = acc[h][v][i];
     __syncthreads();
+    __shared__ float sm_w[GROUPS][GQ], sm_mm[GQ];        // the groups' weights and the largest score
+    for (int i = threadIdx.x; i < GROUPS * GQ; i += NTHREADS) {
+        const int gI = i / GQ, h = i - gI * GQ;
+        float mm = -INFINITY;
+        for (int g2 = 0; g2 < GROUPS; ++g2) mm = fmaxf(mm, sm_m[g2][h]);
+        sm_w[gI][h] = fx_exp<T>(sm_m[gI][h] - mm);
+        if (gI == 0) sm_mm[h] = mm;
+    }
+    __syncthreads();
     for (int o = threadIdx.x; o < nq * head_dim; o += NTHREADS) {
         const int h = o / head_dim, e = o - h * head_dim;
-        float mm = -INFINITY;
-        for (int gI = 0; gI < GROUPS; ++gI) mm = fmaxf(mm, sm_m[gI][h]);
+        const float mm = sm_mm[h];
         float ll = 0.f, a = 0.f;
         if (mm > -INFINITY) {
+#pragma unroll 8
             for (int gI = 0; gI < GROUPS; ++gI) {
-                const float w = fx_exp<T>(sm_m[gI][h] - mm);
+                const float w = sm_w[gI][h];
                 ll += sm_l[gI][h] * w;
                 a += sm_acc[((long)gI * GQ + h) * dpad + e] * w;
             }
@@ -293,16 +326,15 @@ int launch_one(dim3 grid, cudaStream_t s, const T* q, long ldq, const T* k, cons
                int window, float scale, int split_len, int n_splits, float softcap)
 {
     auto kern = decode_split_kernel<T, LPK, VPL, GQ>;
-    const size_t merge_bytes = sizeof(float) * (NTHREADS / LPK) * GQ * (VPL * LPK * Vec<T>::N);
-    const int row_bytes = d * (int)sizeof(T);
-    const int tk = row_bytes <= 256 ? 32 : (row_bytes <= 512 ? 16 : 8);
-    const size_t ring_bytes = (size_t)STAGES * (2 * tk * row_bytes + 128);
+    using S = Shape<T, LPK, VPL, GQ>;
+    const size_t merge_bytes = sizeof(float) * S::GROUPS * GQ * (VPL * LPK * S::N);
+    const size_t ring_bytes = (size_t)S::STAGES * S::stage_bytes(d * (int)sizeof(T));
     const size_t smem = merge_bytes > ring_bytes ? merge_bytes : ring_bytes;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    fx_launch_pdl(kern, grid, NTHREADS, smem, s, q, ldq, k, v, bt, tw, ps, pos, tseq, sslot, pa, pm, nh, nkv, d, window, scale,
+    fx_launch_pdl(kern, grid, S::THREADS, smem, s, q, ldq, k, v, bt, tw, ps, pos, tseq, sslot, pa, pm, nh, nkv, d, window, scale,
                                       split_len, n_splits, softcap);
     return fx_launch_status();
 }

@@ -323,9 +323,12 @@ class GqaAttention(Mixer):
             reach = cache.block_table.shape[1] * cache.page_size
             if s.window is not None:
                 reach = min(reach, (s.window + 63) // 64 * 64 + 64)
-            split_len, n_splits = ops.decode_split_plan(
-                T, kv_blocks, reach, per_sm or 3, single_is_final=per_sm > 0,
-                run_latency=ops.DECODE_RUN_LATENCY if per_sm else 0.0)
+            if qkv.dtype == torch.float32:
+                split_len, n_splits = ops.decode_split_plan_f32(T, kv_blocks, reach)
+            else:
+                split_len, n_splits = ops.decode_split_plan(
+                    T, kv_blocks, reach, per_sm or 3, single_is_final=per_sm > 0,
+                    run_latency=ops.DECODE_RUN_LATENCY if per_sm else 0.0)
             part_acc = self.rt.empty(T, s.n_heads, n_splits, s.head_dim, dtype=torch.float32)
             part_ml = self.rt.empty(T, s.n_heads, n_splits, 2, dtype=torch.float32)
             ops.decode_attention(

@@ -326,3 +326,13 @@ def test_work_of_the_32_bit_prompt_attention():
             assert [it[5] - it[4] for it in items.tolist()] == sorted((it[5] - it[4] for it in items.tolist()), reverse=True)
     assert ops.prefill_f32_tc_fits(3, 517, 576, 16, 16, 128) and not ops.prefill_f32_tc_fits(0, 9, 0, 16, 16, 128)
     assert not ops.prefill_f32_tc_fits(40, 5000, 5056, 16, 16, 128)
+
+
+def test_decode_split_plan_of_the_32_bit_kernel():
+    """Runs of whole 64 keys, in as few rounds of two blocks an SM as their length makes up for."""
+    for tokens in (1, 3, 8, 64, 2000):
+        for kv_blocks in (1, 4, 28):
+            for ctx in (16, 64, 500, 4096, 65536):
+                _, n = ops.decode_split_plan_f32(tokens, kv_blocks, ctx)
+                assert 1 <= n <= min(ops.DECODE_F32_MAX_SPLITS, -(-ctx // 64))
+    assert [ops.decode_split_plan_f32(t, 4, c)[1] for t, c in ((8, 2048), (4, 704), (1, 2048), (400, 2048))] == [8, 11, 32, 2]

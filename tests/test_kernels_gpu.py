@@ -632,6 +632,35 @@ def test_attention_over_pages(dtype, case, kernel):
     _check_attention(out, q, ks, vs, toks, nh, d, window, scale, dtype)
 
 
+@pytest.mark.parametrize("nh,nkv,d,ps,cap", [
+    (4, 4, 8, 3, None), (6, 3, 32, 24, None), (8, 2, 64, 64, None), (5, 5, 64, 16, None), (16, 2, 60, 40, None), (4, 2, 128, 64, 9.0),
+    (9, 9, 96, 7, None), (12, 3, 100, 64, None), (9, 1, 128, 64, None), (6, 3, 200, 48, None),
+])
+def test_decode_attention_f32_forms(nh, nkv, d, ps, cap):
+    """The 32-bit decode kernel with each number of query heads and width of heads that it has a form for: runs that end in a tile,
+    at its end and one past it, against 64 bits."""
+    o = ops()
+    lens = [1, 31, 32, 33, 64, 65, 129, 300]
+    kp, vp, table, ks, vs = build_cache(torch.float32, lens, nkv, d, ps, n_pages=sum(-(-L // ps) for L in lens) + 3)
+    T, scale = len(lens), d ** -0.5
+    q, out = rnd(T, nh * d), torch.empty(T, nh * d, device=DEV)
+    positions, token_seq, slots = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([L - 1 for L in lens], range(T), range(1, T + 1)))
+    for split_len, n_splits in ((0, 1), (0, 5), (16, 19), (33, 10)):
+        pa, pm = torch.full((T, nh, n_splits, d), float("nan"), device=DEV), torch.full((T, nh, n_splits, 2), float("nan"), device=DEV)
+        o.decode_attention(q, kp, vp, table, ps, positions, token_seq, slots, out, nh, nkv, d, None, scale, split_len, n_splits, pa, pm,
+                           softcap=cap)
+        for b, L in enumerate(lens):
+            x = q[b].cpu().double().view(nh, d)
+            k, v = (t[b].double().repeat_interleave(nh // nkv, 1) for t in (ks, vs))
+            s = torch.einsum("hd,khd->hk", x, k) * scale
+            s = cap * torch.tanh(s / cap) if cap else s
+            want = torch.einsum("hk,khd->hd", torch.softmax(s, -1), v)
+            # a sum of d products rounds d times by half a unit of at most |q| |k|, the weights and their sums by some units more
+            unit = 2.0 ** -23
+            es = unit * (d / 2 + 8) * scale * x.norm(dim=-1).max() * k.norm(dim=-1).max()
+            assert float((out[b].cpu().double().view(nh, d) - want).abs().max()) <= v.abs().max() * (2 * es + unit * (8 + L / 2)), (b, n_splits)
+
+
 def _check_attention(out, q, ks, vs, toks, nh, d, window, scale, dtype):
     for i, (s, pos) in enumerate(toks):
         want = plain_attention(q[i, : nh * d].float().cpu().reshape(nh, d), ks[s], vs[s], pos, window, scale)
