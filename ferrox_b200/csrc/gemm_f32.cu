@@ -1,5 +1,5 @@
 // C[M,N] (+)= A[M,K] . W[N,K]^T (+ bias) in true 32-bit arithmetic (FFMA, no tensor core): the products of the 32-bit
-// engine.  Two kernels; kernels/ops.py: gemm_f32_plan chooses.
+// engine that gemm_f32_tc.cu does not take.  Two kernels; kernels/ops.py: gemm_f32_plan chooses.
 //
 //  * `stream`: few rows, or few rows a group.  The time is the time to stream W once, so a block takes R rows of W, its
 //    eight warps share out K in chunks of 128 (a lane four elements, 16-byte loads that bypass L1), the loads of the next
