@@ -25,9 +25,10 @@
 // sub-tile 0's softmax threads and warps 6-9 sub-tile 1's.  The products are issued in the order
 // PV_0(j), S_0(j+1), PV_1(j), S_1(j+1): while one sub-tile's threads work on their block the tensor
 // cores work for the other.  Every wait is bounded (status code 3 on time-out, then the roles leave,
-// tensor memory is freed and the kernel returns).  Keys that are masked for every row are still
-// multiplied (with weight 0); the half of a block that lies beyond the request's pages is read from
-// page 0, which always holds finite values.
+// tensor memory is freed and the kernel returns).  Keys that are masked are still multiplied, with weight 0, and 0 times a
+// value that is infinite or no number is none.  So what lies in a block's place in shared memory for a position that no query of
+// the item sees is zero: where there is no page the TMA fills it in (a page number behind the last), and in the blocks at the
+// edges (behind the last query, before the first one's window) the softmax threads clear the rows of V before their product.
 //
 // A work item is a tile of queries, a head and a run of key blocks [kb_begin, kb_end).  The host cuts the
 // key blocks of long tiles into runs (the last 256 queries of a long prompt see many times the keys the
@@ -117,7 +118,7 @@ __device__ __forceinline__ void cap_any(const Cap& cap, uint32_t* s, float ref) 
 constexpr int ITEM_INTS = 8;   // a work item: first flat token, rows, entry, first position, kb_begin, kb_end, part, kept blocks
 
 struct AttnArgs {
-    const int* block_table; int table_width; int page_size;
+    const int* block_table; int table_width; int page_size, n_pages;
     const int* tiles; const int* seq_slot;
     bf16* out; long ldo;
     float* part_o; float* part_ml;   // partial results of items that hold a run of their tile's key blocks only
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 for (int hk = 0; hk < 2; ++hk) {   // the two runs of 64 keys of the block
                     const int key = j * BKEY + hk * 64;
                     const int p = key <= last_pos ? table[key / a.page_size] : -1;
-                    page[hk] = p >= 0 ? p : 0;      // no page (beyond the request, or before its window): masked anyway
+                    page[hk] = p >= 0 ? p : a.n_pages;      // no page (beyond the request, or before its window): zeros
                     off[hk] = p >= 0 ? key % a.page_size : 0;
                 }
                 mbar_expect_tx(k_full(b), L::K_BYTES);
@@ -348,6 +349,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
             float m = -INFINITY, l = 0.f;
             bool ok = true;
             int cnt = 0;
+            // Zeros for the values of block i, from position kb, that no query of the item sees.  The product of sub-tile 0 comes
+            // first where both have the block, so its threads do it.
+            auto clear_hidden = [&](int i, int kb) {
+                const int lo_item = fx_first_key(pos0, a.window, a.chunk);
+                if (kb + BKEY - 1 <= last_pos && (kb >= lo_item || kb + BKEY <= a.keep_first)) return true;
+                if (t == 1 && active(0, i)) return true;
+                const int vb = L::V_PLACES == 2 ? i & 1 : 0;
+                if (!__all_sync(0xffffffffu, mbar_wait(v_full(vb), (uint32_t)((i / L::V_PLACES) & 1), abort_flag))) return false;
+                for (int c = r; c < L::V_HALVES * BKEY * 8; c += BQ) {          // pieces of 16 bytes, eight a row
+                    const int key = kb + ((c >> 3) & (BKEY - 1));
+                    if (key > last_pos || (key < lo_item && key >= a.keep_first))
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + L::V_OFF + vb * L::V_BYTES + c * 16), "r"(0) : "memory");
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                return true;
+            };
             for (int i = 0; i < n_walk; ++i) {
                 if (!active(t, i)) continue;
                 const int j = block_of(i);
@@ -355,6 +372,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 if (!ok) break;
                 tc_fence_after();
                 if (quad * 32 >= rows_t) {           // none of the warp's rows exists: what its rows of P hold reaches no others
+                    if (!(ok = clear_hidden(i, j * BKEY))) break;
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(p_full(t));
@@ -457,6 +475,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 take_exp(cb, 3, pk + 16);
                 tc_st32(ts + 32, pk);
                 l += sum0 + sum1;
+                if (!interior && !(ok = clear_hidden(i, kb))) break;
                 tc_st_wait();
                 tc_fence_before();
                 __syncwarp();
@@ -687,7 +706,7 @@ extern "C" int fx_prefill_attention_tc(const void* q, long ldq, long ldqh, int n
         if (!encode(v ? &mv : &mk, v ? v_pages : k_pages, 4, dims, strides, box)) return FX_ERR_SIZE;
     }
     AttnArgs a;
-    a.block_table = block_table; a.table_width = table_width; a.page_size = page_size;
+    a.block_table = block_table; a.table_width = table_width; a.page_size = page_size; a.n_pages = n_pages;
     a.tiles = tiles; a.seq_slot = seq_slot; a.out = (bf16*)out; a.ldo = ldo;
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.window = window; a.chunk = chunk; a.value_dim = value_dim;
     a.sinks = sinks; a.gate = (const bf16*)gate; a.ldg = ldg; a.turn = turn;

@@ -1358,6 +1358,56 @@ def test_prefill_attention_tcgen05_keys_and_values_side_by_side():
     assert torch.equal(*outs)
 
 
+# heads, key heads, key heads a value head, D, V, window, keep_first, cap, general: the plain form, capped, kept first keys, shared
+# value heads, the latent form's widths
+HIDDEN_FORMS = [(4, 2, 1, 128, 128, 150, 0, None, False), (4, 2, 1, 128, 128, 150, 0, 20.0, True), (2, 1, 1, 64, 128, 150, 70, None, True),
+                (4, 2, 2, 64, 128, 0, 0, 30.0, True), (2, 2, 1, 192, 128, 0, 0, None, True)]
+
+
+def poisoned(t, mask):
+    """A copy of ``t`` whose elements at ``mask`` are no number, infinite and minus infinite in turn."""
+    bad = torch.tensor([math.nan, math.inf, -math.inf], dtype=t.dtype, device=t.device)
+    at = torch.arange(t.numel(), device=t.device).view(t.shape) % 3
+    return torch.where(mask, bad[at], t)
+
+
+@pytest.mark.parametrize("run_blocks", [0, 1])
+@pytest.mark.parametrize("form", HIDDEN_FORMS)
+def test_prefill_attention_tcgen05_leaves_out_what_nobody_sees(form, run_blocks):
+    """Infinite values and no numbers behind a request's last position, before its window, in pages given back and in page 0, which is
+    nobody's here: the bits are those over zeros.  Ends in the first and in the second half of a key block, tiles of one and two
+    sub-tiles, portions that begin inside a block."""
+    o = ops()
+    H, G, share, D, V, window, keep, cap, general = form
+    ps, lens, starts = 64, [5, 130, 300, 64, 257], [60, 0, 333, 500, 127]
+    T, n, width = sum(lens), len(lens), 11
+    n_pages = n * width + 1
+    table = (1 + torch.arange(n * width).view(n, width)).to(torch.int32).to(DEV)
+    pos = torch.arange(width * ps, device=DEV)
+    hidden = torch.ones(n_pages, ps, dtype=torch.bool, device=DEV)
+    for b, (L, s) in enumerate(zip(lens, starts)):
+        lo = max(0, s - window + 1) if window else 0
+        seen = (pos < s + L) & ((pos >= lo) | (pos < keep))
+        hidden[table[b].long()] = ~seen.view(width, ps)
+        gone = ~seen.view(width, ps).any(1)
+        table[b, gone] = -1
+    mask = hidden[:, None, :, None]
+    kp, vp = rnd(n_pages, G, ps, D, dtype=torch.bfloat16, seed=1), rnd(n_pages, G // share, ps, V, dtype=torch.bfloat16, seed=2)
+    q = rnd(T, H * D, dtype=torch.bfloat16, seed=3)
+    items, merges, parts = o.prefill_tc_plan(list(zip(lens, starts)), window, H, run_blocks=run_blocks, keep_first=keep)
+    outs = []
+    for fill in (lambda t: t.masked_fill(mask, 0), lambda t: poisoned(t, mask)):
+        part_o = torch.full((max(parts, 1), H, 256, o.prefill_value_width(V)), float("nan"), device=DEV)
+        part_ml = torch.full((max(parts, 1), H, 256, 2), float("nan"), device=DEV)
+        status, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty(T, H * V, dtype=torch.bfloat16, device=DEV)
+        o.prefill_attention_tc(q, fill(kp), fill(vp), table, ps, torch.from_numpy(items).to(DEV), torch.arange(n, dtype=torch.int32, device=DEV),
+                               out, H, G, D, window, D ** -0.5, status=status, merges=torch.from_numpy(merges).to(DEV) if parts else None,
+                               part_o=part_o, part_ml=part_ml, value_dim=V, keep_first=keep, softcap=cap, value_share=share, general=general)
+        assert int(status) == 0
+        outs.append(out)
+    assert bool(outs[0].isfinite().all()) and torch.equal(*outs)
+
+
 def test_prefill_attention_tcgen05_refuses_other_sizes():
     o = ops()
     q = rnd(4, 3 * 136, dtype=torch.bfloat16)
