@@ -1,6 +1,7 @@
 """Builds and loads ``csrc/py/fastcall.c``, a small extension module that calls the kernel library's entry points without
 ctypes (3 us a call of two dozen arguments there, half a microsecond here; a step that is not a replayed graph makes some
-sixty).  It needs a C compiler and Python's headers once; without them :func:`bind` returns None and ctypes takes the calls.
+sixty).  It needs a C compiler and Python's headers once; without them, or where the module does not load, :func:`bind` returns
+None and ctypes takes the calls.
 """
 from __future__ import annotations
 
@@ -36,7 +37,8 @@ def build():
                if c and (os.path.exists(c) or shutil.which(c))), None)
     if cc is None:
         return None
-    h = hashlib.sha256(" ".join([*FLAGS, sys.implementation.cache_tag or "", sysconfig.get_platform()]).encode())
+    h = hashlib.sha256(" ".join([*FLAGS, sysconfig.get_config_var("EXT_SUFFIX") or sys.implementation.cache_tag or "",
+                                 sysconfig.get_platform()]).encode())
     with open(SOURCE, "rb") as f:
         h.update(f.read())
     path = os.path.join(build_dir(), f"{NAME}.{h.hexdigest()[:16]}.so")
@@ -51,17 +53,21 @@ def build():
 
 
 def module():
-    """The extension module, or None."""
+    """The extension module, or None where it cannot be built or loaded (a compiler that does not run, a folder that code is not
+    loaded from, a file of another system); built and loaded by the first call."""
     global _module
     with _lock:
         if _module is None:
-            path = build()
             _module = False
-            if path is not None:
-                loader = importlib.machinery.ExtensionFileLoader(NAME, path)
-                spec = importlib.util.spec_from_file_location(NAME, path, loader=loader)
-                _module = importlib.util.module_from_spec(spec)
-                loader.exec_module(_module)
+            try:
+                path = build()
+                if path is not None:
+                    loader = importlib.machinery.ExtensionFileLoader(NAME, path)
+                    m = importlib.util.module_from_spec(importlib.util.spec_from_file_location(NAME, path, loader=loader))
+                    loader.exec_module(m)
+                    _module = m
+            except (OSError, ImportError) as e:
+                _log(f"no extension module, entry points are called by ctypes: {e}")
     return _module or None
 
 

@@ -167,8 +167,15 @@ _fast = {}      # entry points as the extension module calls them: plain ints, f
 def _get_fast(name: str):
     f = _fast.get(name)
     if f is None:
+        _use_extension()
         f = _fast[name] = fastcall.bind(_get(name), _SIGNATURES[name]) or _get(name)
     return f
+
+
+def _answer(name: str, *args) -> int:
+    """What an entry point returns."""
+    rc = (_fast.get(name) or _get_fast(name))(*args)
+    return _get(name)(*args) if rc is NotImplemented else rc         # (a structure or an array among the arguments)
 
 
 def register_signature(name: str, argtypes) -> None:
@@ -181,9 +188,9 @@ def call(name: str, *args) -> None:
     _launches += _KERNELS.get(name, 1)
     if _trace is not None:
         return _call_traced(name, args)
-    rc = (_fast.get(name) or _get_fast(name))(*args)
+    rc = (_fast.get(name) or _get_fast(name))(*args)      # (:func:`_answer`, without its frame)
     if rc != 0:
-        if rc is NotImplemented:         # (a structure or an array among the arguments)
+        if rc is NotImplemented:
             rc = _get(name)(*args)
             if rc == 0:
                 return
@@ -318,16 +325,17 @@ def _rows(t: torch.Tensor) -> int:
     return t.stride(0)
 
 
+_slow = (_ptr, _rows)
+
+
 def _use_extension():
-    """:func:`_ptr` and :func:`_rows` by the extension module where there is one: it calls these for what it does not take."""
+    """:func:`_ptr` and :func:`_rows` by the extension module where there is one, from the first call of an entry point on (an import
+    builds nothing): it calls these for what it does not take."""
     global _ptr, _rows
     m = fastcall.module()
     if m is not None:
-        m.set_slow(_ptr, _rows)
+        m.set_slow(*_slow)
         _ptr, _rows = m.ptr, m.rows
-
-
-_use_extension()
 
 
 def upload(values, device) -> torch.Tensor:
@@ -1334,7 +1342,7 @@ def general_attention_ok(q, ldq, ldqh, k_pages, v_pages, ldk, ldv, out, ldo, ldo
     return int(q.dtype == torch.bfloat16 and k_pages.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
             and ldq % 8 == 0 and ldqh % 8 == 0 and ldk % 8 == 0 and ldv % 8 == 0 and ldo % 2 == 0 and ldoh % 2 == 0
             and q.data_ptr() % 16 == 0 and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0
-            and out.data_ptr() % 4 == 0 and _get_fast("fx_general_attention_ok")(key_dim, value_dim, alias))
+            and out.data_ptr() % 4 == 0 and _answer("fx_general_attention_ok", key_dim, value_dim, alias))
 
 
 def general_attention_fits(key_dim: int, value_dim: int) -> bool:
@@ -1757,7 +1765,7 @@ def slab_ok(x, w) -> bool:
         return False
     if x.stride(0) % 8 or w.stride(0) % 8 or x.data_ptr() % 16 or w.data_ptr() % 16 or x.stride(1) != 1 or w.stride(1) != 1:
         return False
-    return bool(_get_fast("fx_gemm_slab_ok")(w.shape[0], w.shape[1], x.shape[0]))
+    return bool(_answer("fx_gemm_slab_ok", w.shape[0], w.shape[1], x.shape[0]))
 
 
 def gemm_slab(x, w, out, *, bias=None, accumulate=False, status=None, stream=None):

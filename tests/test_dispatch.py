@@ -1,4 +1,6 @@
 """The host-side choices between kernels and launch shapes (pure functions of sizes; no GPU)."""
+import os
+
 import pytest
 import torch
 
@@ -336,3 +338,45 @@ def test_decode_split_plan_of_the_32_bit_kernel():
                 _, n = ops.decode_split_plan_f32(tokens, kv_blocks, ctx)
                 assert 1 <= n <= min(ops.DECODE_F32_MAX_SPLITS, -(-ctx // 64))
     assert [ops.decode_split_plan_f32(t, 4, c)[1] for t, c in ((8, 2048), (4, 704), (1, 2048), (400, 2048))] == [8, 11, 32, 2]
+
+
+def test_an_extension_module_that_does_not_build_or_load_leaves_the_calls_to_ctypes(tmp_path, monkeypatch):
+    """A file that is no library in the module's place, a compiler that does not run: no module, now and when asked again; an import
+    of the wrappers asks for none; an answer that the extension hands back is ctypes' one."""
+    import subprocess
+    import sys
+    import sysconfig
+
+    from ferrox_b200.kernels import fastcall
+
+    monkeypatch.setattr(fastcall, "_module", None)
+    monkeypatch.setattr(fastcall, "build_dir", lambda: str(tmp_path))
+    path = fastcall.build()
+    if path is None:
+        pytest.skip("no C compiler or no Python headers")
+    with open(path, "wb") as f:
+        f.write(b"no library")
+    assert fastcall.module() is None and fastcall.module() is None and fastcall.bind(None, []) is None
+    tool = tmp_path / "cc"
+    tool.write_text("not to be run")
+    tool.chmod(0o600)
+    monkeypatch.setattr(fastcall, "_module", None)
+    monkeypatch.setattr(fastcall, "FLAGS", [*fastcall.FLAGS, "-DOTHER"])
+    monkeypatch.setenv("CC", str(tool))
+    assert fastcall.module() is None
+
+    code = "import ferrox_b200.kernels.fastcall as f; f.build = lambda: 1 / 0; import ferrox_b200, ferrox_b200.kernels.ops"
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+    monkeypatch.setitem(ops._fast, "fx_none", lambda *a: NotImplemented)
+    monkeypatch.setitem(ops._fn, "fx_none", lambda *a: 0)
+    assert ops._answer("fx_none", 3) == 0
+
+    # a module of another interpreter build is another file
+    real = sysconfig.get_config_var
+    monkeypatch.delenv("CC")
+    names = set()
+    for suffix in (".a.so", ".b.so"):
+        monkeypatch.setattr(sysconfig, "get_config_var", lambda n, suffix=suffix: suffix if n == "EXT_SUFFIX" else real(n))
+        names.add(fastcall.build())
+    assert len(names) == 2
