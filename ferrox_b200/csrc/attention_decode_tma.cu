@@ -41,6 +41,7 @@ using namespace fxtc;
 
 constexpr int NCONSUMERS = 128, NTHREADS = 160, TK = 64, MAXQ = 16, MAX_STAGES = 8;
 constexpr int PIECE = TK * 128;        // bytes of a [64 keys][64 dims] piece
+constexpr int SMEM_LIMIT = 220 * 1024;   // (heads of 256 take 202 KB: tma_ring)
 
 struct DecArgs {
     const bf16* q; long ldq;
@@ -500,12 +501,8 @@ template <int DMAX>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecArgs& a, dim3 grid, size_t smem, cudaStream_t s)
 {
     auto kern = decode_tma_kernel<DMAX>;
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = smem;
-    }
+    // of the current device: asked for each time, and for as much as any call takes, so that none takes it from one being captured
+    if (const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT)) return (int)e;
     fx_launch_pdl(kern, grid, NTHREADS, smem, s, mk, mv, a);
     return fx_launch_status();
 }

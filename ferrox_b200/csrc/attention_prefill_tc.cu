@@ -627,12 +627,8 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
            int n_merges, cudaStream_t s)
 {
     auto kern = prefill_attention_tc_kernel<D, V, MODE>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D, V>::TOTAL);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    // of the current device: asked for each time
+    if (const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D, V>::TOTAL)) return (int)e;
     fx_launch_pdl(kern, grid, NTHREADS, Smem<D, V>::TOTAL, s, mq, mk, mv, a);
     const float unit = MODE == CAPPED ? 1.f : a.scale_log2e;
     if (n_merges > 0)

@@ -171,12 +171,8 @@ template <int KSTEPS_MAX>
 int launch(const SlabArgs& a, unsigned blocks, size_t smem, cudaStream_t s)
 {
     auto kern = slab_kernel<KSTEPS_MAX>;
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = smem;
-    }
+    // of the current device: asked for each time, and for as much as any call takes, so that none takes it from one being captured
+    if (const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SLAB_SMEM_MAX)) return (int)e;
     fx_launch_pdl(kern, dim3(blocks), dim3(NTHREADS), smem, s, a);
     return fx_launch_status();
 }

@@ -378,12 +378,8 @@ template <int BN, bool GATED>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, long max_tiles, cudaStream_t s)
 {
     auto kern = gemm_tc_kernel<BN, GATED>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    // of the current device: asked for each time
+    if (const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::SMEM)) return (int)e;
     const unsigned grid = (unsigned)(max_tiles < fx_sm_count() ? max_tiles : fx_sm_count());
     fx_launch_pdl(kern, grid, NTHREADS, Cfg<BN>::SMEM, s, ma, mb, a);
     return fx_launch_status();

@@ -341,12 +341,8 @@ template <int BNH, bool GATED> int launch(const void* X, long ldx, const void* W
     CUtensorMap ma, mb;
     if (!make_map(&ma, X, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)ldx, BM)) return FX_ERR_SIZE;
     if (!make_map(&mb, W, (uint64_t)a.K, (uint64_t)w_rows, (uint64_t)ldw, BNH)) return FX_ERR_SIZE;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<BNH, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BNH>::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    // of the current device: asked for each time
+    if (const cudaError_t e = cudaFuncSetAttribute(gemm_tc2_kernel<BNH, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BNH>::SMEM)) return (int)e;
     const int sms = fx_sm_count();
     const long tiles = fx_cdiv(a.M, 2 * BM) * fx_cdiv(a.N, GATED ? BNH : 2 * BNH);
     const long pairs = tiles < sms / 2 ? tiles : sms / 2;

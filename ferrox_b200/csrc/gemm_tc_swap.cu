@@ -353,12 +353,8 @@ int launch(const void* X, long ldx, const void* W, long ldw, long w_group_stride
         return FX_ERR_SIZE;
     if (!make_map(&mx, X, (uint64_t)a.K, (uint64_t)a.M, 1, (uint64_t)ldx, 0, TNB, 2)) return FX_ERR_SIZE;
     auto kern = gemm_tc_swap_kernel<TNB, GATED>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TNB, GATED>::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    // of the current device: asked for each time
+    if (const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TNB, GATED>::SMEM)) return (int)e;
     const long t_tiles = a.group_offsets ? fx_cdiv(a.M, TNB) + a.n_groups : fx_cdiv(a.M, TNB);   // an upper bound when grouped
     const long max_tiles = t_tiles * fx_cdiv(a.N, BF) * (a.k_splits > 1 ? a.k_splits : 1);
     const long slots = (long)fx_sm_count() * Cfg<TNB, GATED>::CTAS_PER_SM;

@@ -531,14 +531,15 @@ extern "C" int fx_route_small(const float* logits, long ld, int n_tokens, int n_
     return fx_launch_status();
 }
 
+constexpr int FUSED_SMEM_MAX = 200 * 1024;
+
 template <int NT>
 static int launch_route_fused(size_t smem, cudaStream_t s, const FusedArgs& a)
 {
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(route_fused_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {
+        // of the current device: asked for each time, and for as much as any call takes, so that none takes it from one being captured
+        const cudaError_t e = cudaFuncSetAttribute(route_fused_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM_MAX);
         if (e != cudaSuccess) return (int)e;
-        configured = smem;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(FUSED_CTAS);
@@ -575,7 +576,7 @@ extern "C" int fx_route_fused(const void* X, long ldx, const void* W, long ldw, 
     const int nt = n_tokens <= 1 ? 1 : n_tokens <= 2 ? 2 : n_tokens <= 4 ? 4 : 8;
     const size_t smem = (size_t)nt * hidden * sizeof(bf16) + ((size_t)nt * n_route + (size_t)FUSED_WARPS * n_experts) * sizeof(float) +
                         (2 * (size_t)n_experts + 1 + 2 * (size_t)nt * top_k) * sizeof(int);
-    if (smem > 200 * 1024) return FX_ERR_SIZE;
+    if (smem > FUSED_SMEM_MAX) return FX_ERR_SIZE;
     FusedArgs a;
     a.X = (const bf16*)X; a.ldx = ldx; a.W = (const bf16*)W; a.ldw = ldw;
     a.n_tokens = n_tokens; a.n_route = n_route; a.n_experts = n_experts; a.hidden = hidden; a.top_k = top_k; a.renorm = renorm;

@@ -380,3 +380,17 @@ def test_an_extension_module_that_does_not_build_or_load_leaves_the_calls_to_cty
         monkeypatch.setattr(sysconfig, "get_config_var", lambda n, suffix=suffix: suffix if n == "EXT_SUFFIX" else real(n))
         names.add(fastcall.build())
     assert len(names) == 2
+
+
+def test_shared_memory_limits_are_asked_for_without_a_flag():
+    """No launcher remembers in a static that it has asked (the second device of a process would be refused at the launch)."""
+    import re
+
+    from ferrox_b200.kernels import lib
+
+    for name in lib.sources():
+        with open(os.path.join(lib.CSRC, name)) as f:
+            text = f.read()
+        for m in re.finditer(r"cudaFuncSetAttribute", text):
+            before = text[max(0, m.start() - 300):m.start()]
+            assert not re.search(r"static\s+(bool|int|size_t)\s+\w+\s*=\s*(false|0)\s*;", before), name
