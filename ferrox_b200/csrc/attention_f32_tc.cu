@@ -7,9 +7,9 @@
 // attention_kernel: a CTA 128 queries of a request and one head, against blocks of 64 keys.
 //
 //   S = Q K^T     tcgen05.mma 128 x 64 x dim, six for each 16 elements, the small products first, in two sums of half the elements
-//                 each (the tensor core cuts where an FFMA rounds, once for each 16 elements: in one sum the result at 128 keys is
-//                 2.24e-7 off, in two 1.83e-7, with FFMA 1.95e-7); two S in tensor memory, so that the next block's is made while
-//                 this one's softmax runs
+//                 each (the tensor core cuts where an FFMA rounds, once for each 16 elements: with parts that were cut off the result
+//                 at 128 keys was 2.24e-7 off in one sum, 1.83e-7 in two; with rounded ones it is 1.47e-7, with FFMA 2.00e-7); two S in
+//                 tensor memory, so that the next block's is made while this one's softmax runs
 //   P = exp(..)   two threads a query: maximum and sum in 32 bits, P in its three parts into tensor memory
 //   O_j = P V     tcgen05.mma 128 x dim x 64 into an accumulator of the block's own (over all keys' blocks the cuts would add
 //                 up), which the query's threads add to their 32-bit registers, rescaled by the running maximum, when the next
@@ -372,12 +372,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_kernel(const __grid_con
             for (int c = 0; c < HK; c += 16) {
                 uint32_t w[3][8];
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    uint32_t h0, m0, l0, h1, m1, l1;
-                    split3(__uint_as_float(x[c + i]), h0, m0, l0);
-                    split3(__uint_as_float(x[c + i + 1]), h1, m1, l1);
-                    w[0][i / 2] = upper_halves(h0, h1); w[1][i / 2] = upper_halves(m0, m1); w[2][i / 2] = upper_halves(l0, l1);
-                }
+                for (int i = 0; i < 16; i += 2)
+                    split3(__uint_as_float(x[c + i]), __uint_as_float(x[c + i + 1]), w[0][i / 2], w[1][i / 2], w[2][i / 2]);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) tc_st8(lanes + L::P + p * (BK / 2) + (half * HK + c) / 2, w[p]);
             }

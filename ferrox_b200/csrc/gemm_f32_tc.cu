@@ -1,13 +1,17 @@
-// C[M,N] (+)= A[M,K] . W[N,K]^T (+ bias) of 32-bit operands on the tensor cores, no further from the 64-bit sums than the
-// FFMA kernels of gemm_f32.cu.
+// C[M,N] (+)= A[M,K] . W[N,K]^T (+ bias) of 32-bit operands on the tensor cores.
 //
 // A 32-bit value is the sum of three bfloat16 (split3.cuh).  Of the nine products of two such sums six are made: hi.hi,
-// hi.mid, mid.hi, mid.mid, hi.lo, lo.hi; what is left out is below 2^-21 of a product, 2^-24 on average.  Products of two
+// hi.mid, mid.hi, mid.mid, hi.lo, lo.hi; what is left out is up to 2^-24 of a product, 2^-27 on average.  Products of two
 // bfloat16 are exact in 32 bits.  The tensor
 // core adds them up by cutting instead of rounding, which over K = 2,048 would cost 1e-5; so its accumulator holds only 32
 // elements of K (the small products first, then two instructions of large ones), and each thread adds these sums to
 // 32-bit registers of its own, rounding as an FFMA does.  What cannot be had from the parts is done again by a
 // plain loop: an element whose sum is no finite number (an operand that is infinite or no number, or an overflow).
+//
+// How far it is from 64-bit sums (relative 2-norm; the FFMA kernels of gemm_f32.cu in brackets, K of 1,024 to 7,808, 12 to 2,000 rows):
+// operands of both signs 0.9e-7 to 1.7e-7 (1.9e-7 to 5.7e-7), or with magnitudes over four decades 1.0e-7 to 1.6e-7 (2.1e-7 to 4.0e-7).
+// Not nearer everywhere: of one sign, where the cuts all have that sign, 0.7e-7 to 1.0e-7 (0.7e-7 to 2.5e-7), up to 1.3 times as far
+// where FFMA's K is cut into many runs; results of a single product 4.6e-8 (2.5e-8: half a unit in the last place), at most 1.5e-7.
 //
 // What bounds it: six bfloat16 products where an FFMA kernel does one, so a sixth of 1,680 TFLOP/s = 280 against 64.
 // A tile is 128 rows of W in the accumulator's lanes and NT <= 208 rows of A in its columns (M = 517: three tiles of 176, 2
@@ -18,7 +22,7 @@
 // stage g run, the workers take stage g + 1 of W apart and add up stage g - 1.
 // Measured (weights from memory, replayed graphs; before: the FFMA tiles): 517 x 15616 x 2048 805 -> 172 us (192 TFLOP/s), 517 x
 // 2048 x 7808 397 -> 92, 2,000 x 15616 x 2048 2,746 -> 581 (220), 64 x 15616 x 2048 102 -> 54; the three kernels take 14 us however
-// little there is to do.  Error against 64-bit sums (relative 2-norm): 1.3e-7 to 2.9e-7 where the FFMA tiles have 1.6e-7 to 7.9e-7.
+// little there is to do.
 // Every CTA gets the same number of stages: whole tiles as far as they go round, then the rest cut along K into equal
 // shares (`sk_tiles` tiles over `sk_ctas` CTAs), whose sums go to `part`; sum_kernel adds a tile's up in the order of K.
 #include "tc_common.cuh"
@@ -381,13 +385,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_f32_tc_kernel(const __grid_c
 #pragma unroll
                     for (int j = 0; j < 8; ++j, c += a.ldc) old[j] = a.accumulate && j0 + j < cols ? *c : 0.f;
                     c = c8;
+                    asm volatile("" : "+l"(c) :: "memory");          // (or the compiler keeps every column's address,
 #pragma unroll
                     for (int j = 0; j < 8; ++j, c += a.ldc) {
                         const float v = acc[j0 + j] + bias;
                         if (j0 + j < cols && !(odd[j0 / 32] >> ((j0 + j) % 32) & 1)) *c = a.accumulate ? old[j] + v : v;
                     }
                     c8 = c;
-                    asm volatile("" : "+l"(c8) :: "memory");         // (or the compiler keeps every column's address)
+                    asm volatile("" : "+l"(c8) :: "memory");         // of these eight and of the tile)
                 }
             }
 #pragma unroll

@@ -438,8 +438,9 @@ def gemm_f32_tc_tile(M: int, N: int, K: int) -> int:
     Times in microseconds, as measured on a B200: a stage of 32 elements of K takes 0.70 and 0.0018 a row of the tile, the three
     kernels 11 beside that, the shares of the tiles that are cut are written and read at 6 TB/s.  12 x 3072 x 2048: 18 against 25;
     517 x 15616 x 2048: 172 against 805; 64 x 60 x 2048: 16 against 21; 16 x 2048 x 2048 stays with the weight-streaming kernel
-    (13).  Errors against 64-bit sums there: 1.3e-7 to 2.9e-7 (a relative 2-norm), of the FFMA tiles 1.6e-7 to 7.9e-7; with
-    fewer than 1,024 elements of K their chains are as short as this kernel's and their errors no larger, so those stay."""
+    (13).  Errors against 64-bit sums there: 0.9e-7 to 1.7e-7 (a relative 2-norm), of the FFMA tiles 1.9e-7 to 5.7e-7.  Fewer than 1,024
+    elements of K stay with FFMA: the line was drawn while parts were cut off instead of rounded, when the errors there were no
+    smaller (rounded, at K = 256: 0.8e-7 and 2.1e-7); the times below it were not compared."""
     rows = min(M, _f32_tc_rows(K))
     if K < F32_TC_MIN_K or rows < min(M, F32_TC_MAX_TILE):
         return 0
@@ -1233,11 +1234,12 @@ def prefill_f32_tc_plan(entries, window, head_dim):
     queries, the most key blocks first; the positions of every entry that its queries see, in rows of the planes that begin at
     multiples of 64; and the entries that the tensor cores do not take, as the tiles of :func:`prefill_attention_f32`.
 
-    They take an entry that sees 64 keys or more (128 with heads of 64 elements or fewer).  Below, their cut sums are further from
-    64 bits than FFMA's rounded ones, and there is little to gain.  B200, one request from position 0, FFMA and tensor cores, error
-    and time: 16 heads of 128, 33 keys: 1.48e-7 and 1.50e-7, 18 and 11 us; 64: 1.74e-7 and 1.71e-7, 18 and 12 us; 517: 2.62e-7 and
-    2.21e-7, 145 and 42 us; 2000: 3.75e-7 and 2.41e-7, 1299 and 135 us.  8 heads of 64, a window of 150, 64 keys: 1.35e-7 and
-    1.44e-7, 13 and 9 us; 128: 1.61e-7 and 1.58e-7, 23 and 12 us; 2000: 2.60e-7 and 2.14e-7, 87 and 24 us."""
+    They take an entry that sees 64 keys or more (128 with heads of 64 elements or fewer).  The line was drawn while operands' parts
+    were cut off instead of rounded, where the result is then no further from 64 bits than FFMA's; rounded, it is nearer from 9 keys on.
+    B200, one request from position 0, FFMA and tensor cores, error and time: 16 heads of 128, 33 keys: 1.51e-7 and 1.17e-7, 18 and 11
+    us; 64: 1.74e-7 and 1.33e-7, 18 and 12 us; 517: 2.65e-7 and 1.70e-7, 145 and 42 us; 2000: 3.81e-7 and 1.87e-7, 1299 and 135 us.  8
+    heads of 64, a window of 150, 64 keys: 1.39e-7 and 1.07e-7, 13 and 9 us; 128: 1.63e-7 and 1.16e-7, 23 and 12 us; 2000: 2.59e-7 and
+    1.53e-7, 87 and 24 us."""
     import numpy as np
 
     items, spans, rest, flat, row = [], [], [], 0, 0

@@ -99,7 +99,7 @@ def test_gemm_f32_on_tensor_cores_in_slices_of_rows(monkeypatch):
 
 @pytest.mark.parametrize("cut", [False, True])
 def test_gemm_f32_on_tensor_cores_beyond_finite_numbers(cut, monkeypatch):
-    """Infinite operands, no numbers, overflows and values whose lower parts are subnormal: what the FFMA kernels give."""
+    """Infinite operands, no numbers, overflows and small values: what the FFMA kernels give."""
     o = ops()
     monkeypatch.setattr(o, "gemm_f32_plan", lambda *a: (32, 1))
     M, N, K = 20, 128 * (5 if cut else 148), 256
@@ -122,6 +122,61 @@ def test_gemm_f32_on_tensor_cores_beyond_finite_numbers(cut, monkeypatch):
     ok = want.isfinite()
     exact, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
     assert bool(((out.double() - exact).abs() <= 2e-6 * size)[ok].all())
+
+
+def test_gemm_f32_on_tensor_cores_single_products(monkeypatch):
+    """Results of one product each, some of operands whose lower parts are as large as they can be: what the parts leave out is up to
+    2^-24 of it, and the accumulator's cut up to one unit in the last place."""
+    o = ops()
+    M, N, K = 100, 300, 1024
+    a, w, at = torch.zeros(M, K, device=DEV), rnd(N, K), torch.arange(M, device=DEV)
+    a[at, at * 7] = rnd(M, 1)[:, 0]
+    largest = (torch.arange(M, device=DEV, dtype=torch.int32) + 0x3f808000 - M).view(torch.float32)      # 1 + 2^-8 less a few units
+    a[M // 2:, :] = 0
+    a[at[M // 2:], at[M // 2:] * 7] = largest[M // 2:]
+    w[N // 2:, :] = largest[torch.arange(N - N // 2, device=DEV) % M][:, None]
+    out, want = torch.empty(M, N, device=DEV), a.double() @ w.double().T
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *x: (32, 1))
+    monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *x: 112)
+    o.gemm(a, w, out)
+    assert float(((out.double() - want) / want).abs().max()) <= 1.5 * 2 ** -23
+    # the same where cut parts would have the most to leave out, 1 + 2^-7 less a few units
+    a[a != 0], w[:] = 1 + 2 ** -7 - 2 ** -22, 1 + 2 ** -7 - 2 ** -21
+    want = a.double() @ w.double().T
+    o.gemm(a, w, out)
+    assert float(((out.double() - want) / want).abs().max()) <= 1.5 * 2 ** -23
+
+
+def test_gemm_f32_on_tensor_cores_below_the_parts_range(monkeypatch):
+    """Operands whose second and third parts are subnormal or nothing, against weights that make the results large: what is lost of an
+    operand is below 2^-133."""
+    o = ops()
+    M, N, K = 60, 200, 1024
+    a, w = rnd(M, K) * torch.tensor([1e-33, 1e-35, 1e-36, 1e-37, 1e-38], device=DEV).repeat(M // 5)[:, None], rnd(N, K) * 1e30
+    out, size = torch.empty(M, N, device=DEV), w.double().abs()
+    monkeypatch.setattr(o, "gemm_f32_plan", lambda *x: (32, 1))
+    monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *x: 64)
+    o.gemm(a, w, out)
+    err = (out.double() - a.double() @ w.double().T).abs()
+    assert bool((err <= 2.0 ** -133 * size.sum(1) + 2e-6 * (a.double().abs() @ size.T)).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 3072, 2048), (517, 2048, 7808)])
+def test_gemm_f32_on_tensor_cores_sums_of_one_sign(M, N, K, monkeypatch):
+    """Operands of one sign, where every cut of the accumulator has that sign too: two cuts of a stage's sum by up to a unit in its last
+    place, half of it on average (2^-24 to 2^-23 of the result), and the roundings of a chain of K / 32 sums; at most twice as far
+    from 64 bits as the FFMA kernel."""
+    o = ops()
+    a, w = rnd(M, K).abs(), rnd(N, K).abs()
+    want, off = a.double() @ w.double().T, {}
+    tile = o.gemm_f32_tc_tile(M, N, K)
+    assert tile
+    for t in (tile, 0):
+        monkeypatch.setattr(o, "gemm_f32_tc_tile", lambda *x, t=t: t)
+        out = torch.empty(M, N, device=DEV)
+        o.gemm(a, w, out)
+        off[bool(t)] = float((out.double() - want).norm() / want.norm())
+    assert off[True] < 2 ** -22 and off[True] < 2 * off[False], off
 
 
 @pytest.mark.parametrize("form", [-1, -4, -8, 32, 64, 128])
