@@ -22,13 +22,13 @@
 //
 // Warp 0 issues the TMA loads (K and V blocks double-buffered), warp 1 issues the tensor-core
 // instructions and owns the tensor-memory allocation (512 columns: S_0, S_1, O_0, O_1), warps 2-5 are
-// sub-tile 0's softmax threads and warps 6-9 sub-tile 1's.  The products are issued in the order
+// sub-tile 0's softmax threads and warps 6-9 sub-tile 1's, warp 10 clears what nobody sees.  The products are issued in the order
 // PV_0(j), S_0(j+1), PV_1(j), S_1(j+1): while one sub-tile's threads work on their block the tensor
 // cores work for the other.  Every wait is bounded (status code 3 on time-out, then the roles leave,
 // tensor memory is freed and the kernel returns).  Keys that are masked are still multiplied, with weight 0, and 0 times a
 // value that is infinite or no number is none.  So what lies in a block's place in shared memory for a position that no query of
 // the item sees is zero: where there is no page the TMA fills it in (a page number behind the last), and in the blocks at the
-// edges (behind the last query, before the first one's window) the softmax threads clear the rows of V before their product.
+// edges (behind the last query, before the first one's window) warp 10 clears the rows of V before their product.
 //
 // A work item is a tile of queries, a head and a run of key blocks [kb_begin, kb_end).  The host cuts the
 // key blocks of long tiles into runs (the last 256 queries of a long prompt see many times the keys the
@@ -64,7 +64,7 @@ namespace {
 
 using namespace fxtc;
 
-constexpr int BQ = 128, BKEY = 128, NTHREADS = 320, TMEM_COLS = 512;
+constexpr int BQ = 128, BKEY = 128, NTHREADS = 352, TMEM_COLS = 512;
 constexpr float RAISE_MAX_BY = 8.f;   // in powers of two
 
 __device__ __forceinline__ float fast_exp2(float x) {   // 2^x, approximate; -inf gives 0
@@ -196,6 +196,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
         const int j = block_of(i);
         return (j >= lo_of(t) && j <= hi_of(t)) || (j < kept_end && j < blk_lo(t));
     };
+    // walked blocks with positions that no query of the item sees: the last kept one, the window's first, the last
+    const int lo_item = fx_first_key(pos0, a.window, a.chunk);
+    auto is_edge = [&](int i) {
+        const int kb = block_of(i) * BKEY;
+        return i >= 0 && i < n_walk && (kb + BKEY - 1 > last_pos || (kb < lo_item && kb + BKEY > a.keep_first)) && (active(0, i) || active(1, i));
+    };
+    const int edge0 = is_edge(n_kept - 1) ? n_kept - 1 : -1, edge1 = is_edge(n_kept) ? n_kept : -1, edge2 = is_edge(n_walk - 1) ? n_walk - 1 : -1;
+    auto at_edge = [&](int i) { return i == edge0 || i == edge1 || i == edge2; };
     auto last_of = [&](int t) {                            // the last walked block that sub-tile t needs (none: -1)
         int i = n_walk - 1;
         while (i >= 0 && !active(t, i)) --i;
@@ -211,6 +219,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
     auto k_full = [&](int b) { return bar0 + 56 + 8u * b; };
     auto v_full = [&](int b) { return bar0 + 72 + 8u * b; };
     auto kv_empty = [&](int b) { return bar0 + 88 + 8u * b; };
+    // where the loads of a block at an edge arrive: its k_full and v_full are raised when what nobody sees has been cleared
+    auto v_edge = [&](int b) { return bar0 + 104 + 8u * b; };
     volatile int* abort_flag = &abort_flag_s;
 
     if (threadIdx.x == 0) {
@@ -219,6 +229,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
         for (int b = 0; b < 2; ++b) {
             mbar_init(s_full(b), 1); mbar_init(p_full(b), 4); mbar_init(o_done(b), 1);
             mbar_init(k_full(b), 1); mbar_init(v_full(b), 1); mbar_init(kv_empty(b), 1);
+            mbar_init(v_edge(b), 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -245,6 +256,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                     tma_load_3d(base + L::Q_OFF + t * L::Q_BYTES + h * L::SUB, &map_q, h * 64, head, tok0 + t * BQ, q_full);
             const int* table = a.block_table + (long)a.seq_slot[entry] * a.table_width;
             int issued = 0, v_issued = 0;
+            uint32_t v_edges = 0;           // loads at edges so far, odd or even, a bit a place
             for (int i = 0; i < n_walk; ++i) {
                 const int j = block_of(i), b = i & 1, vb = L::V_PLACES == 2 ? b : 0;
                 if (!mbar_wait(kv_empty(b), (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag)) break;
@@ -255,6 +267,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                     page[hk] = p >= 0 ? p : a.n_pages;      // no page (beyond the request, or before its window): zeros
                     off[hk] = p >= 0 ? key % a.page_size : 0;
                 }
+                const bool edge = at_edge(i);
+                const uint32_t v_bar = edge ? v_edge(vb) : v_full(vb);
                 mbar_expect_tx(k_full(b), L::K_BYTES);
                 for (int h = 0; h < L::HALVES; ++h)
                     for (int hk = 0; hk < 2; ++hk)
@@ -263,20 +277,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 issued = i + 1;
                 // (one place of values: free when the block before this one has been multiplied)
                 if (L::V_PLACES == 1 && i > 0 && !mbar_wait(kv_empty((i - 1) & 1), (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) break;
-                mbar_expect_tx(v_full(vb), L::V_BYTES);
+                mbar_expect_tx(v_bar, L::V_BYTES);
                 for (int h = 0; h < L::V_HALVES; ++h)
                     for (int hk = 0; hk < 2; ++hk)
                         tma_load_4d(base + L::V_OFF + vb * L::V_BYTES + h * L::SUB + hk * 8192, &map_v, h * 64, off[hk],
-                                    kvh / a.value_share, page[hk], v_full(vb));
+                                    kvh / a.value_share, page[hk], v_bar);
                 v_issued = i + 1;
+                if (edge) v_edges ^= 1u << vb;
             }
             if (*abort_flag) {   // loads already issued must land before the shared memory is released
+                // (each the last of its place, so that an edge's phase is the one before the next)
                 for (int i = max(0, issued - 2); i < issued; ++i)
                     for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
                         if (mbar_try_wait(k_full(i & 1), (uint32_t)((i >> 1) & 1))) break;
-                for (int i = max(0, v_issued - L::V_PLACES); i < v_issued; ++i)
+                for (int i = max(0, v_issued - L::V_PLACES); i < v_issued; ++i) {
+                    const bool edge = at_edge(i);
+                    const int vb = i % L::V_PLACES;
                     for (uint32_t w = 0; w < WAIT_LIMIT; ++w)
-                        if (mbar_try_wait(v_full(i % L::V_PLACES), (uint32_t)((i / L::V_PLACES) & 1))) break;
+                        if (mbar_try_wait(edge ? v_edge(vb) : v_full(vb), edge ? (v_edges >> vb & 1u) ^ 1u : (uint32_t)((i / L::V_PLACES) & 1))) break;
+                }
             }
         }
     } else if (warp == 1) {
@@ -332,7 +351,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 }
             }
         }
-    } else {
+    } else if (warp < 10) {
         // ---------------- softmax: one query row per thread ----------------
         const int t = (warp - 2) >> 2;
         const int quad = warp & 3;                       // the lanes of tensor memory this warp may touch
@@ -349,22 +368,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
             float m = -INFINITY, l = 0.f;
             bool ok = true;
             int cnt = 0;
-            // Zeros for the values of block i, from position kb, that no query of the item sees.  The product of sub-tile 0 comes
-            // first where both have the block, so its threads do it.
-            auto clear_hidden = [&](int i, int kb) {
-                const int lo_item = fx_first_key(pos0, a.window, a.chunk);
-                if (kb + BKEY - 1 <= last_pos && (kb >= lo_item || kb + BKEY <= a.keep_first)) return true;
-                if (t == 1 && active(0, i)) return true;
-                const int vb = L::V_PLACES == 2 ? i & 1 : 0;
-                if (!__all_sync(0xffffffffu, mbar_wait(v_full(vb), (uint32_t)((i / L::V_PLACES) & 1), abort_flag))) return false;
-                for (int c = r; c < L::V_HALVES * BKEY * 8; c += BQ) {          // pieces of 16 bytes, eight a row
-                    const int key = kb + ((c >> 3) & (BKEY - 1));
-                    if (key > last_pos || (key < lo_item && key >= a.keep_first))
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + L::V_OFF + vb * L::V_BYTES + c * 16), "r"(0) : "memory");
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                return true;
-            };
             for (int i = 0; i < n_walk; ++i) {
                 if (!active(t, i)) continue;
                 const int j = block_of(i);
@@ -372,7 +375,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 if (!ok) break;
                 tc_fence_after();
                 if (quad * 32 >= rows_t) {           // none of the warp's rows exists: what its rows of P hold reaches no others
-                    if (!(ok = clear_hidden(i, j * BKEY))) break;
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(p_full(t));
@@ -385,24 +387,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 // The row of S is read in chunks of 32 columns into two register buffers in turn: the load of the
                 // next chunk is in flight while the current one is worked on.
                 uint32_t ca[32], cb[32], pk[32];
-                auto mask = [&](uint32_t* c, int chunk) {
+                auto mask = [&](uint32_t* c, int chunk, uint32_t with) {
                     if (interior) return;
 #pragma unroll
                     for (int k = 0; k < 32; ++k) {
                         const int key = kb + chunk * 32 + k;
-                        if (key > p_r || (key < lo_r && key >= a.keep_first)) c[k] = 0xff800000u;   // -inf
+                        if (key > p_r || (key < lo_r && key >= a.keep_first)) c[k] = with;
                     }
                 };
+                constexpr uint32_t MINUS_INF = 0xff800000u, NO_NUMBER = 0x7fffffffu;
                 // first pass: the row's maximum
                 float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY, size0 = 0.f, size1 = 0.f;
                 auto take_max = [&](uint32_t* c, int chunk) {
+                    mask(c, chunk, NO_NUMBER);           // (what fmaxf passes over, also where sizes are taken)
                     if (MODE == CAPPED) {
 #pragma unroll
                         for (int k = 0; k < 32; k += 2) {
                             size0 = fmaxf(size0, fabsf(__uint_as_float(c[k]))); size1 = fmaxf(size1, fabsf(__uint_as_float(c[k + 1])));
                         }
                     }
-                    mask(c, chunk);
 #pragma unroll
                     for (int k = 0; k < 32; k += 4) {
                         mx0 = fmaxf(mx0, __uint_as_float(c[k])); mx1 = fmaxf(mx1, __uint_as_float(c[k + 1]));
@@ -416,14 +419,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 tc_ld32(ts + 96, cb); take_max(ca, 2); tc_ld_wait_for(cb);
                 tc_ld32(ts, ca);      take_max(cb, 3);   // chunk 0 again, for the second pass
                 float top = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                const bool all_small = MODE == CAPPED && __all_sync(0xffffffffu, fmaxf(size0, size1) * a.cap.k <= CAP_SMALL);
+                const bool all_small = MODE == CAPPED && __all_sync(0xffffffffu, r >= rows_t || fmaxf(size0, size1) * a.cap.k <= CAP_SMALL);
                 if (MODE == CAPPED && top != -INFINITY) {
                     // (as its weight will be worked out, but for the last place)
                     const float x2 = top * top, q = fmaf(fmaf(fmaf(a.cap.c[3], x2, a.cap.c[2]), x2, a.cap.c[1]), x2, a.cap.c[0]);
                     top = all_small ? fmaf(top * x2, q, top * a.cap.unit) : a.cap.cap * tanhf(a.cap.k * top);
                 }
                 const float mn = fmaxf(m, top);
-                const bool raise = mn > m && (m == -INFINITY || (mn - m) * sl2 > RAISE_MAX_BY);
+                // (rows that do not exist, another request's queries, have no say in the others' references)
+                const bool raise = r < rows_t && mn > m && (m == -INFINITY || (mn - m) * sl2 > RAISE_MAX_BY);
                 if (__any_sync(0xffffffffu, raise)) {
                     const float alpha = m == -INFINITY ? 0.f : fast_exp2((m - mn) * sl2);
                     l *= alpha;
@@ -452,7 +456,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                     if (MODE == CAPPED) {
                         if (all_small) cap_small(a.cap, c, ref); else cap_any(a.cap, c, ref);
                     }
-                    mask(c, chunk);
+                    mask(c, chunk, MINUS_INF);
 #pragma unroll
                     for (int k = 0; k < 32; k += 2) {
                         float e0 = weight(c[k]), e1 = weight(c[k + 1]);
@@ -475,7 +479,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 take_exp(cb, 3, pk + 16);
                 tc_st32(ts + 32, pk);
                 l += sum0 + sum1;
-                if (!interior && !(ok = clear_hidden(i, kb))) break;
                 tc_st_wait();
                 tc_fence_before();
                 __syncwarp();
@@ -538,6 +541,31 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                     }
                 }
             }
+        }
+    } else {
+        // ---------------- zeros where nobody sees a position ----------------
+        // (A warp of its own: among the softmax threads' lines these cost 3 us of 55 in items without an edge.  Its code comes last: before
+        // theirs it cost the plain form 1 to 2 per cent.)
+        auto clear_rows = [&](uint32_t at, int slices, int from, int to) {
+            for (int h = 0; h < slices; ++h)
+#pragma unroll 4
+                for (int c = from * 128 + lane * 16; c < to * 128; c += 512)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + h * L::SUB + c), "r"(0) : "memory");
+        };
+        auto clear = [&](uint32_t at, int slices, int kb) {
+            clear_rows(at, slices, max(0, a.keep_first - kb), min(BKEY, lo_item - kb));
+            clear_rows(at, slices, max(0, last_pos + 1 - kb), BKEY);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+        };
+        uint32_t v_phases = 0;             // a bit a place
+        for (int i = 0; i < n_walk; ++i) {
+            if (!at_edge(i)) continue;
+            const int vb = L::V_PLACES == 2 ? i & 1 : 0, kb = block_of(i) * BKEY;
+            if (!__all_sync(0xffffffffu, mbar_wait(v_edge(vb), v_phases >> vb & 1u, abort_flag))) break;
+            v_phases ^= 1u << vb;
+            clear(base + L::V_OFF + vb * L::V_BYTES, L::V_HALVES, kb);
+            if (lane == 0) mbar_arrive(v_full(vb));
         }
     }
 

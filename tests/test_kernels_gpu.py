@@ -1463,6 +1463,34 @@ def test_prefill_attention_tcgen05_leaves_out_what_nobody_sees(form, run_blocks)
     assert bool(outs[0].isfinite().all()) and torch.equal(*outs)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_prefill_attention_tcgen05_capped_bits_are_the_requests_own(D):
+    """A capped request's bits are the same whatever lies behind its last position, before its window, and in the rows of the
+    request beside it: scores there are nothing, like its own, a thousand times as large (far beyond where the cap's cubic ends), or
+    rise from one key block to the next as its own do not."""
+    o = ops()
+    H, ps, window, lens, starts = 32, 64, 100, [70, 40], [230, 0]
+    n_pages, T = 6, sum(lens)
+    kp, vp = rnd(n_pages, H, ps, D, dtype=torch.bfloat16, seed=1), rnd(n_pages, H, ps, D, dtype=torch.bfloat16, seed=2)
+    table = torch.tensor([[1, 4, 0, 3, 2], [5, 5, 5, 5, 5]], dtype=torch.int32, device=DEV)
+    q = rnd(T, H * D, dtype=torch.bfloat16, seed=3)
+    items, _, _ = o.prefill_tc_plan(list(zip(lens, starts)), window, H, run_blocks=0)
+    outs = []
+    for size in (0, 1, 1000, "rising"):
+        k, x = kp.clone(), q.clone()
+        if size == "rising":
+            x[lens[0]:] = 27 / D ** 0.5 * kp[2, :, 290 - 256].reshape(1, -1)
+        else:
+            k[2, :, 300 - 256:] *= size
+            k[0, :, :(starts[0] - window + 1) - 128] *= size
+            x[lens[0]:] *= size
+        out = torch.empty(T, H * D, dtype=torch.bfloat16, device=DEV)
+        o.prefill_attention_tc(x, k, vp, table, ps, torch.from_numpy(items).to(DEV), torch.arange(2, dtype=torch.int32, device=DEV), out, H, H,
+                               D, window, D ** -0.5, softcap=30.0, general=True)
+        outs.append(out[:lens[0]])
+    assert [torch.equal(outs[0], x) for x in outs[1:]] == [True] * 3
+
+
 def test_prefill_attention_tcgen05_refuses_other_sizes():
     o = ops()
     q = rnd(4, 3 * 136, dtype=torch.bfloat16)
