@@ -76,7 +76,10 @@ __device__ __forceinline__ float fast_exp2(float x) {   // 2^x, approximate; -in
 // How a score becomes a weight: the plain kernel's exponential is the hardware's (weights below 2^-126 are 0), the general
 // forms' is exp2f, and their denominators add up the weights as the second product has them (rounded to bfloat16: a row with
 // one large weight then has none of its rounding).
+// What rescales a row, its sink and the merge of its runs is done the same way: weights below 2^-126 reach a result whose values
+// are large enough.
 enum { FAST = 0, GENERAL = 1, CAPPED = 2 };
+template <int MODE> __device__ __forceinline__ float exp2_of(float x) { return MODE == FAST ? fast_exp2(x) : exp2f(x); }
 
 // A capped score in powers of two, c log2(e) tanh(k s) with k = scale / c.  Up to k s = 1/2, tanh(x) = x + x z p(z), z = x^2, p
 // fitted (weighted least squares towards the smallest largest error, 1.5e-8 of tanh(x); in 32 bits 7.5e-8): a cubic in s^2
@@ -134,11 +137,11 @@ struct AttnArgs {
 };
 
 // What a row's sums are multiplied with at the end: 1 / (l + the head's sink), l being relative to 2^ref.
-__device__ __forceinline__ float inverse_sum(float l, float ref, const float* sinks, int head) {
+template <int MODE> __device__ __forceinline__ float inverse_sum(float l, float ref, const float* sinks, int head) {
     if (!(l > 0.f)) return 0.f;
     if (!sinks) return 1.f / l;
-    const float sk = sinks[head] * 1.4426950408889634f, mm = fmaxf(ref, sk), f = fast_exp2(ref - mm);
-    return f / (l * f + fast_exp2(sk - mm));
+    const float sk = sinks[head] * 1.4426950408889634f, mm = fmaxf(ref, sk), f = exp2_of<MODE>(ref - mm);
+    return f / (l * f + exp2_of<MODE>(sk - mm));
 }
 
 template <int D, int V>
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 // (rows that do not exist, another request's queries, have no say in the others' references)
                 const bool raise = r < rows_t && mn > m && (m == -INFINITY || (mn - m) * sl2 > RAISE_MAX_BY);
                 if (__any_sync(0xffffffffu, raise)) {
-                    const float alpha = m == -INFINITY ? 0.f : fast_exp2((m - mn) * sl2);
+                    const float alpha = m == -INFINITY ? 0.f : exp2_of<MODE>((m - mn) * sl2);
                     l *= alpha;
                     m = mn;
                     if (cnt > 0) {   // the sums so far of this row, in tensor memory, take the new reference too
@@ -508,7 +511,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 }
             } else if (ok && has_blocks) {
                 tc_fence_after();
-                const float inv = inverse_sum(l, m * sl2, a.sinks, head);
+                const float inv = inverse_sum<MODE>(l, m * sl2, a.sinks, head);
                 bf16* dst = a.out + (long)(tok0 + t * BQ + r) * a.ldo + (long)head * a.value_dim;
                 const bf16* gate = a.gate ? a.gate + (long)(tok0 + t * BQ + r) * a.ldg + (long)head * a.value_dim : nullptr;
                 const float* turn = a.turn ? a.turn + (long)(tok0 + t * BQ + r) * a.value_dim : nullptr;
@@ -583,7 +586,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
 // relative to the reference m_c) and the sum of weights l_c; with M = max m_c the result is
 // sum_c o_c 2^((m_c - M) s) / sum_c l_c 2^((m_c - M) s), the runs taken in their order.  A run without visible keys
 // for the row has m_c = -inf and is skipped.  merges: int32 [n, 4] = (first flat token, rows, first part, runs).
-template <int V>
+template <int V, int MODE>
 __global__ void __launch_bounds__(128) prefill_merge_kernel(const int* __restrict__ merges, const float* __restrict__ part_o,
                                                             const float* __restrict__ part_ml, bf16* __restrict__ out, long ldo,
                                                             int n_heads, float scale_log2e, int value_dim,
@@ -608,7 +611,7 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const int* __restric
         m_c = ml.x; l_c = ml.y;
     }
     const float mx = warp_max(m_c);
-    const float w_c = m_c == -INFINITY ? 0.f : fast_exp2((m_c - mx) * scale_log2e);
+    const float w_c = m_c == -INFINITY ? -1.f : exp2_of<MODE>((m_c - mx) * scale_log2e);      // (-1: no visible keys)
     float acc[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i) acc[i] = 0.f;
@@ -616,14 +619,15 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const int* __restric
 #pragma unroll 4
     for (int c = 0; c < runs; ++c) {
         const float w = __shfl_sync(0xffffffffu, w_c, c);
-        l = fmaf(__shfl_sync(0xffffffffu, l_c, c), w, l);
-        if (w == 0.f) continue;    // a run without visible keys for this row wrote no sums
+        const float l_of = __shfl_sync(0xffffffffu, l_c, c);
+        if (w == -1.f) continue;   // a run without visible keys for this row wrote no sums
+        l = fmaf(l_of, w, l);
         const float* src = part_o + (slot0 + c * run_stride) * V + lane * PER;
 #pragma unroll
         for (int i = 0; i < PER; ++i) acc[i] = fmaf(src[i], w, acc[i]);
     }
     if (lane * PER >= value_dim) return;
-    const float inv = inverse_sum(l, mx * scale_log2e, sinks, head);
+    const float inv = inverse_sum<MODE>(l, mx * scale_log2e, sinks, head);
     bf16* dst = out + (long)(tok0 + r) * ldo + (long)head * value_dim + lane * PER;
     const bf16* g = gate ? gate + (long)(tok0 + r) * ldg + (long)head * value_dim + lane * PER : nullptr;
     static_assert(PER % 2 == 0, "a lane holds whole pairs");
@@ -660,7 +664,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
     fx_launch_pdl(kern, grid, NTHREADS, Smem<D, V>::TOTAL, s, mq, mk, mv, a);
     const float unit = MODE == CAPPED ? 1.f : a.scale_log2e;
     if (n_merges > 0)
-        fx_launch_pdl(prefill_merge_kernel<V>, dim3(n_merges, a.n_heads, 2 * BQ / 4), 128, 0, s, merges, (const float*)a.part_o,
+        fx_launch_pdl(prefill_merge_kernel<V, MODE>, dim3(n_merges, a.n_heads, 2 * BQ / 4), 128, 0, s, merges, (const float*)a.part_o,
                       (const float*)a.part_ml, a.out, a.ldo, a.n_heads, unit, a.value_dim, a.sinks, a.gate, a.ldg, a.turn);
     return fx_launch_status();
 }

@@ -1491,6 +1491,43 @@ def test_prefill_attention_tcgen05_capped_bits_are_the_requests_own(D):
     assert [torch.equal(outs[0], x) for x in outs[1:]] == [True] * 3
 
 
+@pytest.mark.parametrize("what", ["raised", "merged", "sink"])
+@pytest.mark.parametrize("cap,shift", [(None, 130.0), (40.0, 104.0)])
+def test_prefill_attention_tcgen05_small_weights_of_large_values(cap, shift, what):
+    """Keys whose weights are 2^-130 of the largest (capped scores: 2^-104, of 2^-115 that they can be) but whose values make up for it
+    are in the result: where the row's reference is raised past them, where their run is merged, and under a large sink."""
+    o = ops()
+    D, ps, T, start = 64, 64, 60, 130
+    scale = math.log(2.0) / 8            # the score of (8, 0, ..) and (x, 0, ..) is x powers of two
+    if cap:
+        half = cap * math.atanh(shift / 2 * math.log(2.0) / cap) / math.log(2.0)
+        low, high = -half, half
+    else:
+        low, high = 0.0, shift
+    n_pages, large = 3, 100 if cap is None else 80
+    kp, vp = torch.zeros(n_pages, 1, ps, D), torch.full((n_pages, 1, ps, D), 2.0 ** large)
+    kp[:, :, :, 0] = low
+    sinks = None
+    if what == "sink":
+        sinks = torch.full((1,), (high if cap is None else shift / 2) * math.log(2.0), device=DEV)
+    else:
+        kp[2, :, :, 0] = high
+        vp[2] = 2.0 ** (large - shift + 5)
+    kp, vp = kp.to(DEV, torch.bfloat16), vp.to(DEV, torch.bfloat16)
+    q = torch.zeros(T, D, dtype=torch.bfloat16, device=DEV)
+    q[:, 0] = 8.0
+    table = torch.arange(n_pages, dtype=torch.int32, device=DEV)[None]
+    items, merges, parts = o.prefill_tc_plan([(T, start)], None, 1, run_blocks=1 if what == "merged" else 0)
+    part_o, part_ml = torch.empty(max(parts, 1), 1, 256, 64, device=DEV), torch.empty(max(parts, 1), 1, 256, 2, device=DEV)
+    out = torch.empty(T, D, dtype=torch.bfloat16, device=DEV)
+    o.prefill_attention_tc(q, kp, vp, table, ps, torch.from_numpy(items).to(DEV), torch.zeros(1, dtype=torch.int32, device=DEV), out, 1, 1, D, None,
+                           scale, merges=torch.from_numpy(merges).to(DEV) if parts else None, part_o=part_o, part_ml=part_ml, sinks=sinks,
+                           softcap=cap, general=True)
+    want = general_attention_in_64_bits(q.view(T, 1, D), kp, vp, table, [T], [start], 1, 1, 1, 0, 0, None, cap, scale, sinks)
+    # the cap's exponent of up to 58 and the scale's of 130 are held to 2^-18: their sum in the weight to 2^-16, the result to 2^-9
+    assert float(((out.view(T, 1, D).double() - want).abs() / want).max()) < 2 ** -8
+
+
 def test_prefill_attention_tcgen05_refuses_other_sizes():
     o = ops()
     q = rnd(4, 3 * 136, dtype=torch.bfloat16)
