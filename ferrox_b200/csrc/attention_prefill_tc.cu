@@ -29,6 +29,9 @@
 // value that is infinite or no number is none.  So what lies in a block's place in shared memory for a position that no query of
 // the item sees is zero: where there is no page the TMA fills it in (a page number behind the last), and in the blocks at the
 // edges (behind the last query, before the first one's window) warp 10 clears the rows of V before their product.
+// What one query sees and another of its sub-tile does not stays: elements of a result that are no finite number while the
+// weights' sum is one are made again from the operands as they are (remake), so that such a value reaches only the queries that see
+// it.  (Looking for them and the call take 0.2 us of a prompt of 53 tokens, 0.3 to 1.1 us of 55 to 110.)
 //
 // A work item is a tile of queries, a head and a run of key blocks [kb_begin, kb_end).  The host cuts the
 // key blocks of long tiles into runs (the last 256 queries of a long prompt see many times the keys the
@@ -123,6 +126,8 @@ constexpr int ITEM_INTS = 8;   // a work item: first flat token, rows, entry, fi
 struct AttnArgs {
     const int* block_table; int table_width; int page_size, n_pages;
     const int* tiles; const int* seq_slot;
+    const bf16 *q, *k, *v; long ldq, ldqh, kv_at[6];      // the operands, for remake; strides of a page, a head, a position: keys, values
+    int head_dim;
     bf16* out; long ldo;
     float* part_o; float* part_ml;   // partial results of items that hold a run of their tile's key blocks only
     int n_heads, n_kv_heads, window, chunk;
@@ -144,6 +149,69 @@ template <int MODE> __device__ __forceinline__ float inverse_sum(float l, float 
     return f / (l * f + exp2_of<MODE>(sk - mm));
 }
 
+// Row `row` of this block's item: the elements of its result (in `out`, or the 32-bit sums of an item that holds a run) that are no finite
+// numbers, made again from the operands as they are, over the keys that the query sees, weights rounded as for the product, against the
+// reference `ref`; `inv`: one over the weights' sum.  Rare, and out of line: it reads anew what it needs to know, so that the kernel keeps no registers for it.
+template <int MODE, int V>
+__device__ __noinline__ void remake(const AttnArgs& a, int row, float ref, float inv)
+{
+    const int* item = a.tiles + (long)blockIdx.y * ITEM_INTS;
+    const int* table = a.block_table + (long)a.seq_slot[item[2]] * a.table_width;
+    const int head = blockIdx.x, kvh = head / (a.n_heads / a.n_kv_heads), pos = item[3] + row, lo = fx_first_key(pos, a.window, a.chunk);
+    const int first_blk = item[4], end_blk = item[5], part = item[6], n_kept = item[7];
+    const long token = item[0] + row;
+    const bf16 *q = a.q + token * a.ldq + head * a.ldqh, *k_head = a.k + kvh * a.kv_at[1], *v_head = a.v + kvh / a.value_share * a.kv_at[4];
+    float* sums = part >= 0 ? a.part_o + (((long)part * a.n_heads + head) * (2 * BQ) + row) * V : nullptr;
+    bf16* dst = a.out + token * a.ldo + (long)head * a.value_dim;
+    const bf16* gate = a.gate ? a.gate + token * a.ldg + (long)head * a.value_dim : nullptr;
+    const float* turn = a.turn ? a.turn + token * a.value_dim : nullptr;
+    for (int c = 0; c < a.value_dim; c += 8) {
+        float o[8];
+        uint32_t odd = 0;
+        for (int d = 0; d < 8; ++d) {
+            const float x = sums ? sums[c + d] : __bfloat162float(dst[c + d]);
+            if (!(fabsf(x) < INFINITY)) odd |= turn && !sums ? 3u << (d & ~1) : 1u << d;       // (a pair that was turned: both)
+            o[d] = 0.f;
+        }
+        uint32_t left = odd;                      // what no key yet made no number
+        for (int j = n_kept > 0 ? 0 : first_blk; j < end_blk && left; j = j + 1 == n_kept ? first_blk : j + 1)
+            for (int key = j * BKEY; key < (j + 1) * BKEY && key <= pos && left; ++key) {
+                if (key < lo && key >= a.keep_first) continue;
+                const int page = table[key / a.page_size], at = key % a.page_size;
+                if (page < 0) continue;
+                const bf16* k = k_head + page * a.kv_at[0] + at * a.kv_at[2];
+                float s = 0.f;
+                for (int d = 0; d < a.head_dim; d += 8) {
+                    float x[8], y[8];
+                    Pack<bf16>::load(q + d, x);
+                    Pack<bf16>::load(k + d, y);
+                    for (int i = 0; i < 8; ++i) s = fmaf(x[i], y[i], s);
+                }
+                const float x = MODE == CAPPED ? fmaf(a.cap.cap, tanhf(a.cap.k * s), -ref) : fmaf(s, a.scale_log2e, -ref);
+                const float w = __bfloat162float(__float2bfloat16_rn(exp2_of<MODE>(x)));
+                float v[8];
+                Pack<bf16>::load(v_head + page * a.kv_at[3] + at * a.kv_at[5] + c, v);
+                left = 0;
+                for (int d = 0; d < 8; ++d) {
+                    o[d] = fmaf(w, v[d], o[d]);
+                    if ((odd >> d & 1) && o[d] == o[d]) left |= 1u << d;
+                }
+            }
+        if (turn && !sums)
+            for (int d = 0; d < 8; d += 2) {
+                o[d] *= inv; o[d + 1] *= inv;
+                fx_turn_back(o[d], o[d + 1], *reinterpret_cast<const float2*>(turn + c + d));
+            }
+        for (int d = 0; d < 8; ++d) {
+            if (!(odd >> d & 1)) continue;
+            if (sums) { sums[c + d] = o[d]; continue; }
+            if (!turn) o[d] *= inv;
+            if (gate) o[d] *= fx_sigmoid_fast(__bfloat162float(gate[c + d]));
+            dst[c + d] = __float2bfloat16_rn(o[d]);
+        }
+    }
+}
+
 template <int D, int V>
 struct Smem {
     static constexpr int HALVES = D / 64, V_HALVES = V / 64;   // 64-element (128-byte) slices of a key's, a value's row
@@ -160,7 +228,7 @@ template <int D, int V, int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                            const __grid_constant__ CUtensorMap map_k,
                                                                            const __grid_constant__ CUtensorMap map_v,
-                                                                           AttnArgs a)
+                                                                           const __grid_constant__ AttnArgs a)
 {
     using L = Smem<D, V>;
     extern __shared__ uint8_t smem_raw[];
@@ -489,6 +557,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                 ++cnt;
             }
             const bool has_blocks = last_of(t) >= 0;
+            float again_inv = 1.f;
+            __nv_bfloat162 zero[4] = {};
+            float none[4] = {0.f, 0.f, 0.f, 0.f};        // no number where an element of this row's result is no finite number
             if (ok && has_blocks) ok = __all_sync(0xffffffffu, mbar_wait(o_done(t), 0, abort_flag));
             if (ok && part >= 0) {
                 // a run of the tile's key blocks: the sums as they are, each row's reference and sum of weights
@@ -503,6 +574,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
                         tc_ld32(to + c * 32, ob);
                         tc_ld_wait();
                         if (r < rows_t) {
+#pragma unroll
+                            for (int k = 0; k < 32; ++k) none[k & 3] = fmaf(__uint_as_float(ob[k]), 0.f, none[k & 3]);
 #pragma unroll
                             for (int k = 0; k < 32; k += 4)
                                 *reinterpret_cast<uint4*>(dst + c * 32 + k) = make_uint4(ob[k], ob[k + 1], ob[k + 2], ob[k + 3]);
@@ -539,11 +612,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_attention_tc_kernel(const
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) x[e] *= fx_sigmoid_fast(g[e]);
                             }
-                            Pack<bf16>::store(dst + c * 32 + k, x);
+                            __nv_bfloat162 y[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                y[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+                                zero[e] = __hfma2(y[e], __nv_bfloat162(0.f, 0.f), zero[e]);
+                            }
+                            *reinterpret_cast<uint4*>(dst + c * 32 + k) = *reinterpret_cast<const uint4*>(y);
                         }
                     }
                 }
+                again_inv = inv;
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) none[e] += __low2float(zero[e]) + __high2float(zero[e]);
+            const float sum = (none[0] + none[1]) + (none[2] + none[3]);
+            if (sum != sum && l > 0.f && l < INFINITY) remake<MODE, V>(a, t * BQ + r, m * sl2, again_inv);
         }
     } else {
         // ---------------- zeros where nobody sees a position ----------------
@@ -714,6 +798,7 @@ extern "C" int fx_prefill_attention_tc(const void* q, long ldq, long ldqh, int n
     if ((gate && (ldg % 8 || (uintptr_t)gate % 16)) || (uintptr_t)turn % 16) return FX_ERR_ALIGN;
     if (n_tiles > 65535) return FX_ERR_SIZE;
     CUtensorMap mq, mk, mv;
+    AttnArgs a;
     {
         cuuint64_t dims[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_heads, (cuuint64_t)n_tokens};
         cuuint64_t strides[2] = {(cuuint64_t)ldqh * 2, (cuuint64_t)ldq * 2};
@@ -727,14 +812,15 @@ extern "C" int fx_prefill_attention_tc(const void* q, long ldq, long ldqh, int n
         for (int i = 0; i < 3; ++i) {
             if (kv_strides) at[i] = kv_strides[3 * v + i];
             if (at[i] % 8) return FX_ERR_ALIGN;
+            a.kv_at[3 * v + i] = at[i];
         }
         cuuint64_t dims[4] = {(cuuint64_t)width, (cuuint64_t)page_size, (cuuint64_t)heads, (cuuint64_t)n_pages};
         cuuint64_t strides[3] = {(cuuint64_t)at[2] * 2, (cuuint64_t)at[1] * 2, (cuuint64_t)at[0] * 2};
         cuuint32_t box[4] = {64, 64, 1, 1};
         if (!encode(v ? &mv : &mk, v ? v_pages : k_pages, 4, dims, strides, box)) return FX_ERR_SIZE;
     }
-    AttnArgs a;
     a.block_table = block_table; a.table_width = table_width; a.page_size = page_size; a.n_pages = n_pages;
+    a.q = (const bf16*)q; a.k = (const bf16*)k_pages; a.v = (const bf16*)v_pages; a.ldq = ldq; a.ldqh = ldqh; a.head_dim = head_dim;
     a.tiles = tiles; a.seq_slot = seq_slot; a.out = (bf16*)out; a.ldo = ldo;
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.window = window; a.chunk = chunk; a.value_dim = value_dim;
     a.sinks = sinks; a.gate = (const bf16*)gate; a.ldg = ldg; a.turn = turn;

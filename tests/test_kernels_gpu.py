@@ -1528,6 +1528,59 @@ def test_prefill_attention_tcgen05_small_weights_of_large_values(cap, shift, wha
     assert float(((out.view(T, 1, D).double() - want).abs() / want).max()) < 2 ** -8
 
 
+@pytest.mark.parametrize("run_blocks", [0, 1])
+@pytest.mark.parametrize("form", [*HIDDEN_FORMS, "turned and gated"])
+def test_prefill_attention_tcgen05_values_reach_only_who_sees_them(form, run_blocks):
+    """Values that are no numbers or infinite at positions that some of a tile's queries see: what sees one has none in that element;
+    what does not has its result, made again in another order of sums (32-bit sums of weights that bfloat16 holds: their rounding, and
+    the result's to bfloat16, which may fall to either side); elements beside them keep their bits."""
+    o = ops()
+    more = form == "turned and gated"
+    H, G, share, D, V, window, keep, cap, general = HIDDEN_FORMS[0] if more else form
+    ps, T, start = 64, 500, 100
+    n_pages = -(-(start + T) // ps)
+    table = torch.randperm(n_pages, generator=torch.Generator().manual_seed(3)).to(torch.int32).to(DEV)[None]
+    kp, vp = rnd(n_pages, G, ps, D, dtype=torch.bfloat16, seed=1), rnd(n_pages, G // share, ps, V, dtype=torch.bfloat16, seed=2)
+    bad, heads = vp.clone(), G // share
+    places = [(30, 1, math.inf), (170, 3, math.nan), (270, 5, -math.inf), (271, 5, math.inf), (599, V - 1, math.nan)]
+    for p, col, x in places:
+        bad[int(table[0, p // ps]), heads - 1, p % ps, col] = x
+    q = rnd(T, H * D, dtype=torch.bfloat16, seed=3)
+    angle = rnd(T, V // 2, seed=5)
+    turn = torch.stack([angle.cos(), angle.sin()], -1).reshape(T, V).contiguous() if more else None
+    gate = rnd(T, H * V, dtype=torch.bfloat16, seed=6) if more else None
+    items, merges, parts = o.prefill_tc_plan([(T, start)], window, H, run_blocks=run_blocks, keep_first=keep)
+    outs = []
+    for v in (vp, bad):
+        part_o = torch.full((max(parts, 1), H, 256, o.prefill_value_width(V)), float("nan"), device=DEV)
+        part_ml = torch.full((max(parts, 1), H, 256, 2), float("nan"), device=DEV)
+        status, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty(T, H * V, dtype=torch.bfloat16, device=DEV)
+        o.prefill_attention_tc(q, kp, v, table, ps, torch.from_numpy(items).to(DEV), torch.zeros(1, dtype=torch.int32, device=DEV), out, H, G, D,
+                               window, D ** -0.5, status=status, merges=torch.from_numpy(merges).to(DEV) if parts else None, part_o=part_o,
+                               part_ml=part_ml, value_dim=V, keep_first=keep, softcap=cap, value_share=share, general=general, turn=turn,
+                               gate=gate)
+        assert int(status) == 0
+        outs.append(out.view(T, heads, H // heads, V).float())
+    clean, got = outs
+    pos = torch.arange(start, start + T, device=DEV)
+    touched = torch.zeros(T, heads, V, dtype=torch.bool, device=DEV)
+    cols = set()
+    for p, col, x in places:
+        sees = (p <= pos) & ((p > pos - (window or 1 << 30)) | (p < keep))
+        for c in ({col, col ^ 1} if more else {col}):         # (a turned pair: both)
+            touched[:, heads - 1, c] |= sees
+            cols.add(c)
+    touched = touched[:, :, None].expand_as(got)
+    assert bool(clean.isfinite().all()) and torch.equal(~got.isfinite(), touched)
+    same = torch.ones(heads, 1, V, dtype=torch.bool, device=DEV)
+    same[heads - 1, :, sorted(cols)] = False
+    assert bool((got == clean)[same.expand_as(got)].all())
+    # a weight's rounding to bfloat16 may fall to the other side where its score's sum differs in the last bit (2^-8 of the weight,
+    # which is at most 1), and so may the result's (2^-8 of it): seldom
+    off, size = (got - clean)[~touched], clean[~touched]
+    assert float((off.abs() - 2 ** -8 * size.abs()).max()) <= 2 ** -8 * float(vp.float().abs().max()) and float(off.norm() / size.norm()) < 1e-3
+
+
 def test_prefill_attention_tcgen05_refuses_other_sizes():
     o = ops()
     q = rnd(4, 3 * 136, dtype=torch.bfloat16)
